@@ -57,15 +57,15 @@ __device__ void grid_barrier(const BatchArgs& A) {
 template <int EGQ, int EGL>
 struct BatchCfg {
   static constexpr int s(int a, int b) { return a > b ? a : b; }
-  static constexpr int SMEM = s(s(s(MixCfg<2, 0, EGL>::SMEM, MixCfg<2, 1, EGL>::SMEM),
-                                  s(MixCfg<3, 0, EGQ>::SMEM, MixCfg<3, 1, EGQ>::SMEM)),
+  static constexpr int SMEM = s(s(s(MixCfg<2, 0, EGL>::SMEM0, MixCfg<2, 1, EGL>::SMEM0),
+                                  s(MixCfg<3, 0, EGQ>::SMEM0, MixCfg<3, 1, EGQ>::SMEM0)),
                                 (int)(BT_WARPS * sizeof(SurfWarpSmem)));
   // The dynamic shared memory a launch needs: the work area of the element
   // types present (mask bit t = type t, bit 4 = surface loads), so that a
   // batch of one type gets the occupancy of that type alone.
   static int smem_for(unsigned mask) {
-    const int sz[5] = {MixCfg<2, 0, EGL>::SMEM, MixCfg<2, 1, EGL>::SMEM, MixCfg<3, 0, EGQ>::SMEM,
-                       MixCfg<3, 1, EGQ>::SMEM, (int)(BT_WARPS * sizeof(SurfWarpSmem))};
+    const int sz[5] = {MixCfg<2, 0, EGL>::SMEM0, MixCfg<2, 1, EGL>::SMEM0, MixCfg<3, 0, EGQ>::SMEM0,
+                       MixCfg<3, 1, EGQ>::SMEM0, (int)(BT_WARPS * sizeof(SurfWarpSmem))};
     int w = 0;
     for (int t = 0; t < 5; ++t)
       if (mask & (1u << t)) w = s(w, sz[t]);
@@ -76,10 +76,10 @@ struct BatchCfg {
 template <int EGQ, int EGL, int TM, class H>
 __device__ __forceinline__ void load_tables(int type, const KParams& P, unsigned char* w) {
   switch (type) {
-    case 0: if constexpr (TM & 1) mix_tables<2, 0, EGL, H>(P, w); break;
-    case 1: if constexpr (TM & 2) mix_tables<2, 1, EGL, H>(P, w); break;
-    case 2: if constexpr (TM & 4) mix_tables<3, 0, EGQ, H>(P, w); break;
-    default: if constexpr (TM & 8) mix_tables<3, 1, EGQ, H>(P, w); break;
+    case 0: if constexpr (TM & 1) mix_tables<2, 0, EGL, float, H>(P, w); break;
+    case 1: if constexpr (TM & 2) mix_tables<2, 1, EGL, float, H>(P, w); break;
+    case 2: if constexpr (TM & 4) mix_tables<3, 0, EGQ, float, H>(P, w); break;
+    default: if constexpr (TM & 8) mix_tables<3, 1, EGQ, float, H>(P, w); break;
   }
 }
 
@@ -91,7 +91,7 @@ __device__ __forceinline__ void member_units(const KParams& P, const int32_t* el
   const int ng = (count + EG - 1) / EG;
   for (int u = j; u < nunits; u += gridDim.x) {
     const int g1 = min(ng, (u + 1) * bg);
-    for (int g = u * bg; g < g1; ++g) mix_group<N1, PM, EG, 3, H>(P, elems, count, g, p4_first, w);
+    for (int g = u * bg; g < g1; ++g) mix_group<N1, PM, EG, float, H>(P, elems, count, g, p4_first, w);
   }
 }
 

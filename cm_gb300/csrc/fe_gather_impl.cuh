@@ -76,12 +76,12 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
       const uint16_t* tab = P.tables + (size_t)__shfl_sync(0xffffffffu, trow, j) * NR;
       if (lane < NPE) {
         const int rk = tab[lane] & 0x7fff;
-        const float* src = S.uu + (size_t)e * cmfe::rec_stride_uu(NPE) + (size_t)la * NU3 + lane;
+        const float* src = S.uu + (size_t)e * cmfe::rec_stride_uu(NPE) + cmfe::rec_uu(NPE, 0, la, 0, lane);
         float v[9];
 #pragma unroll
         for (int m = 0; m < 3; ++m)
 #pragma unroll
-          for (int n = 0; n < 3; ++n) v[m * 3 + n] = rec_load<CG>(src + (size_t)m * NPE * NU3 + n * NPE);
+          for (int n = 0; n < 3; ++n) v[m * 3 + n] = rec_load<CG>(src + (3 * m + n) * NPE);
 #pragma unroll
         for (int m = 0; m < 3; ++m)
 #pragma unroll

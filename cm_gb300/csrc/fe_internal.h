@@ -117,10 +117,16 @@ CMFE_HD constexpr int rec_stride_uu(int npe) { return (9 * npe * npe + 31) / 32 
 CMFE_HD constexpr int rec_stride_cp(int npe, int npp) { return (npp * 3 * npe + 15) / 16 * 16; }  // doubles
 CMFE_HD constexpr int rec_stride_r(int npe, int npp) { return (3 * npe + npp + 15) / 16 * 16; }   // doubles
 
+// Place of entry (component m of node a, component n of node b) in an
+// element's displacement record, [a][m][n][b]: what the gather of node a's
+// rows reads is contiguous.
+CMFE_HD constexpr int rec_uu(int npe, int m, int a, int n, int b) { return ((a * 3 + m) * 3 + n) * npe + b; }
+
 // Per-element records of the staged assembly (mixed kernel with staged
-// output, surface mode 2, row gather): the full displacement block
-// [3 NPE][3 NPE] (FP32, row-major), the pressure-coupling rows [NPP][3 NPE]
-// and the residual [nrow] (FP64) of element e, at e times the strides above.
+// output, surface mode 2, row gather): the full displacement block (FP32,
+// mirrored, in the order of rec_uu), the pressure-coupling rows
+// [NPP][3 NPE] and the residual [nrow] (FP64) of element e, at e times the
+// strides above.
 struct StageOut {
   float* uu;
   double* cp;

@@ -10,28 +10,28 @@
 
 namespace {
 
-template <int N1, int PM, int SPLIT, class H>
+template <int N1, int PM, class H>
 __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB) fe_mixed_kernel(KParams P) {
   using C = MixCfg<N1, PM>;
   extern __shared__ __align__(16) unsigned char sm[];
-  mix_tables<N1, PM, C::EG, H>(P, sm);
+  mix_tables<N1, PM, C::EG, float, H>(P, sm);
   const int ngroups = (P.count + C::EG - 1) / C::EG;
   const bool p4_first = (blockIdx.x / P.wave) & 1;
-  for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) mix_group<N1, PM, C::EG, SPLIT, H>(P, P.elems, P.count, grp, p4_first, sm);
+  for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) mix_group<N1, PM, C::EG, float, H>(P, P.elems, P.count, grp, p4_first, sm);
 }
 
 // The same element code over all elements in element order, each element's
 // entries stored into its staging records instead of the CSR arrays (no
 // colour order is needed: elements write disjoint records).
-template <int N1, int PM, int SPLIT, class H>
+template <int N1, int PM, class H>
 __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB) fe_mixed_staged_kernel(KParams P, cmfe::StageOut so) {
   using C = MixCfg<N1, PM>;
   extern __shared__ __align__(16) unsigned char sm[];
-  mix_tables<N1, PM, C::EG, H>(P, sm);
+  mix_tables<N1, PM, C::EG, float, H>(P, sm);
   const int ngroups = (P.count + C::EG - 1) / C::EG;
   const bool p4_first = (blockIdx.x / P.wave) & 1;
   for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x)
-    mix_group<N1, PM, C::EG, SPLIT, H, 1>(P, nullptr, P.count, grp, p4_first, sm, &so);
+    mix_group<N1, PM, C::EG, float, H, 1>(P, nullptr, P.count, grp, p4_first, sm, &so);
 }
 
 // Staged assembly in one launch: CTAs take element groups in element order
@@ -43,18 +43,18 @@ __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB) fe_mixed_staged_ker
 // another.  Publication follows the release/acquire pattern: every thread
 // fences its record stores before the counting, and a completing count is
 // followed by a fence before the records are read (through L2, not L1).
-template <int N1, int PM, int SPLIT, class H>
+template <int N1, int PM, class H>
 __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB)
     fe_mixed_fused_kernel(KParams P, cmfe::StageOut so, cmfe::FusedArgs F) {
   using C = MixCfg<N1, PM>;
   constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, EG = C::EG;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ int s_grp, s_nready;
-  mix_tables<N1, PM, EG, H>(P, sm);
+  mix_tables<N1, PM, EG, float, H>(P, sm);
   const int ngroups = min((P.count + EG - 1) / EG, F.g1);
   const bool p4_first = (blockIdx.x / P.wave) & 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int* s_node = reinterpret_cast<const int*>(sm + C::O_NODE);
+  const int* s_node = reinterpret_cast<const int*>(sm + C::O_NODE1);
   int* ready = reinterpret_cast<int*>(sm + C::O_READY);
   unsigned char* scratch = sm + C::O_SCRATCH;
   for (;;) {
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB)
     __syncthreads();
     const int grp = s_grp;
     if (grp >= ngroups) break;
-    mix_group<N1, PM, EG, SPLIT, H, 1>(P, nullptr, P.count, grp, p4_first, sm, &so);
+    mix_group<N1, PM, EG, float, H, 1>(P, nullptr, P.count, grp, p4_first, sm, &so);
     const int nvalid = min(EG, P.count - grp * EG);
     __syncthreads();  // the group's records are complete within the CTA; the scratch is free
     if (F.bmask) {
@@ -105,37 +105,38 @@ __global__ void __launch_bounds__(256, MixCfg<N1, PM>::MINB)
 
 // Resident blocks per SM of the fused kernel (its shared-memory attribute set
 // once per device first); 0 on error, with the error in *err.
-template <int N1, int PM, int SPLIT, class H>
+template <int N1, int PM, class H>
 int fused_per_sm(cudaError_t* err) {
   using C = MixCfg<N1, PM>;
+  constexpr int SMEM = C::SMEM1;
   static std::atomic<bool> attr[64];
-  auto kern = fe_mixed_fused_kernel<N1, PM, SPLIT, H>;
+  auto kern = fe_mixed_fused_kernel<N1, PM, H>;
   int dev = 0;
   *err = cudaGetDevice(&dev);
   if (*err != cudaSuccess) return 0;
   if (dev < 0 || dev >= 64 || !attr[dev].load()) {
-    *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    *err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (*err != cudaSuccess) return 0;
     if (dev >= 0 && dev < 64) attr[dev].store(true);
   }
   int per_sm = 0;
-  *err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM);
+  *err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, SMEM);
   if (*err != cudaSuccess) return 0;
   return per_sm < 1 ? 1 : per_sm;
 }
 
-template <int N1, int PM, int SPLIT, class H>
+template <int N1, int PM, class H>
 int launch_fused_t(const KParams& kp, const cmfe::StageOut& so, cmfe::FusedArgs fa, int gather_bytes, int num_sms,
                    cudaStream_t st) {
   using C = MixCfg<N1, PM>;
-  auto kern = fe_mixed_fused_kernel<N1, PM, SPLIT, H>;
+  auto kern = fe_mixed_fused_kernel<N1, PM, H>;
   const int avail = C::O_READY - C::O_SCRATCH;
   fa.gbytes = gather_bytes;
   fa.gwarps = gather_bytes > 0 ? avail / gather_bytes : 0;
   if (fa.gwarps > C::THREADS / 32) fa.gwarps = C::THREADS / 32;
   if (fa.gwarps < 1) return (int)cudaErrorInvalidConfiguration;
   cudaError_t e;
-  const int per_sm = fused_per_sm<N1, PM, SPLIT, H>(&e);
+  const int per_sm = fused_per_sm<N1, PM, H>(&e);
   if (!per_sm) return (int)e;
   const int all = (kp.count + C::EG - 1) / C::EG;
   if (fa.g1 > all) fa.g1 = all;
@@ -146,36 +147,37 @@ int launch_fused_t(const KParams& kp, const cmfe::StageOut& so, cmfe::FusedArgs 
   grid = grid < 1 ? 1 : grid;
   KParams k = kp;
   k.wave = num_sms > 0 ? num_sms : 1;
-  kern<<<grid, C::THREADS, C::SMEM, st>>>(k, so, fa);
+  kern<<<grid, C::THREADS, C::SMEM1, st>>>(k, so, fa);
   return (int)cudaGetLastError();
 }
 
 template <class H>
 int launch_fused_h(const HostSetup& s, const KParams& kp, const cmfe::StageOut& so, const cmfe::FusedArgs& fa,
                    int num_sms, cudaStream_t st) {
-  if (s.n1 == 2 && s.pmode == 0) return launch_fused_t<2, 0, 3, H>(kp, so, fa, s.gather_bytes, num_sms, st);
-  if (s.n1 == 2 && s.pmode == 1) return launch_fused_t<2, 1, 3, H>(kp, so, fa, s.gather_bytes, num_sms, st);
-  if (s.n1 == 3 && s.pmode == 0) return launch_fused_t<3, 0, 3, H>(kp, so, fa, s.gather_bytes, num_sms, st);
-  return launch_fused_t<3, 1, 3, H>(kp, so, fa, s.gather_bytes, num_sms, st);
+  if (s.n1 == 2 && s.pmode == 0) return launch_fused_t<2, 0, H>(kp, so, fa, s.gather_bytes, num_sms, st);
+  if (s.n1 == 2 && s.pmode == 1) return launch_fused_t<2, 1, H>(kp, so, fa, s.gather_bytes, num_sms, st);
+  if (s.n1 == 3 && s.pmode == 0) return launch_fused_t<3, 0, H>(kp, so, fa, s.gather_bytes, num_sms, st);
+  return launch_fused_t<3, 1, H>(kp, so, fa, s.gather_bytes, num_sms, st);
 }
 
-template <int N1, int PM, int SPLIT, class H, bool STAGED = false>
+template <int N1, int PM, class H, bool STAGED = false>
 int launch_t(const KParams& kp, int num_sms, cudaStream_t st, const cmfe::StageOut& so = cmfe::StageOut{}) {
   using C = MixCfg<N1, PM>;
+  constexpr int SMEM = STAGED ? C::SMEM1 : C::SMEM0;
   // the attribute belongs to the device that is current: set once per device
   static std::atomic<bool> attr[64];
-  const void* kern = STAGED ? (const void*)fe_mixed_staged_kernel<N1, PM, SPLIT, H>
-                            : (const void*)fe_mixed_kernel<N1, PM, SPLIT, H>;
+  const void* kern = STAGED ? (const void*)fe_mixed_staged_kernel<N1, PM, H>
+                            : (const void*)fe_mixed_kernel<N1, PM, H>;
   int dev = 0;
   cudaError_t e0 = cudaGetDevice(&dev);
   if (e0 != cudaSuccess) return (int)e0;
   if (dev < 0 || dev >= 64 || !attr[dev].load()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
     if (dev >= 0 && dev < 64) attr[dev].store(true);
   }
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, SMEM);
   if (e != cudaSuccess) return (int)e;
   per_sm = per_sm < 1 ? 1 : per_sm;
   const int groups = (kp.count + C::EG - 1) / C::EG;
@@ -185,19 +187,19 @@ int launch_t(const KParams& kp, int num_sms, cudaStream_t st, const cmfe::StageO
   KParams k = kp;
   k.wave = num_sms > 0 ? num_sms : 1;
   if constexpr (STAGED)
-    fe_mixed_staged_kernel<N1, PM, SPLIT, H><<<grid, C::THREADS, C::SMEM, st>>>(k, so);
+    fe_mixed_staged_kernel<N1, PM, H><<<grid, C::THREADS, SMEM, st>>>(k, so);
   else
-    fe_mixed_kernel<N1, PM, SPLIT, H><<<grid, C::THREADS, C::SMEM, st>>>(k);
+    fe_mixed_kernel<N1, PM, H><<<grid, C::THREADS, SMEM, st>>>(k);
   return (int)cudaGetLastError();
 }
 
 template <class H, bool STAGED = false>
 int launch_h(const HostSetup& s, const KParams& kp, int num_sms, cudaStream_t st,
              const cmfe::StageOut& so = cmfe::StageOut{}) {
-  if (s.n1 == 2 && s.pmode == 0) return launch_t<2, 0, 3, H, STAGED>(kp, num_sms, st, so);
-  if (s.n1 == 2 && s.pmode == 1) return launch_t<2, 1, 3, H, STAGED>(kp, num_sms, st, so);
-  if (s.n1 == 3 && s.pmode == 0) return launch_t<3, 0, 3, H, STAGED>(kp, num_sms, st, so);
-  return launch_t<3, 1, 3, H, STAGED>(kp, num_sms, st, so);
+  if (s.n1 == 2 && s.pmode == 0) return launch_t<2, 0, H, STAGED>(kp, num_sms, st, so);
+  if (s.n1 == 2 && s.pmode == 1) return launch_t<2, 1, H, STAGED>(kp, num_sms, st, so);
+  if (s.n1 == 3 && s.pmode == 0) return launch_t<3, 0, H, STAGED>(kp, num_sms, st, so);
+  return launch_t<3, 1, H, STAGED>(kp, num_sms, st, so);
 }
 
 }  // namespace
@@ -214,11 +216,11 @@ int fused_wave(const HostSetup& s, int num_sms, bool double_float) {
   cudaError_t e;
   int per_sm;
   if (double_float)
-    per_sm = s.n1 == 2 ? (s.pmode ? fused_per_sm<2, 1, 3, dd>(&e) : fused_per_sm<2, 0, 3, dd>(&e))
-                       : (s.pmode ? fused_per_sm<3, 1, 3, dd>(&e) : fused_per_sm<3, 0, 3, dd>(&e));
+    per_sm = s.n1 == 2 ? (s.pmode ? fused_per_sm<2, 1, dd>(&e) : fused_per_sm<2, 0, dd>(&e))
+                       : (s.pmode ? fused_per_sm<3, 1, dd>(&e) : fused_per_sm<3, 0, dd>(&e));
   else
-    per_sm = s.n1 == 2 ? (s.pmode ? fused_per_sm<2, 1, 3, double>(&e) : fused_per_sm<2, 0, 3, double>(&e))
-                       : (s.pmode ? fused_per_sm<3, 1, 3, double>(&e) : fused_per_sm<3, 0, 3, double>(&e));
+    per_sm = s.n1 == 2 ? (s.pmode ? fused_per_sm<2, 1, double>(&e) : fused_per_sm<2, 0, double>(&e))
+                       : (s.pmode ? fused_per_sm<3, 1, double>(&e) : fused_per_sm<3, 0, double>(&e));
   if (!per_sm) return -(int)e;
   return per_sm * (num_sms > 0 ? num_sms : 1);
 }

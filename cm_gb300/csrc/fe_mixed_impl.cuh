@@ -15,21 +15,15 @@
 //    P_g(k,m) with P_g = J_z w_g dxi/dz sigma.  The pressure-coupling block
 //    K(p_q, u_nb) = sum_g psi_q(g) J_z w_g dN_b/dz_n is contracted with the
 //    tensor-product (sum-factorised) form of the trilinear pressure basis.
-//  * The displacement block is FP32 with the contraction on tensor cores.
-//    Per Gauss point the spatial tangent is pulled back to xi space:
-//    D^{mn}(k,l) = sum_ij dxi_k/dz_i SUB^{mn}(i,j) dxi_l/dz_j with the
-//    reference's SUB^{mn} = J_z w (c(T2V(:,m),T2V(:,n)) + delta_mn sigma)
-//    (:1003-1034), so K^{mn}(a,b) = sum_{(g,k)} Phi(g,k;a) W^{mn}(g,k;b) with
-//    W = D Phi and Phi the constant gradient table.  That product runs as
-//    mma.sync m16n8k16 BF16 with FP32 accumulation; with SPLIT = 3 both
-//    operands are split into a BF16 high part and a BF16 residual and three
-//    products are accumulated, which keeps about 16 significant bits.
+//  * The displacement block is FP32: the reference's tangent (:1003-1034) is
+//    pulled back to xi space per Gauss point and contracted over the Gauss
+//    points by sum factorisation on the FP32 pipes (fe_uu.cuh).  Warps do it
+//    on their own, one block of an element (or two symmetric ones) at a time.
 //  * Elements of one colour share no node; a CTA processes EG elements at a
 //    time for the per-Gauss-point work (so 100+ threads do the FP64
 //    kinematics at once) and then contracts them one by one.
 #pragma once
 
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -37,6 +31,7 @@
 #include "fe_dd.cuh"
 #include "fe_internal.h"
 #include "fe_math.cuh"
+#include "fe_uu.cuh"
 
 using cmfe::HostSetup;
 using cmfe::KParams;
@@ -51,7 +46,7 @@ constexpr int align16(int x) { return (x + 15) & ~15; }
 // measured 17 % faster than two CTAs of 4 elements despite the register
 // spills the 80-register budget causes), 4 for element-based pressure, 8 for
 // trilinear elements.
-template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8)>
+template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8), class T = float>
 struct MixCfg {
   static constexpr int MINB = (N1 == 3 && PM) ? 3 : 2;  // CTAs per SM the launch bounds ask for
   static constexpr int NPE = N1 * N1 * N1;
@@ -61,16 +56,7 @@ struct MixCfg {
   static constexpr int NROW = NU3 + NPP;
   static constexpr int THREADS = 256;
   static constexpr int EG = EG_;                // elements per group
-  static constexpr int MT = (NPE + 15) / 16;    // m16 tiles over a
-  static constexpr int NT = (NPE + 7) / 8;      // n8 tiles over b
-  static constexpr int KT = 6;                  // k16 tiles over (g,k): 81 -> 96
-  static constexpr int KPW = 52;                // padded row length in 32-bit words (104 bf16)
-  static constexpr int AROWS = MT * 16;
-  static constexpr int BROWS = NT * 8;
   static constexpr int REC64 = 20;  // P(9), A(9), t1, pad
-  static constexpr int REC32 = 60;  // D^{mn}(k,l) for 6 blocks, padded so Gauss points 2 apart hit banks 24 apart
-  static constexpr int PHS = 4 * NPE;  // per-Gauss-point stride of the FP32 gradient table: [b][d0, d1, d2, 0]
-  static constexpr int KAP = 84;    // contraction length: kappa = 28 k + g, g < 27 (g = 27 is padding)
   static constexpr int O_PSI64 = 0;
   static constexpr int O_L = align16(O_PSI64 + NG * 8 * 8);
   static constexpr int O_W = align16(O_L + 6 * 8);
@@ -78,55 +64,32 @@ struct MixCfg {
   static constexpr int O_LM = align16(O_1D + 6 * N1 * 8);  // L x (1-D value | derivative) products
   // constant tables first, then the per-group scratch from O_Z on (the fused
   // kernel reuses the scratch between groups for its row gathers)
-  static constexpr int O_PHI32 = align16(O_LM + 12 * N1 * 8);
-  static constexpr int O_A = align16(O_PHI32 + NG * PHS * 4);
-  static constexpr int O_Z = align16(O_A + 2 * AROWS * KPW * 4);
+  static constexpr int O_MM = align16(O_LM + 12 * N1 * 8);
+  static constexpr int O_Z = align16(O_MM + UUCfg<N1>::MM * (int)sizeof(T));
   static constexpr int O_P = align16(O_Z + EG * 3 * NPE * 8);
-  static constexpr int O_DZ = align16(O_P + EG * 8 * 8);
-  static constexpr int O_PG = align16(O_DZ + EG * NG * 9 * 8);
+  static constexpr int O_PG = align16(O_P + EG * 8 * 8);
   static constexpr int O_R64 = align16(O_PG + EG * NG * 8);
+  static constexpr int P1S = EG * (18 * N1 * N1 + 81 * N1) * 8;  // scratch of the gradients' first two stages
+  static constexpr int RECS = EG * NG * UU_REC * (int)sizeof(T);
   static constexpr int O_R32 = align16(O_R64 + EG * NG * REC64 * 8);
-  static constexpr int O_F32 = align16(O_R32 + EG * NG * REC32 * 4);
-  static constexpr int O_NODE = align16(O_F32 + EG * NG * 24 * 4);
-  static constexpr int SMEM = align16(O_NODE + EG * (NR + 1) * 4);
+  // the gradients and the FP64 stages' scratch share their space with the
+  // warps' stage-1 values of the displacement block
+  static constexpr int O_DZ = align16(O_R32 + (RECS > P1S ? RECS : P1S));
+  static constexpr int O_F32 = align16(O_DZ + EG * NG * 9 * 8);
+  static constexpr int WS1 = THREADS / 32 * UUCfg<N1>::S1 * (int)sizeof(T);
+  static constexpr int F32_END = align16(O_F32 + EG * NG * 24 * 4);
+  static constexpr int O_BASE = align16(O_DZ + WS1 > F32_END ? O_DZ + WS1 : F32_END);
+  // coloured order only: scatter addresses and rank tables of the group
+  static constexpr int O_TAB = align16(O_BASE + EG * 9 * NPE * 4);
+  static constexpr int O_NODE0 = align16(O_TAB + EG * NPE * NPE * 2);
+  static constexpr int SMEM0 = align16(O_NODE0 + EG * (NR + 1) * 4);
+  // staged order: the node numbers follow the scratch directly; the fused
+  // kernel's list of row nodes a group completed lies just below them
+  static constexpr int O_NODE1 = align16(O_BASE + EG * NR * 4);
+  static constexpr int SMEM1 = align16(O_NODE1 + EG * (NR + 1) * 4);
   static constexpr int O_SCRATCH = O_Z;
-  // fused kernel: the list of row nodes a group completed, just below O_NODE
-  static constexpr int O_READY = O_NODE - align16(EG * NR * 4);
+  static constexpr int O_READY = O_BASE;
 };
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo_elem, float hi_elem) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(lo_elem, hi_elem);  // .x -> low 16 bits
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-// Splits (v0, v1) into BF16 high parts and BF16 residuals.
-__device__ __forceinline__ void split_bf16(float v0, float v1, uint32_t& hi, uint32_t& lo) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
-  const float r0 = v0 - __bfloat162float(h.x);
-  const float r1 = v1 - __bfloat162float(h.y);
-  __nv_bfloat162 l = __floats2bfloat162_rn(r0, r1);
-  hi = *reinterpret_cast<uint32_t*>(&h);
-  lo = *reinterpret_cast<uint32_t*>(&l);
-}
-
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Four 8x8 b16 matrices from shared memory (ldmatrix, not transposed): lane L
-// gives the address of row L % 8 of matrix L / 8 (16-byte aligned); register i
-// receives the thread's element pair of matrix i (row lane / 4, pair lane % 4).
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* row_addr) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(row_addr);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(a));
-}
 
 // Block (m, n) of the lower-triangle displacement blocks: 0..2 diagonal,
 // 3 = (1,0), 4 = (2,0), 5 = (2,1).
@@ -245,6 +208,31 @@ __device__ __forceinline__ void load_geo(const KParams& P, int e, int g, dd dn[9
   jx = {v.x, v.y};
 }
 
+// The same data in the displacement block's type T; FP32 takes the leading
+// parts of the double-float copy, which are the values rounded to FP32.
+__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, double dn[9], double& jx) {
+  load_geo(P, e, g, dn, jx);
+}
+__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, float dn[9], float& jx) {
+  const float2* geo = reinterpret_cast<const float2*>(P.geo_dd) + ((size_t)e * NG + g) * 10;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) dn[i] = geo[i].x;
+  jx = geo[9].x;
+}
+
+template <class T, class H>
+__device__ __forceinline__ T to_t(H v) {
+  if constexpr (sizeof(T) == 4)
+    return hf(v);
+  else
+    return hd(v);
+}
+
+template <class T>
+__device__ __forceinline__ T* stage_uu(const cmfe::StageOut& so) {
+  return so.uu;
+}
+
 // The 3-point Gauss-Legendre abscissae on [0, 1].
 __device__ __forceinline__ double gauss_1d(int gi) {
   return gi == 0 ? (-sqrt(0.6) + 1.0) / 2.0 : (gi == 1 ? 0.5 : (sqrt(0.6) + 1.0) / 2.0);
@@ -262,20 +250,17 @@ __device__ __forceinline__ void lagrange_1d(int a, double t, double& bv, double&
   }
 }
 
-// Constant tables (basis values and derivatives at the Gauss points, the
-// split BF16 gradient table of the tensor-core stage) into shared memory.
-template <int N1, int PM, int EG_, class H>
+// Constant tables (basis values and derivatives at the Gauss points and their
+// products) into shared memory.
+template <int N1, int PM, int EG_, class T, class H>
 __device__ __forceinline__ void mix_tables(const KParams& P, unsigned char* sm) {
-  using C = MixCfg<N1, PM, EG_>;
-  constexpr int NPE = C::NPE, KPW = C::KPW;
+  using C = MixCfg<N1, PM, EG_, T>;
   H* s_psi = reinterpret_cast<H*>(sm + C::O_PSI64);  // [g][q]
   H* s_L = reinterpret_cast<H*>(sm + C::O_L);        // [q][gi]
   H* s_w = reinterpret_cast<H*>(sm + C::O_W);        // [g]
   H* s_B1 = reinterpret_cast<H*>(sm + C::O_1D);      // [gi][a] 1-D values
   H* s_D1 = s_B1 + 3 * N1;                                // [gi][a] 1-D derivatives
   H* s_LM = reinterpret_cast<H*>(sm + C::O_LM);      // [B|D][q][gi][a]: L(q, gi) x 1-D value | derivative
-  float* s_phi32 = reinterpret_cast<float*>(sm + C::O_PHI32);  // [g][b][l], l padded to 4
-  uint32_t* s_A = reinterpret_cast<uint32_t*>(sm + C::O_A);    // [hi/lo][a][KPW]
   const int tid = threadIdx.x;
   // ---- constant tables
   for (int i = tid; i < NG * 8; i += C::THREADS) s_psi[i] = hval<H>(P.gbf_p[i]);
@@ -299,25 +284,7 @@ __device__ __forceinline__ void mix_tables(const KParams& P, unsigned char* sm) 
     lagrange_1d<N1>(a, t, bv, dv);
     s_LM[tid] = hval<H>((q == 0 ? 1.0 - t : t) * (d ? dv : bv));
   }
-  for (int i = tid; i < NG * 3 * NPE; i += C::THREADS) {
-    const int g = i / (3 * NPE), l = (i / NPE) % 3, b = i % NPE;
-    s_phi32[g * C::PHS + 4 * b + l] = (float)P.gbf_u[(g * 4 + l + 1) * NPE + b];
-    if (l == 0) s_phi32[g * C::PHS + 4 * b + 3] = 0.0f;
-  }
-  for (int i = tid; i < C::AROWS * KPW; i += C::THREADS) {
-    const int a = i / KPW, wd = i % KPW;
-    float v[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int kap = 2 * wd + h;
-      const int kk = kap / 28, gg = kap % 28;
-      v[h] = (a < NPE && kap < C::KAP && gg < NG) ? (float)P.gbf_u[(gg * 4 + kk + 1) * NPE + a] : 0.0f;
-    }
-    uint32_t hi, lo;
-    split_bf16(v[0], v[1], hi, lo);
-    s_A[i] = hi;
-    s_A[C::AROWS * KPW + i] = lo;
-  }
+  uu_table<N1, T>(reinterpret_cast<T*>(sm + C::O_MM), tid, C::THREADS);
 }
 
 // Element number of entry i of an element list (NULL: P.first_elem + i).
@@ -326,17 +293,16 @@ __device__ __forceinline__ int elem_at(const KParams& P, const int32_t* elems, i
 }
 
 // One group of up to EG elements, elems[grp*EG ...] of the count elements
-// of the current colour.  p4_first swaps the order of the independent FP64
-// (P3) and tensor-core (P4) stages.  OUT = 0 adds the element's entries into
-// the CSR values and the residual (first contributor in colour order stores,
-// later ones add); OUT = 1 stores them into the element's staging records
-// (*SO), which the row gather sums afterwards.
-template <int N1, int PM, int EG_, int SPLIT, class H, int OUT = 0>
+// of the current colour.  p4_first swaps the order of the independent stages
+// P3 (residual and coupling) and P4 (displacement block).  OUT = 0 adds the
+// element's entries into the CSR values and the residual (first contributor
+// in colour order stores, later ones add); OUT = 1 stores them into the
+// element's staging records (*SO), which the row gather sums afterwards.
+template <int N1, int PM, int EG_, class T, class H, int OUT = 0>
 __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems, int count, int grp, bool p4_first,
                                           unsigned char* sm, const cmfe::StageOut* SO = nullptr) {
-  using C = MixCfg<N1, PM, EG_>;
+  using C = MixCfg<N1, PM, EG_, T>;
   constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, NU3 = C::NU3, NROW = C::NROW, EG = C::EG;
-  constexpr int KPW = C::KPW;
   H* s_psi = reinterpret_cast<H*>(sm + C::O_PSI64);  // [g][q]
   H* s_L = reinterpret_cast<H*>(sm + C::O_L);        // [q][gi]
   H* s_w = reinterpret_cast<H*>(sm + C::O_W);        // [g]
@@ -348,11 +314,10 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   H* s_dz = reinterpret_cast<H*>(sm + C::O_DZ);      // [el][g][c*3+k]
   H* s_pg = reinterpret_cast<H*>(sm + C::O_PG);      // [el][g]
   H* s_r64 = reinterpret_cast<H*>(sm + C::O_R64);    // [el][g][REC64]
-  float* s_phi32 = reinterpret_cast<float*>(sm + C::O_PHI32);  // [g][b][l], l padded to 4
-  float* s_r32 = reinterpret_cast<float*>(sm + C::O_R32);      // [el][g][REC32]
-  uint32_t* s_A = reinterpret_cast<uint32_t*>(sm + C::O_A);    // [hi/lo][a][KPW]
-  float* s_f32 = reinterpret_cast<float*>(sm + C::O_F32);      // scratch of P3 and P4 (EG x 2592 B)
-  int* s_node = reinterpret_cast<int*>(sm + C::O_NODE);        // [el][NR+1]
+  T* s_D = reinterpret_cast<T*>(sm + C::O_R32);                // [el][g][UU_REC]
+  T* s_mm = reinterpret_cast<T*>(sm + C::O_MM);
+  float* s_f32 = reinterpret_cast<float*>(sm + C::O_F32);      // scratch of P3 (EG x 2592 B)
+  int* s_node = reinterpret_cast<int*>(sm + (OUT == 1 ? C::O_NODE1 : C::O_NODE0));  // [el][NR+1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nu = P.nu;
   const int nvalid = min(EG, count - grp * EG);
@@ -438,9 +403,9 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   }
   __syncthreads();
   // ---- P2 (H: kinematics, stress and the residual / coupling records per
-  // Gauss point) and P2b (FP32: the spatial tangent pulled back to xi space)
+  // Gauss point) and P2b (T: the spatial tangent pulled back to xi space)
   // run at the same time on the two halves of the CTA, so that the FP64 and
-  // the FP32 pipes overlap; P2b forms the FP32 kinematics it needs itself from
+  // the FP32 pipes overlap; P2b forms the kinematics it needs itself from
   // the same gradients.
   constexpr int HALF = C::THREADS / 2;
   if (tid < HALF) {
@@ -505,70 +470,21 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
       const int el = t / NG, g = t % NG;
       if (el >= nvalid) continue;
       const int e = elem_at(P, elems, grp * EG + el);
-      float Mf[3][3], Ff[3][3], cf[4], Cf[6][6], Sf[6], inv[3][3];
+      T Mt[3][3], dn[9], jx, ct[4];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) Mf[c][k] = hf(s_dz[t * 9 + c * 3 + k]);
-      H dnh[9], jxh;
-      load_geo(P, e, g, dnh, jxh);
-      float dn[9];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) dn[i] = hf(dnh[i]);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) Ff[i][j] = Mf[i][0] * dn[j] + Mf[i][1] * dn[3 + j] + Mf[i][2] * dn[6 + j];
-      float adj[3][3];
-      adj[0][0] = Mf[1][1] * Mf[2][2] - Mf[1][2] * Mf[2][1];
-      adj[0][1] = Mf[0][2] * Mf[2][1] - Mf[0][1] * Mf[2][2];
-      adj[0][2] = Mf[0][1] * Mf[1][2] - Mf[0][2] * Mf[1][1];
-      adj[1][0] = Mf[1][2] * Mf[2][0] - Mf[1][0] * Mf[2][2];
-      adj[1][1] = Mf[0][0] * Mf[2][2] - Mf[0][2] * Mf[2][0];
-      adj[1][2] = Mf[0][2] * Mf[1][0] - Mf[0][0] * Mf[1][2];
-      adj[2][0] = Mf[1][0] * Mf[2][1] - Mf[1][1] * Mf[2][0];
-      adj[2][1] = Mf[0][1] * Mf[2][0] - Mf[0][0] * Mf[2][1];
-      adj[2][2] = Mf[0][0] * Mf[1][1] - Mf[0][1] * Mf[1][0];
-      const float det = Mf[0][0] * adj[0][0] + Mf[0][1] * adj[1][0] + Mf[0][2] * adj[2][0];
-      const float rdet = 1.0f / det;
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) inv[i][j] = adj[i][j] * rdet;
-      const float jz = fabsf(det);
-      const float jznuf = jz / hf(jxh);
-      const float jgwf = jz * hf(s_w[g]);
-      const float pgf = hf(s_pg[t]);
+        for (int k = 0; k < 3; ++k) Mt[c][k] = to_t<T>(s_dz[t * 9 + c * 3 + k]);
+      load_geo_t(P, e, g, dn, jx);
       const double* cm = P.mat + (P.matpe ? (size_t)e * P.nmat : 0);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) cf[i] = i < P.nmat ? (float)cm[i] : 0.0f;
-      d_gauss_elasticity<float>(P.law, cf, Ff, jznuf, pgf, Cf, Sf);
-      float* r32 = &s_r32[t * C::REC32];
-#pragma unroll
-      for (int blk = 0; blk < 6; ++blk) {
-        int m, n;
-        blk_mn(blk, m, n);
-        float sub[3][3], tmp[3][3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j)
-            sub[i][j] = jgwf * (Cf[t2v(i, m)][t2v(j, n)] + (m == n ? Sf[t2v(i, j)] : 0.0f));
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) tmp[k][j] = inv[k][0] * sub[0][j] + inv[k][1] * sub[1][j] + inv[k][2] * sub[2][j];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int l = 0; l < 3; ++l)
-            r32[blk * 9 + k * 3 + l] = tmp[k][0] * inv[l][0] + tmp[k][1] * inv[l][1] + tmp[k][2] * inv[l][2];
-      }
-      if (!(isfinite(Cf[0][0]) && isfinite(Cf[3][3]))) atomicOr(P.status, 1u);
+      for (int i = 0; i < 4; ++i) ct[i] = i < P.nmat ? (T)cm[i] : T(0);
+      if (!uu_tangent<T>(P.law, ct, Mt, dn, T(1) / jx, to_t<T>(s_w[g]), to_t<T>(s_pg[t]), &s_D[t * UU_REC]))
+        atomicOr(P.status, 1u);
     }
   }
   __syncthreads();
-  // P3 (FP64 pipe) and P4 (tensor cores, scatter) are independent; the
+  // P3 (FP64 pipe) and P4 (displacement block) are independent; the
   // second wave of CTAs runs them in the opposite order so that the two
   // CTAs sharing an SM work on different pipes.
   for (int ph = 0; ph < 2; ++ph) {
@@ -778,28 +694,14 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
         }
       }
     } else {
-      // ---- P4: displacement blocks on tensor cores (FP32 accumulate).
-      // The six lower blocks of one element are stacked along M:
-      //   D'[(blk,b)][a] = sum_kappa W^{blk}[kappa][b] Phi[kappa][a] = K^{blk}(a,b),
-      // kappa = 28k + g (derivative-major, one padding slot per derivative).  Each warp owns (element, m-tile) tasks; it forms its
-      // A fragments (W values) in registers from the per-Gauss-point D^{blk}
-      // records and the gradient table, and takes B = Phi from shared memory.
+      // ---- P4: displacement blocks by sum factorisation, warp by warp
       if (!P.res_only) {
-        // Rows of the stacked blocks: block blk occupies rows [blk * BS, blk * BS + NPE).
-        // For triquadratic elements BS = 32, so that a 16-row tile never spans
-        // two blocks and the two rows a thread holds share the D^{blk} loads.
-        constexpr int BS = NPE > 16 ? 32 : NPE;
-        constexpr int MROWS = 6 * BS;
-        constexpr int MT2 = (MROWS + 15) / 16;
-        const int gq = lane >> 2, tq = lane & 3;
-        const uint32_t* Bhi = s_A;
-        const uint32_t* Blo = s_A + C::AROWS * KPW;
-        // Scatter addresses staged in shared memory (regions P3 does not read
-        // while this stage runs): base[el][3m+n][a] = start of the n-block of
-        // row (m, node a), and the element's rank table over its u nodes.
-        int* s_base = reinterpret_cast<int*>(s_dz);
-        uint16_t* s_tab = reinterpret_cast<uint16_t*>(s_f32);
-        __syncthreads();
+        // Coloured order: scatter addresses staged in shared memory:
+        // base[el][3m+n][a] = start of the n-block of row (m, node a), and the
+        // element's rank table over its u nodes.
+        int* s_base = reinterpret_cast<int*>(sm + C::O_BASE);
+        uint16_t* s_tab = reinterpret_cast<uint16_t*>(sm + C::O_TAB);
+        T* s1 = reinterpret_cast<T*>(sm + C::O_DZ) + (size_t)warp * UUCfg<N1>::S1;
         if constexpr (OUT == 0) {
           for (int i = tid; i < EG * 9 * NPE; i += C::THREADS) {
             const int a = i % NPE, mn = (i / NPE) % 9, el = i / (9 * NPE);
@@ -811,113 +713,58 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
             const int a = ab / NPE, b = ab % NPE;
             s_tab[i] = el < nvalid ? P.tables[(size_t)s_node[el * (NR + 1) + NR] * NR * NR + a * NR + b] : 0;
           }
-          __syncthreads();
         }
-        for (int task = warp; task < nvalid * MT2; task += C::THREADS / 32) {
-          const int el = task / MT2, mt = task % MT2;
-          const int* bs = &s_base[el * 9 * NPE];
-          const uint16_t* tb = &s_tab[el * NPE * NPE];
-          const float* r32 = &s_r32[el * NG * C::REC32];
-          float acc[C::NT][4];
+        __syncthreads();  // the scratch below is free (P3 done or not begun)
+        for (int task = warp; task < UUCfg<N1>::tasks(nvalid); task += C::THREADS / 32) {
+          uu_warp_task<N1, T>(s_D, s_mm, s1, task, nvalid, lane,
+                              [&](int el, int blk, int a12, int b12, const T (&K)[N1][N1]) {
+            int m, n;
+            blk_mn(blk, m, n);
+            // a diagonal block's entries beyond its diagonal are mirrors
+            const bool diag = blk < 3 && a12 == b12;
+            constexpr int NP = N1 * N1;
+            if constexpr (OUT == 1) {
+              T* st = stage_uu<T>(*SO) + (size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_uu(NPE);
+              T* s0 = st + ((a12 * 3 + m) * 3 + n) * NPE + b12;
+              T* s1m = st + ((b12 * 3 + n) * 3 + m) * NPE + a12;
 #pragma unroll
-          for (int nt = 0; nt < C::NT; ++nt)
+              for (int a3 = 0; a3 < N1; ++a3)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) acc[nt][h] = 0.f;
-          const int R0 = 16 * mt + gq, R1 = R0 + 8;
-          const int blk0 = R0 / BS, b0 = R0 % BS, blk1 = R1 / BS, b1 = R1 % BS;
-          const bool v0 = R0 < MROWS && b0 < NPE, v1 = R1 < MROWS && b1 < NPE;
-#pragma unroll 1
-          for (int kt = 0; kt < C::KT; ++kt) {
-            float wv[2][4];  // [row r0/r1][kappa 2t, 2t+1, 2t+8, 2t+9]
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int kap = 16 * kt + 2 * tq + (j & 1) + (j >= 2 ? 8 : 0);
-              const int k = kap / 28, g = kap % 28;
-              const bool kv = kap < C::KAP && g < NG;
-              float w0 = 0.f, w1 = 0.f;
-              if constexpr (BS % 16 == 0) {  // both rows in block blk0
-                if (kv && (v0 || v1)) {
-                  const float* dt = &r32[g * C::REC32 + blk0 * 9 + k * 3];
-                  const float d0 = dt[0], d1 = dt[1], d2 = dt[2];
-                  if (v0) {
-                    const float4 ph = *reinterpret_cast<const float4*>(&s_phi32[g * C::PHS + 4 * b0]);
-                    w0 = d0 * ph.x + d1 * ph.y + d2 * ph.z;
-                  }
-                  if (v1) {
-                    const float4 ph = *reinterpret_cast<const float4*>(&s_phi32[g * C::PHS + 4 * b1]);
-                    w1 = d0 * ph.x + d1 * ph.y + d2 * ph.z;
-                  }
+                for (int b3 = 0; b3 < N1; ++b3) {
+                  if (diag && a3 > b3) continue;
+                  if (N1 == 2 && blk < 3 && a12 + NP * a3 > b12 + NP * b3) continue;
+                  s0[a3 * NP * 9 * NPE + b3 * NP] = K[a3][b3];
+                  if (!(diag && a3 == b3)) s1m[b3 * NP * 9 * NPE + a3 * NP] = K[a3][b3];
                 }
-              } else {
-                if (kv && v0) {
-                  const float* dt = &r32[g * C::REC32 + blk0 * 9 + k * 3];
-                  const float4 ph = *reinterpret_cast<const float4*>(&s_phi32[g * C::PHS + 4 * b0]);
-                  w0 = dt[0] * ph.x + dt[1] * ph.y + dt[2] * ph.z;
+            } else {
+              const int* bs = &s_base[el * 9 * NPE];
+              const uint16_t* tb = &s_tab[el * NPE * NPE];
+#pragma unroll
+              for (int a3 = 0; a3 < N1; ++a3)
+#pragma unroll
+                for (int b3 = 0; b3 < N1; ++b3) {
+                  if (diag && a3 > b3) continue;
+                  const int a = a12 + NP * a3, b = b12 + NP * b3;
+                  if (N1 == 2 && blk < 3 && a > b) continue;
+                  const float v = (float)K[a3][b3];
+                  const uint16_t tab_ab = tb[a * NPE + b];
+                  const int p1 = bs[(m * 3 + n) * NPE + a] + (tab_ab & 0x7fff);
+                  if (tab_ab & 0x8000)
+                    P.vals_uu[p1] = v;
+                  else
+                    atomicAdd(&P.vals_uu[p1], v);
+                  if (diag && a3 == b3) continue;
+                  const uint16_t tab_ba = tb[b * NPE + a];
+                  const int p2 = bs[(n * 3 + m) * NPE + b] + (tab_ba & 0x7fff);
+                  if (tab_ba & 0x8000)
+                    P.vals_uu[p2] = v;
+                  else
+                    atomicAdd(&P.vals_uu[p2], v);
                 }
-                if (kv && v1) {
-                  const float* dt = &r32[g * C::REC32 + blk1 * 9 + k * 3];
-                  const float4 ph = *reinterpret_cast<const float4*>(&s_phi32[g * C::PHS + 4 * b1]);
-                  w1 = dt[0] * ph.x + dt[1] * ph.y + dt[2] * ph.z;
-                }
-              }
-              wv[0][j] = w0;
-              wv[1][j] = w1;
             }
-            uint32_t ah[4], al[4];
-            split_bf16(wv[0][0], wv[0][1], ah[0], al[0]);  // row r0, cols 2t..2t+1
-            split_bf16(wv[1][0], wv[1][1], ah[1], al[1]);  // row r1, cols 2t..2t+1
-            split_bf16(wv[0][2], wv[0][3], ah[2], al[2]);  // row r0, cols 2t+8..
-            split_bf16(wv[1][2], wv[1][3], ah[3], al[3]);  // row r1, cols 2t+8..
-#pragma unroll
-            for (int nt = 0; nt < C::NT; ++nt) {
-              // B fragments of this n-tile: high and low parts, kappa halves
-              // 16 kt .. 16 kt + 7 and 16 kt + 8 .. 16 kt + 15, in one ldmatrix
-              const int mi = lane >> 3;
-              uint32_t bf[4];
-              ldmatrix_x4(bf, (mi < 2 ? Bhi : Blo) + (8 * nt + (lane & 7)) * KPW + 8 * kt + 4 * (mi & 1));
-              mma_bf16(acc[nt], ah[0], ah[1], ah[2], ah[3], bf[0], bf[1]);
-              if (SPLIT == 3) {
-                mma_bf16(acc[nt], ah[0], ah[1], ah[2], ah[3], bf[2], bf[3]);
-                mma_bf16(acc[nt], al[0], al[1], al[2], al[3], bf[0], bf[1]);
-              }
-            }
-          }
-          // scatter K^{blk}(a, b) and its mirror
-#pragma unroll
-          for (int nt = 0; nt < C::NT; ++nt)
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              const bool vr = h < 2 ? v0 : v1;
-              const int blk = h < 2 ? blk0 : blk1, b = h < 2 ? b0 : b1;
-              const int a = 8 * nt + 2 * tq + (h & 1);
-              if (!vr || a >= NPE) continue;
-              int m, n;
-              blk_mn(blk, m, n);
-              if (m == n && a < b) continue;
-              const float v = acc[nt][h];
-              if constexpr (OUT == 1) {
-                float* st = SO->uu + (size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_uu(NPE);
-                st[(size_t)(m * NPE + a) * NU3 + n * NPE + b] = v;
-                if (!(m == n && a == b)) st[(size_t)(n * NPE + b) * NU3 + m * NPE + a] = v;
-                continue;
-              }
-              const uint16_t tab_ab = tb[a * NPE + b];
-              const int p1 = bs[(m * 3 + n) * NPE + a] + (tab_ab & 0x7fff);
-              if (tab_ab & 0x8000)
-                P.vals_uu[p1] = v;
-              else
-                atomicAdd(&P.vals_uu[p1], v);
-              if (!(m == n && a == b)) {
-                const uint16_t tab_ba = tb[b * NPE + a];
-                const int p2 = bs[(n * 3 + m) * NPE + b] + (tab_ba & 0x7fff);
-                if (tab_ba & 0x8000)
-                  P.vals_uu[p2] = v;
-                else
-                  atomicAdd(&P.vals_uu[p2], v);
-              }
-            }
+          });
         }
-        __syncthreads();  // P3 may run next and reuse the staging regions
+        __syncthreads();  // P3 may run next and reuse the scratch
       }
     }
   }

@@ -161,9 +161,8 @@ __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, c
         // the lower block entry and its mirror: distinct entries for distinct
         // (oh, ms, ns), so the lanes never touch the same word
         float* st = SO->uu + (size_t)e * cmfe::rec_stride_uu(NPE);
-        const int R = mh * NPE + a, Cc = nh * NPE + b;
-        st[(size_t)R * (3 * NPE) + Cc] += (float)acc;
-        st[(size_t)Cc * (3 * NPE) + R] += (float)acc;
+        st[cmfe::rec_uu(NPE, mh, a, nh, b)] += (float)acc;
+        st[cmfe::rec_uu(NPE, nh, b, mh, a)] += (float)acc;
         continue;
       }
       if (mode == 1) {
