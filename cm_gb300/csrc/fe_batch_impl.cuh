@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(BT_THREADS, MINB) fe_mixed_batch_kernel(BatchA
         const int i = u * BT_WARPS + warp;
         if (i < nb) {
           if (c_members[s].type >= 2) {
-            if constexpr ((TM & 12) != 0) surface_element<3>(P, belems[i], bmask, 0, 1, ws[warp], lane);
+            if constexpr ((TM & 12) != 0) surface_element<3, 8>(P, belems[i], bmask, 0, 1, ws[warp], lane);
           } else {
-            if constexpr ((TM & 3) != 0) surface_element<2>(P, belems[i], bmask, 0, 1, ws[warp], lane);
+            if constexpr ((TM & 3) != 0) surface_element<2, 8>(P, belems[i], bmask, 0, 1, ws[warp], lane);
           }
         }
       }

@@ -1,30 +1,36 @@
-// libcm_fe: the row gather of the staged assembly, device code shared by the
-// separate gather kernel (fe_gather.cu) and the fused assembly kernel
-// (fe_mixed.cu), which gathers a node's rows as soon as the last element
-// around the node has stored its records.
+// libcm_fe: the row gather of the staged assembly, device code of the fused
+// assembly kernels, which gather a node's rows as soon as the last element
+// around the node has stored its record.
 //
 // One warp forms the rows of one row node from the per-element records
-// (StageOut) of the elements around it, adding them in increasing element
-// number -- a fixed order, so the result is deterministic -- into a
-// shared-memory copy of the rows, and then writes each row once,
-// contiguously.  This is the addition of EQUATIONS_MATRICES_JACOBIAN_ELEMENT_ADD
-// / MATRIX_VALUES_ADD_DP2 (equations_matrices_routines.f90:3174-3225,
-// matrix_vector.f90:2756-2880) and of the residual vector add
-// (distributed_matrix_vector.f90:8853-8927), organised by rows instead of by
-// elements: every matrix sector is written once, in full, and never read.
+// (cmfe::Rec) of the elements around it, adding them in increasing element
+// number -- a fixed order, so the result is deterministic -- and writes each
+// row once, contiguously.  This is the addition of
+// EQUATIONS_MATRICES_JACOBIAN_ELEMENT_ADD / MATRIX_VALUES_ADD_DP2
+// (equations_matrices_routines.f90:3174-3225, matrix_vector.f90:2756-2880) and
+// of the residual vector add (distributed_matrix_vector.f90:8853-8927),
+// organised by rows instead of by elements: every matrix sector is written
+// once, in full, and never read.
 //
-// The incidences of a row node are read 32 at a time, lane i loading
-// incidence i and its element's rank-table row, and handed to the warp by
-// shuffles: the loads of one incidence (its ranks and record values) then
-// depend on no other load.
+// What bounds it is latency (a corner node of a triquadratic box sums eight
+// elements), so nothing waits in a chain: what a row node needs of an element
+// is one contiguous piece of the element's record, the pieces of four
+// elements are copied to shared memory at once (cp.async), and every lane
+// keeps its columns of the rows in registers.  Which of an element's nodes
+// belongs to a column comes from the inverse of the element's rank-table
+// row, built in shared memory while the copies are in flight.  Adding in
+// shared memory instead, one element after the other, took 80 k of the 188 k
+// cycles of an element group of the 32^3 box; this form is in the figures at
+// the fused kernel.
 //
-// Row layout (the mixed split of the handle): a displacement row (m, a)
-// holds [u_x | u_y | u_z] blocks of wu[a] columns in the FP32 array at
+// Row layout of the mixed split: a displacement row (m, a) holds
+// [u_x | u_y | u_z] blocks of wu[a] columns in the FP32 array at
 // uu_row_ptr[m nu + a] and its pressure columns in the FP64 array at
 // cp_row_ptr[m nu + a]; a pressure row q holds [u_x | u_y | u_z] blocks of
 // wp[q] columns and then its pressure-pressure columns (structural zeros) at
-// cp_row_ptr[3 nu + q].  The column of a neighbour inside a block is its rank
-// in the row node's neighbour list, read from the element's rank table.
+// cp_row_ptr[3 nu + q].  With FP64 blocks (T = double) all of a row is in one
+// array at row_ptr: [u_x | u_y | u_z | p].  The column of a neighbour inside a
+// block is its rank in the row node's neighbour list.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,120 +41,277 @@
 
 namespace {
 
-// Record loads: through L2 only (CG = true) when other CTAs of the same
-// launch wrote the records, which this SM's L1 does not see.
-template <bool CG, class T>
-__device__ __forceinline__ T rec_load(const T* p) {
-  if constexpr (CG)
-    return __ldcg(p);
-  else
-    return *p;
-}
+constexpr int GR = 4;           // elements whose pieces are in flight together
+constexpr int GPOS = 128;       // columns of a u block in registers at a time (4 per lane)
+constexpr int GPP = 32;         // pressure columns at a time (1 per lane)
+constexpr int GNONE = 255;      // no local node at this column
+constexpr int GLIST = 8;        // incidences of a ready node read ahead by the whole CTA
 
-// The three displacement rows of u node a, by one warp; `mine` is the warp's
-// shared scratch (36 wu bytes rounded up to 16, then 24 wc bytes).
-template <int NPE, int NPP, bool CG>
-__device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe::StageOut& S, const int32_t* u_inc_ptr,
-                                             const int32_t* u_inc, int a, unsigned char* mine, int lane) {
-  constexpr int NR = NPE + NPP, NU3 = 3 * NPE;
-  const int nu = P.nu;
+// A row node whose elements are all assembled: u node id < nu, else pressure
+// row node id - nu; its incidences [k0, k0 + cnt).
+struct ReadyNode {
+  int id, k0, cnt, pad;
+};
+
+// Shared scratch of one gathering warp: the pieces in flight; u nodes: the
+// local nodes of every column [GPOS][GR], and the sums of the pressure columns
+// and the residual; pressure nodes: the sums of the row instead.
+template <int NPE, int NPP, class T>
+struct GatherCfg {
+  using R = cmfe::Rec<NPE, NPP, T>;
+  static constexpr int O_ACC = GR * R::ROW;                 // u: [3][GPP], residual [3]
+  static constexpr int O_INV = O_ACC + (3 * GPP + 4) * 8;
+  static constexpr int O_ACCP = GR * R::PROW;               // p: [3][GPOS], residual
+  static constexpr int UB = O_INV + GR * GPOS, PB = O_ACCP + (3 * GPOS + 2) * 8;
+  static constexpr int BYTES = UB > PB ? UB : PB;           // multiples of 16
+};
+
+// Copies n bytes (a multiple of 16) from global memory to the warp's shared
+// memory, through L2 only: other CTAs of the same launch wrote them.
+__device__ __forceinline__ void copy_piece(unsigned char* dst, const unsigned char* src, int n, int lane) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  for (int i = 16 * lane; i < n; i += 512)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + i), "l"(src + i) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// One 32-bit word holds the local nodes of the four elements of a round at
+// one column.
+static_assert(GR == 4, "one byte per element of a round");
+__device__ __forceinline__ int inv_at(uint32_t w, int j) { return (w >> (8 * j)) & 255; }
+
+// The three displacement rows of u node a, by one warp.  list: its first
+// GLIST incidences (element and local node, rank-table row).
+template <int NPE, int NPP, class T>
+__device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe::StageOut& S, const cmfe::FusedArgs& F,
+                                             const ReadyNode& rn, const int2* list, unsigned char* mine, int lane) {
+  using R = cmfe::Rec<NPE, NPP, T>;
+  constexpr int NR = NPE + NPP;
+  constexpr bool FULL = sizeof(T) == 8;
+  const int nu = P.nu, a = rn.id;
   const int wu = P.wu[a];
-  const int ru = 3 * wu;  // uu row length
-  const int wc = P.cp_row_ptr[(size_t)a + 1] - P.cp_row_ptr[(size_t)a];  // pressure columns, the same for m = 0..2
-  float* acc_u = reinterpret_cast<float*>(mine);                            // [3][ru]
-  double* acc_c = reinterpret_cast<double*>(mine + ((12 * ru + 15) & ~15));  // [3][wc]
-  for (int i = lane; i < 3 * ru; i += 32) acc_u[i] = 0.f;
-  for (int i = lane; i < 3 * wc; i += 32) acc_c[i] = 0.0;
-  double racc = 0.0;
-  __syncwarp();
-  const int k0 = u_inc_ptr[a], k1 = u_inc_ptr[a + 1];
-  for (int kb = k0; kb < k1; kb += 32) {
-    // up to 32 incidences at once: lane i holds incidence kb + i and its rank-table row
-    const int cnt = min(32, k1 - kb);
-    int pk = 0, trow = 0;
-    if (lane < cnt) {
-      pk = u_inc[kb + lane];
-      trow = P.elem_table[pk >> 5] * NR + (pk & 31);
+  T* du[3];
+  double* dc[3];
+  int wc;
+  if constexpr (FULL) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      du[m] = P.vals + P.row_ptr[(size_t)m * nu + a];
+      dc[m] = du[m] + 3 * wu;
     }
-    for (int j = 0; j < cnt; ++j) {
-      const int packed = __shfl_sync(0xffffffffu, pk, j);
-      const int e = packed >> 5, la = packed & 31;
-      const uint16_t* tab = P.tables + (size_t)__shfl_sync(0xffffffffu, trow, j) * NR;
-      if (lane < NPE) {
-        const int rk = tab[lane] & 0x7fff;
-        const float* src = S.uu + (size_t)e * cmfe::rec_stride_uu(NPE) + cmfe::rec_uu(NPE, 0, la, 0, lane);
-        float v[9];
+    wc = P.row_ptr[(size_t)a + 1] - P.row_ptr[(size_t)a] - 3 * wu;
+  } else {
 #pragma unroll
-        for (int m = 0; m < 3; ++m)
+    for (int m = 0; m < 3; ++m) {
+      du[m] = P.vals_uu + P.uu_row_ptr[(size_t)m * nu + a];
+      dc[m] = P.vals + P.cp_row_ptr[(size_t)m * nu + a];
+    }
+    wc = P.cp_row_ptr[(size_t)a + 1] - P.cp_row_ptr[(size_t)a];  // the same for m = 0..2
+  }
+  using G = GatherCfg<NPE, NPP, T>;
+  uint8_t* inv = mine + G::O_INV;
+  double* cacc = reinterpret_cast<double*>(mine + G::O_ACC);
+  const int passes = max((wu + GPOS - 1) / GPOS, (wc + GPP - 1) / GPP);
+  for (int pass = 0; pass < passes; ++pass) {  // one pass unless the neighbourhood is very large
+    const int p0 = pass * GPOS, q0 = pass * GPP;
+    T acc[GPOS / 32][9];
+    for (int i = lane; i < 3 * GPP + 3; i += 32) cacc[i] = 0.0;
 #pragma unroll
-          for (int n = 0; n < 3; ++n) v[m * 3 + n] = rec_load<CG>(src + (3 * m + n) * NPE);
+    for (int i = 0; i < GPOS / 32; ++i)
 #pragma unroll
-        for (int m = 0; m < 3; ++m)
+      for (int mn = 0; mn < 9; ++mn) acc[i][mn] = T(0);
+    for (int kb = 0; kb < rn.cnt; kb += GR) {
+      const int cnt = min(GR, rn.cnt - kb);
+      int2 in = {0, 0};
+      if (lane < cnt) in = kb + lane < GLIST ? list[kb + lane] : int2{F.u_inc[rn.k0 + kb + lane], F.u_inc_row[rn.k0 + kb + lane]};
 #pragma unroll
-          for (int n = 0; n < 3; ++n) acc_u[m * ru + n * wu + rk] += v[m * 3 + n];
-      }
-      if (lane < NPP) {
-        const int rq = tab[NPE + lane] & 0x7fff;
-        const double* src = S.cp + (size_t)e * cmfe::rec_stride_cp(NPE, NPP) + lane * NU3 + la;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) acc_c[m * wc + rq] += rec_load<CG>(src + m * NPE);
-      }
-      if (lane < 3 && P.r) racc += rec_load<CG>(S.r + (size_t)e * cmfe::rec_stride_r(NPE, NPP) + lane * NPE + la);
+      for (int i = 0; i < GPOS / 32; ++i) reinterpret_cast<uint32_t*>(inv)[32 * i + lane] = 0xffffffffu;
       __syncwarp();
-    }
-  }
+      int rk[GR], rq[GR];
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    float* du = P.vals_uu + P.uu_row_ptr[(size_t)m * nu + a];
-    for (int i = lane; i < ru; i += 32) du[i] = acc_u[m * ru + i];
-    double* dc = P.vals + P.cp_row_ptr[(size_t)m * nu + a];
-    for (int i = lane; i < wc; i += 32) dc[i] = acc_c[m * wc + i];
+      for (int j = 0; j < GR; ++j) {
+        const int packed = __shfl_sync(0xffffffffu, in.x, j);
+        const uint16_t* tab = P.tables + (size_t)__shfl_sync(0xffffffffu, in.y, j) * NR;
+        rk[j] = rq[j] = -1;
+        if (j < cnt) {
+          if (lane < NPE) rk[j] = (tab[lane] & 0x7fff) - p0;
+          if (lane < NPP) rq[j] = (tab[NPE + lane] & 0x7fff) - q0;
+          copy_piece(mine + j * R::ROW, S.rec + (size_t)(packed >> 5) * R::BYTES + (packed & 31) * R::ROW, R::ROW, lane);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < GR; ++j)
+        if (rk[j] >= 0 && rk[j] < GPOS) inv[rk[j] * GR + j] = (uint8_t)lane;
+      copies_done();
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < GPOS / 32; ++i) {
+        if (p0 + 32 * i >= wu) break;
+        const uint32_t w = reinterpret_cast<const uint32_t*>(inv)[32 * i + lane];
+#pragma unroll
+        for (int j = 0; j < GR; ++j) {
+          const int b = inv_at(w, j);
+          if (b != GNONE) {
+            const T* v = reinterpret_cast<const T*>(mine + j * R::ROW) + b;
+#pragma unroll
+            for (int mn = 0; mn < 9; ++mn) acc[i][mn] += v[mn * NPE];
+          }
+        }
+      }
+      // the piece's FP64 values, [m][q] coupling and [m] residual, one per
+      // lane: an FP64 warp instruction costs the same for 3 lanes as for 32
+#pragma unroll
+      for (int j = 0; j < GR; ++j) {
+        if (j >= cnt) break;
+        const int tq = __shfl_sync(0xffffffffu, rq[j], lane % NPP);
+        const int at = lane < 3 * NPP ? (tq >= 0 && tq < GPP ? lane / NPP * GPP + tq : -1) : 3 * GPP + lane - 3 * NPP;
+        if (lane < 3 * NPP + 3 && at >= 0) cacc[at] += reinterpret_cast<const double*>(mine + j * R::ROW + R::OC)[lane];
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < GPOS / 32; ++i) {
+      const int pos = p0 + 32 * i + lane;
+      if (pos < wu) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+#pragma unroll
+          for (int n = 0; n < 3; ++n) du[m][n * wu + pos] = acc[i][3 * m + n];
+      }
+    }
+    if (q0 + lane < wc) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) dc[m][q0 + lane] = cacc[m * GPP + lane];
+    }
+    if (pass == 0 && lane < 3 && P.r) P.r[(size_t)lane * nu + a] = cacc[3 * GPP + lane];
+    __syncwarp();
   }
-  if (lane < 3 && P.r) P.r[(size_t)lane * nu + a] = racc;
-  __syncwarp();
 }
 
-// The row of pressure row node q, by one warp (scratch: 8 bytes per column).
-template <int NPE, int NPP, bool CG>
-__device__ __forceinline__ void gather_pnode(const cmfe::KParams& P, const cmfe::StageOut& S, const int32_t* p_inc_ptr,
-                                             const int32_t* p_inc, int q, unsigned char* mine, int lane) {
-  constexpr int NR = NPE + NPP, NU3 = 3 * NPE;
+// The row of pressure row node q, by one warp.
+template <int NPE, int NPP, class T>
+__device__ __forceinline__ void gather_pnode(const cmfe::KParams& P, const cmfe::StageOut& S, const cmfe::FusedArgs& F,
+                                             const ReadyNode& rn, const int2* list, unsigned char* mine, int lane) {
+  using R = cmfe::Rec<NPE, NPP, T>;
+  constexpr int NR = NPE + NPP;
+  const int q = rn.id - P.nu;
   const size_t row = (size_t)3 * P.nu + q;
+  const int32_t* rp = sizeof(T) == 8 ? P.row_ptr : P.cp_row_ptr;
   const int wp = P.wp[q];
-  const int len = P.cp_row_ptr[row + 1] - P.cp_row_ptr[row];
-  double* acc = reinterpret_cast<double*>(mine);  // [len]
-  for (int i = lane; i < len; i += 32) acc[i] = 0.0;  // pressure-pressure entries stay zero
-  double racc = 0.0;
-  __syncwarp();
-  const int k0 = p_inc_ptr[q], k1 = p_inc_ptr[q + 1];
-  for (int kb = k0; kb < k1; kb += 32) {
-    const int cnt = min(32, k1 - kb);
-    int pk = 0, trow = 0;
-    if (lane < cnt) {
-      pk = p_inc[kb + lane];
-      trow = P.elem_table[pk >> 3] * NR + NPE + (pk & 7);
-    }
-    for (int j = 0; j < cnt; ++j) {
-      const int packed = __shfl_sync(0xffffffffu, pk, j);
-      const int tr = __shfl_sync(0xffffffffu, trow, j);
-      const int e = packed >> 3, lq = packed & 7;
-      if (lane < NPE) {
-        const int rk = P.tables[(size_t)tr * NR + lane] & 0x7fff;
-        const double* src = S.cp + (size_t)e * cmfe::rec_stride_cp(NPE, NPP) + lq * NU3 + lane;
-        double v[3];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) v[n] = rec_load<CG>(src + n * NPE);
-#pragma unroll
-        for (int n = 0; n < 3; ++n) acc[n * wp + rk] += v[n];
-      }
-      if (lane == 0 && P.r) racc += rec_load<CG>(S.r + (size_t)e * cmfe::rec_stride_r(NPE, NPP) + NU3 + lq);
+  const int len = rp[row + 1] - rp[row];
+  double* out = P.vals + rp[row];
+  double* acc = reinterpret_cast<double*>(mine + GatherCfg<NPE, NPP, T>::O_ACCP);
+  constexpr int NV = 3 * NPE + 1;  // values of a piece: [n][b] coupling, residual
+  for (int p0 = 0; p0 < wp || p0 == 0; p0 += GPOS) {
+    for (int i = lane; i < 3 * GPOS + 1; i += 32) acc[i] = 0.0;
+    for (int kb = 0; kb < rn.cnt; kb += GR) {
+      const int cnt = min(GR, rn.cnt - kb);
+      int2 in = {0, 0};
+      if (lane < cnt) in = kb + lane < GLIST ? list[kb + lane] : int2{F.p_inc[rn.k0 + kb + lane], F.p_inc_row[rn.k0 + kb + lane]};
       __syncwarp();
+      int rk[GR];
+#pragma unroll
+      for (int j = 0; j < GR; ++j) {
+        const int packed = __shfl_sync(0xffffffffu, in.x, j);
+        const uint16_t* tab = P.tables + (size_t)__shfl_sync(0xffffffffu, in.y, j) * NR;
+        rk[j] = -1;
+        if (j < cnt) {
+          if (lane < NPE) rk[j] = (tab[lane] & 0x7fff) - p0;
+          copy_piece(mine + j * R::PROW, S.rec + (size_t)(packed >> 3) * R::BYTES + R::P0 + (packed & 7) * R::PROW,
+                     R::PROW, lane);
+        }
+      }
+      copies_done();
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < GR; ++j) {
+        if (j >= cnt) break;
+        const double* v = reinterpret_cast<const double*>(mine + j * R::PROW);
+#pragma unroll
+        for (int s = 0; s < (NV + 31) / 32; ++s) {
+          const int i = 32 * s + lane;
+          const int tk = __shfl_sync(0xffffffffu, rk[j], i % NPE);
+          const int at = i < 3 * NPE ? (tk >= 0 && tk < GPOS ? i / NPE * GPOS + tk : -1) : 3 * GPOS;
+          if (i < NV && at >= 0) acc[at] += v[i];
+        }
+        __syncwarp();
+      }
     }
+    for (int i = lane; i < min(GPOS, wp - p0); i += 32) {
+#pragma unroll
+      for (int n = 0; n < 3; ++n) out[n * wp + p0 + i] = acc[n * GPOS + i];
+    }
+    if (p0 == 0) {
+      for (int i = 3 * wp + lane; i < len; i += 32) out[i] = 0.0;  // pressure-pressure entries
+      if (lane == 0 && P.r) P.r[row] = acc[3 * GPOS];
+    }
+    __syncwarp();
   }
-  double* dc = P.vals + P.cp_row_ptr[row];
-  for (int i = lane; i < len; i += 32) dc[i] = acc[i];
-  if (lane == 0 && P.r) P.r[row] = racc;
-  __syncwarp();
 }
+
+// Counts the finished elements around the row nodes of one element group
+// (nvalid elements, local node numbers s_node[el][NR + 1]) and gathers the
+// rows of the nodes this completes, by all threads of a CTA.  The records of
+// the group are stored; the caller's threads are past a barrier after that.
+// Publication follows the release/acquire pattern: every thread fences its
+// record stores before the counting, and a completing count is followed by a
+// fence before the records are read.  scratch: gather_scratch bytes.
+template <int NPE, int NPP, int EG, int THREADS, class T>
+struct GroupGather {
+  using G = GatherCfg<NPE, NPP, T>;
+  static constexpr int NR = NPE + NPP;
+  static constexpr int O_READY = THREADS / 32 * G::BYTES;
+  static constexpr int O_LIST = O_READY + EG * NR * (int)sizeof(ReadyNode);
+  static constexpr int SCRATCH = O_LIST + EG * NR * GLIST * (int)sizeof(int2);
+
+  static __device__ __forceinline__ void run(const cmfe::KParams& P, const cmfe::StageOut& S, const cmfe::FusedArgs& F,
+                                             const int* s_node, int nvalid, unsigned char* scratch, int* s_count,
+                                             int* s_next) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    ReadyNode* ready = reinterpret_cast<ReadyNode*>(scratch + O_READY);
+    int2* list = reinterpret_cast<int2*>(scratch + O_LIST);
+    __threadfence();  // release: this thread's record stores before the counts below
+    if (tid == 0) *s_count = *s_next = 0;
+    __syncthreads();
+    for (int i = tid; i < nvalid * NR; i += THREADS) {
+      __threadfence();  // cumulative release, after the barrier, for the stores of the whole CTA
+      const int el = i / NR, r = i % NR;
+      const int node = s_node[el * (NR + 1) + r];
+      const bool un = r < NPE;
+      const int id = un ? node : P.nu + node;
+      const int32_t* ptr = un ? F.u_inc_ptr + node : F.p_inc_ptr + node;
+      const int k0 = ptr[0], cnt = ptr[1] - k0;
+      if (atomicAdd(F.node_done + id, 1) + 1 == cnt) {
+        __threadfence();  // acquire: the records of every element around the node
+        ready[atomicAdd(s_count, 1)] = {id, k0, cnt, 0};
+      }
+    }
+    __syncthreads();
+    const int nready = *s_count;
+    // the incidences of all ready nodes in one go
+    for (int i = tid; i < nready * GLIST; i += THREADS) {
+      const ReadyNode rn = ready[i / GLIST];
+      const int j = i % GLIST;
+      if (j < rn.cnt) {
+        const bool un = rn.id < P.nu;
+        list[i] = int2{(un ? F.u_inc : F.p_inc)[rn.k0 + j], (un ? F.u_inc_row : F.p_inc_row)[rn.k0 + j]};
+      }
+    }
+    __syncthreads();
+    unsigned char* mine = scratch + (size_t)warp * G::BYTES;
+    for (;;) {  // nodes differ in cost: each warp takes the next one
+      int j = 0;
+      if (lane == 0) j = atomicAdd(s_next, 1);
+      j = __shfl_sync(0xffffffffu, j, 0);
+      if (j >= nready) break;
+      const ReadyNode rn = ready[j];
+      if (rn.id < P.nu)
+        gather_unode<NPE, NPP, T>(P, S, F, rn, list + j * GLIST, mine, lane);
+      else
+        gather_pnode<NPE, NPP, T>(P, S, F, rn, list + j * GLIST, mine, lane);
+    }
+    __syncthreads();  // the next group reuses the scratch
+  }
+};
 
 }  // namespace

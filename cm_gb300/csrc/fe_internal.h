@@ -52,6 +52,7 @@ struct HostSetup {
   std::vector<uint16_t> tables;          // [ntables][nr][nr]: CSR rank | first-contributor bit 15
   std::vector<int32_t> elem_table;       // [ne]
   std::vector<double> geo;               // [ne][NG][10]: dXi/dNu (row-major) and J_x
+  std::vector<double> geo_rj;            // [ne][NG]: 1 / J_x
   std::vector<double> gbf_u, gbf_p, gw;  // quadrature tables
   // elements with at least one boundary face, grouped by colour, and a mask of
   // their boundary local faces (reference local-face order)
@@ -61,13 +62,12 @@ struct HostSetup {
   // node (sorted by element number, packed e * 32 + local node) and around
   // every pressure row node (e * 8 + local pressure node).
   std::vector<int32_t> u_inc_ptr, u_inc, p_inc_ptr, p_inc;
+  // the incidences' rank-table rows: elem_table[e] * nr + local row node
+  std::vector<int32_t> u_inc_row, p_inc_row;
   // the largest element number around any of the row nodes 0..a (u nodes)
   // and 0..q (pressure row nodes): once the elements below E are assembled,
   // every node a with u_last_prefix[a] < E has its rows complete
   std::vector<int32_t> u_last_prefix, p_last_prefix;
-  // shared memory one gather warp needs: the larger of a u node's three rows
-  // (3 x 3 wu FP32, then 3 x its pressure columns FP64) and a pressure row (FP64)
-  int gather_bytes = 0;
 };
 
 // Arguments of the element kernels (plain data; device pointers).
@@ -76,6 +76,7 @@ struct KParams {
   const int32_t* elem_u;
   const int32_t* elem_p;
   const double* geo;
+  const double* geo_rj;  // 1 / J_x
   const float* geo_dd;  // geo as (hi, lo) FP32 pairs, for the double-float variant
   const double* mat;
   const double* gbf_u;
@@ -109,28 +110,26 @@ struct KParams {
 #define CMFE_HD
 #endif
 
-// Strides of the per-element records of the staged assembly, in elements of
-// each record's type, rounded up to whole 128-byte lines, so that no L2 line
-// holds parts of two elements' records (npe u nodes and npp pressure
-// parameters per element).
-CMFE_HD constexpr int rec_stride_uu(int npe) { return (9 * npe * npe + 31) / 32 * 32; }          // floats
-CMFE_HD constexpr int rec_stride_cp(int npe, int npp) { return (npp * 3 * npe + 15) / 16 * 16; }  // doubles
-CMFE_HD constexpr int rec_stride_r(int npe, int npp) { return (3 * npe + npp + 15) / 16 * 16; }   // doubles
+// The record one element leaves for the row gathers of the staged assembly
+// (npe u nodes, npp pressure parameters, displacement block in T), ordered so
+// that what the gather of one row node reads is contiguous:
+//   for every u node a    [m][n][b] displacement entries (T), [m][q] coupling
+//                         entries and [m] residuals (double), at a * ROW;
+//   for every pressure parameter q  [n][b] coupling entries and the residual
+//                         (double), at P0 + q * PROW.
+// The coupling entries are stored twice, once per reader.
+template <int NPE, int NPP, class T>
+struct Rec {
+  static constexpr int OC = (9 * NPE * (int)sizeof(T) + 7) / 8 * 8;
+  static constexpr int OR = OC + 3 * NPP * 8;
+  static constexpr int ROW = (OR + 3 * 8 + 15) / 16 * 16;
+  static constexpr int PROW = ((3 * NPE + 1) * 8 + 15) / 16 * 16;
+  static constexpr int P0 = NPE * ROW;
+  static constexpr int BYTES = (P0 + NPP * PROW + 127) / 128 * 128;  // whole 128-byte lines
+};
 
-// Place of entry (component m of node a, component n of node b) in an
-// element's displacement record, [a][m][n][b]: what the gather of node a's
-// rows reads is contiguous.
-CMFE_HD constexpr int rec_uu(int npe, int m, int a, int n, int b) { return ((a * 3 + m) * 3 + n) * npe + b; }
-
-// Per-element records of the staged assembly (mixed kernel with staged
-// output, surface mode 2, row gather): the full displacement block (FP32,
-// mirrored, in the order of rec_uu), the pressure-coupling rows
-// [NPP][3 NPE] and the residual [nrow] (FP64) of element e, at e times the
-// strides above.
 struct StageOut {
-  float* uu;
-  double* cp;
-  double* r;
+  unsigned char* rec;  // element e's record at e * Rec::BYTES
 };
 
 // Arguments of the fused staged assembly (fe_mixed.cu): the incidence lists,
@@ -143,12 +142,12 @@ struct FusedArgs {
   const int32_t* u_inc;
   const int32_t* p_inc_ptr;
   const int32_t* p_inc;
+  const int32_t* u_inc_row;  // rank-table row of every incidence
+  const int32_t* p_inc_row;
   int* work;       // this launch's group counter
   int* node_done;
   const uint8_t* bmask;
   int g0, g1;      // element groups of this launch: [g0, g1)
-  int gwarps;  // warps that gather (set by the launcher)
-  int gbytes;  // scratch bytes per gathering warp (set by the launcher)
 };
 
 // Launches the mixed-precision assembly kernel for one colour (fe_mixed.cu),
@@ -163,31 +162,22 @@ int fused_group_size(const HostSetup& s);
 // one wave of the launch takes); a negative cudaError_t on failure.
 int fused_wave(const HostSetup& s, int num_sms, bool double_float);
 
-// Launches the mixed-precision assembly kernel over all elements with its
-// output staged per element (so; fe_mixed.cu), in
-// one launch, without colour order.  Returns a cudaError_t value.
-int launch_mixed_staged(const HostSetup& s, const KParams& kp, const StageOut& so, int num_sms, void* stream,
-                        bool double_float);
-
 // The staged assembly in one launch with the row gathers inside it
-// (fe_mixed.cu); fused_fits() says whether a mesh's largest row node fits the
-// kernel's gather scratch.  Returns a cudaError_t value.
-int fused_fits(const HostSetup& s);
+// (fe_mixed.cu).  Returns a cudaError_t value.
 int launch_mixed_fused(const HostSetup& s, const KParams& kp, const StageOut& so, const FusedArgs& fa, int num_sms,
                        void* stream, bool double_float);
 
-// Sums the staged element outputs into the CSR rows (uu FP32, coupling FP64)
-// and the residual, one row node at a time, in the fixed element order of
-// the incidence lists (fe_gather.cu).  Returns a cudaError_t value.
-int launch_gather(const HostSetup& s, const KParams& kp, const StageOut& so, const int32_t* u_inc_ptr,
-                  const int32_t* u_inc, const int32_t* p_inc_ptr, const int32_t* p_inc, int num_sms, void* stream);
+// Bytes of one element's record.
+inline size_t record_bytes(const HostSetup& s) {
+  if (s.n1 == 2) return s.pmode ? Rec<8, 8, float>::BYTES : Rec<8, 1, float>::BYTES;
+  return s.pmode ? Rec<27, 8, float>::BYTES : Rec<27, 1, float>::BYTES;
+}
 
 // Launches the surface-pressure kernel over boundary elements (fe_surface.cu):
-// mode 0 adds into the CSR values / residual, mode 1 into element outputs,
-// mode 2 into the staged element records (so.uu, so.r).
+// mode 0 adds into the CSR values / residual, mode 1 into element outputs.
 // Returns a cudaError_t value.
 int launch_surface(const HostSetup& s, const KParams& kp, const int32_t* belems, const uint8_t* bmask, int nb,
-                   int mode, int want_jac, int num_sms, void* stream, const StageOut& so = StageOut{});
+                   int mode, int want_jac, int num_sms, void* stream);
 
 // Builds the set-up; returns FE_NO_ERROR or a FE_ERR_* code with msg filled.
 int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg);

@@ -485,7 +485,7 @@ struct fe_equations_set {
           *d_cp_row_ptr = nullptr, *d_wu = nullptr, *d_wp = nullptr, *d_elem_table = nullptr,
           *d_colour_elems = nullptr;
   uint16_t* d_tables = nullptr;
-  double *d_geo = nullptr, *d_mat = nullptr, *d_gbf_u = nullptr, *d_gbf_p = nullptr, *d_gw = nullptr;
+  double *d_geo = nullptr, *d_geo_rj = nullptr, *d_mat = nullptr, *d_gbf_u = nullptr, *d_gbf_p = nullptr, *d_gw = nullptr;
   float* d_geo_dd = nullptr;
   double* d_surfp = nullptr;
   int32_t* d_bnd_elems = nullptr;
@@ -495,9 +495,9 @@ struct fe_equations_set {
   int assembly_order = FE_ASSEMBLY_STAGED;
   // staged assembly: incidence lists (uploaded at creation) and the
   // per-element records (allocated on the first staged evaluation)
-  int32_t *d_u_inc_ptr = nullptr, *d_u_inc = nullptr, *d_p_inc_ptr = nullptr, *d_p_inc = nullptr;
-  float* d_st_uu = nullptr;
-  double *d_st_cp = nullptr, *d_st_r = nullptr;
+  int32_t *d_u_inc_ptr = nullptr, *d_u_inc = nullptr, *d_p_inc_ptr = nullptr, *d_p_inc = nullptr,
+          *d_u_inc_row = nullptr, *d_p_inc_row = nullptr;
+  unsigned char* d_rec = nullptr;
   int* d_fuse = nullptr;  // fused staged assembly: [0, kFuseChunks) group counters, then per-row-node counts
   int host_output = FE_HOST_OUTPUT_STREAMED;
   int stream_chunks = 0;  // launches of a streamed assembly; 0: equal runs of whole waves
@@ -581,6 +581,7 @@ KParams base_params(fe_handle h) {
   k.elem_u = h->d_elem_u;
   k.elem_p = h->d_elem_p;
   k.geo = h->d_geo;
+  k.geo_rj = h->d_geo_rj;
   k.geo_dd = h->d_geo_dd;
   k.nr = s.nr;
   k.pmode = s.pmode;
@@ -646,6 +647,8 @@ int mixed_fused(fe_handle h, const KParams& kp, const cmfe::StageOut& so, bool d
   fa.u_inc = h->d_u_inc;
   fa.p_inc_ptr = h->d_p_inc_ptr;
   fa.p_inc = h->d_p_inc;
+  fa.u_inc_row = h->d_u_inc_row;
+  fa.p_inc_row = h->d_p_inc_row;
   fa.node_done = h->d_fuse + kFuseChunks;
   fa.bmask = h->has_surfp && nb > 0 ? h->d_bnd_mask : nullptr;
   for (int c = 0; c < chunks; ++c) {
@@ -668,13 +671,7 @@ int64_t fused_groups(const HostSetup& s) {
 }
 
 int ensure_records(fe_handle h) {
-  const auto& s = h->hs;
-  int rc;
-  if ((rc = ensure((void**)&h->d_st_uu, sizeof(float) * cmfe::rec_stride_uu(s.npe) * (size_t)s.ne)) ||
-      (rc = ensure((void**)&h->d_st_cp, sizeof(double) * cmfe::rec_stride_cp(s.npe, s.npp) * (size_t)s.ne)) ||
-      (rc = ensure((void**)&h->d_st_r, sizeof(double) * cmfe::rec_stride_r(s.npe, s.npp) * (size_t)s.ne)))
-    return rc;
-  return FE_NO_ERROR;
+  return ensure((void**)&h->d_rec, cmfe::record_bytes(h->hs) * (size_t)h->hs.ne);
 }
 
 KParams staged_params(fe_handle h, const double* dx, float* du, double* dc, double* dr) {
@@ -689,34 +686,18 @@ KParams staged_params(fe_handle h, const double* dx, float* du, double* dc, doub
   return kp;
 }
 
-// The staged mixed assembly into device buffers: one launch over all
-// elements into the per-element records, the surface-pressure faces added to
-// the records of their elements, then the row gather (or all three in the
-// fused kernel where its gather scratch fits).  Adds the number of kernels
-// launched to *count when count is set.
+// The staged mixed assembly into device buffers: the per-element records, the
+// surface-pressure faces added to the records of their elements, and the row
+// gathers, all in one launch.  Adds the number of kernels launched to *count
+// when count is set.
 int mixed_staged(fe_handle h, const double* dx, float* du, double* dc, double* dr, bool double_float,
                  cudaStream_t st, int64_t* count) {
   const auto& s = h->hs;
   int rc;
   if ((rc = ensure_records(h))) return rc;
   const KParams kp = staged_params(h, dx, du, dc, dr);
-  const cmfe::StageOut so{h->d_st_uu, h->d_st_cp, h->d_st_r};
-  if (cmfe::fused_fits(s)) return mixed_fused(h, kp, so, double_float, st, {0, fused_groups(s)}, nullptr, count);
-  const int nb = s.bnd_ptr.empty() ? 0 : s.bnd_ptr[s.ncolours];
-  int e = cmfe::launch_mixed_staged(s, kp, so, h->num_sms, st, double_float);
-  if (e != 0) return set_error(FE_ERR_CUDA, std::string("staged kernel launch: ") + cudaGetErrorString((cudaError_t)e));
-  int64_t n = 1;
-  if (h->has_surfp && nb > 0) {
-    e = cmfe::launch_surface(s, kp, h->d_bnd_elems, h->d_bnd_mask, nb, 2, 1, h->num_sms, st, so);
-    if (e != 0) return set_error(FE_ERR_CUDA, std::string("surface kernel launch: ") + cudaGetErrorString((cudaError_t)e));
-    ++n;
-  }
-  e = cmfe::launch_gather(s, kp, so, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc, h->num_sms, st);
-  if (e != 0) return set_error(FE_ERR_CUDA, std::string("gather kernel launch: ") + cudaGetErrorString((cudaError_t)e));
-  ++n;
-  h->launches += n;
-  if (count) *count += n;
-  return FE_NO_ERROR;
+  const cmfe::StageOut so{h->d_rec};
+  return mixed_fused(h, kp, so, double_float, st, {0, fused_groups(s)}, nullptr, count);
 }
 
 // Streamed host outputs: the fused assembly in chunks of element groups into
@@ -761,7 +742,7 @@ int mixed_streamed(fe_handle h, const double* dx, float* du, double* dc, double*
     h->chunk_events.push_back(ev);
   }
   const KParams kp = staged_params(h, dx, du, dc, dr);
-  const cmfe::StageOut so{h->d_st_uu, h->d_st_cp, h->d_st_r};
+  const cmfe::StageOut so{h->d_rec};
   cudaEvent_t* ev = h->chunk_events.data();
   if ((rc = mixed_fused(h, kp, so, double_float, st, bounds, ev, nullptr))) return rc;
   cudaStream_t cs = h->copy_stream;
@@ -829,7 +810,7 @@ int mixed_colours(fe_handle h, const double* dx, float* du, double* dc, double* 
 // The mixed assembly in the handle's assembly order.
 int mixed_assemble(fe_handle h, const double* dx, float* du, double* dc, double* dr, bool double_float,
                    cudaStream_t st, int64_t* count) {
-  if (h->assembly_order == FE_ASSEMBLY_STAGED && h->hs.gather_bytes > 0)
+  if (h->assembly_order == FE_ASSEMBLY_STAGED)
     return mixed_staged(h, dx, du, dc, dr, double_float, st, count);
   return mixed_colours(h, dx, du, dc, dr, double_float, st, count);
 }
@@ -1107,7 +1088,8 @@ namespace {
 std::vector<void*> shared_arrays(fe_handle h) {
   return {h->d_bnd_elems, h->d_bnd_mask, h->d_geo_dd, h->d_elem_u, h->d_elem_p, h->d_row_ptr, h->d_uu_row_ptr,
           h->d_cp_row_ptr, h->d_wu, h->d_wp, h->d_elem_table, h->d_colour_elems, h->d_tables, h->d_geo,
-          h->d_gbf_u, h->d_gbf_p, h->d_gw, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc};
+          h->d_gbf_u, h->d_gbf_p, h->d_gw, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc,
+          h->d_u_inc_row, h->d_p_inc_row, h->d_geo_rj};
 }
 }  // namespace
 
@@ -1143,7 +1125,7 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
       (rc = dev_upload(&h->d_cp_row_ptr, s.cp_row_ptr)) || (rc = dev_upload(&h->d_wu, s.wu)) ||
       (rc = dev_upload(&h->d_wp, s.wp)) || (rc = dev_upload(&h->d_elem_table, s.elem_table)) ||
       (rc = dev_upload(&h->d_colour_elems, s.colour_elems)) || (rc = dev_upload(&h->d_tables, s.tables)) ||
-      (rc = dev_upload(&h->d_geo, s.geo)) || (rc = dev_upload(&h->d_mat, s.mat)) ||
+      (rc = dev_upload(&h->d_geo, s.geo)) || (rc = dev_upload(&h->d_geo_rj, s.geo_rj)) || (rc = dev_upload(&h->d_mat, s.mat)) ||
       (rc = dev_upload(&h->d_gbf_u, s.gbf_u)) || (rc = dev_upload(&h->d_gbf_p, s.gbf_p)) ||
       (rc = dev_upload(&h->d_gw, s.gw)))
     return fail(rc);
@@ -1158,7 +1140,8 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   }
   if ((rc = dev_upload(&h->d_bnd_elems, s.bnd_elems)) || (rc = dev_upload(&h->d_bnd_mask, s.bnd_mask))) return fail(rc);
   if ((rc = dev_upload(&h->d_u_inc_ptr, s.u_inc_ptr)) || (rc = dev_upload(&h->d_u_inc, s.u_inc)) ||
-      (rc = dev_upload(&h->d_p_inc_ptr, s.p_inc_ptr)) || (rc = dev_upload(&h->d_p_inc, s.p_inc)))
+      (rc = dev_upload(&h->d_p_inc_ptr, s.p_inc_ptr)) || (rc = dev_upload(&h->d_p_inc, s.p_inc)) ||
+      (rc = dev_upload(&h->d_u_inc_row, s.u_inc_row)) || (rc = dev_upload(&h->d_p_inc_row, s.p_inc_row)))
     return fail(rc);
   {
     auto owner = std::make_shared<SharedDeviceSetup>();
@@ -1188,7 +1171,7 @@ int fe_destroy(fe_handle h) {
   }
   // per-handle state: materials, surface load, status word, staging and records
   void* own[] = {h->d_surfp, h->d_mat, h->d_status, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
-                 h->d_col, h->d_st_uu, h->d_st_cp, h->d_st_r, h->d_fuse};
+                 h->d_col, h->d_rec, h->d_fuse};
   for (void* p : own)
     if (p) cudaFree(p);
   for (cudaEvent_t ev : h->chunk_events)
@@ -1222,6 +1205,7 @@ int fe_clone(fe_handle src, fe_handle* out) {
     h->d_colour_elems = src->d_colour_elems;
     h->d_tables = src->d_tables;
     h->d_geo = src->d_geo;
+    h->d_geo_rj = src->d_geo_rj;
     h->d_geo_dd = src->d_geo_dd;
     h->d_gbf_u = src->d_gbf_u;
     h->d_gbf_p = src->d_gbf_p;
@@ -1232,6 +1216,8 @@ int fe_clone(fe_handle src, fe_handle* out) {
     h->d_u_inc = src->d_u_inc;
     h->d_p_inc_ptr = src->d_p_inc_ptr;
     h->d_p_inc = src->d_p_inc;
+    h->d_u_inc_row = src->d_u_inc_row;
+    h->d_p_inc_row = src->d_p_inc_row;
     h->high_precision = src->high_precision;
     h->assembly_order = src->assembly_order;
     h->host_output = src->host_output;
@@ -1432,8 +1418,8 @@ int fe_jacobian_evaluate_mixed(fe_handle h, const double* x, float* values_uu, d
   double* dc = values_coupling;
   double* dr = r;
   bool mapped_out = false;  // some output is host memory written in place: wait before returning
-  const bool staged = h->assembly_order == FE_ASSEMBLY_STAGED && h->hs.gather_bytes > 0;
-  if (staged && (hu || hc || hr) && h->host_output == FE_HOST_OUTPUT_STREAMED && cmfe::fused_fits(h->hs)) {
+  const bool staged = h->assembly_order == FE_ASSEMBLY_STAGED;
+  if (staged && (hu || hc || hr) && h->host_output == FE_HOST_OUTPUT_STREAMED) {
     // the rows each chunk of elements completes go to the host while the
     // next chunks assemble
     if (hu && (rc = ensure((void**)&h->s_uu, sizeof(float) * h->hs.nnz_uu))) return rc;
@@ -1643,6 +1629,7 @@ int fe_batch_create(const fe_handle* handles, int32_t count, fe_batch* out) {
       e.kp.elems = h->d_colour_elems;
       e.kp.count = hs.ne;
       e.kp.surf_p = nullptr;
+      e.kp.wave = b->num_sms;
       e.belems = h->d_bnd_elems;
       e.bmask = h->d_bnd_mask;
       e.type = member_type(hs);

@@ -31,7 +31,9 @@
 #include "fe_dd.cuh"
 #include "fe_internal.h"
 #include "fe_math.cuh"
+#include "fe_line.cuh"
 #include "fe_uu.cuh"
+#include "fe_gather_impl.cuh"
 
 using cmfe::HostSetup;
 using cmfe::KParams;
@@ -46,7 +48,7 @@ constexpr int align16(int x) { return (x + 15) & ~15; }
 // measured 17 % faster than two CTAs of 4 elements despite the register
 // spills the 80-register budget causes), 4 for element-based pressure, 8 for
 // trilinear elements.
-template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8), class T = float>
+template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8), class T = float, int NT = 256>
 struct MixCfg {
   static constexpr int MINB = (N1 == 3 && PM) ? 3 : 2;  // CTAs per SM the launch bounds ask for
   static constexpr int NPE = N1 * N1 * N1;
@@ -54,41 +56,42 @@ struct MixCfg {
   static constexpr int NR = NPE + NPP;
   static constexpr int NU3 = 3 * NPE;
   static constexpr int NROW = NU3 + NPP;
-  static constexpr int THREADS = 256;
+  static constexpr int THREADS = NT;
   static constexpr int EG = EG_;                // elements per group
   static constexpr int REC64 = 20;  // P(9), A(9), t1, pad
   static constexpr int O_PSI64 = 0;
-  static constexpr int O_L = align16(O_PSI64 + NG * 8 * 8);
-  static constexpr int O_W = align16(O_L + 6 * 8);
-  static constexpr int O_1D = align16(O_W + NG * 8);
-  static constexpr int O_LM = align16(O_1D + 6 * N1 * 8);  // L x (1-D value | derivative) products
+  static constexpr int O_W = align16(O_PSI64 + NG * 8 * 8);
   // constant tables first, then the per-group scratch from O_Z on (the fused
   // kernel reuses the scratch between groups for its row gathers)
-  static constexpr int O_MM = align16(O_LM + 12 * N1 * 8);
+  static constexpr int O_MM = align16(O_W + NG * 8);
   static constexpr int O_Z = align16(O_MM + UUCfg<N1>::MM * (int)sizeof(T));
   static constexpr int O_P = align16(O_Z + EG * 3 * NPE * 8);
   static constexpr int O_PG = align16(O_P + EG * 8 * 8);
   static constexpr int O_R64 = align16(O_PG + EG * NG * 8);
   static constexpr int P1S = EG * (18 * N1 * N1 + 81 * N1) * 8;  // scratch of the gradients' first two stages
+  static constexpr int L2 = 2 * N1;                               // linear x 1-D basis products of a line
+  static constexpr int T1S = EG * 3 * L2 * 9 * 8;                 // coupling, per component: stage 1
+  static constexpr int W2S = EG * L2 * L2 * 3 * 8;                //   and each of the two stage-2 arrays
+  static constexpr int P3S = PM ? 3 * T1S + 6 * W2S : 0;
   static constexpr int RECS = EG * NG * UU_REC * (int)sizeof(T);
   static constexpr int O_R32 = align16(O_R64 + EG * NG * REC64 * 8);
   // the gradients and the FP64 stages' scratch share their space with the
   // warps' stage-1 values of the displacement block
   static constexpr int O_DZ = align16(O_R32 + (RECS > P1S ? RECS : P1S));
-  static constexpr int O_F32 = align16(O_DZ + EG * NG * 9 * 8);
+  static constexpr int P3R = EG * (9 * N1 * 9 + 6 * N1 * N1 * 3 + 64) * 8;  // scratch of the residual stages
+  static constexpr int O_U1 = O_DZ, O_U2 = O_U1 + EG * 9 * N1 * 9 * 8, O_U3 = O_U2 + EG * 6 * N1 * N1 * 3 * 8;
   static constexpr int WS1 = THREADS / 32 * UUCfg<N1>::S1 * (int)sizeof(T);
-  static constexpr int F32_END = align16(O_F32 + EG * NG * 24 * 4);
-  static constexpr int O_BASE = align16(O_DZ + WS1 > F32_END ? O_DZ + WS1 : F32_END);
+  static constexpr int big(int x, int y) { return x > y ? x : y; }
+  static constexpr int O_BASE = align16(O_DZ + big(big(EG * NG * 9 * 8, WS1), big(P3R, P3S)));
   // coloured order only: scatter addresses and rank tables of the group
   static constexpr int O_TAB = align16(O_BASE + EG * 9 * NPE * 4);
   static constexpr int O_NODE0 = align16(O_TAB + EG * NPE * NPE * 2);
   static constexpr int SMEM0 = align16(O_NODE0 + EG * (NR + 1) * 4);
-  // staged order: the node numbers follow the scratch directly; the fused
-  // kernel's list of row nodes a group completed lies just below them
-  static constexpr int O_NODE1 = align16(O_BASE + EG * NR * 4);
+  // staged order: the node numbers follow the scratch, which the row gathers
+  // reuse from O_Z on
+  static constexpr int GATHER_END = align16(O_Z + GroupGather<NPE, NPP, EG, THREADS, T>::SCRATCH);
+  static constexpr int O_NODE1 = O_BASE > GATHER_END ? O_BASE : GATHER_END;
   static constexpr int SMEM1 = align16(O_NODE1 + EG * (NR + 1) * 4);
-  static constexpr int O_SCRATCH = O_Z;
-  static constexpr int O_READY = O_BASE;
 };
 
 // Block (m, n) of the lower-triangle displacement blocks: 0..2 diagonal,
@@ -102,36 +105,35 @@ __device__ __forceinline__ void blk_mn(int blk, int& m, int& n) {
 // F (material frame) and J = Jznu: sigma = dev(F_bar S_bar F_bar^T / J) + p I.
 template <class H>
 __device__ void mix_stress(int law, const H* c, const H F[3][3], H J, H p, H sig[3][3]) {
-  const H s = hrcbrt(J);
+  const H s = hrcbrt(J), s2 = s * s, rJ = s * s2;
   const H zero = hval<H>(0.0), one = hval<H>(1.0), two = hval<H>(2.0), half = hval<H>(0.5);
   if (law == FE_LAW_MOONEY_RIVLIN) {
-    // S_bar = al I + be C_bar, so F_bar S_bar F_bar^T = al B_bar + be B_bar^2 with
-    // B_bar = F_bar F_bar^T (and tr C_bar = tr B_bar): fewer FP64 operations
-    // than forming C_bar and both products
-    const H s2 = s * s;
-    H Bb[3][3];
+    // S_bar = al I + be C_bar, so F_bar S_bar F_bar^T = al B_bar + be B_bar^2
+    // with B_bar = J^(-2/3) F F^T (and tr C_bar = tr B_bar); the powers of J
+    // and 1/J go into the two coefficients
+    H B[3][3];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = i; j < 3; ++j) {
-        Bb[i][j] = s2 * (F[i][0] * F[j][0] + F[i][1] * F[j][1] + F[i][2] * F[j][2]);
-        Bb[j][i] = Bb[i][j];
+        B[i][j] = hfma(F[i][2], F[j][2], hfma(F[i][1], F[j][1], F[i][0] * F[j][0]));
+        B[j][i] = B[i][j];
       }
-    const H I1 = Bb[0][0] + Bb[1][1] + Bb[2][2];
-    const H al = two * (c[0] + I1 * c[1]);
-    const H be = -(two * c[1]);
-    const H rJ = one / J;
+    const H I1 = s2 * (B[0][0] + B[1][1] + B[2][2]);
+    const H q = two * rJ * s2;
+    const H al = q * hfma(I1, c[1], c[0]);
+    const H be = -(q * s2 * c[1]);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
       for (int j = i; j < 3; ++j) {
-        const H b2 = Bb[i][0] * Bb[0][j] + Bb[i][1] * Bb[1][j] + Bb[i][2] * Bb[2][j];
-        sig[i][j] = (al * Bb[i][j] + be * b2) * rJ;
+        const H b2 = hfma(B[i][2], B[2][j], hfma(B[i][1], B[1][j], B[i][0] * B[0][j]));
+        sig[i][j] = hfma(be, b2, al * B[i][j]);
         sig[j][i] = sig[i][j];
       }
-    const H tr3 = (sig[0][0] + sig[1][1] + sig[2][2]) * hval<H>(1.0 / 3.0);
+    const H sh = hfma(hval<H>(-1.0 / 3.0), sig[0][0] + sig[1][1] + sig[2][2], p);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) sig[i][i] = sig[i][i] - tr3 + p;
+    for (int i = 0; i < 3; ++i) sig[i][i] = sig[i][i] + sh;
     return;
   }
   H Fb[3][3], Cb[3][3], S[3][3], T[3][3];
@@ -143,61 +145,51 @@ __device__ void mix_stress(int law, const H* c, const H F[3][3], H J, H p, H sig
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = i; j < 3; ++j) {
-      Cb[i][j] = Fb[0][i] * Fb[0][j] + Fb[1][i] * Fb[1][j] + Fb[2][i] * Fb[2][j];
+      Cb[i][j] = hfma(Fb[2][i], Fb[2][j], hfma(Fb[1][i], Fb[1][j], Fb[0][i] * Fb[0][j]));
       Cb[j][i] = Cb[i][j];
     }
-  if (law == FE_LAW_MOONEY_RIVLIN) {
-    const H I1 = Cb[0][0] + Cb[1][1] + Cb[2][2];
-    const H al = two * (c[0] + I1 * c[1]);
-    const H be = -(two * c[1]);
+  const H B[6] = {two * c[1], two * c[2], two * c[2], c[3], c[3], c[2]};
+  const H E[6] = {half * (Cb[0][0] - one), half * (Cb[1][1] - one), half * (Cb[2][2] - one), Cb[1][0], Cb[2][0],
+                  Cb[2][1]};
+  H DQ[6], dot = zero;
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) S[i][j] = i == j ? be * Cb[i][j] + al : be * Cb[i][j];
-  } else {
-    const H B[6] = {two * c[1], two * c[2], two * c[2], c[3], c[3], c[2]};
-    const H E[6] = {half * (Cb[0][0] - one), half * (Cb[1][1] - one), half * (Cb[2][2] - one), Cb[1][0], Cb[2][0],
-                    Cb[2][1]};
-    H DQ[6], dot = zero;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      DQ[i] = B[i] * E[i];
-      dot = dot + E[i] * DQ[i];
-    }
-    const H t1 = half * c[0] * hexp(half * dot);
-    S[0][0] = t1 * DQ[0];
-    S[1][1] = t1 * DQ[1];
-    S[2][2] = t1 * DQ[2];
-    S[0][1] = S[1][0] = t1 * DQ[3];
-    S[0][2] = S[2][0] = t1 * DQ[4];
-    S[1][2] = S[2][1] = t1 * DQ[5];
+  for (int i = 0; i < 6; ++i) {
+    DQ[i] = B[i] * E[i];
+    dot = hfma(E[i], DQ[i], dot);
   }
-  // sigma_bar = F_bar S F_bar^T / J
+  const H t1 = half * c[0] * hexp(half * dot) * rJ;
+  S[0][0] = t1 * DQ[0];
+  S[1][1] = t1 * DQ[1];
+  S[2][2] = t1 * DQ[2];
+  S[0][1] = S[1][0] = t1 * DQ[3];
+  S[0][2] = S[2][0] = t1 * DQ[4];
+  S[1][2] = S[2][1] = t1 * DQ[5];
+  // sigma_bar = F_bar (S / J) F_bar^T
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) T[i][j] = Fb[i][0] * S[0][j] + Fb[i][1] * S[1][j] + Fb[i][2] * S[2][j];
-  const H rJ = one / J;
+    for (int j = 0; j < 3; ++j) T[i][j] = hfma(Fb[i][2], S[2][j], hfma(Fb[i][1], S[1][j], Fb[i][0] * S[0][j]));
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = i; j < 3; ++j) {
-      sig[i][j] = (T[i][0] * Fb[j][0] + T[i][1] * Fb[j][1] + T[i][2] * Fb[j][2]) * rJ;
+      sig[i][j] = hfma(T[i][2], Fb[j][2], hfma(T[i][1], Fb[j][1], T[i][0] * Fb[j][0]));
       sig[j][i] = sig[i][j];
     }
-  const H tr3 = (sig[0][0] + sig[1][1] + sig[2][2]) * hval<H>(1.0 / 3.0);
+  const H sh = hfma(hval<H>(-1.0 / 3.0), sig[0][0] + sig[1][1] + sig[2][2], p);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) sig[i][i] = sig[i][i] - tr3 + p;
+  for (int i = 0; i < 3; ++i) sig[i][i] = sig[i][i] + sh;
 }
 
-// Geometric Gauss-point data (dXi/dNu row-major, J_x) in H.
-__device__ __forceinline__ void load_geo(const KParams& P, int e, int g, double dn[9], double& jx) {
+// Geometric Gauss-point data (dXi/dNu row-major, J_x, 1 / J_x) in H.
+__device__ __forceinline__ void load_geo(const KParams& P, int e, int g, double dn[9], double& jx, double& rjx) {
   const double* geo = &P.geo[((size_t)e * NG + g) * 10];
 #pragma unroll
   for (int i = 0; i < 9; ++i) dn[i] = geo[i];
   jx = geo[9];
+  rjx = P.geo_rj[(size_t)e * NG + g];
 }
-__device__ __forceinline__ void load_geo(const KParams& P, int e, int g, dd dn[9], dd& jx) {
+__device__ __forceinline__ void load_geo(const KParams& P, int e, int g, dd dn[9], dd& jx, dd& rjx) {
   const float2* geo = reinterpret_cast<const float2*>(P.geo_dd) + ((size_t)e * NG + g) * 10;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
@@ -206,18 +198,20 @@ __device__ __forceinline__ void load_geo(const KParams& P, int e, int g, dd dn[9
   }
   const float2 v = geo[9];
   jx = {v.x, v.y};
+  rjx = to_dd(P.geo_rj[(size_t)e * NG + g]);
 }
-
 // The same data in the displacement block's type T; FP32 takes the leading
-// parts of the double-float copy, which are the values rounded to FP32.
-__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, double dn[9], double& jx) {
-  load_geo(P, e, g, dn, jx);
+// parts of the double-float copy, which are the values rounded to FP32 (a
+// conversion takes the FP64 pipe as long as an FP64 operation).
+__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, double dn[9], double& rjx) {
+  double jx;
+  load_geo(P, e, g, dn, jx, rjx);
 }
-__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, float dn[9], float& jx) {
+__device__ __forceinline__ void load_geo_t(const KParams& P, int e, int g, float dn[9], float& rjx) {
   const float2* geo = reinterpret_cast<const float2*>(P.geo_dd) + ((size_t)e * NG + g) * 10;
 #pragma unroll
   for (int i = 0; i < 9; ++i) dn[i] = geo[i].x;
-  jx = geo[9].x;
+  rjx = 1.0f / geo[9].x;
 }
 
 template <class T, class H>
@@ -228,62 +222,17 @@ __device__ __forceinline__ T to_t(H v) {
     return hd(v);
 }
 
-template <class T>
-__device__ __forceinline__ T* stage_uu(const cmfe::StageOut& so) {
-  return so.uu;
-}
-
-// The 3-point Gauss-Legendre abscissae on [0, 1].
-__device__ __forceinline__ double gauss_1d(int gi) {
-  return gi == 0 ? (-sqrt(0.6) + 1.0) / 2.0 : (gi == 1 ? 0.5 : (sqrt(0.6) + 1.0) / 2.0);
-}
-
-// 1-D Lagrange basis function a of degree N1 - 1 on [0, 1] and its derivative at t.
-template <int N1>
-__device__ __forceinline__ void lagrange_1d(int a, double t, double& bv, double& dv) {
-  if (N1 == 2) {
-    bv = a == 0 ? 1.0 - t : t;
-    dv = a == 0 ? -1.0 : 1.0;
-  } else {
-    bv = a == 0 ? 1.0 - 3.0 * t + 2.0 * t * t : (a == 1 ? 4.0 * t * (1.0 - t) : t * (t + t - 1.0));
-    dv = a == 0 ? 4.0 * t - 3.0 : (a == 1 ? 4.0 - 8.0 * t : 4.0 * t - 1.0);
-  }
-}
-
-// Constant tables (basis values and derivatives at the Gauss points and their
-// products) into shared memory.
-template <int N1, int PM, int EG_, class T, class H>
+// Constant tables (pressure basis and weights at the Gauss points, products of
+// the 1-D basis functions) into shared memory.
+template <int N1, int PM, int EG_, class T, class H, int NT = 256>
 __device__ __forceinline__ void mix_tables(const KParams& P, unsigned char* sm) {
-  using C = MixCfg<N1, PM, EG_, T>;
+  using C = MixCfg<N1, PM, EG_, T, NT>;
   H* s_psi = reinterpret_cast<H*>(sm + C::O_PSI64);  // [g][q]
-  H* s_L = reinterpret_cast<H*>(sm + C::O_L);        // [q][gi]
   H* s_w = reinterpret_cast<H*>(sm + C::O_W);        // [g]
-  H* s_B1 = reinterpret_cast<H*>(sm + C::O_1D);      // [gi][a] 1-D values
-  H* s_D1 = s_B1 + 3 * N1;                                // [gi][a] 1-D derivatives
-  H* s_LM = reinterpret_cast<H*>(sm + C::O_LM);      // [B|D][q][gi][a]: L(q, gi) x 1-D value | derivative
   const int tid = threadIdx.x;
   // ---- constant tables
   for (int i = tid; i < NG * 8; i += C::THREADS) s_psi[i] = hval<H>(P.gbf_p[i]);
   for (int i = tid; i < NG; i += C::THREADS) s_w[i] = hval<H>(P.gw[i]);
-  if (tid < 6) {
-    const int q = tid / 3, gi = tid % 3;
-    const double t = gauss_1d(gi);
-    s_L[tid] = hval<H>(q == 0 ? 1.0 - t : t);
-  }
-  if (tid < 3 * N1) {  // 1-D Lagrange values and derivatives at the Gauss points
-    const int gi = tid / N1, a = tid % N1;
-    double bv, dv;
-    lagrange_1d<N1>(a, gauss_1d(gi), bv, dv);
-    s_B1[tid] = hval<H>(bv);
-    s_D1[tid] = hval<H>(dv);
-  }
-  if (tid < 12 * N1) {  // their products with the linear pressure basis (nodal-pressure coupling)
-    const int a = tid % N1, gi = (tid / N1) % 3, q = (tid / (3 * N1)) % 2, d = tid / (6 * N1);
-    const double t = gauss_1d(gi);
-    double bv, dv;
-    lagrange_1d<N1>(a, t, bv, dv);
-    s_LM[tid] = hval<H>((q == 0 ? 1.0 - t : t) * (d ? dv : bv));
-  }
   uu_table<N1, T>(reinterpret_cast<T*>(sm + C::O_MM), tid, C::THREADS);
 }
 
@@ -298,17 +247,14 @@ __device__ __forceinline__ int elem_at(const KParams& P, const int32_t* elems, i
 // element's entries into the CSR values and the residual (first contributor
 // in colour order stores, later ones add); OUT = 1 stores them into the
 // element's staging records (*SO), which the row gather sums afterwards.
-template <int N1, int PM, int EG_, class T, class H, int OUT = 0>
+template <int N1, int PM, int EG_, class T, class H, int OUT = 0, int NT = 256>
 __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems, int count, int grp, bool p4_first,
                                           unsigned char* sm, const cmfe::StageOut* SO = nullptr) {
-  using C = MixCfg<N1, PM, EG_, T>;
-  constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, NU3 = C::NU3, NROW = C::NROW, EG = C::EG;
+  using C = MixCfg<N1, PM, EG_, T, NT>;
+  constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, NU3 = C::NU3, EG = C::EG;
+  using R = cmfe::Rec<NPE, NPP, T>;
   H* s_psi = reinterpret_cast<H*>(sm + C::O_PSI64);  // [g][q]
-  H* s_L = reinterpret_cast<H*>(sm + C::O_L);        // [q][gi]
   H* s_w = reinterpret_cast<H*>(sm + C::O_W);        // [g]
-  H* s_B1 = reinterpret_cast<H*>(sm + C::O_1D);      // [gi][a] 1-D values
-  H* s_D1 = s_B1 + 3 * N1;                                // [gi][a] 1-D derivatives
-  H* s_LM = reinterpret_cast<H*>(sm + C::O_LM);      // [B|D][q][gi][a]: L(q, gi) x 1-D value | derivative
   H* s_z = reinterpret_cast<H*>(sm + C::O_Z);        // [el][c][a]
   H* s_p = reinterpret_cast<H*>(sm + C::O_P);        // [el][q]
   H* s_dz = reinterpret_cast<H*>(sm + C::O_DZ);      // [el][g][c*3+k]
@@ -316,9 +262,12 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   H* s_r64 = reinterpret_cast<H*>(sm + C::O_R64);    // [el][g][REC64]
   T* s_D = reinterpret_cast<T*>(sm + C::O_R32);                // [el][g][UU_REC]
   T* s_mm = reinterpret_cast<T*>(sm + C::O_MM);
-  float* s_f32 = reinterpret_cast<float*>(sm + C::O_F32);      // scratch of P3 (EG x 2592 B)
   int* s_node = reinterpret_cast<int*>(sm + (OUT == 1 ? C::O_NODE1 : C::O_NODE0));  // [el][NR+1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // FP64 items are dealt to the warps from a different first warp in each
+  // CTA of an SM: an SM sub-partition takes 64 cycles per FP64 warp
+  // instruction, and most stages have fewer items than threads
+  const int vt = ((warp + blockIdx.x / P.wave) % (C::THREADS / 32)) * 32 + lane;
   const int nu = P.nu;
   const int nvalid = min(EG, count - grp * EG);
   __syncthreads();
@@ -348,48 +297,67 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   }
   __syncthreads();
   // ---- P1: dz/dxi at the Gauss points by sum factorisation over the
-  // tensor-product basis (FP64): xi1, then xi2, then xi3 contractions with
-  // the 1-D value (B) and derivative (D) tables.
+  // tensor-product basis: xi1, then xi2, then xi3, one line of nodes or points
+  // per item (fe_line.cuh; B = values, D = derivatives).
   {
     constexpr int N2 = N1 * N1;
-    H* S1 = reinterpret_cast<H*>(sm + C::O_R32);  // [el][c][B|D][g1][a2a3]
-    H* S2 = S1 + EG * 3 * 2 * 3 * N2;                  // [el][c][BB|BD|DB][g1][g2][a3]
-    for (int i = tid; i < EG * 3 * 2 * 3 * N2; i += C::THREADS) {
-      const int j = i % N2, g1 = (i / N2) % 3, typ = (i / (3 * N2)) % 2, ec = i / (6 * N2);
-      const H* M = typ ? s_D1 : s_B1;
-      const H* zr = &s_z[ec * NPE + N1 * j];
-      H acc = hval<H>(0.0);
+    H* S1 = reinterpret_cast<H*>(sm + C::O_R32);  // [B|D][ec][g1][a2a3]
+    H* S2 = S1 + EG * 3 * 2 * 3 * N2;             // [BB|BD|DB][ec][g1][g2][a3]
+    constexpr int S1T = EG * 3 * 3 * N2, S2T = EG * 3 * 9 * N1;
+    for (int i = vt; i < EG * 3 * N2; i += C::THREADS) {
+      const int j = i % N2, ec = i / N2;
+      H z[N1], B[3], D[3];
 #pragma unroll
-      for (int a1 = 0; a1 < N1; ++a1) acc = hfma(M[g1 * N1 + a1], zr[a1], acc);
-      S1[i] = acc;
+      for (int a1 = 0; a1 < N1; ++a1) z[a1] = s_z[ec * NPE + N1 * j + a1];
+      line_BD<N1, H>(z, B, D);
+#pragma unroll
+      for (int g = 0; g < 3; ++g) {
+        S1[(ec * 3 + g) * N2 + j] = B[g];
+        S1[S1T + (ec * 3 + g) * N2 + j] = D[g];
+      }
     }
     __syncthreads();
-    for (int i = tid; i < EG * 3 * 3 * 9 * N1; i += C::THREADS) {
-      const int a3 = i % N1, g2 = (i / N1) % 3, g1 = (i / (3 * N1)) % 3, typ2 = (i / (9 * N1)) % 3,
-                ec = i / (27 * N1);
-      const int src = typ2 == 2 ? 1 : 0;                     // DB reads the D stage-1 output
-      const H* M = typ2 == 1 ? s_D1 : s_B1;             // BD applies D along xi2
-      const H* sr = &S1[((ec * 2 + src) * 3 + g1) * N2 + N1 * a3];
-      H acc = hval<H>(0.0);
+    constexpr int L2I = EG * 3 * 3 * N1;  // (ec, g1, a3)
+    for (int i = vt; i < 2 * L2I; i += C::THREADS) {
+      const bool d1 = i >= L2I;
+      const int r = d1 ? i - L2I : i;
+      const int a3 = r % N1, eg = r / N1;  // eg = ec * 3 + g1
+      const H* s = S1 + (d1 ? S1T : 0) + eg * N2 + N1 * a3;
+      H z[N1], B[3];
 #pragma unroll
-      for (int a2 = 0; a2 < N1; ++a2) acc = hfma(M[g2 * N1 + a2], sr[a2], acc);
-      S2[i] = acc;
+      for (int a2 = 0; a2 < N1; ++a2) z[a2] = s[a2];
+      if (d1) {
+        line_B<N1, H>(z, B);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) S2[2 * S2T + (eg * 3 + g) * N1 + a3] = B[g];
+      } else {
+        H D[3];
+        line_BD<N1, H>(z, B, D);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+          S2[(eg * 3 + g) * N1 + a3] = B[g];
+          S2[S2T + (eg * 3 + g) * N1 + a3] = D[g];
+        }
+      }
     }
     __syncthreads();
-    for (int i = tid; i < EG * 3 * 3 * NG; i += C::THREADS) {
-      const int g = i % NG, k = (i / NG) % 3, ec = i / (3 * NG);
-      const int g1 = g % 3, g2 = (g / 3) % 3, g3 = g / 9;
-      const int typ2 = k == 0 ? 2 : (k == 1 ? 1 : 0);        // d/dxi1: DB, d/dxi2: BD, d/dxi3: BB
-      const H* M = k == 2 ? s_D1 : s_B1;
-      const H* sr = &S2[(((ec * 3 + typ2) * 3 + g1) * 3 + g2) * N1];
-      H acc = hval<H>(0.0);
+    constexpr int L3I = EG * 3 * 9;  // (ec, g1, g2)
+    for (int i = vt; i < 3 * L3I; i += C::THREADS) {
+      const int k = i / L3I, r = i % L3I;  // d/dxi1: DB, d/dxi2: BD, d/dxi3: BB
+      const int g2 = r % 3, g1 = (r / 3) % 3, ec = r / 9, el = ec / 3, c = ec % 3;
+      const H* s = S2 + (2 - k) * S2T + r * N1;
+      H z[N1], o[3];
 #pragma unroll
-      for (int a3 = 0; a3 < N1; ++a3) acc = hfma(M[g3 * N1 + a3], sr[a3], acc);
-      const int el = ec / 3, c = ec % 3;
-      s_dz[(el * NG + g) * 9 + c * 3 + k] = acc;
+      for (int a3 = 0; a3 < N1; ++a3) z[a3] = s[a3];
+      if (k == 2)
+        line_D<N1, H>(z, o);
+      else
+        line_B<N1, H>(z, o);
+#pragma unroll
+      for (int g3 = 0; g3 < 3; ++g3) s_dz[(el * NG + g1 + 3 * g2 + 9 * g3) * 9 + c * 3 + k] = o[g3];
     }
   }
-  for (int i = tid; i < EG * NG; i += C::THREADS) {
+  for (int i = vt; i < EG * NG; i += C::THREADS) {
     const int el = i / NG, g = i % NG;
     H pg;
     if (PM) {
@@ -408,8 +376,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   // the FP32 pipes overlap; P2b forms the kinematics it needs itself from
   // the same gradients.
   constexpr int HALF = C::THREADS / 2;
-  if (tid < HALF) {
-    for (int t = tid; t < EG * NG; t += HALF) {
+  if (vt < HALF) {
+    for (int t = vt; t < EG * NG; t += HALF) {
       const int el = t / NG, g = t % NG;
       if (el >= nvalid) continue;
       const int e = elem_at(P, elems, grp * EG + el);
@@ -428,58 +396,59 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
       adj[2][1] = M[0][1] * M[2][0] - M[0][0] * M[2][1];
       adj[2][2] = M[0][0] * M[1][1] - M[0][1] * M[1][0];
       const H det = M[0][0] * adj[0][0] + M[0][1] * adj[1][0] + M[0][2] * adj[2][0];
-      H dn[9], jx;
-      load_geo(P, e, g, dn, jx);
-      H F[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) F[i][j] = M[i][0] * dn[j] + M[i][1] * dn[3 + j] + M[i][2] * dn[6 + j];
+      H dn[9], jx, rjx;
+      load_geo(P, e, g, dn, jx, rjx);
       const H jz = habs(det);
-      const H jznu = jz / jx;
       const H w = s_w[g];
       const bool dpos = hpos(det);
       const H sw = dpos ? w : -w;  // J_z w dxi/dz = sign(det) w adj
-      const double* cm = P.mat + (P.matpe ? (size_t)e * P.nmat : 0);
-      const H cc[4] = {hval<H>(cm[0]), hval<H>(cm[1]), hval<H>(P.nmat > 2 ? cm[2] : 0.0),
-                       hval<H>(P.nmat > 3 ? cm[3] : 0.0)};
       const H pgv = s_pg[t];
       H* rec = &s_r64[t * C::REC64];
       bool ok = dpos;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          adj[k][n] = sw * adj[k][n];
+          rec[9 + k * 3 + n] = adj[k][n];
+        }
       if (P.r != nullptr) {
-        H sig[3][3];
-        mix_stress<H>(P.law, cc, F, jznu, pgv, sig);
+        H F[3][3], sig[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) F[i][j] = hfma(M[i][2], dn[6 + j], hfma(M[i][1], dn[3 + j], M[i][0] * dn[j]));
+        const double* cm = P.mat + (P.matpe ? (size_t)e * P.nmat : 0);
+        const H cc[4] = {hval<H>(cm[0]), hval<H>(cm[1]), hval<H>(P.nmat > 2 ? cm[2] : 0.0),
+                         hval<H>(P.nmat > 3 ? cm[3] : 0.0)};
+        mix_stress<H>(P.law, cc, F, jz * rjx, pgv, sig);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
           for (int m = 0; m < 3; ++m) {
-            const H v = sw * (adj[k][0] * sig[0][m] + adj[k][1] * sig[1][m] + adj[k][2] * sig[2][m]);
+            const H v = hfma(adj[k][2], sig[2][m], hfma(adj[k][1], sig[1][m], adj[k][0] * sig[0][m]));
             rec[k * 3 + m] = v;
             ok = ok && hfinite(v);
           }
-        rec[18] = jx * w * (jznu - hval<H>(1.0));
+        rec[18] = w * (jz - jx);  // J_x w (J - 1)
       }
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int n = 0; n < 3; ++n) rec[9 + k * 3 + n] = sw * adj[k][n];
       if (!ok) atomicOr(P.status, 1u);
     }
   } else {
-    for (int t = tid - HALF; t < (P.res_only ? 0 : EG * NG); t += HALF) {
+    for (int t = vt - HALF; t < (P.res_only ? 0 : EG * NG); t += HALF) {
       const int el = t / NG, g = t % NG;
       if (el >= nvalid) continue;
       const int e = elem_at(P, elems, grp * EG + el);
-      T Mt[3][3], dn[9], jx, ct[4];
+      T Mt[3][3], dn[9], rjx, ct[4];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int k = 0; k < 3; ++k) Mt[c][k] = to_t<T>(s_dz[t * 9 + c * 3 + k]);
-      load_geo_t(P, e, g, dn, jx);
+      load_geo_t(P, e, g, dn, rjx);
       const double* cm = P.mat + (P.matpe ? (size_t)e * P.nmat : 0);
 #pragma unroll
       for (int i = 0; i < 4; ++i) ct[i] = i < P.nmat ? (T)cm[i] : T(0);
-      if (!uu_tangent<T>(P.law, ct, Mt, dn, T(1) / jx, to_t<T>(s_w[g]), to_t<T>(s_pg[t]), &s_D[t * UU_REC]))
+      if (!uu_tangent<T>(P.law, ct, Mt, dn, rjx, to_t<T>(s_w[g]), to_t<T>(s_pg[t]), &s_D[t * UU_REC]))
         atomicOr(P.status, 1u);
     }
   }
@@ -491,105 +460,137 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
     if ((ph == 0) != p4_first) {
       // ---- P3: residual rows and pressure-coupling columns (high precision H)
       __syncthreads();
-      // Sum factorisation over the tensor-product basis:
-      //   RK[el][mk][a] = sum_g M_k(g; a) V_g(k, m),  V_g(k, m) = rec_g[roff + 3 k + m],
-      // with M_k the product of the 1-D derivative table along xi_k and the
-      // 1-D value table along the other two directions; one xi direction
-      // contracted per stage.  roff = 0: V = P, the residual rows are
-      // sum_k RK; roff = 9: V = A = J_z w dxi/dz, the element-based pressure
-      // coupling column of (n, b) is sum_k RK[el][3 n + k][b].
       constexpr int N2 = N1 * N1;
-      auto sumfact = [&](int roff) {
-        H* U1 = s_dz;                         // [el][mk][a1][g2 + 3 g3]
-        H* U2 = reinterpret_cast<H*>(s_f32);  // [el][mk][a1 + N1 a2][g3]
-        H* RK = s_dz;                         // [el][mk][a]
-        for (int i = tid; i < EG * 9 * N1 * 9; i += C::THREADS) {
-          const int j = i % 9, a1 = (i / 9) % N1, mk = (i / (9 * N1)) % 9, el = i / (81 * N1);
-          const int m = mk / 3, k = mk % 3;
-          const H* M = k == 0 ? s_D1 : s_B1;
+      // Sum factorisation over the tensor-product basis, line by line: for
+      // V = rec[roff + 3 k + m],
+      //   R(m, a) = sum_g sum_k M_k(g; a) V_g(k, m),
+      // M_k the product of the 1-D derivatives along xi_k and the 1-D values
+      // along the other two.  xi1 is contracted for each k, xi2 with the k = 0
+      // and k = 1 terms merged (both take values along xi3), xi3 with all
+      // merged.  roff = 0: V = P, the residual rows; roff = 9: V = A = J_z w
+      // dxi/dz, the element-based pressure coupling column.
+      H* U1 = reinterpret_cast<H*>(sm + C::O_U1);  // [el][m][k][a1][g2 + 3 g3]
+      H* U2 = reinterpret_cast<H*>(sm + C::O_U2);  // [W|U][el][m][a1 + N1 a2][g3]
+      H* Lq = reinterpret_cast<H*>(sm + C::O_U3);  // residual pressure rows: [el][q1][j], then [el][q1 q2][g3]
+      auto sumfact = [&](int roff, bool prows, auto emit, auto emit_p) {
+        for (int i = vt; i < EG * 81; i += C::THREADS) {
+          const int j = i % 9, k = (i / 9) % 3, m = (i / 27) % 3, el = i / 81;
           const H* rec = &s_r64[(el * NG + 3 * j) * C::REC64 + roff + k * 3 + m];
-          H acc = hval<H>(0.0);
+          const H v[3] = {rec[0], rec[C::REC64], rec[2 * C::REC64]};
+          H o[N1];
+          if (k == 0)
+            line_Dt<N1, H>(v, o);
+          else
+            line_Bt<N1, H>(v, o);
 #pragma unroll
-          for (int g1 = 0; g1 < 3; ++g1) acc = hfma(M[g1 * N1 + a1], rec[g1 * C::REC64], acc);
-          U1[i] = acc;
+          for (int a = 0; a < N1; ++a) U1[((i / 9) * N1 + a) * 9 + j] = o[a];
+        }
+        if (PM && prows) {  // the pressure rows, on the warps the lines leave over
+          for (int i = C::THREADS - 1 - vt; i < EG * 9; i += C::THREADS) {
+            const H* rec = &s_r64[(i / 9 * NG + 3 * (i % 9)) * C::REC64 + 18];
+            const H v[3] = {rec[0], rec[C::REC64], rec[2 * C::REC64]};
+            H o[2];
+            line_Lt<H>(v, o);
+            Lq[(i / 9 * 2) * 9 + i % 9] = o[0];
+            Lq[(i / 9 * 2 + 1) * 9 + i % 9] = o[1];
+          }
         }
         __syncthreads();
-        for (int i = tid; i < EG * 9 * N2 * 3; i += C::THREADS) {
-          const int g3 = i % 3, a1 = (i / 3) % N1, a2 = (i / (3 * N1)) % N1, mk = (i / (3 * N2)) % 9,
-                    el = i / (27 * N2);
-          const H* M = mk % 3 == 1 ? s_D1 : s_B1;
-          const H* u = &U1[((el * 9 + mk) * N1 + a1) * 9 + 3 * g3];
-          H acc = hval<H>(0.0);
+        constexpr int I2 = EG * 9 * N1;  // (el, m, a1, g3)
+        for (int i = vt; i < 2 * I2; i += C::THREADS) {
+          const bool third = i >= I2;
+          const int r = third ? i - I2 : i;
+          const int g3 = r % 3, a1 = (r / 3) % N1, em = r / (3 * N1);
+          const H* u = U1 + (em * 3 * N1 + a1) * 9 + 3 * g3;
+          H o[N1];
+          if (third)
+            line_Bt<N1, H>(u + 2 * N1 * 9, o);
+          else
+            line_BtDt<N1, H>(u, u + N1 * 9, o);
 #pragma unroll
-          for (int g2 = 0; g2 < 3; ++g2) acc = hfma(M[g2 * N1 + a2], u[g2], acc);
-          U2[i] = acc;
+          for (int a = 0; a < N1; ++a) U2[((third ? EG * 3 : 0) + em) * N2 * 3 + (a1 + N1 * a) * 3 + g3] = o[a];
+        }
+        if (PM && prows) {
+          H* Lq2 = Lq + EG * 18;
+          for (int i = C::THREADS - 1 - vt; i < EG * 6; i += C::THREADS) {  // (el, q1, g3)
+            H o[2];
+            line_Lt<H>(Lq + (i / 3) * 9 + 3 * (i % 3), o);
+            const int q1 = (i / 3) % 2, el = i / 6;
+            Lq2[(el * 4 + q1) * 3 + i % 3] = o[0];
+            Lq2[(el * 4 + q1 + 2) * 3 + i % 3] = o[1];
+          }
         }
         __syncthreads();
-        for (int i = tid; i < EG * 9 * NPE; i += C::THREADS) {
-          const int a = i % NPE, mk = (i / NPE) % 9, el = i / (9 * NPE);
-          const int a12 = a % N2, a3 = a / N2;
-          const H* M = mk % 3 == 2 ? s_D1 : s_B1;
-          const H* u = &U2[((el * 9 + mk) * N2 + a12) * 3];
-          H acc = hval<H>(0.0);
-#pragma unroll
-          for (int g3 = 0; g3 < 3; ++g3) acc = hfma(M[g3 * N1 + a3], u[g3], acc);
-          RK[i] = acc;
+        for (int i = vt; i < EG * 3 * N2; i += C::THREADS) {
+          const int a12 = i % N2, m = (i / N2) % 3, el = i / (3 * N2);
+          H o[N1];
+          line_BtDt<N1, H>(U2 + i * 3, U2 + (EG * 3 * N2 + i) * 3, o);
+          if (el < nvalid) emit(el, m, a12, o);
+        }
+        if (prows) {
+          if (PM) {
+            const H* Lq2 = Lq + EG * 18;
+            for (int i = C::THREADS - 1 - vt; i < EG * 4; i += C::THREADS) {  // (el, q1 q2)
+              H o[2];
+              line_Lt<H>(Lq2 + i * 3, o);
+              if (i / 4 < nvalid) {
+                emit_p(i / 4, i % 4, o[0]);
+                emit_p(i / 4, i % 4 + 4, o[1]);
+              }
+            }
+          } else {
+            for (int el = C::THREADS - 1 - vt; el < nvalid; el += C::THREADS) {
+              H acc = hval<H>(0.0);
+              for (int g = 0; g < NG; ++g) acc = acc + s_r64[(el * NG + g) * C::REC64 + 18];
+              emit_p(el, 0, acc);
+            }
+          }
         }
         __syncthreads();
       };
       if (P.r != nullptr) {
-        sumfact(0);
-        for (int it = tid; it < EG * NROW; it += C::THREADS) {
-          const int el = it / NROW, row = it % NROW;
-          if (el >= nvalid) continue;
-          const H* rec = &s_r64[el * NG * C::REC64];
+        auto add_r = [&](int el, int ln, size_t gr, double v) {
           const int* nd = &s_node[el * (NR + 1)];
           const uint16_t* tab = P.tables + (size_t)nd[NR] * NR * NR;
-          H acc = hval<H>(0.0);
-          int ln;
-          size_t R;
-          if (row < NU3) {
-            const int m = row / NPE, a = row % NPE;
-            const H* rk = &s_dz[(el * 9 + m * 3) * NPE + a];
-            acc = rk[0] + rk[NPE] + rk[2 * NPE];
-            ln = a;
-            R = (size_t)m * nu + nd[a];
-          } else {
-            const int q = row - NU3;
-            for (int g = 0; g < NG; ++g) acc = PM ? hfma(s_psi[g * 8 + q], rec[g * C::REC64 + 18], acc)
-                                                  : acc + rec[g * C::REC64 + 18];
-            ln = NPE + q;
-            R = (size_t)3 * nu + nd[ln];
-          }
-          const double accd = hd(acc);
-          if constexpr (OUT == 1) {
-            SO->r[(size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_r(NPE, NPP) + row] = accd;
-          } else {
-            const bool first = tab[ln * NR + ln] & 0x8000;
-            if (first)
-              P.r[R] = accd;
-            else
-              atomicAdd(&P.r[R], accd);
-          }
-        }
+          if (tab[ln * NR + ln] & 0x8000)
+            P.r[gr] = v;
+          else
+            atomicAdd(&P.r[gr], v);
+        };
+        sumfact(
+            0, true,
+            [&](int el, int m, int a12, const H (&o)[N1]) {
+#pragma unroll
+              for (int a3 = 0; a3 < N1; ++a3) {
+                const int a = a12 + N2 * a3;
+                if constexpr (OUT == 1) {
+                  unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
+                  reinterpret_cast<double*>(er + a * R::ROW + R::OR)[m] = hd(o[a3]);
+                } else {
+                  add_r(el, a, (size_t)m * nu + s_node[el * (NR + 1) + a], hd(o[a3]));
+                }
+              }
+            },
+            [&](int el, int q, H v) {
+              if constexpr (OUT == 1) {
+                unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
+                reinterpret_cast<double*>(er + R::P0 + q * R::PROW)[NU3] = hd(v);
+              } else {
+                add_r(el, NPE + q, (size_t)3 * nu + s_node[el * (NR + 1) + NPE + q], hd(v));
+              }
+            });
       }
-      if (!PM && !P.res_only) {
-        __syncthreads();  // the residual rows have read RK
-        sumfact(9);
-        for (int it = tid; it < EG * NU3; it += C::THREADS) {
-          const int el = it / NU3, col = it % NU3;
-          if (el >= nvalid) continue;
-          const int n = col / NPE, b = col % NPE;
+      // one pressure-coupling entry K(q, (n, b)) and its mirror
+      auto emit_c = [&](int el, int q, int n, int b, double kv) {
+        if constexpr (OUT == 1) {
+          unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
+          reinterpret_cast<double*>(er + R::P0 + q * R::PROW)[n * NPE + b] = kv;
+          reinterpret_cast<double*>(er + b * R::ROW + R::OC)[n * NPP + q] = kv;
+        } else {
           const int* nd = &s_node[el * (NR + 1)];
           const uint16_t* tab = P.tables + (size_t)nd[NR] * NR * NR;
-          const H* rk = &s_dz[(el * 9 + n * 3) * NPE + b];
-          const double kv = hd(rk[0] + rk[NPE] + rk[2 * NPE]);
-          if constexpr (OUT == 1) {
-            SO->cp[(size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_cp(NPE, NPP) + col] = kv;
-            continue;
-          }
-          const int nb = nd[b], pq = nd[NPE];
-          const uint16_t tqb = tab[NPE * NR + b], tbq = tab[b * NR + NPE];
+          const int lq = NPE + q, pq = nd[lq], nb = nd[b];
+          const uint16_t tqb = tab[lq * NR + b], tbq = tab[b * NR + lq];
           const size_t p1 = (size_t)P.cp_row_ptr[(size_t)3 * nu + pq] + (size_t)n * P.wp[pq] + (tqb & 0x7fff);
           if (tqb & 0x8000)
             P.vals[p1] = kv;
@@ -601,85 +602,63 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
           else
             atomicAdd(&P.vals[p2], kv);
         }
-      }
+      };
+      if (!PM && !P.res_only)
+        sumfact(
+            9, false,
+            [&](int el, int n, int b12, const H (&o)[N1]) {
+#pragma unroll
+              for (int b3 = 0; b3 < N1; ++b3) emit_c(el, 0, n, b12 + N2 * b3, hd(o[b3]));
+            },
+            [](int, int, H) {});
       // Pressure-coupling block for nodal (trilinear) pressure,
       //   K(q, n, b) = sum_k sum_g psi_q(g) A_g(k, n) dN_b/dxi_k(g),  A_g = J_z w dxi/dz,
-      // psi_q = L(q1) L(q2) L(q3), dN_b/dxi_k = M1k(b1) M2k(b2) M3k(b3) (M = 1-D
-      // derivative along xi_k, 1-D value otherwise), by sum factorisation with
-      // the products LB = L x value, LD = L x derivative of the 1-D tables.
-      // Stage 1 contracts g1 for every (n, k) into T1_n[el][k][q1][b1][g2 + 3 g3]
-      // (n = 0, 1 in the s_f32 scratch region, n = 2 in the gradient region,
-      // both free by now); then one thread per (n, el, q1, b1, q2, b2)
-      // contracts g2 -- the k = 0 and k = 1 terms, which share the value table
-      // along xi3, summed into w, the k = 2 term into u -- and g3.
+      // psi_q = L(q1) L(q2) L(q3), dN_b/dxi_k = M1k(b1) M2k(b2) M3k(b3), line by
+      // line with the products of the linear and the 1-D basis functions
+      // (line_L): xi1 for every k, xi2 with k = 0 and 1 merged, xi3 with all.
       if (PM && !P.res_only) {
-        constexpr int NT1 = 3 * 2 * N1 * 9;  // T1 entries per element and n
-        H* T1f = reinterpret_cast<H*>(s_f32);
-        const H* LB = s_LM;
-        const H* LD = s_LM + 6 * N1;
-        __syncthreads();  // the residual rows have read the gradient region
-        for (int i = tid; i < 3 * EG * NT1; i += C::THREADS) {
-          const int n = i / (EG * NT1), r = i % (EG * NT1);
-          const int j = r % 9, b1 = (r / 9) % N1, q1 = (r / (9 * N1)) % 2, k = (r / (18 * N1)) % 3,
-                    el = r / NT1;
-          const H* lm = (k == 0 ? LD : LB) + q1 * 3 * N1 + b1;
+        constexpr int L2 = C::L2;
+        H* T1 = reinterpret_cast<H*>(sm + C::O_DZ);  // [n][el][k][q1 b1][g2 + 3 g3]
+        H* W2 = T1 + EG * 9 * L2 * 9;                // [n][el][q1 b1][q2 b2][g3]
+        H* V2 = W2 + EG * 3 * L2 * L2 * 3;           // the k = 2 terms
+        for (int i = vt; i < EG * 81; i += C::THREADS) {
+          const int j = i % 9, k = (i / 9) % 3, el = (i / 27) % EG, n = i / (27 * EG);
           const H* a = &s_r64[(el * NG + 3 * j) * C::REC64 + 9 + 3 * k + n];
-          H* T1 = n < 2 ? T1f + n * EG * NT1 : s_dz;
-          T1[r] = hfma(lm[0], a[0], hfma(lm[N1], a[C::REC64], lm[2 * N1] * a[2 * C::REC64]));
+          const H v[3] = {a[0], a[C::REC64], a[2 * C::REC64]};
+          H o[L2];
+          if (k == 0)
+            line_L<N1, 0, 1, H>(v, v, o);
+          else
+            line_L<N1, 1, 0, H>(v, v, o);
+#pragma unroll
+          for (int b = 0; b < L2; ++b) T1[((i / 9) * L2 + b) * 9 + j] = o[b];
         }
         __syncthreads();
-        for (int tt = tid; tt < 3 * EG * 4 * N2; tt += C::THREADS) {
-          const int n = tt / (EG * 4 * N2), t = tt % (EG * 4 * N2);
-          const int b2 = t % N1, q2 = (t / N1) % 2, b1 = (t / (2 * N1)) % N1, q1 = (t / (2 * N2)) % 2,
-                    el = t / (4 * N2);
+        constexpr int I2 = EG * 3 * L2 * 3;  // (n, el, q1 b1, g3)
+        for (int i = vt; i < 2 * I2; i += C::THREADS) {
+          const bool third = i >= I2;
+          const int r = third ? i - I2 : i;
+          const int g3 = r % 3, b1 = (r / 3) % L2, ne = r / (3 * L2);
+          const H* t = T1 + (ne * 3 * L2 + b1) * 9 + 3 * g3;
+          H o[L2];
+          if (third)
+            line_L<N1, 1, 0, H>(t + 2 * L2 * 9, t, o);
+          else
+            line_L<N1, 1, 1, H>(t, t + L2 * 9, o);
+          H* out = (third ? V2 : W2) + (ne * L2 + b1) * L2 * 3 + g3;
+#pragma unroll
+          for (int b = 0; b < L2; ++b) out[b * 3] = o[b];
+        }
+        __syncthreads();
+        for (int i = vt; i < EG * 3 * L2 * L2; i += C::THREADS) {
+          const int qb2 = i % L2, qb1 = (i / L2) % L2, el = (i / (L2 * L2)) % EG, n = i / (L2 * L2 * EG);
+          H o[L2];
+          line_L<N1, 1, 1, H>(W2 + i * 3, V2 + i * 3, o);
           if (el >= nvalid) continue;
-          const H* T1 = n < 2 ? T1f + n * EG * NT1 : s_dz;
-          const H* t0 = &T1[el * NT1 + (q1 * N1 + b1) * 9];  // k stride 18 N1
-          const H* lb2 = LB + q2 * 3 * N1 + b2;
-          const H* ld2 = LD + q2 * 3 * N1 + b2;
-          H w[3], u[3];
+          const int q12 = qb1 / N1 + 2 * (qb2 / N1), b12 = qb1 % N1 + N1 * (qb2 % N1);
 #pragma unroll
-          for (int g3 = 0; g3 < 3; ++g3) {
-            H wa = hval<H>(0.0), ua = hval<H>(0.0);
-#pragma unroll
-            for (int g2 = 0; g2 < 3; ++g2) {
-              const int jj = g2 + 3 * g3;
-              wa = hfma(lb2[g2 * N1], t0[jj], wa);
-              wa = hfma(ld2[g2 * N1], t0[18 * N1 + jj], wa);
-              ua = hfma(lb2[g2 * N1], t0[36 * N1 + jj], ua);
-            }
-            w[g3] = wa;
-            u[g3] = ua;
-          }
-          const int* nd = &s_node[el * (NR + 1)];
-          const uint16_t* tab = P.tables + (size_t)nd[NR] * NR * NR;
-#pragma unroll
-          for (int q3 = 0; q3 < 2; ++q3)
-#pragma unroll
-            for (int b3 = 0; b3 < N1; ++b3) {
-              H acc = hval<H>(0.0);
-#pragma unroll
-              for (int g3 = 0; g3 < 3; ++g3)
-                acc = hfma(LD[(q3 * 3 + g3) * N1 + b3], u[g3], hfma(LB[(q3 * 3 + g3) * N1 + b3], w[g3], acc));
-              const int q = q1 + 2 * q2 + 4 * q3, b = b1 + N1 * b2 + N2 * b3;
-              const double kv = hd(acc);
-              if constexpr (OUT == 1) {
-                SO->cp[(size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_cp(NPE, NPP) + q * NU3 + n * NPE + b] = kv;
-                continue;
-              }
-              const int lq = NPE + q, pq = nd[lq], nb = nd[b];
-              const uint16_t tqb = tab[lq * NR + b], tbq = tab[b * NR + lq];
-              const size_t p1 = (size_t)P.cp_row_ptr[(size_t)3 * nu + pq] + (size_t)n * P.wp[pq] + (tqb & 0x7fff);
-              if (tqb & 0x8000)
-                P.vals[p1] = kv;
-              else
-                atomicAdd(&P.vals[p1], kv);
-              const size_t p2 = (size_t)P.cp_row_ptr[(size_t)n * nu + nb] + (tbq & 0x7fff);
-              if (tbq & 0x8000)
-                P.vals[p2] = kv;
-              else
-                atomicAdd(&P.vals[p2], kv);
-            }
+          for (int qb3 = 0; qb3 < L2; ++qb3)
+            emit_c(el, q12 + 4 * (qb3 / N1), n, b12 + N2 * (qb3 % N1), hd(o[qb3]));
         }
       }
       // structurally zero pressure-pressure entries, stored by their first contributor
@@ -724,17 +703,18 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
             const bool diag = blk < 3 && a12 == b12;
             constexpr int NP = N1 * N1;
             if constexpr (OUT == 1) {
-              T* st = stage_uu<T>(*SO) + (size_t)elem_at(P, elems, grp * EG + el) * cmfe::rec_stride_uu(NPE);
-              T* s0 = st + ((a12 * 3 + m) * 3 + n) * NPE + b12;
-              T* s1m = st + ((b12 * 3 + n) * 3 + m) * NPE + a12;
+              unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
+              T* s0 = reinterpret_cast<T*>(er + a12 * R::ROW) + (3 * m + n) * NPE + b12;
+              T* s1m = reinterpret_cast<T*>(er + b12 * R::ROW) + (3 * n + m) * NPE + a12;
+              constexpr int A3 = NP * (R::ROW / (int)sizeof(T));  // next a3: NP node rows on
 #pragma unroll
               for (int a3 = 0; a3 < N1; ++a3)
 #pragma unroll
                 for (int b3 = 0; b3 < N1; ++b3) {
                   if (diag && a3 > b3) continue;
                   if (N1 == 2 && blk < 3 && a12 + NP * a3 > b12 + NP * b3) continue;
-                  s0[a3 * NP * 9 * NPE + b3 * NP] = K[a3][b3];
-                  if (!(diag && a3 == b3)) s1m[b3 * NP * 9 * NPE + a3 * NP] = K[a3][b3];
+                  s0[a3 * A3 + b3 * NP] = K[a3][b3];
+                  if (!(diag && a3 == b3)) s1m[b3 * A3 + a3 * NP] = K[a3][b3];
                 }
             } else {
               const int* bs = &s_base[el * 9 * NPE];

@@ -322,23 +322,6 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
   s.nnz = nnz;
   s.nnz_uu = nuu;
   s.nnz_cp = ncp;
-  {
-    // scratch of one gathering warp: the larger of a u node's three rows
-    // (3 x 3 wu FP32, padded to 16 bytes, then 3 x its pressure columns FP64)
-    // and a pressure row (FP64)
-    int64_t need = 0;
-    for (int n = 0; n < s.nu; ++n) {
-      const int64_t wc = s.cp_row_ptr[(size_t)n + 1] - s.cp_row_ptr[(size_t)n];
-      need = std::max<int64_t>(need, ((36 * (int64_t)s.wu[n] + 15) & ~(int64_t)15) + 3 * wc * 8);
-    }
-    for (int q = 0; q < s.npn; ++q) {
-      const size_t row = (size_t)3 * s.nu + q;
-      need = std::max<int64_t>(need, (int64_t)(s.cp_row_ptr[row + 1] - s.cp_row_ptr[row]) * 8);
-    }
-    s.gather_bytes = (int)std::min<int64_t>((need + 15) & ~(int64_t)15, 1 << 30);
-  }
-
-
   s.col.allocate(nnz);
   parallel_for((int)s.ndofs, [&](int r) {
     const bool urow = r < 3ll * s.nu;
@@ -461,6 +444,12 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     }
     s.ntables = (int)seen.size();
   }
+  if ((int64_t)s.ntables * nr >= (1ll << 31)) return fail(msg, "too many distinct rank tables");
+  s.u_inc_row.resize(s.u_inc.size());
+  s.p_inc_row.resize(s.p_inc.size());
+  parallel_for((int)s.u_inc.size(), [&](int k) { s.u_inc_row[k] = s.elem_table[s.u_inc[k] >> 5] * nr + (s.u_inc[k] & 31); });
+  parallel_for((int)s.p_inc.size(),
+               [&](int k) { s.p_inc_row[k] = s.elem_table[s.p_inc[k] >> 3] * nr + s.npe + (s.p_inc[k] & 7); });
 
   // Boundary faces: a local face (reference order -xi1, -xi2, -xi3, +xi1,
   // +xi2, +xi3) whose four corner nodes no other element holds.
@@ -519,6 +508,7 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
 
   // Geometric Gauss-point data.
   s.geo.assign((size_t)s.ne * NG * 10, 0.0);
+  s.geo_rj.assign((size_t)s.ne * NG, 0.0);
   std::vector<char> degenerate(s.ne, 0);
   parallel_for(s.ne, [&](int e) {
     for (int g = 0; g < NG; ++g) {
@@ -548,6 +538,7 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
         for (int j = 0; j < 3; ++j) out[i * 3 + j] = dn[i][j];
       out[9] = std::sqrt(std::fabs(det_gl));
       if (!(out[9] > 0.0)) degenerate[e] = 1;
+      s.geo_rj[(size_t)e * NG + g] = 1.0 / out[9];
     }
   });
   for (int e = 0; e < s.ne; ++e)

@@ -53,13 +53,14 @@ struct SurfWarpSmem {
 // All loaded faces of boundary element e, by one warp (S is the warp's
 // shared scratch).  mode: 0 = CSR (FP64 values, or FP32 uu values when
 // P.vals_uu), 1 = element outputs (P.elem_out, elements first_elem ..
-// first_elem + count - 1), 2 = the element's staging records (SO->uu,
-// SO->r), which only this warp touches, so it adds without atomics.
-template <int N1>
+// first_elem + count - 1), 2 = the element's record (displacement block in
+// T), which only this warp touches, so it adds without atomics.
+template <int N1, int NPP, class T = float>
 __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, const uint8_t* bmask, int mode,
                                                 int want_jac, SurfWarpSmem& S, int lane,
                                                 const cmfe::StageOut* SO = nullptr) {
   constexpr int NPE = N1 * N1 * N1, NF = N1 * N1;
+  using R = cmfe::Rec<NPE, NPP, T>;
   const int nr = P.nr, nrow = 3 * NPE + (P.pmode ? 8 : 1);
   const uint8_t mask = bmask[e];
   for (int lf = 0; lf < 6; ++lf) {
@@ -130,7 +131,7 @@ __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, c
         }
         const int a = S.node[f];
         if (mode == 2) {
-          SO->r[(size_t)e * cmfe::rec_stride_r(NPE, nrow - 3 * NPE) + c * NPE + a] += acc;
+          reinterpret_cast<double*>(SO->rec + (size_t)e * R::BYTES + a * R::ROW + R::OR)[c] += acc;
         } else if (mode == 1) {
           P.elem_out[(size_t)(e - P.first_elem) * nrow + c * NPE + a] += acc;
         } else {
@@ -160,16 +161,16 @@ __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, c
       if (mode == 2) {
         // the lower block entry and its mirror: distinct entries for distinct
         // (oh, ms, ns), so the lanes never touch the same word
-        float* st = SO->uu + (size_t)e * cmfe::rec_stride_uu(NPE);
-        st[cmfe::rec_uu(NPE, mh, a, nh, b)] += (float)acc;
-        st[cmfe::rec_uu(NPE, nh, b, mh, a)] += (float)acc;
+        unsigned char* er = SO->rec + (size_t)e * R::BYTES;
+        reinterpret_cast<T*>(er + a * R::ROW)[(3 * mh + nh) * NPE + b] += (T)acc;
+        reinterpret_cast<T*>(er + b * R::ROW)[(3 * nh + mh) * NPE + a] += (T)acc;
         continue;
       }
       if (mode == 1) {
         double* out = P.elem_out + (size_t)(e - P.first_elem) * nrow * nrow;
-        const int R = mh * NPE + a, Cc = nh * NPE + b;
-        out[(size_t)Cc * nrow + R] += acc;
-        out[(size_t)R * nrow + Cc] += acc;
+        const int row = mh * NPE + a, col = nh * NPE + b;
+        out[(size_t)col * nrow + row] += acc;
+        out[(size_t)row * nrow + col] += acc;
         continue;
       }
       const int na = en[a], nb2 = en[b];
