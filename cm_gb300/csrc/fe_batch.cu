@@ -72,10 +72,6 @@ int batch_smem(int v, unsigned mask) {
 int launch_mixed_batch(int variant, unsigned mask, const BatchMember* members, int n, const BatchArgs& a,
                        int ctas_per_sm, int num_sms, void* stream) {
   if (n < 1 || n > BATCH_MAX_MEMBERS) return (int)cudaErrorInvalidValue;
-  // one element type: the kernel compiled for that type alone (a smaller
-  // body, register-allocated for that type only)
-  for (int t = 0; t < 4; ++t)
-    if ((mask & 15u) == (1u << t)) return launch_batch_typed(variant, t, mask, members, n, a, ctas_per_sm, num_sms, stream);
   cudaStream_t st = (cudaStream_t)stream;
   switch (variant) {
     case 0: return launch_variant<4, 8>(members, n, a, mask, ctas_per_sm, num_sms, st);

@@ -1,9 +1,6 @@
 // libcm_fe: device code of the batched mixed-precision assembly (the
-// persistent kernel, its grid barrier and the member constant table),
-// included by the translation units that instantiate it: fe_batch.cu (kernels
-// for batches of mixed element types) and fe_batch_typed.cu (one element
-// type).  Each translation unit is its own module with its own constant
-// table, written by the launch helper of that unit before its kernel runs.
+// persistent kernel, its grid barrier and the member constant table, written
+// by the launch helper before the kernel runs), instantiated in fe_batch.cu.
 #pragma once
 #include "fe_mixed_impl.cuh"
 #include "fe_surface_impl.cuh"

@@ -17,11 +17,8 @@
 // is one contiguous piece of the element's record, the pieces of four
 // elements are copied to shared memory at once (cp.async), and every lane
 // keeps its columns of the rows in registers.  Which of an element's nodes
-// belongs to a column comes from the inverse of the element's rank-table
-// row, built in shared memory while the copies are in flight.  Adding in
-// shared memory instead, one element after the other, took 80 k of the 188 k
-// cycles of an element group of the 32^3 box; this form is in the figures at
-// the fused kernel.
+// belongs to a column is read from the node's pattern (HostSetup::pat), which
+// nodes with equal surroundings share, while the copies are in flight.
 //
 // Row layout of the mixed split: a displacement row (m, a) holds
 // [u_x | u_y | u_z] blocks of wu[a] columns in the FP32 array at
@@ -54,15 +51,14 @@ struct ReadyNode {
 };
 
 // Shared scratch of one gathering warp: the pieces in flight; u nodes: the
-// local nodes of every column [GPOS][GR], and the sums of the pressure columns
-// and the residual; pressure nodes: the sums of the row instead.
+// sums of the pressure columns and the residual; pressure nodes: the sums of
+// the row.
 template <int NPE, int NPP, class T>
 struct GatherCfg {
   using R = cmfe::Rec<NPE, NPP, T>;
-  static constexpr int O_ACC = GR * R::ROW;                 // u: [3][GPP], residual [3]
-  static constexpr int O_INV = O_ACC + (3 * GPP + 4) * 8;
+  static constexpr int O_ACC = GR * R::ROW;                 // u: [3][GPP], residual [3], then FP64 blocks [9][GPOS]
   static constexpr int O_ACCP = GR * R::PROW;               // p: [3][GPOS], residual
-  static constexpr int UB = O_INV + GR * GPOS, PB = O_ACCP + (3 * GPOS + 2) * 8;
+  static constexpr int UB = O_ACC + (3 * GPP + 4 + (sizeof(T) == 8 ? 9 * GPOS : 0)) * 8, PB = O_ACCP + (3 * GPOS + 2) * 8;
   static constexpr int BYTES = UB > PB ? UB : PB;           // multiples of 16
 };
 
@@ -80,7 +76,7 @@ __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;
 static_assert(GR == 4, "one byte per element of a round");
 __device__ __forceinline__ int inv_at(uint32_t w, int j) { return (w >> (8 * j)) & 255; }
 
-// The three displacement rows of u node a, by one warp.  list: its first
+// The three displacement rows of a u node, by one warp.  list: its first
 // GLIST incidences (element and local node, rank-table row).
 template <int NPE, int NPP, class T>
 __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe::StageOut& S, const cmfe::FusedArgs& F,
@@ -109,52 +105,80 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
     wc = P.cp_row_ptr[(size_t)a + 1] - P.cp_row_ptr[(size_t)a];  // the same for m = 0..2
   }
   using G = GatherCfg<NPE, NPP, T>;
-  uint8_t* inv = mine + G::O_INV;
   double* cacc = reinterpret_cast<double*>(mine + G::O_ACC);
+  const uint32_t* pat = F.pat + F.u_pat[a];
   const int passes = max((wu + GPOS - 1) / GPOS, (wc + GPP - 1) / GPP);
   for (int pass = 0; pass < passes; ++pass) {  // one pass unless the neighbourhood is very large
     const int p0 = pass * GPOS, q0 = pass * GPP;
-    T acc[GPOS / 32][9];
+    T acc[FULL ? 1 : GPOS / 32][9];
+    double* uacc = cacc + 3 * GPP + 4;
     for (int i = lane; i < 3 * GPP + 3; i += 32) cacc[i] = 0.0;
+    if constexpr (FULL) {
+      for (int i = lane; i < 9 * GPOS; i += 32) uacc[i] = 0.0;
+    } else {
 #pragma unroll
-    for (int i = 0; i < GPOS / 32; ++i)
+      for (int i = 0; i < GPOS / 32; ++i)
 #pragma unroll
-      for (int mn = 0; mn < 9; ++mn) acc[i][mn] = T(0);
+        for (int mn = 0; mn < 9; ++mn) acc[i][mn] = T(0);
+    }
     for (int kb = 0; kb < rn.cnt; kb += GR) {
       const int cnt = min(GR, rn.cnt - kb);
       int2 in = {0, 0};
       if (lane < cnt) in = kb + lane < GLIST ? list[kb + lane] : int2{F.u_inc[rn.k0 + kb + lane], F.u_inc_row[rn.k0 + kb + lane]};
-#pragma unroll
-      for (int i = 0; i < GPOS / 32; ++i) reinterpret_cast<uint32_t*>(inv)[32 * i + lane] = 0xffffffffu;
       __syncwarp();
-      int rk[GR], rq[GR];
 #pragma unroll
       for (int j = 0; j < GR; ++j) {
         const int packed = __shfl_sync(0xffffffffu, in.x, j);
-        const uint16_t* tab = P.tables + (size_t)__shfl_sync(0xffffffffu, in.y, j) * NR;
-        rk[j] = rq[j] = -1;
-        if (j < cnt) {
-          if (lane < NPE) rk[j] = (tab[lane] & 0x7fff) - p0;
-          if (lane < NPP) rq[j] = (tab[NPE + lane] & 0x7fff) - q0;
+        if (j < cnt)
           copy_piece(mine + j * R::ROW, S.rec + (size_t)(packed >> 5) * R::BYTES + (packed & 31) * R::ROW, R::ROW, lane);
-        }
       }
-#pragma unroll
-      for (int j = 0; j < GR; ++j)
-        if (rk[j] >= 0 && rk[j] < GPOS) inv[rk[j] * GR + j] = (uint8_t)lane;
-      copies_done();
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < GPOS / 32; ++i) {
-        if (p0 + 32 * i >= wu) break;
-        const uint32_t w = reinterpret_cast<const uint32_t*>(inv)[32 * i + lane];
+      // the columns' local nodes (FP64: the local nodes' columns) and the
+      // pressure parameters' ranks
+      const uint32_t* pr = pat + (size_t)(kb / GR) * (wu + 2 * NPP);
+      int rq = -1;
+      if (lane < 4 * NPP) rq = (int)reinterpret_cast<const uint16_t*>(pr + wu)[lane] - q0;
+      if constexpr (FULL) {
+        int rk[GR];
 #pragma unroll
         for (int j = 0; j < GR; ++j) {
-          const int b = inv_at(w, j);
-          if (b != GNONE) {
-            const T* v = reinterpret_cast<const T*>(mine + j * R::ROW) + b;
+          const int row = __shfl_sync(0xffffffffu, in.y, j);
+          rk[j] = j < cnt && lane < NPE ? (P.tables[(size_t)row * NR + lane] & 0x7fff) - p0 : -1;
+        }
+        copies_done();
+        __syncwarp();
+        // value i of a piece, [m][n][b], to its column: added in shared
+        // memory, where every lane holds a value (the columns of one element
+        // are a quarter of a corner node's, so sums per column would issue
+        // three times the FP64 instructions)
 #pragma unroll
-            for (int mn = 0; mn < 9; ++mn) acc[i][mn] += v[mn * NPE];
+        for (int j = 0; j < GR; ++j) {
+          if (j >= cnt) break;
+          const double* v = reinterpret_cast<const double*>(mine + j * R::ROW);
+#pragma unroll
+          for (int s = 0; s < (9 * NPE + 31) / 32; ++s) {
+            const int i = 32 * s + lane;
+            const int tk = __shfl_sync(0xffffffffu, rk[j], i % NPE);
+            if (i < 9 * NPE && tk >= 0 && tk < GPOS) uacc[i / NPE * GPOS + tk] += v[i];
+          }
+          __syncwarp();
+        }
+      } else {
+        uint32_t w[GPOS / 32];
+#pragma unroll
+        for (int i = 0; i < GPOS / 32; ++i) w[i] = p0 + 32 * i + lane < wu ? pr[p0 + 32 * i + lane] : 0xffffffffu;
+        copies_done();
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < GPOS / 32; ++i) {
+          if (p0 + 32 * i >= wu) break;
+#pragma unroll
+          for (int j = 0; j < GR; ++j) {
+            const int b = inv_at(w[i], j);
+            if (b != GNONE) {
+              const T* v = reinterpret_cast<const T*>(mine + j * R::ROW) + b;
+#pragma unroll
+              for (int mn = 0; mn < 9; ++mn) acc[i][mn] += v[mn * NPE];
+            }
           }
         }
       }
@@ -163,7 +187,7 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
 #pragma unroll
       for (int j = 0; j < GR; ++j) {
         if (j >= cnt) break;
-        const int tq = __shfl_sync(0xffffffffu, rq[j], lane % NPP);
+        const int tq = __shfl_sync(0xffffffffu, rq, j * NPP + lane % NPP);
         const int at = lane < 3 * NPP ? (tq >= 0 && tq < GPP ? lane / NPP * GPP + tq : -1) : 3 * GPP + lane - 3 * NPP;
         if (lane < 3 * NPP + 3 && at >= 0) cacc[at] += reinterpret_cast<const double*>(mine + j * R::ROW + R::OC)[lane];
         __syncwarp();
@@ -176,7 +200,8 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
 #pragma unroll
         for (int m = 0; m < 3; ++m)
 #pragma unroll
-          for (int n = 0; n < 3; ++n) du[m][n * wu + pos] = acc[i][3 * m + n];
+          for (int n = 0; n < 3; ++n)
+            du[m][n * wu + pos] = FULL ? (T)uacc[(3 * m + n) * GPOS + 32 * i + lane] : acc[FULL ? 0 : i][3 * m + n];
       }
     }
     if (q0 + lane < wc) {

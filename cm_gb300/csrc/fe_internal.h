@@ -62,8 +62,16 @@ struct HostSetup {
   // node (sorted by element number, packed e * 32 + local node) and around
   // every pressure row node (e * 8 + local pressure node).
   std::vector<int32_t> u_inc_ptr, u_inc, p_inc_ptr, p_inc;
-  // the incidences' rank-table rows: elem_table[e] * nr + local row node
+  // the incidences' rank-table rows, elem_table[e] * nr + local row node
   std::vector<int32_t> u_inc_row, p_inc_row;
+  // u nodes: which local node of which element belongs to a column of the
+  // node's rows.  Nodes with the same rank-table rows around them share a
+  // pattern; u_pat[n] is node n's offset in pat (32-bit words), where every
+  // round of four incidences has wu words (one byte per incidence: its local
+  // node at that column, 255 = none) followed by the ranks of its pressure
+  // parameters, 4 * npp 16-bit values (0xffff past the last incidence).
+  std::vector<int32_t> u_pat;
+  std::vector<uint32_t> pat;
   // the largest element number around any of the row nodes 0..a (u nodes)
   // and 0..q (pressure row nodes): once the elements below E are assembled,
   // every node a with u_last_prefix[a] < E has its rows complete
@@ -144,6 +152,8 @@ struct FusedArgs {
   const int32_t* p_inc;
   const int32_t* u_inc_row;  // rank-table row of every incidence
   const int32_t* p_inc_row;
+  const int32_t* u_pat;      // offset of every u node's pattern
+  const uint32_t* pat;
   int* work;       // this launch's group counter
   int* node_done;
   const uint8_t* bmask;
@@ -167,7 +177,15 @@ int fused_wave(const HostSetup& s, int num_sms, bool double_float);
 int launch_mixed_fused(const HostSetup& s, const KParams& kp, const StageOut& so, const FusedArgs& fa, int num_sms,
                        void* stream, bool double_float);
 
-// Bytes of one element's record.
+// The FP64 Jacobian (and residual when kp.r) the same way (fe_fp64.cu), with
+// records of record_bytes_fp64() each; fp64_groups: its element groups, and
+// whether the mesh is one that leaves SMs without a group.
+int launch_fp64_fused(const HostSetup& s, const KParams& kp, const StageOut& so, const FusedArgs& fa, int num_sms,
+                      void* stream);
+int fp64_groups(const HostSetup& s, int num_sms, bool* small);
+size_t record_bytes_fp64(const HostSetup& s);
+
+// Bytes of one element's record (mixed precision).
 inline size_t record_bytes(const HostSetup& s) {
   if (s.n1 == 2) return s.pmode ? Rec<8, 8, float>::BYTES : Rec<8, 1, float>::BYTES;
   return s.pmode ? Rec<27, 8, float>::BYTES : Rec<27, 1, float>::BYTES;
@@ -220,10 +238,6 @@ int batch_smem(int v, unsigned mask);
 // Copies the member table (device memory, n entries) into the constant table
 // and launches the persistent kernel, both on stream; returns a cudaError_t.
 int launch_mixed_batch(int variant, unsigned mask, const BatchMember* members, int n, const BatchArgs& a,
-                       int ctas_per_sm, int num_sms, void* stream);
-// The same for a batch whose members all have element type `type`
-// (fe_batch_typed.cu).
-int launch_batch_typed(int variant, int type, unsigned mask, const BatchMember* members, int n, const BatchArgs& a,
                        int ctas_per_sm, int num_sms, void* stream);
 
 // Device CSR pattern (0-based row pointers and columns) and sizes of a handle

@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -496,8 +497,15 @@ struct fe_equations_set {
   // staged assembly: incidence lists (uploaded at creation) and the
   // per-element records (allocated on the first staged evaluation)
   int32_t *d_u_inc_ptr = nullptr, *d_u_inc = nullptr, *d_p_inc_ptr = nullptr, *d_p_inc = nullptr,
-          *d_u_inc_row = nullptr, *d_p_inc_row = nullptr;
+          *d_u_inc_row = nullptr, *d_p_inc_row = nullptr, *d_u_pat = nullptr;
+  uint32_t* d_pat = nullptr;
   unsigned char* d_rec = nullptr;
+  // FP64 assembly: its records and counters, and the order of their uses
+  unsigned char* d_rec64 = nullptr;
+  int* d_fuse64 = nullptr;
+  cudaEvent_t order_event = nullptr;
+  std::vector<cudaStream_t> side_streams;  // parts of a small mesh's FP64 assembly
+  std::vector<cudaEvent_t> side_events;
   int* d_fuse = nullptr;  // fused staged assembly: [0, kFuseChunks) group counters, then per-row-node counts
   int host_output = FE_HOST_OUTPUT_STREAMED;
   int stream_chunks = 0;  // launches of a streamed assembly; 0: equal runs of whole waves
@@ -625,6 +633,111 @@ constexpr int kFuseChunks = 64;
 constexpr int kStreamChunks = 16;
 constexpr int kStreamAuto = 12;
 
+// The arguments of a fused launch of this handle, its counters (*fuse,
+// allocated on first use) set to zero on the stream.
+int fused_args(fe_handle h, int** fuse, cudaStream_t st, cmfe::FusedArgs* fa) {
+  const auto& s = h->hs;
+  const size_t counters = kFuseChunks + (size_t)s.nu + (size_t)s.npn;
+  int rc;
+  if ((rc = ensure((void**)fuse, sizeof(int) * counters))) return rc;
+  CUDA_TRY(cudaMemsetAsync(*fuse, 0, sizeof(int) * counters, st));
+  const int nb = s.bnd_ptr.empty() ? 0 : s.bnd_ptr[s.ncolours];
+  std::memset(fa, 0, sizeof(*fa));
+  fa->u_inc_ptr = h->d_u_inc_ptr;
+  fa->u_inc = h->d_u_inc;
+  fa->p_inc_ptr = h->d_p_inc_ptr;
+  fa->p_inc = h->d_p_inc;
+  fa->u_inc_row = h->d_u_inc_row;
+  fa->p_inc_row = h->d_p_inc_row;
+  fa->u_pat = h->d_u_pat;
+  fa->pat = h->d_pat;
+  fa->work = *fuse;
+  fa->node_done = *fuse + kFuseChunks;
+  fa->bmask = h->has_surfp && nb > 0 ? h->d_bnd_mask : nullptr;
+  fa->g0 = 0;
+  fa->g1 = INT32_MAX;
+  return FE_NO_ERROR;
+}
+
+// A stream whose work is being captured into a graph (an error while asking
+// counts as one).
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) == cudaSuccess) return c != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
+// Work that uses buffers of the handle, on whatever streams, in call order:
+// the stream waits for the handle's previous such work, and the destructor
+// marks the end of what was queued since.
+struct HandleOrder {
+  fe_handle h;
+  cudaStream_t st;
+  HandleOrder(fe_handle h_, cudaStream_t st_) : h(h_), st(st_) {
+    if (!h->order_event) cudaEventCreateWithFlags(&h->order_event, cudaEventDisableTiming);
+    if (h->order_event) cudaStreamWaitEvent(st, h->order_event, 0);
+  }
+  ~HandleOrder() {
+    if (h->order_event) cudaEventRecord(h->order_event, st);
+  }
+};
+
+// The FP64 Jacobian (and the residual when kp.r) by the fused assembly.
+// *taken = false, without an error, where the records cannot be had (no
+// memory left, or the stream is being captured and its replays may run
+// beside other work of the handle): the caller then launches colour by colour.
+int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
+  const auto& s = h->hs;
+  *taken = false;
+  if (capturing(st)) return FE_NO_ERROR;
+  if (ensure((void**)&h->d_rec64, cmfe::record_bytes_fp64(s) * (size_t)s.ne)) return FE_NO_ERROR;
+  HandleOrder order(h, st);
+  cmfe::FusedArgs fa;
+  int rc;
+  if ((rc = fused_args(h, &h->d_fuse64, st, &fa))) return rc == FE_ERR_OUT_OF_MEMORY ? FE_NO_ERROR : rc;
+  kp.elems = nullptr;
+  kp.first_elem = 0;
+  kp.count = s.ne;
+  const cmfe::StageOut so{h->d_rec64};
+  bool small = false;
+  const int groups = cmfe::fp64_groups(s, h->num_sms, &small);
+  // A small mesh: as many launches as it has element colours, as the
+  // colour-ordered assembly has (callers count them; a box has 8), side by side on streams
+  // of the handle -- one after the other they would take one element's 50 us
+  // each.
+  const int n = small ? std::min(std::min(s.ncolours, groups), 8) : 1;
+  std::vector<cudaStream_t>& side = h->side_streams;
+  std::vector<cudaEvent_t>& ev = h->side_events;
+  while ((int)side.size() < n - 1) {
+    cudaStream_t ss;
+    CUDA_TRY(cudaStreamCreateWithFlags(&ss, cudaStreamNonBlocking));
+    side.push_back(ss);
+  }
+  while ((int)ev.size() < n) {
+    cudaEvent_t e;
+    CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ev.push_back(e);
+  }
+  int* const work = fa.work;
+  if (n > 1) CUDA_TRY(cudaEventRecord(ev[0], st));
+  int err = 0;
+  for (int c = n - 1; c >= 0 && !err; --c) {  // the last part on the caller's stream
+    fa.work = work + c;
+    fa.g0 = (int)((int64_t)groups * c / n);
+    fa.g1 = (int)((int64_t)groups * (c + 1) / n);
+    cudaStream_t t = c ? side[c - 1] : st;
+    if (c) CUDA_TRY(cudaStreamWaitEvent(t, ev[0], 0));
+    err = cmfe::launch_fp64_fused(s, kp, so, fa, h->num_sms, t);
+    if (!err) h->launches++;
+    if (c) CUDA_TRY(cudaEventRecord(ev[c], t));
+  }
+  for (int c = 1; c < n; ++c) CUDA_TRY(cudaStreamWaitEvent(st, ev[c], 0));
+  if (err) return set_error(FE_ERR_CUDA, std::string("FP64 kernel launch: ") + cudaGetErrorString((cudaError_t)err));
+  *taken = true;
+  return FE_NO_ERROR;
+}
+
 // The fused staged assembly (element records and row gathers in one kernel)
 // in launches over consecutive ranges of element groups, launch c taking
 // groups [bounds[c], bounds[c + 1]); when `done` is given, done[c] is
@@ -637,20 +750,8 @@ int mixed_fused(fe_handle h, const KParams& kp, const cmfe::StageOut& so, bool d
   int rc;
   const int chunks = (int)bounds.size() - 1;
   if (chunks < 1 || chunks > kFuseChunks) return set_error(FE_ERR_INVALID_ARGUMENT, "fused launches: 1..64");
-  const size_t counters = kFuseChunks + (size_t)s.nu + (size_t)s.npn;
-  if ((rc = ensure((void**)&h->d_fuse, sizeof(int) * counters))) return rc;
-  CUDA_TRY(cudaMemsetAsync(h->d_fuse, 0, sizeof(int) * counters, st));
-  const int nb = s.bnd_ptr.empty() ? 0 : s.bnd_ptr[s.ncolours];
   cmfe::FusedArgs fa;
-  std::memset(&fa, 0, sizeof(fa));
-  fa.u_inc_ptr = h->d_u_inc_ptr;
-  fa.u_inc = h->d_u_inc;
-  fa.p_inc_ptr = h->d_p_inc_ptr;
-  fa.p_inc = h->d_p_inc;
-  fa.u_inc_row = h->d_u_inc_row;
-  fa.p_inc_row = h->d_p_inc_row;
-  fa.node_done = h->d_fuse + kFuseChunks;
-  fa.bmask = h->has_surfp && nb > 0 ? h->d_bnd_mask : nullptr;
+  if ((rc = fused_args(h, &h->d_fuse, st, &fa))) return rc;
   for (int c = 0; c < chunks; ++c) {
     fa.work = h->d_fuse + c;
     fa.g0 = (int)bounds[c];
@@ -1089,7 +1190,7 @@ std::vector<void*> shared_arrays(fe_handle h) {
   return {h->d_bnd_elems, h->d_bnd_mask, h->d_geo_dd, h->d_elem_u, h->d_elem_p, h->d_row_ptr, h->d_uu_row_ptr,
           h->d_cp_row_ptr, h->d_wu, h->d_wp, h->d_elem_table, h->d_colour_elems, h->d_tables, h->d_geo,
           h->d_gbf_u, h->d_gbf_p, h->d_gw, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc,
-          h->d_u_inc_row, h->d_p_inc_row, h->d_geo_rj};
+          h->d_u_inc_row, h->d_p_inc_row, h->d_u_pat, h->d_pat, h->d_geo_rj};
 }
 }  // namespace
 
@@ -1141,7 +1242,8 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   if ((rc = dev_upload(&h->d_bnd_elems, s.bnd_elems)) || (rc = dev_upload(&h->d_bnd_mask, s.bnd_mask))) return fail(rc);
   if ((rc = dev_upload(&h->d_u_inc_ptr, s.u_inc_ptr)) || (rc = dev_upload(&h->d_u_inc, s.u_inc)) ||
       (rc = dev_upload(&h->d_p_inc_ptr, s.p_inc_ptr)) || (rc = dev_upload(&h->d_p_inc, s.p_inc)) ||
-      (rc = dev_upload(&h->d_u_inc_row, s.u_inc_row)) || (rc = dev_upload(&h->d_p_inc_row, s.p_inc_row)))
+      (rc = dev_upload(&h->d_u_inc_row, s.u_inc_row)) || (rc = dev_upload(&h->d_p_inc_row, s.p_inc_row)) || (rc = dev_upload(&h->d_u_pat, s.u_pat)) ||
+      (rc = dev_upload(&h->d_pat, s.pat)))
     return fail(rc);
   {
     auto owner = std::make_shared<SharedDeviceSetup>();
@@ -1171,11 +1273,14 @@ int fe_destroy(fe_handle h) {
   }
   // per-handle state: materials, surface load, status word, staging and records
   void* own[] = {h->d_surfp, h->d_mat, h->d_status, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
-                 h->d_col, h->d_rec, h->d_fuse};
+                 h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64};
   for (void* p : own)
     if (p) cudaFree(p);
   for (cudaEvent_t ev : h->chunk_events)
     if (ev) cudaEventDestroy(ev);
+  if (h->order_event) cudaEventDestroy(h->order_event);
+  for (cudaEvent_t ev : h->side_events) cudaEventDestroy(ev);
+  for (cudaStream_t ss : h->side_streams) cudaStreamDestroy(ss);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   delete h;  // releases this handle's share of the mesh arrays
   return FE_NO_ERROR;
@@ -1217,6 +1322,8 @@ int fe_clone(fe_handle src, fe_handle* out) {
     h->d_p_inc_ptr = src->d_p_inc_ptr;
     h->d_p_inc = src->d_p_inc;
     h->d_u_inc_row = src->d_u_inc_row;
+    h->d_u_pat = src->d_u_pat;
+    h->d_pat = src->d_pat;
     h->d_p_inc_row = src->d_p_inc_row;
     h->high_precision = src->high_precision;
     h->assembly_order = src->assembly_order;
@@ -1395,7 +1502,9 @@ int fe_jacobian_evaluate(fe_handle h, const double* x, double* values, double* r
   kp.x = dx;
   kp.vals = dv;
   kp.r = dr;
-  if ((rc = run_colours<M_JAC>(h, kp, st))) return rc;
+  bool taken = false;
+  if ((rc = fp64_fused(h, kp, st, &taken))) return rc;
+  if (!taken && (rc = run_colours<M_JAC>(h, kp, st))) return rc;
   if (hv) CUDA_TRY(cudaMemcpyAsync(values, dv, sizeof(double) * h->hs.nnz, cudaMemcpyDeviceToHost, st));
   if (hr) CUDA_TRY(cudaMemcpyAsync(r, dr, sizeof(double) * h->hs.ndofs, cudaMemcpyDeviceToHost, st));
   if (hv || hr) return finish_status(h, st);

@@ -451,6 +451,60 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
   parallel_for((int)s.p_inc.size(),
                [&](int k) { s.p_inc_row[k] = s.elem_table[s.p_inc[k] >> 3] * nr + s.npe + (s.p_inc[k] & 7); });
 
+  // Column patterns of the u nodes' rows, shared by nodes with equal
+  // rank-table rows (a node's incidences in element order).
+  {
+    struct Seen {
+      int32_t node;  // a node with this pattern
+      int32_t next;  // next pattern with the same hash, or -1
+    };
+    std::unordered_map<uint64_t, int32_t> head;
+    std::vector<Seen> seen;
+    std::vector<int32_t> owner(s.nu);  // number of the pattern
+    auto row_of = [&](int32_t k) { return s.u_inc_row[k]; };
+    for (int n = 0; n < s.nu; ++n) {
+      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
+      uint64_t hash = 1469598103934665603ull;
+      for (int32_t j = 0; j < cnt; ++j) hash = (hash ^ (uint64_t)(uint32_t)row_of(k0 + j)) * 1099511628211ull;
+      auto it = head.emplace(hash, -1).first;
+      int32_t id = it->second;
+      for (; id >= 0; id = seen[id].next) {
+        const int32_t o0 = s.u_inc_ptr[seen[id].node];
+        bool same = s.u_inc_ptr[seen[id].node + 1] - o0 == cnt;
+        for (int32_t j = 0; same && j < cnt; ++j) same = row_of(o0 + j) == row_of(k0 + j);
+        if (same) break;
+      }
+      if (id < 0) {
+        id = (int32_t)seen.size();
+        seen.push_back({n, it->second});
+        it->second = id;
+      }
+      owner[n] = id;
+    }
+    const int pwords = 2 * s.npp;  // 4 * npp 16-bit ranks
+    std::vector<int64_t> at(seen.size() + 1, 0);
+    for (size_t i = 0; i < seen.size(); ++i) {
+      const int n = seen[i].node;
+      const int rounds = (s.u_inc_ptr[n + 1] - s.u_inc_ptr[n] + 3) / 4;
+      at[i + 1] = at[i] + (int64_t)rounds * (s.wu[n] + pwords);
+    }
+    if (at[seen.size()] >= (1ll << 31)) return fail(msg, "too many distinct node patterns");
+    s.pat.assign((size_t)at[seen.size()], 0xffffffffu);
+    parallel_for((int)seen.size(), [&](int i) {
+      const int n = seen[i].node;
+      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
+      for (int32_t j = 0; j < cnt; ++j) {
+        uint32_t* w = &s.pat[(size_t)at[i] + (size_t)(j / 4) * (s.wu[n] + pwords)];
+        const uint16_t* T = &s.tables[(size_t)row_of(k0 + j) * nr];
+        for (int b = 0; b < s.npe; ++b) reinterpret_cast<uint8_t*>(w + (T[b] & 0x7fff))[j % 4] = (uint8_t)b;
+        for (int q = 0; q < s.npp; ++q)
+          reinterpret_cast<uint16_t*>(w + s.wu[n])[(j % 4) * s.npp + q] = T[s.npe + q] & 0x7fff;
+      }
+    });
+    s.u_pat.resize(s.nu);
+    for (int n = 0; n < s.nu; ++n) s.u_pat[n] = (int32_t)at[owner[n]];
+  }
+
   // Boundary faces: a local face (reference order -xi1, -xi2, -xi3, +xi1,
   // +xi2, +xi3) whose four corner nodes no other element holds.
   {

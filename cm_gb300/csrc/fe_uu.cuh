@@ -13,14 +13,15 @@
 //   stage 1  S1[kl][a1 b1][g2 g3] = sum_g1 MM_{t1(kl)}(a1, b1; g1) D_kl(g1, g2, g3)
 //   stage 2  w[t3][g3] = sum_{kl with type t3 along xi3} sum_g2 MM_{t2(kl)}(a2, b2; g2) S1[kl][a1 b1][g2, g3]
 //   stage 3  K(a, b) = sum_t3 sum_g3 MM_{t3}(a3, b3; g3) w[t3][g3].
-// A triquadratic element takes 82 k multiply-adds this way (105 k without the
-// symmetry of the diagonal blocks) instead of the 354 k of the 81 x 81 x 81
-// product over (Gauss point, derivative) pairs, in full T precision.
+// A triquadratic element takes about 70 k multiply-adds this way instead of the
+// 354 k of the 81 x 81 x 81 product over (Gauss point, derivative) pairs, in
+// full T precision.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include "../../include/cm_fe.h"
+#include "fe_dd.cuh"
 
 namespace {
 
@@ -53,7 +54,9 @@ __device__ __forceinline__ T uu_rcbrt(T x);
 template <>
 __device__ __forceinline__ float uu_rcbrt<float>(float x) { return rcbrtf(x); }
 template <>
-__device__ __forceinline__ double uu_rcbrt<double>(double x) { return rcbrt(x); }
+__device__ __forceinline__ double uu_rcbrt<double>(double x) { return hrcbrt(x); }
+__device__ __forceinline__ bool uu_finite(float v) { return isfinite(v); }
+__device__ __forceinline__ bool uu_finite(double v) { return hfinite(v); }
 template <class T>
 __device__ __forceinline__ T uu_exp(T x);
 template <>
@@ -173,25 +176,30 @@ __device__ __forceinline__ bool uu_tangent(int law, const T* c, const T M[3][3],
       if (v < 3) t += h;
     }
   }
+  // every term of D is linear in what follows: J_z w goes in here
   const T tr = sb[0] + sb[1] + sb[2];
-  T sg[6];
+  const T jw3 = third * jw;
+  T sg[6];  // J_z w (sigma + mu/2 1), mu/2 = tr / 3 - p: the delta_mn part
+  const T mu2 = jw * (third * tr - p);
 #pragma unroll
   for (int v = 0; v < 6; ++v) {
     const T sd = v < 3 ? sb[v] - third * tr : sb[v];
-    q[v] = -third * q[v] - (two * third) * sd;
-    sg[v] = v < 3 ? sd + p : sd;
+    q[v] = -jw3 * (q[v] + two * sd);
+    sg[v] = v < 3 ? jw * (sd + p) + mu2 : jw * sd;
   }
-  const T kap = t * T(1.0 / 9.0) - T(2.0 / 9.0) * tr + p;
-  const T mu2 = third * tr - p;  // mu / 2
-  T r[3][3], rho[3][3], b[3][3], sG[3][3];
+  const T kap = jw * (t * T(1.0 / 9.0) - T(2.0 / 9.0) * tr + p);
+  e0 = jw * e0;
+#pragma unroll
+  for (int v = 0; v < 6; ++v) eb[v] = jw * eb[v];
+  T r[3][3], rho[3][3], b[3][3], sG[3][3], mG[3][3], ob[3][3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     r[k][0] = q[0] * G[k][0] + q[3] * G[k][1] + q[4] * G[k][2];
     r[k][1] = q[3] * G[k][0] + q[1] * G[k][1] + q[5] * G[k][2];
     r[k][2] = q[4] * G[k][0] + q[5] * G[k][1] + q[2] * G[k][2];
-    sG[k][0] = sg[0] * G[k][0] + sg[3] * G[k][1] + sg[4] * G[k][2] + mu2 * G[k][0];
-    sG[k][1] = sg[3] * G[k][0] + sg[1] * G[k][1] + sg[5] * G[k][2] + mu2 * G[k][1];
-    sG[k][2] = sg[4] * G[k][0] + sg[5] * G[k][1] + sg[2] * G[k][2] + mu2 * G[k][2];
+    sG[k][0] = sg[0] * G[k][0] + sg[3] * G[k][1] + sg[4] * G[k][2];
+    sG[k][1] = sg[3] * G[k][0] + sg[1] * G[k][1] + sg[5] * G[k][2];
+    sG[k][2] = sg[4] * G[k][0] + sg[5] * G[k][1] + sg[2] * G[k][2];
     if (law == FE_LAW_MOONEY_RIVLIN) {
 #pragma unroll
       for (int m = 0; m < 3; ++m) b[k][m] = F[m][0] * f[k][0] + F[m][1] * f[k][1] + F[m][2] * f[k][2];
@@ -201,27 +209,35 @@ __device__ __forceinline__ bool uu_tangent(int law, const T* c, const T M[3][3],
       b[k][2] = Bv[4] * G[k][0] + Bv[5] * G[k][1] + Bv[2] * G[k][2];
     }
 #pragma unroll
-    for (int m = 0; m < 3; ++m) rho[k][m] = r[k][m] + kap * G[k][m];
+    for (int m = 0; m < 3; ++m) {
+      mG[k][m] = mu2 * G[k][m];
+      rho[k][m] = r[k][m] + kap * G[k][m];
+      ob[k][m] = e0 * b[k][m];
+    }
   }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 3; ++k)
 #pragma unroll
     for (int l = 0; l < 3; ++l) {
-      const T iso = G[l][0] * sG[k][0] + G[l][1] * sG[k][1] + G[l][2] * sG[k][2];  // delta_mn part
-      T bkl = T(0);  // MR: dxi_k/dz . B_bar . dxi_l/dz
-      if (law == FE_LAW_MOONEY_RIVLIN) bkl = -half * e0 * (G[l][0] * b[k][0] + G[l][1] * b[k][1] + G[l][2] * b[k][2]);
+      // delta_mn part, and MR's -e0/2 (dxi_k/dz . B_bar . dxi_l/dz) B_bar
+      const T iso = G[l][0] * sG[k][0] + G[l][1] * sG[k][1] + G[l][2] * sG[k][2];
+      T bkl = T(0);
+      if (law == FE_LAW_MOONEY_RIVLIN) bkl = -half * (G[l][0] * ob[k][0] + G[l][1] * ob[k][1] + G[l][2] * ob[k][2]);
 #pragma unroll
       for (int blk = 0; blk < 6; ++blk) {
         if (blk < 3 && k > l) continue;
         const int m = blk < 3 ? blk : (blk == 3 ? 1 : 2), n = blk < 3 ? blk : (blk == 5 ? 1 : 0);
-        T v = G[k][m] * rho[l][n] + r[k][m] * G[l][n] + mu2 * G[k][n] * G[l][m];
-        v += e0 * (b[k][m] * b[l][n]);
+        T v = G[k][m] * rho[l][n] + r[k][m] * G[l][n] + mG[k][n] * G[l][m];
         if (law == FE_LAW_MOONEY_RIVLIN) {
-          v -= half * e0 * (b[k][n] * b[l][m]);
           const int vm = m == n ? m : (m + n == 1 ? 3 : (m + n == 2 ? 4 : 5));
           v += bkl * Bv[vm];
+          if (m == n)
+            v += (half * ob[k][m]) * b[l][m];
+          else
+            v += ob[k][m] * b[l][n] - (half * ob[k][n]) * b[l][m];
         } else {
+          v += ob[k][m] * b[l][n];
 #pragma unroll
           for (int u = 0; u < 6; ++u) {
             const int I = V0[u], J2 = V1[u];
@@ -234,8 +250,7 @@ __device__ __forceinline__ bool uu_tangent(int law, const T* c, const T M[3][3],
           }
         }
         if (m == n) v += iso;
-        v *= jw;
-        if (blk == 0 && k == l) ok = ok && isfinite(v);
+        if (blk == 0 && k == l) ok = ok && uu_finite(v);
         rec[uu_slot(blk, k, l)] = v;
       }
     }
@@ -423,17 +438,37 @@ __device__ __forceinline__ void uu_warp_task(const T* s_D, const T* s_mm, T* s1,
     }
 #pragma unroll
     for (int j = 0; j < JW; ++j) {
-      T K[N1][N1];
+      // stage 3 in even and odd combinations: the reflection of xi3 takes
+      // (a3, b3) to (N1 - 1 - a3, N1 - 1 - b3) and changes the sign of the
+      // types with one derivative, so the entries come in pairs P + Q, P - Q
+      T K[N1][N1], e[4], o[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        e[t] = w[j][t][0] + w[j][t][2];
+        o[t] = w[j][t][0] - w[j][t][2];
+      }
 #pragma unroll
       for (int a3 = 0; a3 < N1; ++a3)
 #pragma unroll
         for (int b3 = 0; b3 < N1; ++b3) {
-          T v = T(0);
+          const int ma = N1 - 1 - a3, mb = N1 - 1 - b3;
+          if (ma * N1 + mb < a3 * N1 + b3) continue;
+          T P = T(0), Q = T(0);
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-#pragma unroll
-            for (int g = 0; g < 3; ++g) v += T(uu_mm(N1, t, a3, b3, g)) * w[j][t][g];
-          K[a3][b3] = v;
+          for (int t = 0; t < 4; ++t) {
+            const double m0 = uu_mm(N1, t, a3, b3, 0), m1 = uu_mm(N1, t, a3, b3, 1), m2 = uu_mm(N1, t, a3, b3, 2);
+            const double me = 0.5 * (m0 + m2), mo = 0.5 * (m0 - m2);
+            T& E = t == 0 || t == 3 ? P : Q;
+            T& O = t == 0 || t == 3 ? Q : P;
+            const bool self = ma == a3 && mb == b3;
+            if (!(self && (t == 1 || t == 2))) {
+              E += T(me) * e[t];
+              if (m1 != 0.0) E += T(m1) * w[j][t][1];
+            }
+            if (!(self && (t == 0 || t == 3))) O += T(mo) * o[t];
+          }
+          K[a3][b3] = P + Q;
+          if (ma != a3 || mb != b3) K[ma][mb] = P - Q;
         }
       if (work) out(el, blk, a1 + N1 * a2[j0 + j], b1 + N1 * b2[j0 + j], K);
     }
