@@ -16,6 +16,16 @@
 // sum, so a solve is bit-identical from run to run.  The host drives the
 // iteration; it reads one small array per GMRES iteration (the new
 // Hessenberg column) to update the Givens rotations.
+//
+// On the meshes this solver suits (its preconditioner is diagonal) a GMRES
+// iteration is a handful of vectors of a few thousand entries, bound by
+// launches and by the latency of FP64 reductions.  So an iteration is four
+// launches: dots, update with the second pass's dots, update with the norm,
+// the preconditioning and the Hessenberg column, matrix-vector product with
+// the scaling; a block owns a chunk of rows and its warps take different basis vectors, so
+// no dot waits on a block-wide reduction, and the sums over the at most 64
+// chunks are formed by the kernel that uses them.  The next iteration is queued
+// before the host waits for a column.
 #include "fe_internal.h"
 
 #include <cuda_runtime.h>
@@ -30,26 +40,60 @@
 namespace {
 
 constexpr int NT = 256;
-constexpr int RED_BLOCKS = 304;  // partial sums per reduction: two per SM
+constexpr int NWARP = NT / 32;
+constexpr int MAX_CHUNKS = 64;  // row chunks of a reduction: one block each
 
-// y = P A P x on the free dofs (P: the free-dof mask), 0 on the fixed ones;
-// one warp per row, lanes over the row's entries, a fixed shuffle tree.
-__global__ void k_spmv(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                       const double* __restrict__ val, const uint8_t* __restrict__ free_dof,
-                       const double* __restrict__ x, double* __restrict__ y) {
+// y = P A x on the free rows (P: the free-dof mask), 0 on the fixed ones, for
+// x zero on the fixed dofs; with scale: y and v scaled by *scale.  One warp
+// takes two rows, lanes over the entries, and reduces both with five
+// additions instead of ten: the FP64 pipe (19 cycles of an SM per warp
+// instruction) and two waits for memory bind it.  A row of a triquadratic box
+// has 100 to 400 entries; eight a lane are loaded at once.
+__global__ void __launch_bounds__(NT) k_spmv(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                             const double* __restrict__ val, const uint8_t* __restrict__ free_dof,
+                                             const double* __restrict__ x, double* __restrict__ y,
+                                             const double* __restrict__ scale, double* __restrict__ v) {
   const int lane = threadIdx.x & 31;
+  const double sc = scale ? *scale : 1.0;
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw) {
-    double s = 0.0;
-    if (free_dof[i]) {
-      for (int64_t j = rp[i] + lane; j < rp[i + 1]; j += 32) {
-        const int c = col[j];
-        if (free_dof[c]) s = fma(val[j], x[c], s);
+  for (int64_t i = 2 * ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); i < n; i += 2 * nw) {
+    double s[2] = {0.0, 0.0};
+    int at[2], end[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const bool in = i + r < n && free_dof[i + r];
+      at[r] = in ? rp[i + r] + lane : 0;
+      end[r] = in ? rp[i + r + 1] : 0;
+    }
+    while (__any_sync(0xffffffffu, at[0] < end[0] || at[1] < end[1])) {
+      double a[2][8];
+      int c[2][8];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool in = at[r] + 32 * u < end[r];
+          a[r][u] = in ? val[at[r] + 32 * u] : 0.0;
+          c[r][u] = in ? col[at[r] + 32 * u] : 0;
+        }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (at[r] + 32 * u < end[r]) s[r] = fma(a[r][u], x[c[r][u]], s[r]);
+        at[r] += 256;
       }
     }
+    // lanes 0..15 go on with the first row, 16..31 with the second
+    const bool hi = lane & 16;
+    double t = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) y[i] = s;
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const int64_t row = i + (hi ? 1 : 0);
+    if ((lane & 15) == 0 && row < n) {
+      y[row] = scale ? sc * t : t;
+      if (scale) v[row] *= sc;
+    }
   }
 }
 
@@ -97,59 +141,176 @@ __global__ void k_precond(int64_t n, int64_t nu3, const int32_t* __restrict__ rp
   }
 }
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sh[k];
-  return t;  // valid in thread 0
+  return v;  // valid in lane 0
 }
 
-// part[j * gridDim.x + b] = block b's share of V_j . w for j < m (V row-major,
-// leading dimension ld); with V = w and m = 1 it is the squared norm.
-__global__ void k_mdot_part(int64_t n, const double* __restrict__ V, int64_t ld, int m, const double* __restrict__ w,
-                            double* __restrict__ part) {
-  __shared__ double sh[NT / 32];
-  for (int j = 0; j < m; ++j) {
+// Chunk blockIdx.x of gridDim.x of the rows: [r0, r1).
+__device__ __forceinline__ void chunk_rows(int64_t n, int64_t& r0, int64_t& r1) {
+  const int64_t len = (n + gridDim.x - 1) / gridDim.x;
+  r0 = blockIdx.x * len;
+  r1 = r0 + len < n ? r0 + len : n;
+}
+
+// part[j * gridDim.x + chunk] = the chunk's share of V_j . w, j < m (V
+// row-major, leading dimension ld), each by one warp.
+__device__ __forceinline__ void chunk_dots(int64_t r0, int64_t r1, const double* __restrict__ V, int64_t ld, int m,
+                                           const double* w, double* __restrict__ part) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int j = warp; j < m; j += NWARP) {
     double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-      s = fma(V[j * ld + i], w[i], s);
-    const double t = block_sum(s, sh);
-    if (threadIdx.x == 0) part[j * gridDim.x + blockIdx.x] = t;
+    const double* v = V + j * ld;
+#pragma unroll 4
+    for (int64_t i = r0 + lane; i < r1; i += 32) s = fma(v[i], w[i], s);
+    s = warp_sum(s);
+    if (lane == 0) part[j * (int)gridDim.x + blockIdx.x] = s;
   }
 }
 
-// out[j] = sum_b part[j * nb + b], one block per j.
-__global__ void k_mdot_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  __shared__ double sh[NT / 32];
+// Sum of v over each group of G neighbouring lanes (G a power of two), in
+// every lane of the group, by a fixed tree.
+template <int G>
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// h[j] = sum of the chunks' shares for j < m (shared memory): eight lanes to a
+// j, as a chain of FP64 additions waits 64 cycles for each.
+__device__ __forceinline__ void sum_parts(const double* __restrict__ part, int m, double* h) {
+  const int q = threadIdx.x & 7;
+  for (int j0 = 0; j0 < m; j0 += NT / 8) {
+    const int j = j0 + (threadIdx.x >> 3);
+    double s = 0.0;
+    if (j < m)
+      for (int c = q; c < (int)gridDim.x; c += 8) s += part[j * (int)gridDim.x + c];
+    s = group_sum<8>(s);
+    if (j < m && q == 0) h[j] = s;
+  }
+}
+
+constexpr int MAX_BASIS = 208;  // restart limit 200 and a few
+
+// Dots of m vectors with w; V = w and m = 1 give the squared norm.
+__global__ void __launch_bounds__(NT) k_dots(int64_t n, const double* __restrict__ V, int64_t ld, int m,
+                                             const double* __restrict__ w, double* __restrict__ part) {
+  int64_t r0, r1;
+  chunk_rows(n, r0, r1);
+  chunk_dots(r0, r1, V, ld, m, w, part);
+}
+
+// *out = sum over the chunks (one block of one warp).
+__global__ void k_sum(const double* __restrict__ part, int chunks, double* __restrict__ out) {
   double s = 0.0;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) s += part[blockIdx.x * nb + b];
-  const double t = block_sum(s, sh);
-  if (threadIdx.x == 0) out[blockIdx.x] = t;
+  for (int c = threadIdx.x; c < chunks; c += 32) s += part[c];
+  s = warp_sum(s);
+  if (threadIdx.x == 0) *out = s;
 }
 
-// w -= sum_{j < m} h[j] V_j, and acc[j] += h[j] (first thread) when acc is set.
-__global__ void k_gs_update(int64_t n, const double* __restrict__ V, int64_t ld, int m, const double* __restrict__ h,
-                            double* __restrict__ w, double* __restrict__ acc) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double s = w[i];
-    for (int j = 0; j < m; ++j) s = fma(-h[j], V[j * ld + i], s);
-    w[i] = s;
+// w -= sum_j h[j] V_j on the block's chunk (and z = minv .* w): four lanes to a
+// row.  Returns this thread's share of the new w's squared norm.
+__device__ __forceinline__ double chunk_update(int64_t r0, int64_t r1, const double* __restrict__ V, int64_t ld, int m,
+                                               const double* h, double* w, const double* __restrict__ minv = nullptr,
+                                               double* __restrict__ z = nullptr) {
+  const int q = threadIdx.x & 3;
+  double nrm = 0.0;
+  for (int64_t b = r0; b < r1; b += NT / 4) {
+    const int64_t i = b + (threadIdx.x >> 2);
+    double s = 0.0;
+    if (i < r1) {
+#pragma unroll 8
+      for (int j = q; j < m; j += 4) s = fma(h[j], V[j * ld + i], s);
+    }
+    s = group_sum<4>(s);
+    if (i < r1 && q == 0) {
+      const double t = w[i] - s;
+      w[i] = t;
+      if (z) z[i] = minv[i] * t;
+      nrm = fma(t, t, nrm);
+    }
   }
-  if (acc && blockIdx.x == 0 && threadIdx.x < m) acc[threadIdx.x] += h[threadIdx.x];
+  return nrm;
 }
 
-// y = a * x, or y = x / sqrt(*den) when den is set (0 when *den is 0: an
-// Arnoldi breakdown, after which the vector is not used).
-__global__ void k_scale(int64_t n, double a, const double* __restrict__ den, const double* x, double* y) {
-  const double s = den ? (*den > 0.0 ? 1.0 / sqrt(*den) : 0.0) : a;
+// First Gram-Schmidt update and the second pass's dots.  col[j] = h[j].
+__global__ void __launch_bounds__(NT) k_update_dots(int64_t n, const double* __restrict__ V, int64_t ld, int m,
+                                                    const double* __restrict__ part, double* w, double* __restrict__ col,
+                                                    double* __restrict__ part2) {
+  __shared__ double h[MAX_BASIS];
+  int64_t r0, r1;
+  chunk_rows(n, r0, r1);
+  sum_parts(part, m, h);
+  __syncthreads();
+  chunk_update(r0, r1, V, ld, m, h, w);
+  if (blockIdx.x == 0)
+    for (int j = threadIdx.x; j < m; j += NT) col[j] = h[j];
+  __syncthreads();
+  chunk_dots(r0, r1, V, ld, m, w, part2);
+}
+
+// Second Gram-Schmidt update, the result preconditioned (z = minv .* w), and
+// its squared norm.  The last block to finish writes the Hessenberg column to
+// the host (page-locked memory): col[j] + h[j], and the squared norm; col[m] =
+// 1 / norm (0 when it is 0: an Arnoldi breakdown, after which the vector is
+// not used).
+__global__ void __launch_bounds__(NT) k_update_norm(int64_t n, const double* __restrict__ V, int64_t ld, int m,
+                                                    const double* __restrict__ part2, double* w, double* __restrict__ col,
+                                                    double* __restrict__ npart, int* __restrict__ done,
+                                                    const double* __restrict__ minv, double* __restrict__ z, double* host) {
+  __shared__ double h[MAX_BASIS];
+  __shared__ double sh[NWARP];
+  __shared__ bool last;
+  int64_t r0, r1;
+  chunk_rows(n, r0, r1);
+  sum_parts(part2, m, h);
+  __syncthreads();
+  const double s = warp_sum(chunk_update(r0, r1, V, ld, m, h, w, minv, z));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    double t = sh[threadIdx.x];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffu, t, o);
+    if (threadIdx.x == 0) {
+      npart[blockIdx.x] = t;
+      __threadfence();
+      last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int j = threadIdx.x; j < m; j += NT) host[j] = col[j] + h[j];
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    for (int c = threadIdx.x; c < (int)gridDim.x; c += 32) t += __ldcg(npart + c);
+    t = warp_sum(t);
+    if (threadIdx.x == 0) {
+      host[m] = t;
+      col[m] = t > 0.0 ? 1.0 / sqrt(t) : 0.0;
+      *done = 0;
+    }
+  }
+}
+
+// v = a * x, z = minv .* v
+__global__ void __launch_bounds__(NT) k_scale_precond(int64_t n, double a, const double* __restrict__ minv,
+                                                      const double* __restrict__ x, double* __restrict__ v,
+                                                      double* __restrict__ z) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double t = a * x[i];
+    v[i] = t;
+    z[i] = minv[i] * t;
+  }
+}
+
+// y = a * x
+__global__ void k_scale(int64_t n, double a, const double* x, double* y) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = s * x[i];
+    y[i] = a * x[i];
 }
 
 // y = a * x + b * y
@@ -158,19 +319,15 @@ __global__ void k_axpby(int64_t n, double a, const double* __restrict__ x, doubl
     y[i] = a * x[i] + b * y[i];
 }
 
-// z = minv .* v
-__global__ void k_precond_apply(int64_t n, const double* __restrict__ minv, const double* __restrict__ v,
-                                double* __restrict__ z) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    z[i] = minv[i] * v[i];
-}
-
-// x += sum_{j < m} y[j] Z_j
-__global__ void k_combine(int64_t n, const double* __restrict__ Z, int64_t ld, int m, const double* __restrict__ y,
-                          double* __restrict__ x) {
+// x += sum_{j < m} y[j] (minv .* V_j)
+__global__ void __launch_bounds__(NT) k_combine(int64_t n, const double* __restrict__ V, int64_t ld, int m,
+                                                const double* __restrict__ minv, const double* __restrict__ y,
+                                                double* __restrict__ x) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double s = x[i];
-    for (int j = 0; j < m; ++j) s = fma(y[j], Z[j * ld + i], s);
+    const double mi = minv[i];
+#pragma unroll 8
+    for (int j = 0; j < m; ++j) s = fma(y[j], mi * V[j * ld + i], s);
     x[i] = s;
   }
 }
@@ -195,6 +352,7 @@ int blocks_for(int64_t n) {
   return (int)(b < 4096 ? (b < 1 ? 1 : b) : 4096);
 }
 
+// Blocks for one row per warp, and for k_spmv's two.
 int warp_blocks_for(int64_t n) {
   const int64_t b = (n + (NT / 32) - 1) / (NT / 32);
   return (int)(b < 8192 ? (b < 1 ? 1 : b) : 8192);
@@ -206,21 +364,39 @@ int warp_blocks_for(int64_t n) {
     if (e_ != cudaSuccess) return cmfe::record_error(FE_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-// Device work space of one call, freed on scope exit.
+// Device work space of one call in one allocation, freed on scope exit: the
+// arrays are announced with add() and placed by alloc().
 struct Work {
-  std::vector<void*> ptrs;
+  struct Slot {
+    void** p;
+    size_t at;
+  };
+  std::vector<Slot> slots;
+  size_t bytes = 0;
+  void* base = nullptr;
+  double* pinned = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
   ~Work() {
-    for (void* p : ptrs) cudaFree(p);
+    if (base) cudaFree(base);
+    if (pinned) cudaFreeHost(pinned);
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
   }
   template <class T>
-  int alloc(T** p, size_t count) {
-    *p = nullptr;
-    const cudaError_t e = cudaMalloc(p, count * sizeof(T) + 16);
+  void add(T** p, size_t count) {
+    slots.push_back({reinterpret_cast<void**>(p), bytes});
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+  }
+  int alloc(size_t host_doubles) {
+    cudaError_t e = cudaMalloc(&base, bytes);
+    if (e == cudaSuccess) e = cudaMallocHost(&pinned, host_doubles * sizeof(double));
+    for (cudaEvent_t& v : ev)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return cmfe::record_error(FE_ERR_OUT_OF_MEMORY, std::string("Newton work space: ") + cudaGetErrorString(e));
     }
-    ptrs.push_back(*p);
+    for (const Slot& s : slots) *s.p = static_cast<char*>(base) + s.at;
     return FE_NO_ERROR;
   }
 };
@@ -230,29 +406,38 @@ struct Solver {
   cudaStream_t st;
   int64_t n, nnz, nu3;
   const int32_t *rp, *col;
-  double *vals, *r, *rn, *d, *xs, *w, *minv, *diag, *V, *Z, *hbuf, *part, *scal;
+  double *vals, *r, *rn, *d, *xs, *w, *minv, *diag, *V, *z, *col_d, *part, *part2, *npart, *scal;
+  int* done;
   uint8_t* free_dof;
-  int restart;
+  double* pinned;   // page-locked: the Hessenberg column, and single sums
+  const cudaEvent_t* ev;  // two: the columns' copies
+  int restart, chunks;
+  std::vector<cudaGraphExec_t> graphs;  // iteration k of a cycle
+  cudaStream_t capture = nullptr;
+  int64_t cycles = 0;
+  bool no_graphs = false;
 
-  int spmv(const double* x, double* y) {
-    k_spmv<<<warp_blocks_for(n), NT, 0, st>>>(n, rp, col, vals, free_dof, x, y);
-    NT_TRY(cudaGetLastError());
-    return FE_NO_ERROR;
+  Solver() = default;
+  Solver(const Solver&) = delete;
+  ~Solver() {
+    for (cudaGraphExec_t g : graphs)
+      if (g) cudaGraphExecDestroy(g);
+    if (capture) cudaStreamDestroy(capture);
   }
 
-  // out[0..m) = V_j . w on the device
-  int mdot(const double* Vm, int m, const double* wv, double* out) {
-    k_mdot_part<<<RED_BLOCKS, NT, 0, st>>>(n, Vm, n, m, wv, part);
-    k_mdot_final<<<m, NT, 0, st>>>(part, RED_BLOCKS, out);
+  int spmv(const double* x, double* y) {
+    k_spmv<<<warp_blocks_for((n + 1) / 2), NT, 0, st>>>(n, rp, col, vals, free_dof, x, y, nullptr, nullptr);
     NT_TRY(cudaGetLastError());
     return FE_NO_ERROR;
   }
 
   int dot_host(const double* a, const double* b, double* out) {
-    int rc = mdot(a, 1, b, scal);
-    if (rc) return rc;
-    NT_TRY(cudaMemcpyAsync(out, scal, sizeof(double), cudaMemcpyDeviceToHost, st));
+    k_dots<<<chunks, NT, 0, st>>>(n, a, n, 1, b, npart);
+    k_sum<<<1, 32, 0, st>>>(npart, chunks, scal);
+    NT_TRY(cudaGetLastError());
+    NT_TRY(cudaMemcpyAsync(pinned, scal, sizeof(double), cudaMemcpyDeviceToHost, st));
     NT_TRY(cudaStreamSynchronize(st));
+    *out = *pinned;
     return FE_NO_ERROR;
   }
 
@@ -273,6 +458,54 @@ struct Solver {
     return FE_NO_ERROR;
   }
 
+  // GMRES iteration k on the stream t: orthogonalise V_{k+1} (holding
+  // A M^-1 v_k), its Hessenberg column to the host, then scale it and form the
+  // next product.
+  int iteration_kernels(int k, cudaStream_t t) {
+    const int m = k + 1;
+    double* wv = V + (size_t)m * n;
+    double* cd = col_d + (size_t)(k & 1) * (restart + 2);
+    // classical Gram-Schmidt, twice
+    k_dots<<<chunks, NT, 0, t>>>(n, V, n, m, wv, part);
+    k_update_dots<<<chunks, NT, 0, t>>>(n, V, n, m, part, wv, cd, part2);
+    k_update_norm<<<chunks, NT, 0, t>>>(n, V, n, m, part2, wv, cd, npart, done, minv, z,
+                                        pinned + (size_t)(k & 1) * (restart + 2));
+    if (m < restart)
+      k_spmv<<<warp_blocks_for((n + 1) / 2), NT, 0, t>>>(n, rp, col, vals, free_dof, z, V + (size_t)(m + 1) * n, cd + m, wv);
+    NT_TRY(cudaGetLastError());
+    return FE_NO_ERROR;
+  }
+
+  // The same, from the second cycle on as one graph launch: single launches
+  // from the host take longer than the work of a few thousand rows.
+  // The buffers stay the same over the whole load step; a graph is recorded
+  // when its iteration comes up again.
+  int queue_iteration(int k) {
+    if (cycles > 0 && !graphs[k] && !no_graphs) {
+      cudaGraph_t g = nullptr;
+      bool ok = cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+      if (ok) {
+        const int rc = iteration_kernels(k, capture);
+        ok = cudaStreamEndCapture(capture, &g) == cudaSuccess && rc == FE_NO_ERROR;
+      }
+      ok = ok && cudaGraphInstantiate(&graphs[k], g, 0) == cudaSuccess;
+      if (g) cudaGraphDestroy(g);
+      if (!ok) {
+        cudaGetLastError();
+        graphs[k] = nullptr;
+        no_graphs = true;
+      }
+    }
+    if (graphs[k]) {
+      NT_TRY(cudaGraphLaunch(graphs[k], st));
+    } else {
+      const int rc = iteration_kernels(k, st);
+      if (rc) return rc;
+    }
+    NT_TRY(cudaEventRecord(ev[k & 1], st));
+    return FE_NO_ERROR;
+  }
+
   // Right-preconditioned GMRES(restart) for A dx = b (b on free dofs, dx
   // zero on fixed ones); returns the iterations in *its.
   int gmres(const double* b, double* dx, double rtol, int max_it, int64_t* its) {
@@ -290,28 +523,20 @@ struct Solver {
     std::vector<double> col_h(restart + 2);
     while (*its < max_it) {
       if (beta <= rtol * bnorm) break;
-      k_scale<<<blocks_for(n), NT, 0, st>>>(n, 1.0 / beta, nullptr, res, V);
       std::fill(g.begin(), g.end(), 0.0);
       g[0] = beta;
       int k = 0;
-      bool done = false;
+      bool done_it = false;
+      k_scale_precond<<<blocks_for(n), NT, 0, st>>>(n, 1.0 / beta, minv, res, V, z);
+      if ((rc = spmv(z, V + n))) return rc;
+      int queued = 0;  // iterations queued: one ahead of the column the host waits for
       while (k < restart && *its < max_it) {
-        double* vk = V + (size_t)k * n;
-        double* zk = Z + (size_t)k * n;
-        double* wv = V + (size_t)(k + 1) * n;
-        k_precond_apply<<<blocks_for(n), NT, 0, st>>>(n, minv, vk, zk);
-        if ((rc = spmv(zk, wv))) return rc;
-        // classical Gram-Schmidt, twice; hbuf[0..k] accumulates the column
-        NT_TRY(cudaMemsetAsync(hbuf, 0, sizeof(double) * (restart + 2), st));
-        for (int pass = 0; pass < 2; ++pass) {
-          if ((rc = mdot(V, k + 1, wv, hbuf + restart + 2))) return rc;
-          k_gs_update<<<blocks_for(n), NT, 0, st>>>(n, V, n, k + 1, hbuf + restart + 2, wv, hbuf);
+        for (; queued < restart && queued <= k + 1 && *its + (queued - k) < max_it; ++queued) {
+          if ((rc = queue_iteration(queued))) return rc;
         }
-        if ((rc = mdot(wv, 1, wv, hbuf + k + 1))) return rc;  // squared norm
-        k_scale<<<blocks_for(n), NT, 0, st>>>(n, 0.0, hbuf + k + 1, wv, wv);
-        NT_TRY(cudaGetLastError());
-        NT_TRY(cudaMemcpyAsync(col_h.data(), hbuf, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
-        NT_TRY(cudaStreamSynchronize(st));
+        NT_TRY(cudaEventSynchronize(ev[k & 1]));
+        const double* hc = pinned + (size_t)(k & 1) * (restart + 2);
+        std::copy(hc, hc + k + 2, col_h.begin());
         col_h[k + 1] = std::sqrt(col_h[k + 1]);
         // apply the previous rotations, then a new one that zeroes H[k+1][k]
         for (int i = 0; i < k; ++i) {
@@ -330,7 +555,7 @@ struct Solver {
         ++k;
         ++*its;
         if (std::fabs(g[k]) <= rtol * bnorm || bb <= 1e-14 * beta) {
-          done = true;
+          done_it = true;
           break;
         }
       }
@@ -341,15 +566,16 @@ struct Solver {
         const double hii = H[(size_t)i * restart + i];
         y[i] = hii != 0.0 ? s / hii : 0.0;
       }
-      NT_TRY(cudaMemcpyAsync(hbuf, y.data(), sizeof(double) * k, cudaMemcpyHostToDevice, st));
-      k_combine<<<blocks_for(n), NT, 0, st>>>(n, Z, n, k, hbuf, dx);
+      NT_TRY(cudaMemcpyAsync(col_d, y.data(), sizeof(double) * k, cudaMemcpyHostToDevice, st));
+      k_combine<<<blocks_for(n), NT, 0, st>>>(n, V, n, k, minv, col_d, dx);
       // true residual of the cycle
       if ((rc = spmv(dx, res))) return rc;
       k_axpby<<<blocks_for(n), NT, 0, st>>>(n, 1.0, b, -1.0, res);
       double r2 = 0.0;
       if ((rc = dot_host(res, res, &r2))) return rc;
       beta = std::sqrt(r2);
-      if (done && beta <= rtol * bnorm) break;
+      ++cycles;
+      if (done_it && beta <= rtol * bnorm) break;
     }
     return FE_NO_ERROR;
   }
@@ -396,13 +622,26 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   double *dx_state, *fvals;
   int32_t* fdofs;
   const size_t rs = (size_t)S.restart;
-  if ((rc = W.alloc(&S.vals, (size_t)S.nnz)) || (rc = W.alloc(&S.r, n)) || (rc = W.alloc(&S.rn, n)) ||
-      (rc = W.alloc(&S.d, n)) || (rc = W.alloc(&S.xs, n)) || (rc = W.alloc(&S.w, n)) || (rc = W.alloc(&S.minv, n)) ||
-      (rc = W.alloc(&S.diag, n)) || (rc = W.alloc(&S.V, (rs + 1) * n)) || (rc = W.alloc(&S.Z, rs * n)) ||
-      (rc = W.alloc(&S.hbuf, 2 * rs + 4)) || (rc = W.alloc(&S.part, (rs + 2) * RED_BLOCKS)) ||
-      (rc = W.alloc(&S.scal, 4)) || (rc = W.alloc(&S.free_dof, n)) || (rc = W.alloc(&dx_state, n)) ||
-      (rc = W.alloc(&fvals, num_fixed > 0 ? num_fixed : 1)) || (rc = W.alloc(&fdofs, num_fixed > 0 ? num_fixed : 1)))
-    return rc;
+  const size_t basis = rs + 1;
+  int64_t chunks = (n + 63) / 64;
+  S.chunks = (int)(chunks < MAX_CHUNKS ? chunks : MAX_CHUNKS);
+  W.add(&S.vals, (size_t)S.nnz);
+  for (double** p : {&S.r, &S.rn, &S.d, &S.xs, &S.w, &S.minv, &S.diag, &S.z, &dx_state}) W.add(p, (size_t)n);
+  W.add(&S.V, (basis + 1) * n);
+  W.add(&S.col_d, 2 * (rs + 2));
+  W.add(&S.part, (basis + 1) * MAX_CHUNKS);
+  W.add(&S.part2, (basis + 1) * MAX_CHUNKS);
+  W.add(&S.npart, MAX_CHUNKS);
+  W.add(&S.scal, 4);
+  W.add(&S.done, 4);
+  W.add(&S.free_dof, (size_t)n);
+  W.add(&fvals, num_fixed > 0 ? num_fixed : 1);
+  W.add(&fdofs, num_fixed > 0 ? num_fixed : 1);
+  if ((rc = W.alloc(2 * (rs + 2)))) return rc;
+  S.graphs.assign(rs, nullptr);
+  S.no_graphs = cudaStreamCreateWithFlags(&S.capture, cudaStreamNonBlocking) != cudaSuccess;
+  S.pinned = W.pinned;
+  S.ev = W.ev;
   cudaStream_t st = S.st;
   // the state on the device (x may be host memory)
   cudaPointerAttributes pa;
@@ -414,6 +653,7 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   double* xd = host_x ? dx_state : x;
   if (host_x) NT_TRY(cudaMemcpyAsync(xd, x, sizeof(double) * n, cudaMemcpyHostToDevice, st));
   NT_TRY(cudaMemsetAsync(S.free_dof, 1, n, st));
+  NT_TRY(cudaMemsetAsync(S.done, 0, sizeof(int), st));
   if (num_fixed > 0) {
     NT_TRY(cudaMemcpyAsync(fdofs, fixed_dofs, sizeof(int32_t) * num_fixed, cudaMemcpyHostToDevice, st));
     NT_TRY(cudaMemcpyAsync(fvals, fixed_values, sizeof(double) * num_fixed, cudaMemcpyHostToDevice, st));
@@ -461,7 +701,7 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
     report->linear_iterations += lits;
     double dn2 = 0.0;
     if ((rc = S.dot_host(S.d, S.d, &dn2))) return finish(rc);
-    if (std::sqrt(dn2) > o.max_step) k_scale<<<blocks_for(n), NT, 0, st>>>(n, o.max_step / std::sqrt(dn2), nullptr, S.d, S.d);
+    if (std::sqrt(dn2) > o.max_step) k_scale<<<blocks_for(n), NT, 0, st>>>(n, o.max_step / std::sqrt(dn2), S.d, S.d);
     // slope of f = 1/2 ||r||^2 along d: r . (A d)
     if ((rc = S.spmv(S.d, S.w))) return finish(rc);
     double slope = 0.0;
