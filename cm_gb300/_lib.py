@@ -109,6 +109,9 @@ SIGNATURES = {
     "fe_batch_launch_count": [_vp, C.POINTER(_i64)],
     # include/cm_warmstart.h
     "ws_gemm_f32": [_i32, _i32, _i32, _vp, _i64, _i64, _vp, _i64, _i64, _vp, _i64, C.c_float, _vp],
+    "ws_linear_f32": [_i32, _i32, _i32, _vp, _vp, _vp, _i32, _vp, _vp],
+    "ws_mlp_workspace": [_i32, _i32, _vp],
+    "ws_mlp_loss_grad": [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "ws_bias_act": [_vp, _vp, _i32, _i32, _i32, _vp],
     "ws_act_backward": [_vp, _vp, _vp, _i64, _i32, _vp],
     "ws_column_sum": [_vp, _vp, _i32, _i32, _vp],
@@ -120,9 +123,12 @@ SIGNATURES = {
 
 # Functions of the C ABI that return nothing.
 VOID_FUNCTIONS = {"fe_newton_options_default"}
+# Functions that return a size.
+SIZE_FUNCTIONS = {"ws_mlp_workspace"}
 
 WS_ACT_IDENTITY = 0
 WS_ACT_TANH = 1
+WS_MAX_LAYERS = 8
 
 _lib = None
 
@@ -141,7 +147,7 @@ def load(path: str | None = None):
     for name, args in SIGNATURES.items():
         f = getattr(L, name)
         f.argtypes = args
-        f.restype = None if name in VOID_FUNCTIONS else C.c_int
+        f.restype = None if name in VOID_FUNCTIONS else C.c_int64 if name in SIZE_FUNCTIONS else C.c_int
     _lib = L
     return L
 

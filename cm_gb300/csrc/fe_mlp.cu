@@ -1,13 +1,15 @@
 // libcm_fe: kernels of the learned Newton warm start (include/cm_warmstart.h).
 //
 // Training runs in FP32 on the CUDA cores (the network is 4-256-256-256-64,
-// so one training step is a few tens of MFLOP); inference runs the whole
+// so one training step is a few tens of MFLOP), one launch per layer and
+// direction; inference runs the whole
 // network in one launch with BF16 weights on the tensor cores
 // (mma.sync m16n8k16, FP32 accumulation), one CTA per 16 input rows with the
 // activations held in shared memory between layers.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -74,6 +76,226 @@ __global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const fl
         *c = beta == 0.0f ? acc[i][j] : acc[i][j] + beta * *c;
       }
     }
+}
+
+// ------------------------------------------------- FP32 network training
+// One tile of C = A B^T over the whole contraction length: TBM x TBN outputs by
+// eight warps, each over an eighth of every 256-long chunk of the contraction,
+// their sums added in warp order (deterministic).  On the networks trained
+// here (256 x 256 layers, minibatches of 256) a product is a few hundred
+// thousand multiply-adds per SM and its time is latency: one wait for the
+// operands of a chunk and one reduction, where 64 x 64 tiles walking the
+// contraction 16 at a time left 16 CTAs 33 us.
+constexpr int TBM = 32, TBN = 16, TBK = 256, TWARPS = 8;
+constexpr int TLDA = TBM + 1, TLDB = TBN + 4;
+constexpr int TSMEM = ((TBK + 4) * (TLDA + TLDB)) * 4;  // operands; the warps' sums reuse it
+static_assert(TWARPS * TBM * (TBN + 1) * 4 <= TSMEM, "reduction scratch");
+
+// Rows r0 .. r0 + ROWS of an operand (R rows in all), chunk [k0, k0 + TBK) of the
+// contraction (K long): all loads first (fetch), then into s[k][row] (put).  KC:
+// stored [row][K] (contraction contiguous), else [K][row].  Four values at a
+// time where the alignment and the sizes allow (vec).
+template <bool KC, int ROWS, int LD>
+struct TileOperand {
+  static constexpr int Q = ROWS * TBK / 4 / (32 * TWARPS);
+  float4 v[Q];
+  static __device__ __forceinline__ bool vec(const float* src, int64_t ld, int R, int K) {
+    return (reinterpret_cast<uintptr_t>(src) & 15) == 0 && ld % 4 == 0 && (KC ? K : R) % 4 == 0;
+  }
+  static __device__ __forceinline__ void at(int u, int& r, int& k) {
+    const int i = u * 32 * TWARPS + threadIdx.x;
+    r = KC ? i / (TBK / 4) : i % (ROWS / 4) * 4;
+    k = KC ? i % (TBK / 4) * 4 : i / (ROWS / 4);
+  }
+  __device__ __forceinline__ void fetch(const float* __restrict__ src, int64_t ld, int r0, int R, int k0, int K, bool vec) {
+#pragma unroll
+    for (int u = 0; u < Q; ++u) {
+      int r, k;
+      at(u, r, k);
+      const float* p = KC ? src + (int64_t)(r0 + r) * ld + k0 + k : src + (int64_t)(k0 + k) * ld + r0 + r;
+      v[u] = float4{0.f, 0.f, 0.f, 0.f};
+      if (r0 + r < R && k0 + k < K) {
+        if (vec) {
+          v[u] = *reinterpret_cast<const float4*>(p);
+        } else {
+          const int left = KC ? K - k0 - k : R - r0 - r;
+          v[u].x = p[0];
+          if (left > 1) v[u].y = p[1];
+          if (left > 2) v[u].z = p[2];
+          if (left > 3) v[u].w = p[3];
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void put(float* __restrict__ s, int kn) const {
+#pragma unroll
+    for (int u = 0; u < Q; ++u) {
+      int r, k;
+      at(u, r, k);
+      if (k >= kn) continue;
+      float* d = s + k * LD + r;
+      constexpr int st = KC ? LD : 1;
+      d[0] = v[u].x;
+      d[st] = v[u].y;
+      d[2 * st] = v[u].z;
+      d[3 * st] = v[u].w;
+    }
+  }
+};
+
+// The tile at (m0, n0).  Outputs go to out(m, n, value) for m < M, n < N; with
+// colsum, sum over the contraction of A's rows to csum(m, value).
+template <bool AKC, bool BKC, class Out, class Sum>
+__device__ __forceinline__ void tile_product(int M, int N, int K, const float* A, int64_t lda, const float* B,
+                                             int64_t ldb, int m0, int n0, bool colsum, Out out, Sum csum) {
+  extern __shared__ __align__(16) float tsm[];
+  float* As = tsm;
+  float* Bs = tsm + (TBK + 4) * TLDA;  // a chunk's last quadruple may pass its end
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tr = lane >> 2, tc = lane & 3;  // rows tr + 8 i, columns 4 tc + j
+  float acc[4][4] = {}, asum = 0.0f;
+  TileOperand<AKC, TBM, TLDA> ta;
+  TileOperand<BKC, TBN, TLDB> tb;
+  const bool va = ta.vec(A, lda, M, K), vb = tb.vec(B, ldb, N, K);
+  for (int k0 = 0; k0 < K; k0 += TBK) {
+    const int kn = min(TBK, K - k0);
+    ta.fetch(A, lda, m0, M, k0, K, va);
+    tb.fetch(B, ldb, n0, N, k0, K, vb);
+    if (k0) __syncthreads();
+    ta.put(As, kn);
+    tb.put(Bs, kn);
+    __syncthreads();
+    const int kw = warp * (TBK / TWARPS);
+    const int ke = min(TBK / TWARPS, K - k0 - kw);
+#pragma unroll 8
+    for (int kk = 0; kk < ke; ++kk) {
+      const float* a = As + (kw + kk) * TLDA + tr;
+      const float4 b = *reinterpret_cast<const float4*>(Bs + (kw + kk) * TLDB + 4 * tc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float v = a[8 * i];
+        acc[i][0] = fmaf(v, b.x, acc[i][0]);
+        acc[i][1] = fmaf(v, b.y, acc[i][1]);
+        acc[i][2] = fmaf(v, b.z, acc[i][2]);
+        acc[i][3] = fmaf(v, b.w, acc[i][3]);
+      }
+    }
+    if (colsum)
+      for (int kk = 0; kk < ke; ++kk) asum += As[(kw + kk) * TLDA + lane];
+  }
+  __syncthreads();
+  constexpr int LDR = TBN + 1;
+  float* red = tsm + warp * TBM * LDR;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) red[(tr + 8 * i) * LDR + 4 * tc + j] = acc[i][j];
+  red[lane * LDR + TBN] = asum;
+  __syncthreads();
+  for (int i = threadIdx.x; i < TBM * TBN; i += 32 * TWARPS) {
+    const int m = i / TBN, n = i % TBN;
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < TWARPS; ++w) v += tsm[w * TBM * LDR + m * LDR + n];
+    if (m0 + m < M && n0 + n < N) out(m0 + m, n0 + n, v);
+  }
+  if (colsum && threadIdx.x < TBM && m0 + (int)threadIdx.x < M) {
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < TWARPS; ++w) v += tsm[w * TBM * LDR + threadIdx.x * LDR + TBN];
+    csum(m0 + threadIdx.x, v);
+  }
+}
+
+__device__ __forceinline__ float act_fwd(float x, int act);
+
+// y = act(x W^T + b), x: [n][in], W: [out][in].  With target (the last layer of
+// a training step): dz = 2 (y - target) / (n out) and this CTA's share of
+// sum (y - target)^2 in part.
+__global__ void __launch_bounds__(32 * TWARPS) linear_kernel(int n, int in, int out, const float* __restrict__ x,
+                                                             const float* __restrict__ W, const float* __restrict__ b,
+                                                             int act, float* __restrict__ y,
+                                                             const float* __restrict__ target, float* __restrict__ dz,
+                                                             float* __restrict__ part) {
+  __shared__ float sq[TWARPS];
+  const int tn = (out + TBN - 1) / TBN;
+  const float inv2 = target ? 2.0f / ((float)n * (float)out) : 0.0f;
+  float s = 0.0f;
+  tile_product<true, true>(
+      n, out, in, x, in, W, in, blockIdx.x / tn * TBM, blockIdx.x % tn * TBN, false,
+      [&](int m, int c, float v) {
+        v = act_fwd(v + (b ? b[c] : 0.0f), act);
+        const int64_t at = (int64_t)m * out + c;
+        if (y) y[at] = v;
+        if (target) {
+          const float d = v - target[at];
+          s = fmaf(d, d, s);
+          dz[at] = d * inv2;
+        }
+      },
+      [](int, float) {});
+  if (target) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sq[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float t = 0.0f;
+      for (int w = 0; w < TWARPS; ++w) t += sq[w];
+      part[blockIdx.x] = t;
+    }
+  }
+}
+
+// Backward of one layer from dz: [n][out]: dW = dz^T h, db = column sums of dz
+// (first tw CTAs), and with dprev the previous layer's dz = (dz W) act'(h) (the
+// others).  With part: the loss from the last layer's shares, in order.
+__global__ void __launch_bounds__(32 * TWARPS) backward_kernel(int n, int in, int out, const float* __restrict__ dz,
+                                                               const float* __restrict__ h, const float* __restrict__ W,
+                                                               int act, float* __restrict__ dW, float* __restrict__ db,
+                                                               float* __restrict__ dprev, int tw,
+                                                               const float* __restrict__ part, int parts,
+                                                               float* __restrict__ loss) {
+  if ((int)blockIdx.x < tw) {
+    const int tn = (in + TBN - 1) / TBN;
+    const int tm = blockIdx.x / tn, tc = blockIdx.x % tn;
+    tile_product<false, false>(
+        out, in, n, dz, out, h, in, tm * TBM, tc * TBN, tc == 0,
+        [&](int o, int i, float v) { dW[(int64_t)o * in + i] = v; }, [&](int o, float v) { db[o] = v; });
+    if (part && blockIdx.x == 0 && threadIdx.x < 32) {
+      float s = 0.0f;
+      for (int c = threadIdx.x; c < parts; c += 32) s += part[c];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (threadIdx.x == 0) *loss = s / ((float)n * (float)out);
+    }
+    return;
+  }
+  const int t = blockIdx.x - tw, tn = (in + TBN - 1) / TBN;
+  tile_product<true, false>(
+      n, in, out, dz, out, W, in, t / tn * TBM, t % tn * TBN, false,
+      [&](int m, int i, float v) {
+        const int64_t at = (int64_t)m * in + i;
+        const float a = h[at];
+        dprev[at] = act == WS_ACT_TANH ? v * (1.0f - a * a) : v;
+      },
+      [](int, float) {});
+}
+
+int tiles(int m, int n) { return ((m + TBM - 1) / TBM) * ((n + TBN - 1) / TBN); }
+
+// The kernels' shared memory, set once per device.
+int tile_attributes() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev < 0 || dev >= 64 || !done[dev].load())) {
+    e = cudaFuncSetAttribute(linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TSMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TSMEM);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev].store(true);
+  }
+  return e == cudaSuccess ? FE_NO_ERROR
+                          : cmfe::record_error(FE_ERR_CUDA, std::string("training kernels: ") + cudaGetErrorString(e));
 }
 
 __device__ __forceinline__ float act_fwd(float x, int act) { return act == WS_ACT_TANH ? tanhf(x) : x; }
@@ -226,6 +448,67 @@ int ws_gemm_f32(int32_t m, int32_t n, int32_t k, const float* a, int64_t a_sm, i
   const dim3 grid((n + TN - 1) / TN, (m + TM - 1) / TM);
   gemm_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(m, n, k, a, a_sm, a_sk, b, b_sk, b_sn, c, ldc, beta);
   return cuda_status("ws_gemm_f32");
+}
+
+int ws_linear_f32(int32_t n, int32_t in, int32_t out, const float* x, const float* w, const float* bias, int32_t act,
+                  float* y, void* stream) {
+  if (n < 0 || in <= 0 || out <= 0 || !x || !w || !y || (act != WS_ACT_IDENTITY && act != WS_ACT_TANH))
+    return bad("ws_linear_f32: bad arguments");
+  if (n == 0) return FE_NO_ERROR;
+  const int rc = tile_attributes();
+  if (rc) return rc;
+  linear_kernel<<<tiles(n, out), 32 * TWARPS, TSMEM, (cudaStream_t)stream>>>(n, in, out, x, w, bias, act, y, nullptr,
+                                                                             nullptr, nullptr);
+  return cuda_status("ws_linear_f32");
+}
+
+int64_t ws_mlp_workspace(int32_t n, int32_t layers, const int32_t* widths) {
+  if (n <= 0 || layers < 1 || layers > WS_MAX_LAYERS || !widths) return 0;
+  int64_t floats = tiles(n, widths[layers]);
+  for (int l = 1; l <= layers; ++l) floats += 2 * (int64_t)n * widths[l];
+  return floats;
+}
+
+int ws_mlp_loss_grad(int32_t n, int32_t layers, const int32_t* widths, const float* params, float* grad, const float* x,
+                     const float* target, float* loss, float* workspace, void* stream) {
+  if (n <= 0 || layers < 1 || layers > WS_MAX_LAYERS || !widths || !params || !grad || !x || !target || !loss || !workspace)
+    return bad("ws_mlp_loss_grad: bad arguments");
+  for (int l = 0; l <= layers; ++l)
+    if (widths[l] <= 0) return bad("ws_mlp_loss_grad: widths must be positive");
+  int rc = tile_attributes();
+  if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  const float* h[WS_MAX_LAYERS + 1];   // layer outputs
+  float* dz[WS_MAX_LAYERS + 1];        // gradients before the activations
+  int64_t off[WS_MAX_LAYERS + 1];      // W_l, b_l in params and grad
+  float* ws = workspace;
+  h[0] = x;
+  off[0] = 0;
+  for (int l = 0; l < layers; ++l) {
+    off[l + 1] = off[l] + (int64_t)widths[l + 1] * (widths[l] + 1);
+    h[l + 1] = ws;
+    ws += (int64_t)n * widths[l + 1];
+    dz[l + 1] = ws;
+    ws += (int64_t)n * widths[l + 1];
+  }
+  float* part = ws;
+  for (int l = 0; l < layers; ++l) {
+    const int in = widths[l], out = widths[l + 1];
+    const float* W = params + off[l];
+    const bool last = l + 1 == layers;
+    linear_kernel<<<tiles(n, out), 32 * TWARPS, TSMEM, st>>>(
+        n, in, out, h[l], W, W + (int64_t)out * in, last ? WS_ACT_IDENTITY : WS_ACT_TANH,
+        last ? nullptr : const_cast<float*>(h[l + 1]), last ? target : nullptr, dz[l + 1], part);
+  }
+  for (int l = layers - 1; l >= 0; --l) {
+    const int in = widths[l], out = widths[l + 1], tw = tiles(out, in);
+    float* dW = grad + off[l];
+    const bool last = l + 1 == layers;
+    backward_kernel<<<tw + (l > 0 ? tiles(n, in) : 0), 32 * TWARPS, TSMEM, st>>>(
+        n, in, out, dz[l + 1], h[l], params + off[l], WS_ACT_TANH, dW, dW + (int64_t)out * in, l > 0 ? dz[l] : nullptr,
+        tw, last ? part : nullptr, tiles(n, widths[layers]), loss);
+  }
+  return cuda_status("ws_mlp_loss_grad");
 }
 
 int ws_bias_act(float* y, const float* bias, int32_t rows, int32_t cols, int32_t act, void* stream) {

@@ -44,6 +44,7 @@ class MLP:
 
     def __init__(self, widths=(4, 256, 256, 256, 64), seed=0, device="cuda"):
         self.widths = tuple(int(w) for w in widths)
+        self._widths_c = (C.c_int32 * len(self.widths))(*self.widths)
         self.device = torch.device(device)
         self.L = _lib.load()
         sizes = []
@@ -84,9 +85,8 @@ class MLP:
             i, o = self.widths[l], self.widths[l + 1]
             h = torch.empty(n, o, dtype=torch.float32, device=self.device)
             W = self.W(l)
-            check(self.L.ws_gemm_f32(n, o, i, _p(hs[-1]), i, 1, _p(W), 1, i, _p(h), o, 0.0, _s(h)))
             act = WS_ACT_TANH if l + 1 < self.layers else WS_ACT_IDENTITY
-            check(self.L.ws_bias_act(_p(h), _p(self.b(l)), n, o, act, _s(h)))
+            check(self.L.ws_linear_f32(n, i, o, _p(hs[-1]), _p(W), _p(self.b(l)), act, _p(h), _s(h)))
             hs.append(h)
         return hs
 
@@ -108,11 +108,20 @@ class MLP:
                 dh = dprev
 
     def loss_and_grad(self, x, y):
-        hs = self.forward(x)
-        dy = torch.empty_like(hs[-1])
+        """Mean squared error against y and, in self.grad, its gradient."""
+        x, y = x.contiguous(), y.contiguous()
+        n = x.shape[0]
         loss = torch.empty(1, dtype=torch.float32, device=self.device)
-        check(self.L.ws_mse(_p(hs[-1]), _p(y.contiguous()), _p(dy), _p(loss), dy.numel(), _s(dy)))
-        self.backward(hs, dy)
+        if n == 0 or self.layers > _lib.WS_MAX_LAYERS:
+            hs = self.forward(x)
+            dy = torch.empty_like(hs[-1])
+            check(self.L.ws_mse(_p(hs[-1]), _p(y), _p(dy), _p(loss), dy.numel(), _s(dy)))
+            self.backward(hs, dy)
+            return loss
+        work = torch.empty(self.L.ws_mlp_workspace(n, self.layers, self._widths_c), dtype=torch.float32,
+                           device=self.device)
+        check(self.L.ws_mlp_loss_grad(n, self.layers, self._widths_c, self.flat.data_ptr(), self.grad.data_ptr(),
+                                      x.data_ptr(), y.data_ptr(), loss.data_ptr(), work.data_ptr(), _s(work)))
         return loss
 
     def adam_step(self, lr, beta1=0.9, beta2=0.999, eps=1e-8):

@@ -33,6 +33,20 @@ extern "C" {
 int ws_gemm_f32(int32_t m, int32_t n, int32_t k, const float* a, int64_t a_sm, int64_t a_sk, const float* b,
                 int64_t b_sk, int64_t b_sn, float* c, int64_t ldc, float beta, void* stream);
 
+/* y = act(x W^T + b) in FP32: x [n][in], W [out][in], b [out] or NULL,
+ * y [n][out]. */
+int ws_linear_f32(int32_t n, int32_t in, int32_t out, const float* x, const float* w, const float* bias, int32_t act,
+                  float* y, void* stream);
+
+/* Mean squared error of the tanh network with a linear last layer and its
+ * gradient, one launch per layer and direction: params and grad hold W_0, b_0,
+ * W_1, b_1, ... (W_l [widths[l+1]][widths[l]]); x [n][widths[0]], target
+ * [n][widths[layers]]; *loss = sum (y - target)^2 / (n widths[layers]).
+ * workspace: ws_mlp_workspace(n, layers, widths) floats of device memory. */
+int64_t ws_mlp_workspace(int32_t n, int32_t layers, const int32_t* widths);
+int ws_mlp_loss_grad(int32_t n, int32_t layers, const int32_t* widths, const float* params, float* grad,
+                     const float* x, const float* target, float* loss, float* workspace, void* stream);
+
 /* y[i][j] = act(y[i][j] + bias[j]) for a rows x cols row-major block. */
 int ws_bias_act(float* y, const float* bias, int32_t rows, int32_t cols, int32_t act, void* stream);
 
