@@ -119,6 +119,7 @@ SIGNATURES = {
     "ws_adam": [_vp, _vp, _vp, _vp, _i64, C.c_float, C.c_float, C.c_float, C.c_float, _i32, _vp],
     "ws_to_bf16": [_vp, _vp, _i64, _vp],
     "ws_mlp_forward_bf16": [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _i32, _vp],
+    "ws_mlp_forward_bf16_cols": [_i32, _i32, _vp, _vp, _vp, _vp, _i32, _vp, _i32, _vp],
 }
 
 # Functions of the C ABI that return nothing.

@@ -4,8 +4,9 @@
 // so one training step is a few tens of MFLOP), one launch per layer and
 // direction; inference runs the whole
 // network in one launch with BF16 weights on the tensor cores
-// (mma.sync m16n8k16, FP32 accumulation), one CTA per 16 input rows with the
-// activations held in shared memory between layers.
+// (mma.sync m16n8k16, FP32 accumulation), one cluster of eight CTAs per 16 input
+// rows with the activations held in shared memory between layers.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -364,7 +365,9 @@ __global__ void to_bf16_kernel(const float* s, uint16_t* d, int64_t n) {
 
 // ------------------------------------------------------ BF16 inference
 constexpr int MAXW = 256;
-constexpr int IW = 8;  // warps per CTA
+constexpr int ICLUSTER = 8;                  // CTAs that share 16 input rows
+constexpr int IW = MAXW / 8 / ICLUSTER;      // warps per CTA: one per tile of 8 features
+constexpr int ILD = MAXW / 2 + 4;  // activation row in 32-bit words (BF16 pairs), padded off the banks
 
 struct MlpArgs {
   int layers;
@@ -378,57 +381,85 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-__global__ void __launch_bounds__(32 * IW) mlp_bf16_kernel(MlpArgs a, int n, const float* __restrict__ x,
-                                                           float* __restrict__ y, int act) {
-  __shared__ float buf[2][16][MAXW + 4];
+// The whole network for 16 input rows by a cluster of eight CTAs.  A few rows
+// are a latency problem: one CTA walking 256 x 256 layers waits for its weights
+// at every step (26 us for the 4-256-256-256-64 network on 256 rows).  Here each
+// warp has at most one tile of 8 features of a layer; its weights are at most
+// 32 registers and are loaded one layer ahead, and the activations, rounded to
+// BF16 as the products take them, go to all eight CTAs' shared memory.  Every
+// output is summed over the contraction in order by one warp.
+__global__ void __cluster_dims__(ICLUSTER, 1, 1) __launch_bounds__(32 * IW)
+    mlp_bf16_kernel(MlpArgs a, int n, const float* __restrict__ x, int xcols, float* __restrict__ y, int act) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ uint32_t buf[2][16][ILD];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
-  const int row0 = blockIdx.x * 16;
-  const int w0 = a.widths[0];
-  for (int i = threadIdx.x; i < 16 * w0; i += blockDim.x) {
-    const int r = i / w0, c = i % w0;
-    buf[0][r][c] = (row0 + r < n) ? x[(int64_t)(row0 + r) * w0 + c] : 0.0f;
-  }
-  __syncthreads();
-  int cur = 0;
-  for (int l = 0; l < a.layers; ++l) {
-    const int in = a.widths[l], out = a.widths[l + 1];
-    const uint32_t* W = a.w[l];
-    const float* bias = a.b[l];
-    const bool last = l + 1 == a.layers;
-    for (int nt = warp; nt < out / 8; nt += IW) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      const int ncol = 8 * nt + gq;  // B column (output feature) this thread loads
-      for (int k0 = 0; k0 < in; k0 += 16) {
-        const float* A0 = &buf[cur][gq][k0 + 2 * tq];
-        const float* A1 = &buf[cur][gq + 8][k0 + 2 * tq];
-        const uint32_t a0 = pack2(A0[0], A0[1]);
-        const uint32_t a1 = pack2(A1[0], A1[1]);
-        const uint32_t a2 = pack2(A0[8], A0[9]);
-        const uint32_t a3 = pack2(A1[8], A1[9]);
-        const uint32_t* wr = W + ((int64_t)ncol * in + k0) / 2;
-        const uint32_t b0 = wr[tq], b1 = wr[tq + 4];
-        asm volatile(
-            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-            "{%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-      }
-      const int c0 = 8 * nt + 2 * tq;
+  const int tile = cluster.block_rank() * IW + warp;  // of every layer that has as many
+  const int row0 = blockIdx.x / ICLUSTER * 16;
+  constexpr int MAXS = MAXW / 16;  // k16 steps
+  uint32_t w[2][2 * MAXS];
+  auto load = [&](int l, uint32_t (&f)[2 * MAXS]) {
+    const int steps = 8 * tile < a.widths[l + 1] ? a.widths[l] / 16 : 0;
+    const uint32_t* wr = a.w[l] + (int64_t)(8 * tile + gq) * a.widths[l] / 2;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const int r = gq + (h >= 2 ? 8 : 0), c = c0 + (h & 1);
-        float v = d[h] + bias[c];
-        if (!last) v = act_fwd(v, act);
+    for (int k = 0; k < MAXS; ++k)
+      if (k < steps) {
+        f[2 * k] = wr[8 * k + tq];
+        f[2 * k + 1] = wr[8 * k + tq + 4];
+      }
+  };
+  load(0, w[0]);
+  for (int i = threadIdx.x; i < 16 * a.widths[0] / 2; i += blockDim.x) {
+    const int r = i / (a.widths[0] / 2), c = 2 * (i % (a.widths[0] / 2));
+    const float* xr = x + (int64_t)(row0 + r) * xcols;
+    const bool in = row0 + r < n;
+    buf[0][r][c / 2] = pack2(in && c < xcols ? xr[c] : 0.0f, in && c + 1 < xcols ? xr[c + 1] : 0.0f);
+  }
+  cluster.sync();  // every CTA of the cluster has started: its shared memory may be written
+  auto layer = [&](int l, uint32_t (&f)[2 * MAXS], uint32_t (&next)[2 * MAXS]) {
+    const bool last = l + 1 == a.layers;
+    if (!last) load(l + 1, next);
+    const int out = a.widths[l + 1], steps = a.widths[l] / 16;
+    if (8 * tile < out) {
+      const uint32_t(*in)[ILD] = buf[l & 1];
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < MAXS; ++k)
+        if (k < steps) {
+          const int c = 8 * k + tq;
+          asm volatile(
+              "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+              "{%0,%1,%2,%3};\n"
+              : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+              : "r"(in[gq][c]), "r"(in[gq + 8][c]), "r"(in[gq][c + 4]), "r"(in[gq + 8][c + 4]), "r"(f[2 * k]),
+                "r"(f[2 * k + 1]));
+        }
+      const int c = 8 * tile + 2 * tq;
+      const float b0 = a.b[l][c], b1 = a.b[l][c + 1];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = gq + 8 * h;
+        const float v0 = d[2 * h] + b0, v1 = d[2 * h + 1] + b1;
         if (last) {
-          if (row0 + r < n) y[(int64_t)(row0 + r) * out + c] = v;
+          if (row0 + r < n) {
+            y[(int64_t)(row0 + r) * out + c] = v0;
+            y[(int64_t)(row0 + r) * out + c + 1] = v1;
+          }
         } else {
-          buf[cur ^ 1][r][c] = v;
+          const uint32_t v = pack2(act_fwd(v0, act), act_fwd(v1, act));
+          uint32_t* dst = &buf[(l + 1) & 1][r][c / 2];
+#pragma unroll
+          for (int q = 0; q < ICLUSTER; ++q) *cluster.map_shared_rank(dst, q) = v;
         }
       }
     }
-    __syncthreads();
-    cur ^= 1;
+    // the activations are everywhere; and nobody writes a CTA that has ended
+    if (!last) cluster.sync();
+  };
+  for (int l = 0; l < a.layers; l += 2) {
+    layer(l, w[0], w[1]);
+    if (l + 1 < a.layers) layer(l + 1, w[1], w[0]);
   }
 }
 
@@ -555,6 +586,12 @@ int ws_to_bf16(const float* src, uint16_t* dst, int64_t count, void* stream) {
 
 int ws_mlp_forward_bf16(int32_t n, int32_t layers, const int32_t* widths, const uint16_t* const* weights,
                         const float* const* bias, const float* x, float* y, int32_t act, void* stream) {
+  return ws_mlp_forward_bf16_cols(n, layers, widths, weights, bias, x, widths ? widths[0] : 0, y, act, stream);
+}
+
+int ws_mlp_forward_bf16_cols(int32_t n, int32_t layers, const int32_t* widths, const uint16_t* const* weights,
+                             const float* const* bias, const float* x, int32_t x_cols, float* y, int32_t act,
+                             void* stream) {
   if (n < 0 || layers < 1 || layers > WS_MAX_LAYERS || !widths || !weights || !bias || !x || !y)
     return bad("ws_mlp_forward_bf16: bad arguments");
   MlpArgs a;
@@ -570,8 +607,9 @@ int ws_mlp_forward_bf16(int32_t n, int32_t layers, const int32_t* widths, const 
     a.w[l] = reinterpret_cast<const uint32_t*>(weights[l]);
     a.b[l] = bias[l];
   }
+  if (x_cols <= 0 || x_cols > widths[0]) return bad("ws_mlp_forward_bf16: x has 1 to widths[0] columns");
   if (n == 0) return FE_NO_ERROR;
-  mlp_bf16_kernel<<<(n + 15) / 16, 32 * IW, 0, (cudaStream_t)stream>>>(a, n, x, y, act);
+  mlp_bf16_kernel<<<(n + 15) / 16 * ICLUSTER, 32 * IW, 0, (cudaStream_t)stream>>>(a, n, x, x_cols, y, act);
   return cuda_status("ws_mlp_forward_bf16");
 }
 

@@ -160,20 +160,22 @@ class MLP:
             bp[:self.widths[l + 1]] = self.b(l)
             ws.append(Wb)
             bs.append(bp)
-        self._bf16 = (widths, ws, bs)
+        n = self.layers
+        self._bf16 = (widths, ws, bs, (C.c_int32 * len(widths))(*widths), (C.c_void_p * n)(*[t.data_ptr() for t in ws]),
+                      (C.c_void_p * n)(*[t.data_ptr() for t in bs]))
 
     def infer_bf16(self, x):
         if self._bf16 is None:
             self._prepare_bf16()
-        widths, ws, bs = self._bf16
-        n = x.shape[0]
-        xp = torch.zeros(n, widths[0], dtype=torch.float32, device=self.device)
-        xp[:, :x.shape[1]] = x
+        widths, _, _, W, Wp, Bp = self._bf16
+        n, cols = x.shape
+        if x.dtype != torch.float32 or x.device != self.flat.device or not x.is_contiguous():
+            xp = torch.empty(n, cols, dtype=torch.float32, device=self.device)
+            xp.copy_(x)
+            x = xp
         y = torch.empty(n, widths[-1], dtype=torch.float32, device=self.device)
-        W = (C.c_int32 * len(widths))(*widths)
-        Wp = (C.c_void_p * self.layers)(*[w.data_ptr() for w in ws])
-        Bp = (C.c_void_p * self.layers)(*[b.data_ptr() for b in bs])
-        check(self.L.ws_mlp_forward_bf16(n, self.layers, W, Wp, Bp, _p(xp), _p(y), WS_ACT_TANH, _s(y)))
+        check(self.L.ws_mlp_forward_bf16_cols(n, self.layers, W, Wp, Bp, x.data_ptr(), cols, y.data_ptr(), WS_ACT_TANH,
+                                              _s(y)))
         return y[:, :self.widths[-1]]
 
 

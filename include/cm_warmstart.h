@@ -76,6 +76,11 @@ int ws_to_bf16(const float* src, uint16_t* dst, int64_t count, void* stream);
 int ws_mlp_forward_bf16(int32_t n, int32_t layers, const int32_t* widths, const uint16_t* const* weights,
                         const float* const* bias, const float* x, float* y, int32_t act, void* stream);
 
+/* The same with x: [n][x_cols], x_cols <= widths[0], the missing columns zero. */
+int ws_mlp_forward_bf16_cols(int32_t n, int32_t layers, const int32_t* widths, const uint16_t* const* weights,
+                             const float* const* bias, const float* x, int32_t x_cols, float* y, int32_t act,
+                             void* stream);
+
 #ifdef __cplusplus
 }
 #endif
