@@ -62,6 +62,9 @@ struct HostSetup {
   // node (sorted by element number, packed e * 32 + local node) and around
   // every pressure row node (e * 8 + local pressure node).
   std::vector<int32_t> u_inc_ptr, u_inc, p_inc_ptr, p_inc;
+  // the same incidences in colour order, for the residual, whose sums have
+  // the order of the colour-by-colour assembly
+  std::vector<int32_t> u_inc_col, p_inc_col;
   // the incidences' rank-table rows, elem_table[e] * nr + local row node
   std::vector<int32_t> u_inc_row, p_inc_row;
   // u nodes: which local node of which element belongs to a column of the
@@ -140,6 +143,13 @@ struct StageOut {
   unsigned char* rec;  // element e's record at e * Rec::BYTES
 };
 
+// The residual record of one element: [a][m] for its u nodes, then [q].
+template <int NPE, int NPP>
+struct RecR {
+  static constexpr int N = (3 * NPE + NPP + 3) / 4 * 4;  // doubles, whole 32-byte sectors
+  static CMFE_HD double* of(const StageOut& so, int e) { return reinterpret_cast<double*>(so.rec) + (size_t)e * N; }
+};
+
 // Arguments of the fused staged assembly (fe_mixed.cu): the incidence lists,
 // a work counter (next element group, zero before the launch), the per-row-
 // node counts of finished elements around the node (u nodes, then pressure
@@ -184,6 +194,13 @@ int launch_fp64_fused(const HostSetup& s, const KParams& kp, const StageOut& so,
                       void* stream);
 int fp64_groups(const HostSetup& s, int num_sms, bool* small);
 size_t record_bytes_fp64(const HostSetup& s);
+
+// The residual in one launch (fe_residual.cu): residual records of
+// record_bytes_residual() each, and fa.node_done, zero before the first launch
+// and left zero.  Returns a cudaError_t value.
+int launch_residual_fused(const HostSetup& s, const KParams& kp, const StageOut& so, const FusedArgs& fa, int num_sms,
+                          void* stream, bool double_float);
+size_t record_bytes_residual(const HostSetup& s);
 
 // Bytes of one element's record (mixed precision).
 inline size_t record_bytes(const HostSetup& s) {

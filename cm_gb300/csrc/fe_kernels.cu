@@ -497,13 +497,18 @@ struct fe_equations_set {
   // staged assembly: incidence lists (uploaded at creation) and the
   // per-element records (allocated on the first staged evaluation)
   int32_t *d_u_inc_ptr = nullptr, *d_u_inc = nullptr, *d_p_inc_ptr = nullptr, *d_p_inc = nullptr,
-          *d_u_inc_row = nullptr, *d_p_inc_row = nullptr, *d_u_pat = nullptr;
+          *d_u_inc_row = nullptr, *d_p_inc_row = nullptr, *d_u_pat = nullptr,
+          *d_u_inc_col = nullptr, *d_p_inc_col = nullptr;
   uint32_t* d_pat = nullptr;
   unsigned char* d_rec = nullptr;
   // FP64 assembly: its records and counters, and the order of their uses
   unsigned char* d_rec64 = nullptr;
   int* d_fuse64 = nullptr;
   cudaEvent_t order_event = nullptr;
+  // residual: its records and node counts (allocated at creation), and their order
+  unsigned char* d_rec_r = nullptr;
+  int* d_done_r = nullptr;
+  cudaEvent_t residual_event = nullptr;
   std::vector<cudaStream_t> side_streams;  // parts of a small mesh's FP64 assembly
   std::vector<cudaEvent_t> side_events;
   int* d_fuse = nullptr;  // fused staged assembly: [0, kFuseChunks) group counters, then per-row-node counts
@@ -672,14 +677,14 @@ bool capturing(cudaStream_t st) {
 // the stream waits for the handle's previous such work, and the destructor
 // marks the end of what was queued since.
 struct HandleOrder {
-  fe_handle h;
+  cudaEvent_t* ev;
   cudaStream_t st;
-  HandleOrder(fe_handle h_, cudaStream_t st_) : h(h_), st(st_) {
-    if (!h->order_event) cudaEventCreateWithFlags(&h->order_event, cudaEventDisableTiming);
-    if (h->order_event) cudaStreamWaitEvent(st, h->order_event, 0);
+  HandleOrder(cudaEvent_t* ev_, cudaStream_t st_) : ev(ev_), st(st_) {
+    if (!*ev) cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    if (*ev) cudaStreamWaitEvent(st, *ev, 0);
   }
   ~HandleOrder() {
-    if (h->order_event) cudaEventRecord(h->order_event, st);
+    if (*ev) cudaEventRecord(*ev, st);
   }
 };
 
@@ -692,7 +697,7 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   *taken = false;
   if (capturing(st)) return FE_NO_ERROR;
   if (ensure((void**)&h->d_rec64, cmfe::record_bytes_fp64(s) * (size_t)s.ne)) return FE_NO_ERROR;
-  HandleOrder order(h, st);
+  HandleOrder order(&h->order_event, st);
   cmfe::FusedArgs fa;
   int rc;
   if ((rc = fused_args(h, &h->d_fuse64, st, &fa))) return rc == FE_ERR_OUT_OF_MEMORY ? FE_NO_ERROR : rc;
@@ -735,6 +740,59 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   for (int c = 1; c < n; ++c) CUDA_TRY(cudaStreamWaitEvent(st, ev[c], 0));
   if (err) return set_error(FE_ERR_CUDA, std::string("FP64 kernel launch: ") + cudaGetErrorString((cudaError_t)err));
   *taken = true;
+  return FE_NO_ERROR;
+}
+
+// The residual's records, node counts and event, at handle creation: residual
+// evaluations allocate nothing.
+int residual_buffers(fe_handle h) {
+  const auto& s = h->hs;
+  const size_t counts = sizeof(int) * ((size_t)s.nu + (size_t)s.npn);
+  int rc;
+  if ((rc = ensure((void**)&h->d_rec_r, cmfe::record_bytes_residual(s) * (size_t)s.ne)) ||
+      (rc = ensure((void**)&h->d_done_r, counts)))
+    return rc;
+  CUDA_TRY(cudaMemset(h->d_done_r, 0, counts));
+  CUDA_TRY(cudaEventCreateWithFlags(&h->residual_event, cudaEventDisableTiming));
+  return FE_NO_ERROR;
+}
+
+// r = residual at dx (device memory): one launch, or, on a stream being
+// captured (its replays may run beside other work of the handle), one per
+// element colour.
+int residual_run(fe_handle h, const double* dx, double* dr, cudaStream_t st) {
+  const auto& s = h->hs;
+  const bool double_float = h->high_precision == FE_HIGH_PRECISION_DOUBLE_FLOAT;
+  KParams kp = base_params(h);
+  kp.x = dx;
+  kp.r = dr;
+  kp.res_only = 1;
+  int rc;
+  if (!capturing(st)) {
+    HandleOrder order(&h->residual_event, st);
+    const int nb = s.bnd_ptr.empty() ? 0 : s.bnd_ptr[s.ncolours];
+    cmfe::FusedArgs fa;
+    std::memset(&fa, 0, sizeof(fa));
+    fa.u_inc_ptr = h->d_u_inc_ptr;
+    fa.u_inc = h->d_u_inc_col;
+    fa.p_inc_ptr = h->d_p_inc_ptr;
+    fa.p_inc = h->d_p_inc_col;
+    fa.node_done = h->d_done_r;
+    fa.bmask = h->has_surfp && nb > 0 ? h->d_bnd_mask : nullptr;
+    kp.count = s.ne;
+    const int e = cmfe::launch_residual_fused(s, kp, cmfe::StageOut{h->d_rec_r}, fa, h->num_sms, st, double_float);
+    if (e != 0) return set_error(FE_ERR_CUDA, std::string("residual kernel launch: ") + cudaGetErrorString((cudaError_t)e));
+    h->launches++;
+    return FE_NO_ERROR;
+  }
+  for (int c = 0; c < s.ncolours; ++c) {
+    kp.elems = h->d_colour_elems + s.colour_ptr[c];
+    kp.count = s.colour_ptr[c + 1] - s.colour_ptr[c];
+    const int e = cmfe::launch_mixed(s, kp, h->num_sms, st, double_float);
+    if (e != 0) return set_error(FE_ERR_CUDA, std::string("residual kernel launch: ") + cudaGetErrorString((cudaError_t)e));
+    h->launches++;
+    if ((rc = surface_after(h, kp, c, 0, st))) return rc;
+  }
   return FE_NO_ERROR;
 }
 
@@ -1190,7 +1248,8 @@ std::vector<void*> shared_arrays(fe_handle h) {
   return {h->d_bnd_elems, h->d_bnd_mask, h->d_geo_dd, h->d_elem_u, h->d_elem_p, h->d_row_ptr, h->d_uu_row_ptr,
           h->d_cp_row_ptr, h->d_wu, h->d_wp, h->d_elem_table, h->d_colour_elems, h->d_tables, h->d_geo,
           h->d_gbf_u, h->d_gbf_p, h->d_gw, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc,
-          h->d_u_inc_row, h->d_p_inc_row, h->d_u_pat, h->d_pat, h->d_geo_rj};
+          h->d_u_inc_row, h->d_p_inc_row, h->d_u_pat, h->d_pat, h->d_geo_rj,
+          h->d_u_inc_col, h->d_p_inc_col};
 }
 }  // namespace
 
@@ -1242,6 +1301,7 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   if ((rc = dev_upload(&h->d_bnd_elems, s.bnd_elems)) || (rc = dev_upload(&h->d_bnd_mask, s.bnd_mask))) return fail(rc);
   if ((rc = dev_upload(&h->d_u_inc_ptr, s.u_inc_ptr)) || (rc = dev_upload(&h->d_u_inc, s.u_inc)) ||
       (rc = dev_upload(&h->d_p_inc_ptr, s.p_inc_ptr)) || (rc = dev_upload(&h->d_p_inc, s.p_inc)) ||
+      (rc = dev_upload(&h->d_u_inc_col, s.u_inc_col)) || (rc = dev_upload(&h->d_p_inc_col, s.p_inc_col)) ||
       (rc = dev_upload(&h->d_u_inc_row, s.u_inc_row)) || (rc = dev_upload(&h->d_p_inc_row, s.p_inc_row)) || (rc = dev_upload(&h->d_u_pat, s.u_pat)) ||
       (rc = dev_upload(&h->d_pat, s.pat)))
     return fail(rc);
@@ -1253,6 +1313,7 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   if (cudaMalloc(&h->d_status, sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess)
     return fail(set_error(FE_ERR_CUDA, "status allocation failed"));
+  if ((rc = residual_buffers(h))) return fail(rc);
   {
     // Resolving the address of the allocation-free entry point's array loads
     // the module that holds it, which commits its 16 MiB on this device now,
@@ -1273,12 +1334,14 @@ int fe_destroy(fe_handle h) {
   }
   // per-handle state: materials, surface load, status word, staging and records
   void* own[] = {h->d_surfp, h->d_mat, h->d_status, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
-                 h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64};
+                 h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64, h->d_rec_r,
+                 h->d_done_r};
   for (void* p : own)
     if (p) cudaFree(p);
   for (cudaEvent_t ev : h->chunk_events)
     if (ev) cudaEventDestroy(ev);
   if (h->order_event) cudaEventDestroy(h->order_event);
+  if (h->residual_event) cudaEventDestroy(h->residual_event);
   for (cudaEvent_t ev : h->side_events) cudaEventDestroy(ev);
   for (cudaStream_t ss : h->side_streams) cudaStreamDestroy(ss);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
@@ -1324,6 +1387,8 @@ int fe_clone(fe_handle src, fe_handle* out) {
     h->d_u_inc_row = src->d_u_inc_row;
     h->d_u_pat = src->d_u_pat;
     h->d_pat = src->d_pat;
+    h->d_u_inc_col = src->d_u_inc_col;
+    h->d_p_inc_col = src->d_p_inc_col;
     h->d_p_inc_row = src->d_p_inc_row;
     h->high_precision = src->high_precision;
     h->assembly_order = src->assembly_order;
@@ -1340,6 +1405,7 @@ int fe_clone(fe_handle src, fe_handle* out) {
       cudaMalloc(&h->d_status, sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess)
     return fail(set_error(FE_ERR_CUDA, "clone: device allocation failed"));
+  if ((rc = residual_buffers(h))) return fail(rc);
   if (src->has_surfp) {
     const size_t bytes = sizeof(double) * 3 * (size_t)h->hs.nu;
     if (cudaMalloc(&h->d_surfp, bytes) != cudaSuccess ||
@@ -1416,18 +1482,7 @@ int fe_residual_evaluate(fe_handle h, const double* x, double* r, void* stream) 
     if ((rc = ensure((void**)&h->s_r, sizeof(double) * h->hs.ndofs))) return rc;
     dr = h->s_r;
   }
-  KParams kp = base_params(h);
-  kp.x = dx;
-  kp.r = dr;
-  kp.res_only = 1;
-  for (int c = 0; c < h->hs.ncolours; ++c) {
-    kp.elems = h->d_colour_elems + h->hs.colour_ptr[c];
-    kp.count = h->hs.colour_ptr[c + 1] - h->hs.colour_ptr[c];
-    const int e = cmfe::launch_mixed(h->hs, kp, h->num_sms, st, h->high_precision == FE_HIGH_PRECISION_DOUBLE_FLOAT);
-    if (e != 0) return set_error(FE_ERR_CUDA, std::string("residual kernel launch: ") + cudaGetErrorString((cudaError_t)e));
-    h->launches++;
-    if ((rc = surface_after(h, kp, c, 0, st))) return rc;
-  }
+  if ((rc = residual_run(h, dx, dr, st))) return rc;
   if (hr) {
     CUDA_TRY(cudaMemcpyAsync(r, dr, sizeof(double) * h->hs.ndofs, cudaMemcpyDeviceToHost, st));
     return finish_status(h, st);
@@ -1461,18 +1516,7 @@ int fe_residual_evaluate_noalloc(fe_handle h, const double* x, double* r, void* 
     }
   } drain{st};
   CUDA_TRY(cudaMemcpyAsync(dx, x, bytes, cudaMemcpyDefault, st));
-  KParams kp = base_params(h);
-  kp.x = dx;
-  kp.r = dr;
-  kp.res_only = 1;
-  for (int c = 0; c < h->hs.ncolours; ++c) {
-    kp.elems = h->d_colour_elems + h->hs.colour_ptr[c];
-    kp.count = h->hs.colour_ptr[c + 1] - h->hs.colour_ptr[c];
-    const int e = cmfe::launch_mixed(h->hs, kp, h->num_sms, st, h->high_precision == FE_HIGH_PRECISION_DOUBLE_FLOAT);
-    if (e != 0) return set_error(FE_ERR_CUDA, std::string("residual kernel launch: ") + cudaGetErrorString((cudaError_t)e));
-    h->launches++;
-    if ((rc = surface_after(h, kp, c, 0, st))) return rc;
-  }
+  if ((rc = residual_run(h, dx, dr, st))) return rc;
   CUDA_TRY(cudaMemcpyAsync(r, dr, bytes, cudaMemcpyDefault, st));
   return finish_status(h, st);
 }

@@ -48,7 +48,8 @@ constexpr int align16(int x) { return (x + 15) & ~15; }
 // measured 17 % faster than two CTAs of 4 elements despite the register
 // spills the 80-register budget causes), 4 for element-based pressure, 8 for
 // trilinear elements.
-template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8), class T = float, int NT = 256>
+// RES: the residual alone (no displacement block, no coupling).
+template <int N1, int PM, int EG_ = (N1 == 3 ? (PM ? 3 : 4) : 8), class T = float, int NT = 256, bool RES = false>
 struct MixCfg {
   static constexpr int MINB = (N1 == 3 && PM) ? 3 : 2;  // CTAs per SM the launch bounds ask for
   static constexpr int NPE = N1 * N1 * N1;
@@ -58,7 +59,8 @@ struct MixCfg {
   static constexpr int NROW = NU3 + NPP;
   static constexpr int THREADS = NT;
   static constexpr int EG = EG_;                // elements per group
-  static constexpr int REC64 = 20;  // P(9), A(9), t1, pad
+  static constexpr int REC64 = RES ? 11 : 20;  // P(9), A(9), t1, pad; RES: P(9), t1, pad
+  static constexpr int T1 = RES ? 9 : 18;      // place of t1
   static constexpr int O_PSI64 = 0;
   static constexpr int O_W = align16(O_PSI64 + NG * 8 * 8);
   // constant tables first, then the per-group scratch from O_Z on (the fused
@@ -72,15 +74,15 @@ struct MixCfg {
   static constexpr int L2 = 2 * N1;                               // linear x 1-D basis products of a line
   static constexpr int T1S = EG * 3 * L2 * 9 * 8;                 // coupling, per component: stage 1
   static constexpr int W2S = EG * L2 * L2 * 3 * 8;                //   and each of the two stage-2 arrays
-  static constexpr int P3S = PM ? 3 * T1S + 6 * W2S : 0;
-  static constexpr int RECS = EG * NG * UU_REC * (int)sizeof(T);
+  static constexpr int P3S = PM && !RES ? 3 * T1S + 6 * W2S : 0;
+  static constexpr int RECS = RES ? 0 : EG * NG * UU_REC * (int)sizeof(T);
   static constexpr int O_R32 = align16(O_R64 + EG * NG * REC64 * 8);
   // the gradients and the FP64 stages' scratch share their space with the
   // warps' stage-1 values of the displacement block
   static constexpr int O_DZ = align16(O_R32 + (RECS > P1S ? RECS : P1S));
   static constexpr int P3R = EG * (9 * N1 * 9 + 6 * N1 * N1 * 3 + 64) * 8;  // scratch of the residual stages
   static constexpr int O_U1 = O_DZ, O_U2 = O_U1 + EG * 9 * N1 * 9 * 8, O_U3 = O_U2 + EG * 6 * N1 * N1 * 3 * 8;
-  static constexpr int WS1 = THREADS / 32 * UUCfg<N1>::S1 * (int)sizeof(T);
+  static constexpr int WS1 = RES ? 0 : THREADS / 32 * UUCfg<N1>::S1 * (int)sizeof(T);
   static constexpr int big(int x, int y) { return x > y ? x : y; }
   static constexpr int O_BASE = align16(O_DZ + big(big(EG * NG * 9 * 8, WS1), big(P3R, P3S)));
   // coloured order only: scatter addresses and rank tables of the group
@@ -92,6 +94,9 @@ struct MixCfg {
   static constexpr int GATHER_END = align16(O_Z + GroupGather<NPE, NPP, EG, THREADS, T>::SCRATCH);
   static constexpr int O_NODE1 = O_BASE > GATHER_END ? O_BASE : GATHER_END;
   static constexpr int SMEM1 = align16(O_NODE1 + EG * (NR + 1) * 4);
+  // residual alone: no row gathers in the scratch
+  static constexpr int O_NODE2 = O_BASE;
+  static constexpr int SMEM2 = align16(O_NODE2 + EG * (NR + 1) * 4);
 };
 
 // Block (m, n) of the lower-triangle displacement blocks: 0..2 diagonal,
@@ -246,13 +251,17 @@ __device__ __forceinline__ int elem_at(const KParams& P, const int32_t* elems, i
 // P3 (residual and coupling) and P4 (displacement block).  OUT = 0 adds the
 // element's entries into the CSR values and the residual (first contributor
 // in colour order stores, later ones add); OUT = 1 stores them into the
-// element's staging records (*SO), which the row gather sums afterwards.
+// element's staging records (*SO), which the row gather sums afterwards;
+// OUT = 2 forms the residual alone and stores it into the element's residual
+// record (cmfe::RecR).
 template <int N1, int PM, int EG_, class T, class H, int OUT = 0, int NT = 256>
 __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems, int count, int grp, bool p4_first,
                                           unsigned char* sm, const cmfe::StageOut* SO = nullptr) {
-  using C = MixCfg<N1, PM, EG_, T, NT>;
+  constexpr bool RES = OUT == 2;
+  using C = MixCfg<N1, PM, EG_, T, NT, RES>;
   constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, NU3 = C::NU3, EG = C::EG;
   using R = cmfe::Rec<NPE, NPP, T>;
+  using RR = cmfe::RecR<NPE, NPP>;
   H* s_psi = reinterpret_cast<H*>(sm + C::O_PSI64);  // [g][q]
   H* s_w = reinterpret_cast<H*>(sm + C::O_W);        // [g]
   H* s_z = reinterpret_cast<H*>(sm + C::O_Z);        // [el][c][a]
@@ -262,7 +271,7 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   H* s_r64 = reinterpret_cast<H*>(sm + C::O_R64);    // [el][g][REC64]
   T* s_D = reinterpret_cast<T*>(sm + C::O_R32);                // [el][g][UU_REC]
   T* s_mm = reinterpret_cast<T*>(sm + C::O_MM);
-  int* s_node = reinterpret_cast<int*>(sm + (OUT == 1 ? C::O_NODE1 : C::O_NODE0));  // [el][NR+1]
+  int* s_node = reinterpret_cast<int*>(sm + (OUT == 2 ? C::O_NODE2 : OUT == 1 ? C::O_NODE1 : C::O_NODE0));  // [el][NR+1]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // FP64 items are dealt to the warps from a different first warp in each
   // CTA of an SM: an SM sub-partition takes 64 cycles per FP64 warp
@@ -375,7 +384,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   // run at the same time on the two halves of the CTA, so that the FP64 and
   // the FP32 pipes overlap; P2b forms the kinematics it needs itself from
   // the same gradients.
-  constexpr int HALF = C::THREADS / 2;
+  // (The residual alone: P2 on all warps.)
+  constexpr int HALF = RES ? C::THREADS : C::THREADS / 2;
   if (vt < HALF) {
     for (int t = vt; t < EG * NG; t += HALF) {
       const int el = t / NG, g = t % NG;
@@ -410,7 +420,7 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
 #pragma unroll
         for (int n = 0; n < 3; ++n) {
           adj[k][n] = sw * adj[k][n];
-          rec[9 + k * 3 + n] = adj[k][n];
+          if (!RES) rec[9 + k * 3 + n] = adj[k][n];
         }
       if (P.r != nullptr) {
         H F[3][3], sig[3][3];
@@ -430,11 +440,11 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
             rec[k * 3 + m] = v;
             ok = ok && hfinite(v);
           }
-        rec[18] = w * (jz - jx);  // J_x w (J - 1)
+        rec[C::T1] = w * (jz - jx);  // J_x w (J - 1)
       }
       if (!ok) atomicOr(P.status, 1u);
     }
-  } else {
+  } else if constexpr (!RES) {
     for (int t = vt - HALF; t < (P.res_only ? 0 : EG * NG); t += HALF) {
       const int el = t / NG, g = t % NG;
       if (el >= nvalid) continue;
@@ -456,8 +466,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   // P3 (FP64 pipe) and P4 (displacement block) are independent; the
   // second wave of CTAs runs them in the opposite order so that the two
   // CTAs sharing an SM work on different pipes.
-  for (int ph = 0; ph < 2; ++ph) {
-    if ((ph == 0) != p4_first) {
+  for (int ph = 0; ph < (RES ? 1 : 2); ++ph) {
+    if (RES || (ph == 0) != p4_first) {
       // ---- P3: residual rows and pressure-coupling columns (high precision H)
       __syncthreads();
       constexpr int N2 = N1 * N1;
@@ -487,7 +497,7 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
         }
         if (PM && prows) {  // the pressure rows, on the warps the lines leave over
           for (int i = C::THREADS - 1 - vt; i < EG * 9; i += C::THREADS) {
-            const H* rec = &s_r64[(i / 9 * NG + 3 * (i % 9)) * C::REC64 + 18];
+            const H* rec = &s_r64[(i / 9 * NG + 3 * (i % 9)) * C::REC64 + C::T1];
             const H v[3] = {rec[0], rec[C::REC64], rec[2 * C::REC64]};
             H o[2];
             line_Lt<H>(v, o);
@@ -541,7 +551,7 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
           } else {
             for (int el = C::THREADS - 1 - vt; el < nvalid; el += C::THREADS) {
               H acc = hval<H>(0.0);
-              for (int g = 0; g < NG; ++g) acc = acc + s_r64[(el * NG + g) * C::REC64 + 18];
+              for (int g = 0; g < NG; ++g) acc = acc + s_r64[(el * NG + g) * C::REC64 + C::T1];
               emit_p(el, 0, acc);
             }
           }
@@ -566,6 +576,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
                 if constexpr (OUT == 1) {
                   unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
                   reinterpret_cast<double*>(er + a * R::ROW + R::OR)[m] = hd(o[a3]);
+                } else if constexpr (OUT == 2) {
+                  RR::of(*SO, elem_at(P, elems, grp * EG + el))[3 * a + m] = hd(o[a3]);
                 } else {
                   add_r(el, a, (size_t)m * nu + s_node[el * (NR + 1) + a], hd(o[a3]));
                 }
@@ -575,12 +587,15 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
               if constexpr (OUT == 1) {
                 unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
                 reinterpret_cast<double*>(er + R::P0 + q * R::PROW)[NU3] = hd(v);
+              } else if constexpr (OUT == 2) {
+                RR::of(*SO, elem_at(P, elems, grp * EG + el))[NU3 + q] = hd(v);
               } else {
                 add_r(el, NPE + q, (size_t)3 * nu + s_node[el * (NR + 1) + NPE + q], hd(v));
               }
             });
       }
       // one pressure-coupling entry K(q, (n, b)) and its mirror
+      if constexpr (!RES) {
       auto emit_c = [&](int el, int q, int n, int b, double kv) {
         if constexpr (OUT == 1) {
           unsigned char* er = SO->rec + (size_t)elem_at(P, elems, grp * EG + el) * R::BYTES;
@@ -672,7 +687,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
           P.vals[(size_t)P.cp_row_ptr[(size_t)3 * nu + pq] + 3 * (size_t)P.wp[pq] + (t & 0x7fff)] = 0.0;
         }
       }
-    } else {
+      }
+    } else if constexpr (!RES) {
       // ---- P4: displacement blocks by sum factorisation, warp by warp
       if (!P.res_only) {
         // Coloured order: scatter addresses staged in shared memory:

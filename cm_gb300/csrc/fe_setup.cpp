@@ -364,6 +364,17 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     for (int e = 0; e < s.ne; ++e) s.colour_elems[fillp[colour[e]]++] = e;
   }
 
+  s.u_inc_col = s.u_inc;
+  s.p_inc_col = s.p_inc;
+  parallel_for(s.nu, [&](int n) {
+    std::sort(s.u_inc_col.begin() + s.u_inc_ptr[n], s.u_inc_col.begin() + s.u_inc_ptr[n + 1],
+              [&](int32_t a, int32_t b) { return colour[a >> 5] < colour[b >> 5]; });
+  });
+  parallel_for(s.npn, [&](int q) {
+    std::sort(s.p_inc_col.begin() + s.p_inc_ptr[q], s.p_inc_col.begin() + s.p_inc_ptr[q + 1],
+              [&](int32_t a, int32_t b) { return colour[a >> 3] < colour[b >> 3]; });
+  });
+
   // Per-element rank / first-contributor tables.
   const int nr = s.nr;
   std::vector<uint16_t> etab((size_t)s.ne * nr * nr);

@@ -54,7 +54,8 @@ struct SurfWarpSmem {
 // shared scratch).  mode: 0 = CSR (FP64 values, or FP32 uu values when
 // P.vals_uu), 1 = element outputs (P.elem_out, elements first_elem ..
 // first_elem + count - 1), 2 = the element's record (displacement block in
-// T), which only this warp touches, so it adds without atomics.
+// T), which only this warp touches, so it adds without atomics; 3 = the
+// element's residual record.
 template <int N1, int NPP, class T = float>
 __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, const uint8_t* bmask, int mode,
                                                 int want_jac, SurfWarpSmem& S, int lane,
@@ -120,7 +121,7 @@ __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, c
     const uint16_t* tab = P.tables + (size_t)P.elem_table[e] * nr * nr;
     const int* en = P.elem_u + (size_t)e * NPE;
     // residual rows
-    if (P.r != nullptr || (mode == 1 && !want_jac) || mode == 2) {
+    if (P.r != nullptr || (mode == 1 && !want_jac) || mode >= 2) {
       if (lane < 3 * NF) {
         const int c = lane / NF, f = lane % NF;
         const double x3[3] = {(-sqrt(0.6) + 1.0) / 2.0, 0.5, (sqrt(0.6) + 1.0) / 2.0};
@@ -130,7 +131,9 @@ __device__ __forceinline__ void surface_element(const cmfe::KParams& P, int e, c
           acc = fma(S.gq[ng][0] * S.gq[ng][1 + c], N, acc);
         }
         const int a = S.node[f];
-        if (mode == 2) {
+        if (mode == 3) {
+          cmfe::RecR<NPE, NPP>::of(*SO, e)[3 * a + c] += acc;
+        } else if (mode == 2) {
           reinterpret_cast<double*>(SO->rec + (size_t)e * R::BYTES + a * R::ROW + R::OR)[c] += acc;
         } else if (mode == 1) {
           P.elem_out[(size_t)(e - P.first_elem) * nrow + c * NPE + a] += acc;
