@@ -33,6 +33,7 @@
 #include <new>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 
 #include "fe_internal.h"
 #include "fe_math.cuh"
@@ -466,6 +467,41 @@ int dev_upload(T** dst, const std::vector<T>& src) {
 
 }  // namespace
 
+namespace {
+// Host arrays to device memory in one allocation: small sets packed and copied
+// at once (an allocation and a copy take about 10 us each, and a mesh has
+// thirty arrays), large ones array by array.
+struct Upload {
+  struct Item {
+    void** dst;
+    const void* src;
+    size_t bytes, at;
+  };
+  std::vector<Item> items;
+  size_t total = 0;
+  template <class T>
+  void add(T** dst, const std::vector<T>& src) {
+    *dst = nullptr;
+    if (src.empty()) return;
+    items.push_back({reinterpret_cast<void**>(dst), src.data(), src.size() * sizeof(T), total});
+    total += (src.size() * sizeof(T) + 255) / 256 * 256;
+  }
+  int run(void** base) {
+    CUDA_TRY(cudaMalloc(base, total ? total : 256));
+    char* b = static_cast<char*>(*base);
+    if (total <= (size_t)8 << 20) {
+      std::vector<char> host(total);
+      for (const Item& i : items) std::memcpy(host.data() + i.at, i.src, i.bytes);
+      CUDA_TRY(cudaMemcpy(b, host.data(), total, cudaMemcpyHostToDevice));
+    } else {
+      for (const Item& i : items) CUDA_TRY(cudaMemcpy(b + i.at, i.src, i.bytes, cudaMemcpyHostToDevice));
+    }
+    for (const Item& i : items) *i.dst = b + i.at;
+    return FE_NO_ERROR;
+  }
+};
+}  // namespace
+
 // Device arrays that depend only on the mesh (connectivity, pattern, rank
 // tables, geometry cache, quadrature, colouring, incidence lists): owned
 // together and shared by the handles fe_clone makes from one set-up.
@@ -488,6 +524,7 @@ struct fe_equations_set {
   uint16_t* d_tables = nullptr;
   double *d_geo = nullptr, *d_geo_rj = nullptr, *d_mat = nullptr, *d_gbf_u = nullptr, *d_gbf_p = nullptr, *d_gw = nullptr;
   float* d_geo_dd = nullptr;
+  void* d_mesh = nullptr;  // the allocation that holds the mesh-only arrays (owned by `shared`)
   double* d_surfp = nullptr;
   int32_t* d_bnd_elems = nullptr;
   uint8_t* d_bnd_mask = nullptr;
@@ -544,6 +581,11 @@ struct fe_batch_s {
   unsigned barrier_polls = 0, barrier_extra = 0;  // grid-barrier limits (fe_batch_set_barrier_limits)
   unsigned type_mask = 0;             // element types present (bit 4: surface loads)
   double tuned_ms = -1.0;
+  // one launch per member: the stream of every slot (0: the caller's) and the
+  // batch's own streams and events
+  std::vector<int> slot_lane;
+  std::vector<cudaStream_t> lanes;
+  std::vector<cudaEvent_t> lane_events;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   int64_t graph_kernels = 0;  // kernels in the captured graph
@@ -1149,15 +1191,25 @@ int sync_table(fe_batch b, cudaStream_t st) {
 // launch copies into constant memory.
 int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t st) {
   if (b->variant == cmfe::batch_variants()) {
-    // one launch per member and colour: the single-set kernels, in member order
-    for (size_t s = 0; s < b->members.size(); ++s) {
+    // the single-set assembly of every member.  The members are independent,
+    // so they run on several streams and small ones share the GPU (24 boxes of
+    // 4 to 24 elements an edge: one after the other 3.4 ms, side by side 2.4)
+    const int nl = (int)b->lanes.size();
+    if (nl) CUDA_TRY(cudaEventRecord(b->lane_events[0], st));
+    for (int l = 0; l < nl; ++l) CUDA_TRY(cudaStreamWaitEvent(b->lanes[l], b->lane_events[0], 0));
+    int rc = FE_NO_ERROR;
+    for (size_t s = 0; s < b->members.size() && !rc; ++s) {
       const KParams& k = b->h_table[s].kp;
       fe_handle h = b->members[b->slot_member[s]];
+      cudaStream_t t = b->slot_lane[s] ? b->lanes[b->slot_lane[s] - 1] : st;
       std::lock_guard<std::mutex> lk(h->mu);
-      const int rc = mixed_assemble(h, k.x, k.vals_uu, k.vals, k.r, false, st, &b->launches);
-      if (rc) return rc;
+      rc = mixed_assemble(h, k.x, k.vals_uu, k.vals, k.r, false, t, &b->launches);
     }
-    return FE_NO_ERROR;
+    for (int l = 0; l < nl; ++l) {  // also after an error: the caller's stream follows what was queued
+      CUDA_TRY(cudaEventRecord(b->lane_events[l + 1], b->lanes[l]));
+      CUDA_TRY(cudaStreamWaitEvent(st, b->lane_events[l + 1], 0));
+    }
+    return rc;
   }
   CUDA_TRY(cudaMemsetAsync(b->d_sync, 0, 2 * sizeof(unsigned), st));
   cmfe::BatchArgs a;
@@ -1175,6 +1227,42 @@ int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t s
                                          b->num_sms, st);
   if (e != 0) return set_error(FE_ERR_CUDA, std::string("batched kernel launch: ") + cudaGetErrorString((cudaError_t)e));
   b->launches++;
+  return FE_NO_ERROR;
+}
+
+// Deals the members to at most kLanes streams, the largest first, each to the
+// stream with the fewest elements so far; one handle stays on one stream (its
+// records and counters serve one launch at a time).
+constexpr int kLanes = 8;
+int batch_lanes(fe_batch b) {
+  const size_t n = b->members.size();
+  std::vector<int> order(n);
+  for (size_t i = 0; i < n; ++i) order[i] = (int)i;
+  auto ne = [&](int slot) { return b->members[b->slot_member[slot]]->hs.ne; };
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return ne(x) > ne(y); });
+  std::vector<int64_t> load(kLanes, 0);
+  std::unordered_map<fe_handle, int> lane_of;
+  b->slot_lane.assign(n, 0);
+  int used = 0;
+  for (int slot : order) {
+    fe_handle h = b->members[b->slot_member[slot]];
+    auto it = lane_of.find(h);
+    const int l = it != lane_of.end() ? it->second : (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    lane_of[h] = l;
+    load[l] += ne(slot);
+    b->slot_lane[slot] = l;
+    used = std::max(used, l);
+  }
+  for (int l = 0; l < used; ++l) {
+    cudaStream_t s;
+    CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    b->lanes.push_back(s);
+  }
+  for (int l = 0; l <= used; ++l) {
+    cudaEvent_t e;
+    CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    b->lane_events.push_back(e);
+  }
   return FE_NO_ERROR;
 }
 
@@ -1242,17 +1330,6 @@ int device_pattern(fe_handle h, const int32_t** row_ptr, const int32_t** col, in
 }
 }  // namespace cmfe
 
-namespace {
-// The mesh-only device arrays of a handle (shared with its clones).
-std::vector<void*> shared_arrays(fe_handle h) {
-  return {h->d_bnd_elems, h->d_bnd_mask, h->d_geo_dd, h->d_elem_u, h->d_elem_p, h->d_row_ptr, h->d_uu_row_ptr,
-          h->d_cp_row_ptr, h->d_wu, h->d_wp, h->d_elem_table, h->d_colour_elems, h->d_tables, h->d_geo,
-          h->d_gbf_u, h->d_gbf_p, h->d_gw, h->d_u_inc_ptr, h->d_u_inc, h->d_p_inc_ptr, h->d_p_inc,
-          h->d_u_inc_row, h->d_p_inc_row, h->d_u_pat, h->d_pat, h->d_geo_rj,
-          h->d_u_inc_col, h->d_p_inc_col};
-}
-}  // namespace
-
 extern "C" {
 
 int fe_last_error(char* buf, int32_t size) {
@@ -1280,34 +1357,45 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   if (cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
     return fail(set_error(FE_ERR_CUDA, "cannot query the device"));
   const auto& s = h->hs;
-  if ((rc = dev_upload(&h->d_elem_u, s.elem_u)) || (rc = dev_upload(&h->d_elem_p, s.elem_p)) ||
-      (rc = dev_upload(&h->d_row_ptr, s.row_ptr)) || (rc = dev_upload(&h->d_uu_row_ptr, s.uu_row_ptr)) ||
-      (rc = dev_upload(&h->d_cp_row_ptr, s.cp_row_ptr)) || (rc = dev_upload(&h->d_wu, s.wu)) ||
-      (rc = dev_upload(&h->d_wp, s.wp)) || (rc = dev_upload(&h->d_elem_table, s.elem_table)) ||
-      (rc = dev_upload(&h->d_colour_elems, s.colour_elems)) || (rc = dev_upload(&h->d_tables, s.tables)) ||
-      (rc = dev_upload(&h->d_geo, s.geo)) || (rc = dev_upload(&h->d_geo_rj, s.geo_rj)) || (rc = dev_upload(&h->d_mat, s.mat)) ||
-      (rc = dev_upload(&h->d_gbf_u, s.gbf_u)) || (rc = dev_upload(&h->d_gbf_p, s.gbf_p)) ||
-      (rc = dev_upload(&h->d_gw, s.gw)))
-    return fail(rc);
-  {
-    std::vector<float> gdd(s.geo.size() * 2);
-    for (size_t i = 0; i < s.geo.size(); ++i) {
-      const float hi = (float)s.geo[i];
-      gdd[2 * i] = hi;
-      gdd[2 * i + 1] = (float)(s.geo[i] - (double)hi);
-    }
-    if ((rc = dev_upload(&h->d_geo_dd, gdd))) return fail(rc);
+  std::vector<float> gdd(s.geo.size() * 2);  // geo as (hi, lo) FP32 pairs
+  for (size_t i = 0; i < s.geo.size(); ++i) {
+    const float hi = (float)s.geo[i];
+    gdd[2 * i] = hi;
+    gdd[2 * i + 1] = (float)(s.geo[i] - (double)hi);
   }
-  if ((rc = dev_upload(&h->d_bnd_elems, s.bnd_elems)) || (rc = dev_upload(&h->d_bnd_mask, s.bnd_mask))) return fail(rc);
-  if ((rc = dev_upload(&h->d_u_inc_ptr, s.u_inc_ptr)) || (rc = dev_upload(&h->d_u_inc, s.u_inc)) ||
-      (rc = dev_upload(&h->d_p_inc_ptr, s.p_inc_ptr)) || (rc = dev_upload(&h->d_p_inc, s.p_inc)) ||
-      (rc = dev_upload(&h->d_u_inc_col, s.u_inc_col)) || (rc = dev_upload(&h->d_p_inc_col, s.p_inc_col)) ||
-      (rc = dev_upload(&h->d_u_inc_row, s.u_inc_row)) || (rc = dev_upload(&h->d_p_inc_row, s.p_inc_row)) || (rc = dev_upload(&h->d_u_pat, s.u_pat)) ||
-      (rc = dev_upload(&h->d_pat, s.pat)))
-    return fail(rc);
+  Upload up;
+  up.add(&h->d_elem_u, s.elem_u);
+  up.add(&h->d_elem_p, s.elem_p);
+  up.add(&h->d_row_ptr, s.row_ptr);
+  up.add(&h->d_uu_row_ptr, s.uu_row_ptr);
+  up.add(&h->d_cp_row_ptr, s.cp_row_ptr);
+  up.add(&h->d_wu, s.wu);
+  up.add(&h->d_wp, s.wp);
+  up.add(&h->d_elem_table, s.elem_table);
+  up.add(&h->d_colour_elems, s.colour_elems);
+  up.add(&h->d_tables, s.tables);
+  up.add(&h->d_geo, s.geo);
+  up.add(&h->d_geo_rj, s.geo_rj);
+  up.add(&h->d_geo_dd, gdd);
+  up.add(&h->d_gbf_u, s.gbf_u);
+  up.add(&h->d_gbf_p, s.gbf_p);
+  up.add(&h->d_gw, s.gw);
+  up.add(&h->d_bnd_elems, s.bnd_elems);
+  up.add(&h->d_bnd_mask, s.bnd_mask);
+  up.add(&h->d_u_inc_ptr, s.u_inc_ptr);
+  up.add(&h->d_u_inc, s.u_inc);
+  up.add(&h->d_p_inc_ptr, s.p_inc_ptr);
+  up.add(&h->d_p_inc, s.p_inc);
+  up.add(&h->d_u_inc_col, s.u_inc_col);
+  up.add(&h->d_p_inc_col, s.p_inc_col);
+  up.add(&h->d_u_inc_row, s.u_inc_row);
+  up.add(&h->d_p_inc_row, s.p_inc_row);
+  up.add(&h->d_u_pat, s.u_pat);
+  up.add(&h->d_pat, s.pat);
+  if ((rc = up.run(&h->d_mesh)) || (rc = dev_upload(&h->d_mat, s.mat))) return fail(rc);
   {
     auto owner = std::make_shared<SharedDeviceSetup>();
-    owner->ptrs = shared_arrays(h);
+    owner->ptrs = {h->d_mesh};
     h->shared = owner;
   }
   if (cudaMalloc(&h->d_status, sizeof(unsigned)) != cudaSuccess ||
@@ -1328,10 +1416,7 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
 
 int fe_destroy(fe_handle h) {
   if (!h) return FE_NO_ERROR;
-  if (!h->shared) {  // a handle whose creation failed part-way owns what it uploaded
-    for (void* p : shared_arrays(h))
-      if (p) cudaFree(p);
-  }
+  if (!h->shared && h->d_mesh) cudaFree(h->d_mesh);  // a handle whose creation failed part-way owns what it uploaded
   // per-handle state: materials, surface load, status word, staging and records
   void* own[] = {h->d_surfp, h->d_mat, h->d_status, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
                  h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64, h->d_rec_r,
@@ -1793,6 +1878,7 @@ int fe_batch_create(const fe_handle* handles, int32_t count, fe_batch* out) {
         o[b->ncol + 1 + c] = hs.bnd_ptr[std::min(c, hs.ncolours)];
       }
     }
+    if (!rc) rc = batch_lanes(b);
     b->surf_sig.assign((size_t)count, nullptr);
     if (!rc) rc = fail(cudaMalloc(&b->d_offsets, offsets.size() * sizeof(int32_t)));
     if (!rc) rc = fail(cudaMemcpy(b->d_offsets, offsets.data(), offsets.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -1815,6 +1901,8 @@ int fe_batch_destroy(fe_batch b) {
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_table) cudaFreeHost(b->h_table);
+  for (cudaEvent_t e : b->lane_events) cudaEventDestroy(e);
+  for (cudaStream_t s : b->lanes) cudaStreamDestroy(s);
   delete b;
   return FE_NO_ERROR;
 }
