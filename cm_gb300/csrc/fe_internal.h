@@ -170,13 +170,13 @@ struct FusedArgs {
   int g0, g1;      // element groups of this launch: [g0, g1)
 };
 
-// Launches the mixed-precision assembly kernel for one colour (fe_mixed.cu),
+// Launches the mixed-precision assembly kernel for one colour (fe_mixed_coloured.cu),
 // with the high-precision phases in FP64 or in double-float arithmetic.
 // Returns a cudaError_t value.
 int launch_mixed(const HostSetup& s, const KParams& kp, int num_sms, void* stream, bool double_float);
 
-// Elements per group of the fused kernel for this element type.
-int fused_group_size(const HostSetup& s);
+// Elements per group of the fused kernel for this element type and mesh size.
+int fused_group_size(const HostSetup& s, int num_sms, bool double_float);
 
 // Blocks of the fused kernel resident on the whole GPU at once (the groups
 // one wave of the launch takes); a negative cudaError_t on failure.

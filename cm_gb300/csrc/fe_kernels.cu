@@ -866,9 +866,9 @@ int mixed_fused(fe_handle h, const KParams& kp, const cmfe::StageOut& so, bool d
   return FE_NO_ERROR;
 }
 
-int64_t fused_groups(const HostSetup& s) {
-  const int eg = cmfe::fused_group_size(s);
-  return (s.ne + eg - 1) / eg;
+int64_t fused_groups(fe_handle h, bool double_float) {
+  const int eg = cmfe::fused_group_size(h->hs, h->num_sms, double_float);
+  return (h->hs.ne + eg - 1) / eg;
 }
 
 int ensure_records(fe_handle h) {
@@ -893,12 +893,11 @@ KParams staged_params(fe_handle h, const double* dx, float* du, double* dc, doub
 // when count is set.
 int mixed_staged(fe_handle h, const double* dx, float* du, double* dc, double* dr, bool double_float,
                  cudaStream_t st, int64_t* count) {
-  const auto& s = h->hs;
   int rc;
   if ((rc = ensure_records(h))) return rc;
   const KParams kp = staged_params(h, dx, du, dc, dr);
   const cmfe::StageOut so{h->d_rec};
-  return mixed_fused(h, kp, so, double_float, st, {0, fused_groups(s)}, nullptr, count);
+  return mixed_fused(h, kp, so, double_float, st, {0, fused_groups(h, double_float)}, nullptr, count);
 }
 
 // Streamed host outputs: the fused assembly in chunks of element groups into
@@ -912,7 +911,7 @@ int mixed_streamed(fe_handle h, const double* dx, float* du, double* dc, double*
   const auto& s = h->hs;
   int rc;
   if ((rc = ensure_records(h))) return rc;
-  const int64_t groups = fused_groups(s);
+  const int64_t groups = fused_groups(h, double_float);
   const int wave = cmfe::fused_wave(s, h->num_sms, double_float);
   if (wave <= 0)
     return set_error(FE_ERR_CUDA, std::string("fused kernel occupancy: ") + cudaGetErrorString((cudaError_t)-wave));
@@ -947,7 +946,7 @@ int mixed_streamed(fe_handle h, const double* dx, float* du, double* dc, double*
   cudaEvent_t* ev = h->chunk_events.data();
   if ((rc = mixed_fused(h, kp, so, double_float, st, bounds, ev, nullptr))) return rc;
   cudaStream_t cs = h->copy_stream;
-  const int nu = s.nu, npn = s.npn, EG = cmfe::fused_group_size(s);
+  const int nu = s.nu, npn = s.npn, EG = cmfe::fused_group_size(s, h->num_sms, double_float);
   auto copy_rows = [&](int64_t r0, int64_t r1) -> int {
     if (r1 <= r0) return FE_NO_ERROR;
     if (hu && r0 < 3 * (int64_t)nu) {

@@ -364,17 +364,6 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     for (int e = 0; e < s.ne; ++e) s.colour_elems[fillp[colour[e]]++] = e;
   }
 
-  s.u_inc_col = s.u_inc;
-  s.p_inc_col = s.p_inc;
-  parallel_for(s.nu, [&](int n) {
-    std::sort(s.u_inc_col.begin() + s.u_inc_ptr[n], s.u_inc_col.begin() + s.u_inc_ptr[n + 1],
-              [&](int32_t a, int32_t b) { return colour[a >> 5] < colour[b >> 5]; });
-  });
-  parallel_for(s.npn, [&](int q) {
-    std::sort(s.p_inc_col.begin() + s.p_inc_ptr[q], s.p_inc_col.begin() + s.p_inc_ptr[q + 1],
-              [&](int32_t a, int32_t b) { return colour[a >> 3] < colour[b >> 3]; });
-  });
-
   // Per-element rank / first-contributor tables.
   const int nr = s.nr;
   std::vector<uint16_t> etab((size_t)s.ne * nr * nr);
@@ -456,11 +445,29 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     s.ntables = (int)seen.size();
   }
   if ((int64_t)s.ntables * nr >= (1ll << 31)) return fail(msg, "too many distinct rank tables");
+  // The incidences of every node: rank-table rows in element order, the
+  // incidences again in colour order, and a hash of a u node's rows.
   s.u_inc_row.resize(s.u_inc.size());
   s.p_inc_row.resize(s.p_inc.size());
-  parallel_for((int)s.u_inc.size(), [&](int k) { s.u_inc_row[k] = s.elem_table[s.u_inc[k] >> 5] * nr + (s.u_inc[k] & 31); });
-  parallel_for((int)s.p_inc.size(),
-               [&](int k) { s.p_inc_row[k] = s.elem_table[s.p_inc[k] >> 3] * nr + s.npe + (s.p_inc[k] & 7); });
+  s.u_inc_col = s.u_inc;
+  s.p_inc_col = s.p_inc;
+  std::vector<uint64_t> row_hash(s.nu);
+  parallel_for(s.nu + s.npn, [&](int i) {
+    const bool un = i < s.nu;
+    const int n = un ? i : i - s.nu, bits = un ? 5 : 3, off = un ? 0 : s.npe;
+    const auto& ptr = un ? s.u_inc_ptr : s.p_inc_ptr;
+    const auto& inc = un ? s.u_inc : s.p_inc;
+    auto& row = un ? s.u_inc_row : s.p_inc_row;
+    auto& col = un ? s.u_inc_col : s.p_inc_col;
+    uint64_t hash = 1469598103934665603ull;
+    for (int32_t k = ptr[n]; k < ptr[n + 1]; ++k) {
+      row[k] = s.elem_table[inc[k] >> bits] * nr + off + (inc[k] & ((1 << bits) - 1));
+      hash = (hash ^ (uint64_t)(uint32_t)row[k]) * 1099511628211ull;
+    }
+    if (un) row_hash[n] = hash;
+    std::sort(col.begin() + ptr[n], col.begin() + ptr[n + 1],
+              [&](int32_t x, int32_t y) { return colour[x >> bits] < colour[y >> bits]; });
+  });
 
   // Column patterns of the u nodes' rows, shared by nodes with equal
   // rank-table rows (a node's incidences in element order).
@@ -475,9 +482,7 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     auto row_of = [&](int32_t k) { return s.u_inc_row[k]; };
     for (int n = 0; n < s.nu; ++n) {
       const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
-      uint64_t hash = 1469598103934665603ull;
-      for (int32_t j = 0; j < cnt; ++j) hash = (hash ^ (uint64_t)(uint32_t)row_of(k0 + j)) * 1099511628211ull;
-      auto it = head.emplace(hash, -1).first;
+      auto it = head.emplace(row_hash[n], -1).first;
       int32_t id = it->second;
       for (; id >= 0; id = seen[id].next) {
         const int32_t o0 = s.u_inc_ptr[seen[id].node];
