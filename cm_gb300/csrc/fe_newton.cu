@@ -296,6 +296,358 @@ __global__ void __launch_bounds__(NT) k_update_norm(int64_t n, const double* __r
   }
 }
 
+// One GMRES cycle in one cooperative launch, for systems whose rows fit the
+// SMs' shared memory: block b holds the matrix entries of rows [bound[b],
+// bound[b + 1]) (as many as fit; the rest is read from L2), the basis vectors'
+// and w's entries of these rows, and one more block turns the Hessenberg
+// columns into the triangular system while the others form the next product.
+// What crosses SMs is the preconditioned vector z and the blocks' shares of
+// the dots: three grid barriers an iteration.
+struct CycleArgs {
+  int n, nb, restart, kmax, cap;
+  int* bound;  // [nb + 1]
+  double beta, tol, breakdown;
+  const int32_t *rp, *col;
+  const double *vals, *minv, *b;
+  const uint8_t* free_dof;
+  double *res, *dx, *z, *part, *part2, *npart, *y;
+  int* ctl;      // [0] barrier arrivals, [1] the cycle has converged; zeroed before the launch
+  double* host;  // page-locked: squared norm of the true residual, iterations, converged
+};
+
+constexpr int CT = 512;                  // threads
+constexpr int CYCLE_ROWS = 64;           // rows of a block at most
+constexpr int LD = CYCLE_ROWS + 1;       // between basis vectors in shared memory
+constexpr int MAX_SHARES = 160;          // blocks at most
+constexpr unsigned CYCLE_POLLS = 1u << 21;  // a barrier gives up after about a second
+
+// Row bounds of k_cycle's blocks: equal shares of entries + 64 x rows (a row's
+// reduction takes as long as 64 entries), no block above CYCLE_ROWS rows.
+__global__ void __launch_bounds__(MAX_SHARES + 32) k_cycle_bounds(int n, int nb, const int32_t* __restrict__ rp,
+                                                                  int* __restrict__ bound) {
+  __shared__ int at[MAX_SHARES + 1];
+  const int b = threadIdx.x;
+  if (b <= nb) {
+    const int64_t target = ((int64_t)rp[n] + 64 * (int64_t)n) * b / nb;
+    int lo = 0, hi = n;  // first row whose share starts at or after the target
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (rp[mid] + 64 * (int64_t)mid < target) lo = mid + 1;
+      else hi = mid;
+    }
+    at[b] = lo;
+  }
+  __syncthreads();
+  if (b == 0) {
+    int prev = 0;
+    bound[0] = 0;
+    for (int i = 1; i <= nb; ++i) {
+      const int least = max(prev, n - (nb - i) * CYCLE_ROWS);
+      bound[i] = prev = min(max(at[i], least), min(prev + CYCLE_ROWS, n));
+    }
+  }
+}
+
+// Grid barrier number k = 1, 2, ... of the launch; false when it gave up.
+__device__ __forceinline__ bool cycle_barrier(int* arrivals, int k) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrivals, 1);
+    const int target = k * (int)gridDim.x;
+    unsigned polls = 0;
+    int v;
+    do {
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(arrivals) : "memory");
+    } while (v < target && ++polls < CYCLE_POLLS);
+    ok = v >= target;
+    __threadfence();
+  }
+  __syncthreads();
+  return ok;
+}
+
+// Squared norm of the vector whose blocks' shares npart holds (one warp).
+__device__ __forceinline__ double cycle_norm(const double* __restrict__ npart, int nb) {
+  double v[MAX_SHARES / 32], t = 0.0;
+#pragma unroll
+  for (int u = 0; u < MAX_SHARES / 32; ++u) {
+    const int c = (threadIdx.x & 31) + 32 * u;
+    v[u] = c < nb ? __ldcg(npart + c) : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < MAX_SHARES / 32; ++u) t += v[u];
+  return group_sum<32>(t);
+}
+
+// h[j] = sum over the blocks of part[j nb + block], j < m: eight lanes to a j.
+__device__ __forceinline__ void cycle_sums(const double* __restrict__ part, int nb, int m, double* h) {
+  const int q = threadIdx.x & 7;
+  for (int j0 = 0; j0 < m; j0 += CT / 8) {
+    const int j = j0 + (threadIdx.x >> 3);
+    if ((threadIdx.x >> 5) * 4 + j0 >= m) continue;  // whole warps
+    double v[MAX_SHARES / 8], s = 0.0;
+#pragma unroll
+    for (int u = 0; u < MAX_SHARES / 8; ++u) v[u] = j < m && q + 8 * u < nb ? __ldcg(part + j * nb + q + 8 * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < MAX_SHARES / 8; ++u) s += v[u];
+    s = group_sum<8>(s);
+    if (j < m && q == 0) h[j] = s;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleArgs A) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ double red[CYCLE_ROWS / 8], s_scale;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = tid & 3, grp = tid >> 2;
+  const bool givens = (int)blockIdx.x == A.nb;
+  const int r0 = givens ? A.n : A.bound[blockIdx.x];
+  const int rows = givens ? 0 : A.bound[blockIdx.x + 1] - r0;
+  const bool row_warp = warp * 8 < rows;  // warps with a row in combine()
+  int bar = 0;
+  double* h = sm;              // [MAX_BASIS]
+  double* c = h + MAX_BASIS;   // [MAX_BASIS]: the Hessenberg column (the last block)
+  double* V = c + MAX_BASIS;   // [restart][LD]
+  double* w = V + (size_t)A.restart * LD;
+  double* wn = w + LD;         // the product
+  double* mi = wn + LD;
+  double* sval = mi + LD;      // [cap]
+  int32_t* rps = reinterpret_cast<int32_t*>(sval + A.cap);  // [CYCLE_ROWS + 1]
+  uint16_t* scol = reinterpret_cast<uint16_t*>(rps + CYCLE_ROWS + 1);
+  // the last block's arrays take the place of the matrix
+  double *cs = V, *sn = cs + A.restart, *g = sn + A.restart, *xs = g + A.restart + 1, *pr = xs + A.restart + 1,
+         *U = pr + A.restart;  // U: packed columns of the triangular matrix
+
+  if (!givens) {
+    for (int r = tid; r <= rows; r += CT) rps[r] = A.rp[r0 + r];
+    __syncthreads();
+    const int e0 = rps[0], cnt = min(rps[rows] - e0, A.cap);
+    for (int e = tid; e < cnt; e += CT) {
+      sval[e] = A.vals[e0 + e];
+      scol[e] = (uint16_t)A.col[e0 + e];
+    }
+    for (int r = tid; r < rows; r += CT) {
+      const double m = A.minv[r0 + r], v = A.res[r0 + r] * (1.0 / A.beta);
+      mi[r] = m;
+      V[r] = v;
+      A.z[r0 + r] = m * v;
+    }
+  } else if (tid == 0) {
+    g[0] = A.beta;
+  }
+
+  // wn = P A x on the block's rows: a warp takes two rows (k_spmv)
+  auto product = [&](const double* x) {
+    const int e0 = rps[0];
+    for (int i = 2 * warp; i < rows; i += 2 * (CT / 32)) {
+      double s[2] = {0.0, 0.0};
+      int at[2], end[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const bool in = i + r < rows && A.free_dof[r0 + i + r];
+        at[r] = in ? rps[i + r] - e0 + lane : lane;
+        end[r] = in ? rps[i + r + 1] - e0 : 0;
+      }
+      while (__any_sync(0xffffffffu, at[0] < end[0] || at[1] < end[1])) {
+        double xv[2][8], av[2][8];
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int e = at[r] + 32 * u;
+            const bool in = e < end[r], near = e < A.cap;
+            xv[r][u] = in ? __ldcg(x + (near ? (int)scol[e] : A.col[e0 + e])) : 0.0;
+            av[r][u] = in ? (near ? sval[e] : A.vals[e0 + e]) : 0.0;
+          }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (at[r] - lane + 32 * u < end[r]) s[r] = fma(av[r][u], xv[r][u], s[r]);  // whole warps
+          at[r] += 256;
+        }
+      }
+      const bool hi = lane & 16;
+      double t = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if ((lane & 15) == 0 && i + (hi ? 1 : 0) < rows) wn[i + (hi ? 1 : 0)] = t;
+    }
+    __syncthreads();
+  };
+  // the block's shares of V_j . w, j < m
+  auto dots = [&](int m, double* part) {
+    for (int j0 = 0; j0 < m; j0 += CT / 4) {
+      const int j = j0 + grp;
+      if (warp * 8 + j0 >= m) continue;
+      double s = 0.0;
+      if (j < m) {
+#pragma unroll 8
+        for (int r = q; r < rows; r += 4) s = fma(V[j * LD + r], w[r], s);
+      }
+      s = group_sum<4>(s);
+      if (j < m && q == 0) part[j * A.nb + blockIdx.x] = s;
+    }
+  };
+  // sum_j h[j] V_j on row grp (the row's four lanes; whole warps)
+  auto combine = [&](int m) {
+    double s = 0.0;
+    if (grp < rows) {
+#pragma unroll 8
+      for (int j = q; j < m; j += 4) s = fma(h[j], V[j * LD + grp], s);
+    }
+    return group_sum<4>(s);
+  };
+  // the block's share of a squared norm, v on the threads with q == 0
+  auto norm_share = [&](double v) {
+    if (row_warp) {
+      double t = (q == 0 && grp < rows) ? v * v : 0.0;
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) red[warp] = t;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const double t = group_sum<8>(lane < 8 && lane * 8 < rows ? red[lane] : 0.0);
+      if (lane == 0) A.npart[blockIdx.x] = t;
+    }
+  };
+  // column k of the Hessenberg matrix: the previous rotations, then the one
+  // that zeroes its last entry (the last block, all threads); true when the
+  // cycle has converged or broken down
+  auto rotate = [&](int k) -> bool {
+    __syncthreads();
+    for (int i = tid; i < k; i += CT) pr[i] = cs[i] * c[i + 1];
+    __syncthreads();
+    double* Uk = U + k * (k + 1) / 2;
+    if (tid == 0) {
+      double x = c[0];
+      xs[0] = x;
+      for (int i = 0; i < k; ++i) xs[i + 1] = x = fma(-sn[i], x, pr[i]);
+      const double bb = c[k + 1], den = hypot(x, bb);
+      const double ck = den > 0.0 ? x / den : 1.0, sk = den > 0.0 ? bb / den : 0.0;
+      Uk[k] = den;
+      cs[k] = ck;
+      sn[k] = sk;
+      g[k + 1] = -sk * g[k];
+      g[k] = ck * g[k];
+    }
+    __syncthreads();
+    for (int i = tid; i < k; i += CT) Uk[i] = fma(cs[i], xs[i], sn[i] * c[i + 1]);
+    return fabs(g[k + 1]) <= A.tol || c[k + 1] <= A.breakdown;
+  };
+
+  if (!cycle_barrier(A.ctl, ++bar)) return;
+  int K = 0;
+  bool converged = false;
+  for (int k = 0;; ++k) {
+    const int m = k + 1;
+    if (!givens) {
+      // the last warp, which has the fewest rows, scales by the norm first
+      if (warp == CT / 32 - 1) {
+        const double t = k ? cycle_norm(A.npart, A.nb) : 1.0;
+        if (lane == 0) s_scale = t > 0.0 ? rsqrt(t) : 0.0;
+      }
+      product(A.z);
+      for (int r = tid; r < rows; r += CT) {
+        if (k) V[k * LD + r] = s_scale * w[r];
+        w[r] = s_scale * wn[r];
+      }
+      __syncthreads();
+      dots(m, A.part);
+    } else if (k) {
+      if (warp == 0) {
+        const double t = cycle_norm(A.npart, A.nb);
+        if (lane == 0) c[k] = sqrt(t);
+      }
+      converged = rotate(k - 1);
+      if (converged && tid == 0) A.ctl[1] = 1;
+    }
+    if (!cycle_barrier(A.ctl, ++bar)) return;
+    if (k && __ldcg(A.ctl + 1)) {  // column k - 1 was the last one
+      K = k;
+      break;
+    }
+    cycle_sums(A.part, A.nb, m, h);
+    if (!givens) {
+      if (row_warp) {
+        const double s = combine(m);
+        if (grp < rows && q == 0) w[grp] -= s;
+      }
+      __syncthreads();
+      dots(m, A.part2);
+    } else {
+      for (int j = tid; j < m; j += CT) c[j] = h[j];
+    }
+    if (!cycle_barrier(A.ctl, ++bar)) return;
+    cycle_sums(A.part2, A.nb, m, h);
+    if (!givens) {
+      double t = 0.0;
+      if (row_warp) {
+        const double s = combine(m);
+        if (grp < rows && q == 0) {
+          t = w[grp] - s;
+          w[grp] = t;
+          A.z[r0 + grp] = mi[grp] * t;
+        }
+      }
+      norm_share(t);
+    } else {
+      for (int j = tid; j < m; j += CT) c[j] += h[j];
+    }
+    if (!cycle_barrier(A.ctl, ++bar)) return;
+    if (m == A.kmax) {
+      if (givens) {
+        if (warp == 0) {
+          const double t = cycle_norm(A.npart, A.nb);
+          if (lane == 0) c[m] = sqrt(t);
+        }
+        converged = rotate(k);
+      }
+      K = m;
+      break;
+    }
+  }
+  // the cycle's correction: U y = g, dx += M^-1 V y
+  if (givens) {
+    __syncthreads();
+    for (int i = K - 1; i >= 0; --i) {
+      const double* Ui = U + i * (i + 1) / 2;
+      const double yi = Ui[i] != 0.0 ? g[i] / Ui[i] : 0.0;
+      __syncthreads();
+      if (tid == 0) A.y[i] = yi;
+      for (int j = tid; j < i; j += CT) g[j] = fma(-Ui[j], yi, g[j]);
+      __syncthreads();
+    }
+  }
+  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (!givens) {
+    for (int j = tid; j < K; j += CT) h[j] = __ldcg(A.y + j);
+    __syncthreads();
+    const double s = row_warp ? combine(K) : 0.0;
+    if (grp < rows && q == 0) A.dx[r0 + grp] = fma(mi[grp], s, A.dx[r0 + grp]);
+  }
+  if (!cycle_barrier(A.ctl, ++bar)) return;
+  // the true residual and its norm
+  if (!givens) {
+    product(A.dx);
+    double t = 0.0;
+    if (grp < rows && q == 0) A.res[r0 + grp] = t = A.b[r0 + grp] - wn[grp];
+    norm_share(t);
+  }
+  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (givens && warp == 0) {
+    const double r2 = cycle_norm(A.npart, A.nb);
+    if (lane == 0) {
+      A.host[0] = r2;
+      A.host[1] = K;
+      A.host[2] = converged ? 1.0 : 0.0;
+    }
+  }
+}
+
 // v = a * x, z = minv .* v
 __global__ void __launch_bounds__(NT) k_scale_precond(int64_t n, double a, const double* __restrict__ minv,
                                                       const double* __restrict__ x, double* __restrict__ v,
@@ -416,6 +768,8 @@ struct Solver {
   cudaStream_t capture = nullptr;
   int64_t cycles = 0;
   bool no_graphs = false;
+  CycleArgs cyc{};     // of k_cycle, when the system takes it
+  size_t cyc_smem = 0;  // 0: it does not
 
   Solver() = default;
   Solver(const Solver&) = delete;
@@ -506,6 +860,79 @@ struct Solver {
     return FE_NO_ERROR;
   }
 
+  // Rows and shared memory of k_cycle for this system; cyc_smem stays 0 when
+  // it has more rows than the blocks take.
+  void plan_cycle(int* ctl, int* bound) {
+    int dev = 0, sms = 0, smem = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop || sms < 2)
+      return;
+    // a block has 16 rows or more while that many blocks are not all in use
+    const int nb = (int)std::min<int64_t>(std::min(sms - 1, MAX_SHARES), (n + 15) / 16);
+    if (n > (int64_t)nb * CYCLE_ROWS || n > 65535 || nnz > INT32_MAX) return;
+    const int64_t fixed = 8 * (2 * MAX_BASIS + (restart + 3) * LD) + 4 * (CYCLE_ROWS + 1);
+    const int64_t last = 8 * (2 * (int64_t)MAX_BASIS + 5 * (restart + 1) + (int64_t)restart * (restart + 1) / 2);
+    const int64_t room = smem - 1024;  // the kernel's static arrays
+    const int64_t cap = (room - fixed) / 10;
+    if (cap < 0 || last > room) return;
+    if (cudaFuncSetAttribute(k_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    CycleArgs& a = cyc;
+    a.n = (int)n;
+    a.nb = nb;
+    a.restart = restart;
+    a.cap = (int)cap;
+    a.rp = rp;
+    a.col = col;
+    a.vals = vals;
+    a.minv = minv;
+    a.free_dof = free_dof;
+    a.z = z;
+    a.part = part;
+    a.part2 = part2;
+    a.npart = npart;
+    a.y = col_d;
+    a.ctl = ctl;
+    a.bound = bound;
+    a.host = pinned;
+    k_cycle_bounds<<<1, MAX_SHARES + 32, 0, st>>>((int)n, nb, rp, bound);
+    if (cudaGetLastError() == cudaSuccess) cyc_smem = (size_t)room;
+  }
+
+  // One cycle of at most kmax iterations by k_cycle; *ran false when the GPU
+  // cannot hold its blocks at once.
+  int cycle(const double* b, double* res, double* dx, double beta, double tol, int kmax, bool* ran, int* K,
+            bool* converged, double* r2) {
+    CycleArgs a = cyc;
+    a.b = b;
+    a.res = res;
+    a.dx = dx;
+    a.beta = beta;
+    a.tol = tol;
+    a.breakdown = 1e-14 * beta;
+    a.kmax = kmax;
+    NT_TRY(cudaMemsetAsync(a.ctl, 0, 2 * sizeof(int), st));
+    pinned[1] = -1.0;
+    void* args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_cycle, dim3(a.nb + 1), dim3(CT), args, cyc_smem, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      cudaGetLastError();
+      *ran = false;
+      return FE_NO_ERROR;
+    }
+    NT_TRY(e);
+    NT_TRY(cudaStreamSynchronize(st));
+    if (pinned[1] < 0.0) return cmfe::record_error(FE_ERR_CUDA, "a grid barrier of the GMRES cycle gave up");
+    *ran = true;
+    *r2 = pinned[0];
+    *K = (int)pinned[1];
+    *converged = pinned[2] != 0.0;
+    return FE_NO_ERROR;
+  }
+
   // Right-preconditioned GMRES(restart) for A dx = b (b on free dofs, dx
   // zero on fixed ones); returns the iterations in *its.
   int gmres(const double* b, double* dx, double rtol, int max_it, int64_t* its) {
@@ -523,6 +950,20 @@ struct Solver {
     std::vector<double> col_h(restart + 2);
     while (*its < max_it) {
       if (beta <= rtol * bnorm) break;
+      if (cyc_smem) {
+        bool ran = false, conv = false;
+        int K = 0;
+        double r2 = 0.0;
+        const int kmax = (int)std::min<int64_t>(restart, max_it - *its);
+        if ((rc = cycle(b, res, dx, beta, rtol * bnorm, kmax, &ran, &K, &conv, &r2))) return rc;
+        if (ran) {
+          *its += K;
+          beta = std::sqrt(r2);
+          if (conv && beta <= rtol * bnorm) break;
+          continue;
+        }
+        cyc_smem = 0;
+      }
       std::fill(g.begin(), g.end(), 0.0);
       g[0] = beta;
       int k = 0;
@@ -621,6 +1062,7 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   Work W;
   double *dx_state, *fvals;
   int32_t* fdofs;
+  int* bound;
   const size_t rs = (size_t)S.restart;
   const size_t basis = rs + 1;
   int64_t chunks = (n + 63) / 64;
@@ -629,19 +1071,28 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   for (double** p : {&S.r, &S.rn, &S.d, &S.xs, &S.w, &S.minv, &S.diag, &S.z, &dx_state}) W.add(p, (size_t)n);
   W.add(&S.V, (basis + 1) * n);
   W.add(&S.col_d, 2 * (rs + 2));
-  W.add(&S.part, (basis + 1) * MAX_CHUNKS);
-  W.add(&S.part2, (basis + 1) * MAX_CHUNKS);
-  W.add(&S.npart, MAX_CHUNKS);
+  int sms = 0;
+  {
+    int dev = 0;
+    NT_TRY(cudaGetDevice(&dev));
+    NT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const size_t shares = (size_t)std::max(MAX_CHUNKS, sms);
+  W.add(&S.part, (basis + 1) * shares);
+  W.add(&S.part2, (basis + 1) * shares);
+  W.add(&S.npart, shares);
   W.add(&S.scal, 4);
   W.add(&S.done, 4);
+  W.add(&bound, MAX_SHARES + 1);
   W.add(&S.free_dof, (size_t)n);
   W.add(&fvals, num_fixed > 0 ? num_fixed : 1);
   W.add(&fdofs, num_fixed > 0 ? num_fixed : 1);
-  if ((rc = W.alloc(2 * (rs + 2)))) return rc;
+  if ((rc = W.alloc(2 * (rs + 2) + 4))) return rc;
   S.graphs.assign(rs, nullptr);
   S.no_graphs = cudaStreamCreateWithFlags(&S.capture, cudaStreamNonBlocking) != cudaSuccess;
   S.pinned = W.pinned;
   S.ev = W.ev;
+  S.plan_cycle(S.done + 1, bound);
   cudaStream_t st = S.st;
   // the state on the device (x may be host memory)
   cudaPointerAttributes pa;
