@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(NT) k_update_norm(int64_t n, const double* __r
 // and w's entries of these rows, and one more block turns the Hessenberg
 // columns into the triangular system while the others form the next product.
 // What crosses SMs is the preconditioned vector z and the blocks' shares of
-// the dots: three grid barriers an iteration.
+// the dots and the norm: three grid barriers an iteration (blocks that poll
+// the shares themselves until all have come take twice the time).
 struct CycleArgs {
   int n, nb, restart, kmax, cap;
   int* bound;  // [nb + 1]
@@ -311,7 +312,8 @@ struct CycleArgs {
   const double *vals, *minv, *b;
   const uint8_t* free_dof;
   double *res, *dx, *z, *part, *part2, *npart, *y;
-  int* ctl;      // [0] barrier arrivals, [1] the cycle has converged; zeroed before the launch
+  double* scale;  // 1 / norm of the newest basis vector, -1: converged
+  int* ctl;       // barrier arrivals; zeroed before the launch
   double* host;  // page-locked: squared norm of the true residual, iterations, converged
 };
 
@@ -319,20 +321,20 @@ constexpr int CT = 512;                  // threads
 constexpr int CYCLE_ROWS = 64;           // rows of a block at most
 constexpr int LD = CYCLE_ROWS + 1;       // between basis vectors in shared memory
 constexpr int MAX_SHARES = 160;          // blocks at most
-constexpr unsigned CYCLE_POLLS = 1u << 21;  // a barrier gives up after about a second
+constexpr unsigned CYCLE_POLLS = 1u << 21;  // a wait gives up after about a second
 
-// Row bounds of k_cycle's blocks: equal shares of entries + 64 x rows (a row's
-// reduction takes as long as 64 entries), no block above CYCLE_ROWS rows.
+// Row bounds of k_cycle's blocks: equal shares of entries + 24 x rows (a row's
+// reduction takes as long as 24 entries), no block above CYCLE_ROWS rows.
 __global__ void __launch_bounds__(MAX_SHARES + 32) k_cycle_bounds(int n, int nb, const int32_t* __restrict__ rp,
                                                                   int* __restrict__ bound) {
   __shared__ int at[MAX_SHARES + 1];
   const int b = threadIdx.x;
   if (b <= nb) {
-    const int64_t target = ((int64_t)rp[n] + 64 * (int64_t)n) * b / nb;
+    const int64_t target = ((int64_t)rp[n] + 24 * (int64_t)n) * b / nb;
     int lo = 0, hi = n;  // first row whose share starts at or after the target
     while (lo < hi) {
       const int mid = (lo + hi) / 2;
-      if (rp[mid] + 64 * (int64_t)mid < target) lo = mid + 1;
+      if (rp[mid] + 24 * (int64_t)mid < target) lo = mid + 1;
       else hi = mid;
     }
     at[b] = lo;
@@ -381,52 +383,82 @@ __device__ __forceinline__ double cycle_norm(const double* __restrict__ npart, i
   return group_sum<32>(t);
 }
 
-// h[j] = sum over the blocks of part[j nb + block], j < m: eight lanes to a j.
-__device__ __forceinline__ void cycle_sums(const double* __restrict__ part, int nb, int m, double* h) {
+// Sums over the blocks of part[j nb + block], j < m, eight lanes to a j:
+// done(j, sum) on one of them.
+template <class F>
+__device__ __forceinline__ void cycle_sums(const double* part, int nb, int m, F done) {
   const int q = threadIdx.x & 7;
   for (int j0 = 0; j0 < m; j0 += CT / 8) {
     const int j = j0 + (threadIdx.x >> 3);
-    if ((threadIdx.x >> 5) * 4 + j0 >= m) continue;  // whole warps
+    if ((threadIdx.x >> 5) * 4 + j0 >= m) break;  // whole warps
     double v[MAX_SHARES / 8], s = 0.0;
 #pragma unroll
     for (int u = 0; u < MAX_SHARES / 8; ++u) v[u] = j < m && q + 8 * u < nb ? __ldcg(part + j * nb + q + 8 * u) : 0.0;
 #pragma unroll
     for (int u = 0; u < MAX_SHARES / 8; ++u) s += v[u];
     s = group_sum<8>(s);
-    if (j < m && q == 0) h[j] = s;
+    if (j < m && q == 0) done(j, s);
   }
-  __syncthreads();
 }
 
 __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleArgs A) {
   extern __shared__ __align__(16) double sm[];
-  __shared__ double red[CYCLE_ROWS / 8], s_scale;
+  __shared__ double red[CYCLE_ROWS / 8];
+  __shared__ int groups;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = tid & 3, grp = tid >> 2;
   const bool givens = (int)blockIdx.x == A.nb;
   const int r0 = givens ? A.n : A.bound[blockIdx.x];
   const int rows = givens ? 0 : A.bound[blockIdx.x + 1] - r0;
   const bool row_warp = warp * 8 < rows;  // warps with a row in combine()
   int bar = 0;
+  bool near = false;           // the matrix entries are in shared memory
   double* h = sm;              // [MAX_BASIS]
   double* c = h + MAX_BASIS;   // [MAX_BASIS]: the Hessenberg column (the last block)
-  double* V = c + MAX_BASIS;   // [restart][LD]
-  double* w = V + (size_t)A.restart * LD;
-  double* wn = w + LD;         // the product
+  double* V = c + MAX_BASIS;   // [restart + 1][LD]; the last vector found is not scaled yet
+  double* wn = V + (size_t)(A.restart + 1) * LD;  // the product
   double* mi = wn + LD;
-  double* sval = mi + LD;      // [cap]
-  int32_t* rps = reinterpret_cast<int32_t*>(sval + A.cap);  // [CYCLE_ROWS + 1]
-  uint16_t* scol = reinterpret_cast<uint16_t*>(rps + CYCLE_ROWS + 1);
+  double* sval = mi + LD + (~A.restart & 1);  // [cap], 16-byte aligned
+  int32_t* rps = reinterpret_cast<int32_t*>(sval + A.cap);  // [CYCLE_ROWS]: a row's first entry there
+  int32_t* rpe = rps + CYCLE_ROWS;  // and its groups of 32
+  uint16_t* scol = reinterpret_cast<uint16_t*>(rpe + CYCLE_ROWS);
   // the last block's arrays take the place of the matrix
   double *cs = V, *sn = cs + A.restart, *g = sn + A.restart, *xs = g + A.restart + 1, *pr = xs + A.restart + 1,
          *U = pr + A.restart;  // U: packed columns of the triangular matrix
 
   if (!givens) {
-    for (int r = tid; r <= rows; r += CT) rps[r] = A.rp[r0 + r];
+    // groups of 32 entries of every free row, the last one filled up with
+    // zeros; a lane's four are neighbours and eight apart in the row
+    if (warp == 0) {
+      int first = 1;
+      for (int r = lane; r < CYCLE_ROWS; r += 32) {
+        const int ng = r < rows && A.free_dof[r0 + r] ? (A.rp[r0 + r + 1] - A.rp[r0 + r] + 31) / 32 : 0;
+        int sum = ng;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += t;
+        }
+        rps[r] = 32 * (first + sum - ng);
+        rpe[r] = ng;
+        first += __shfl_sync(0xffffffffu, sum, 31);
+      }
+      if (lane == 0) groups = first;
+    }
     __syncthreads();
-    const int e0 = rps[0], cnt = min(rps[rows] - e0, A.cap);
-    for (int e = tid; e < cnt; e += CT) {
-      sval[e] = A.vals[e0 + e];
-      scol[e] = (uint16_t)A.col[e0 + e];
+    near = 32 * groups <= A.cap;
+    if (near) {
+      if (tid < 32) {
+        sval[tid] = 0.0;
+        scol[tid] = 0;
+      }
+      for (int r = warp; r < rows; r += CT / 32) {
+        const int e0 = A.rp[r0 + r], len = A.rp[r0 + r + 1] - e0;
+        for (int g = 0; g < rpe[r]; ++g) {
+          const int e = 32 * g + lane, to = rps[r] + 32 * g + 4 * (lane & 7) + (lane >> 3);
+          sval[to] = e < len ? A.vals[e0 + e] : 0.0;
+          scol[to] = e < len ? (uint16_t)A.col[e0 + e] : (uint16_t)0;
+        }
+      }
     }
     for (int r = tid; r < rows; r += CT) {
       const double m = A.minv[r0 + r], v = A.res[r0 + r] * (1.0 / A.beta);
@@ -438,47 +470,51 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
     g[0] = A.beta;
   }
 
-  // wn = P A x on the block's rows: a warp takes two rows (k_spmv)
+  // wn = P A x on the block's rows: eight lanes to a row, 32 entries at a time.
+  // x goes through L1 (the barrier before makes the other blocks' part
+  // visible), as a block's rows share most of their columns.
+  static_assert(CYCLE_ROWS * 8 == CT, "one row per eight threads");
   auto product = [&](const double* x) {
-    const int e0 = rps[0];
-    for (int i = 2 * warp; i < rows; i += 2 * (CT / 32)) {
-      double s[2] = {0.0, 0.0};
-      int at[2], end[2];
+    const int r = tid >> 3, l = tid & 7;
+    if (warp * 4 < rows) {
+      double s0 = 0.0, s1 = 0.0;
+      const int start = r < rows ? rps[r] : 0, ng = r < rows ? rpe[r] : 0;
+      if (near) {
+        const int most = __reduce_max_sync(0xffffffffu, ng);
+        for (int g0 = 0; g0 < most; g0 += 4) {
+          int at[4];
+          double xv[4][4];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const bool in = i + r < rows && A.free_dof[r0 + i + r];
-        at[r] = in ? rps[i + r] - e0 + lane : lane;
-        end[r] = in ? rps[i + r + 1] - e0 : 0;
-      }
-      while (__any_sync(0xffffffffu, at[0] < end[0] || at[1] < end[1])) {
-        double xv[2][8], av[2][8];
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int e = at[r] + 32 * u;
-            const bool in = e < end[r], near = e < A.cap;
-            xv[r][u] = in ? __ldcg(x + (near ? (int)scol[e] : A.col[e0 + e])) : 0.0;
-            av[r][u] = in ? (near ? sval[e] : A.vals[e0 + e]) : 0.0;
+          for (int g = 0; g < 4; ++g) {
+            at[g] = (g0 + g < ng ? start + 32 * (g0 + g) : 0) + 4 * l;  // the first group holds zeros
+            const ushort4 cc = *reinterpret_cast<const ushort4*>(scol + at[g]);
+            xv[g][0] = x[cc.x];
+            xv[g][1] = x[cc.y];
+            xv[g][2] = x[cc.z];
+            xv[g][3] = x[cc.w];
           }
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (at[r] - lane + 32 * u < end[r]) s[r] = fma(av[r][u], xv[r][u], s[r]);  // whole warps
-          at[r] += 256;
+          for (int g = 0; g < 4; ++g) {
+            if (g0 + g >= most) break;
+            const double2 a = *reinterpret_cast<const double2*>(sval + at[g]);
+            const double2 b = *reinterpret_cast<const double2*>(sval + at[g] + 2);
+            s0 = fma(a.x, xv[g][0], s0);
+            s1 = fma(a.y, xv[g][1], s1);
+            s0 = fma(b.x, xv[g][2], s0);
+            s1 = fma(b.y, xv[g][3], s1);
+          }
         }
+      } else if (ng) {
+        for (int e = A.rp[r0 + r] + l; e < A.rp[r0 + r + 1]; e += 8) s0 = fma(A.vals[e], x[A.col[e]], s0);
       }
-      const bool hi = lane & 16;
-      double t = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if ((lane & 15) == 0 && i + (hi ? 1 : 0) < rows) wn[i + (hi ? 1 : 0)] = t;
+      __syncwarp();
+      const double s = group_sum<8>(s0 + s1);
+      if (l == 0 && r < rows) wn[r] = s;
     }
     __syncthreads();
   };
   // the block's shares of V_j . w, j < m
-  auto dots = [&](int m, double* part) {
+  auto dots = [&](int m, const double* w, double* part) {
     for (int j0 = 0; j0 < m; j0 += CT / 4) {
       const int j = j0 + grp;
       if (warp * 8 + j0 >= m) continue;
@@ -544,45 +580,47 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
   bool converged = false;
   for (int k = 0;; ++k) {
     const int m = k + 1;
+    double* w = V + m * LD;
     if (!givens) {
-      // the last warp, which has the fewest rows, scales by the norm first
-      if (warp == CT / 32 - 1) {
-        const double t = k ? cycle_norm(A.npart, A.nb) : 1.0;
-        if (lane == 0) s_scale = t > 0.0 ? rsqrt(t) : 0.0;
-      }
       product(A.z);
-      for (int r = tid; r < rows; r += CT) {
-        if (k) V[k * LD + r] = s_scale * w[r];
-        w[r] = s_scale * wn[r];
-      }
-      __syncthreads();
-      dots(m, A.part);
+      dots(m, wn, A.part);
     } else if (k) {
       if (warp == 0) {
         const double t = cycle_norm(A.npart, A.nb);
-        if (lane == 0) c[k] = sqrt(t);
+        if (lane == 0) {
+          c[k] = sqrt(t);
+          red[0] = t > 0.0 ? rsqrt(t) : 0.0;
+        }
       }
       converged = rotate(k - 1);
-      if (converged && tid == 0) A.ctl[1] = 1;
+      if (tid == 0) *A.scale = converged ? -1.0 : red[0];
     }
     if (!cycle_barrier(A.ctl, ++bar)) return;
-    if (k && __ldcg(A.ctl + 1)) {  // column k - 1 was the last one
+    // V_k, the product and its dots still lack the scale of V_k
+    const double a = k ? __ldcg(A.scale) : 1.0;
+    cycle_sums(A.part, A.nb, m, [&](int j, double s) { h[j] = j == k ? s * a * a : s * a; });
+    for (int r = tid; r < rows; r += CT) {
+      V[k * LD + r] *= a;
+      w[r] = a * wn[r];
+    }
+    if (a < 0.0) {  // column k - 1 was the last one
       K = k;
       break;
     }
-    cycle_sums(A.part, A.nb, m, h);
+    __syncthreads();
     if (!givens) {
       if (row_warp) {
         const double s = combine(m);
         if (grp < rows && q == 0) w[grp] -= s;
       }
       __syncthreads();
-      dots(m, A.part2);
+      dots(m, w, A.part2);
     } else {
       for (int j = tid; j < m; j += CT) c[j] = h[j];
     }
     if (!cycle_barrier(A.ctl, ++bar)) return;
-    cycle_sums(A.part2, A.nb, m, h);
+    cycle_sums(A.part2, A.nb, m, [&](int j, double s) { h[j] = s; });
+    __syncthreads();
     if (!givens) {
       double t = 0.0;
       if (row_warp) {
@@ -871,10 +909,10 @@ struct Solver {
     // a block has 16 rows or more while that many blocks are not all in use
     const int nb = (int)std::min<int64_t>(std::min(sms - 1, MAX_SHARES), (n + 15) / 16);
     if (n > (int64_t)nb * CYCLE_ROWS || n > 65535 || nnz > INT32_MAX) return;
-    const int64_t fixed = 8 * (2 * MAX_BASIS + (restart + 3) * LD) + 4 * (CYCLE_ROWS + 1);
+    const int64_t fixed = 8 * (2 * MAX_BASIS + (restart + 3) * LD + 1) + 8 * CYCLE_ROWS;
     const int64_t last = 8 * (2 * (int64_t)MAX_BASIS + 5 * (restart + 1) + (int64_t)restart * (restart + 1) / 2);
     const int64_t room = smem - 1024;  // the kernel's static arrays
-    const int64_t cap = (room - fixed) / 10;
+    const int64_t cap = (room - fixed) / 10 & ~(int64_t)31;
     if (cap < 0 || last > room) return;
     if (cudaFuncSetAttribute(k_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess) {
       cudaGetLastError();
@@ -891,9 +929,10 @@ struct Solver {
     a.minv = minv;
     a.free_dof = free_dof;
     a.z = z;
+    a.npart = npart;
     a.part = part;
     a.part2 = part2;
-    a.npart = npart;
+    a.scale = scal;
     a.y = col_d;
     a.ctl = ctl;
     a.bound = bound;
@@ -914,7 +953,7 @@ struct Solver {
     a.tol = tol;
     a.breakdown = 1e-14 * beta;
     a.kmax = kmax;
-    NT_TRY(cudaMemsetAsync(a.ctl, 0, 2 * sizeof(int), st));
+    NT_TRY(cudaMemsetAsync(a.ctl, 0, sizeof(int), st));
     pinned[1] = -1.0;
     void* args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_cycle, dim3(a.nb + 1), dim3(CT), args, cyc_smem, st);
@@ -1071,13 +1110,7 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   for (double** p : {&S.r, &S.rn, &S.d, &S.xs, &S.w, &S.minv, &S.diag, &S.z, &dx_state}) W.add(p, (size_t)n);
   W.add(&S.V, (basis + 1) * n);
   W.add(&S.col_d, 2 * (rs + 2));
-  int sms = 0;
-  {
-    int dev = 0;
-    NT_TRY(cudaGetDevice(&dev));
-    NT_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  }
-  const size_t shares = (size_t)std::max(MAX_CHUNKS, sms);
+  const size_t shares = std::max(MAX_CHUNKS, MAX_SHARES);
   W.add(&S.part, (basis + 1) * shares);
   W.add(&S.part2, (basis + 1) * shares);
   W.add(&S.npart, shares);
