@@ -690,7 +690,7 @@ def loadstep_leg(dev, n=8, n_train=48, n_test=4, increments=8, modes=64, train_s
         "mixed_learned": {"newton_iterations": mean("learned_iters"), "krylov_iterations": mean("learned_krylov"),
                           "solve_ms": 1e3 * mean("learned_s"),
                           "load_step_ms": 1e3 * mean("learned_s"), "increments": 1,
-                          "jacobian": "FP32 uu (BF16x3 tensor cores) + FP64 coupling/residual",
+                          "jacobian": "FP32 uu (sum-factorised) + FP64 coupling/residual",
                           "guess": "POD-MLP prediction (BF16 tensor-core inference)",
                           "accepted_guesses": int(sum(r["accepted"] for r in rows)),
                           "krylov_tolerance": "Eisenstat-Walker forcing"},

@@ -18,8 +18,10 @@
 // Elements of one colour share no node, so P6 needs no atomics and the
 // result does not depend on scheduling.
 //
-// The mixed-precision variant keeps P1-P4 and the pressure coupling in FP64
-// and runs the tangent (elasticity tensor, uu block) in FP32.
+// It serves the element-level calls, and the FP64 Jacobian where fe_fp64.cu's
+// launch has no records (no memory left, a stream under capture).  The other assemblies: fe_fp64.cu (FP64 Jacobian),
+// fe_residual.cu, fe_mixed.cu and fe_mixed_coloured.cu (mixed precision),
+// fe_batch.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -58,8 +60,7 @@ int set_error(int code, const std::string& msg) {
       return set_error(FE_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(err__));      \
   } while (0)
 
-enum Mode { M_RES = 0, M_JAC = 1, M_MIX = 2, M_ERES = 3, M_EJAC = 4 };
-
+enum Mode { M_JAC, M_ERES, M_EJAC };
 
 
 template <int N1, int PM>
@@ -99,9 +100,7 @@ template <int N1, int PM, int MODE>
 __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
   using C = Cfg<N1, PM>;
   constexpr int NPE = C::NPE, NPP = C::NPP, NR = C::NR, NU3 = C::NU3, NROW = C::NROW;
-  constexpr bool JAC = (MODE == M_JAC || MODE == M_MIX || MODE == M_EJAC);
-  constexpr bool MIX = (MODE == M_MIX);
-  using TT = typename std::conditional<MIX, float, double>::type;  // tangent precision
+  constexpr bool JAC = MODE != M_ERES;
   extern __shared__ __align__(16) double smem[];
   double* s_gbf = smem + C::O_GBF;
   double* s_gbfp = smem + C::O_GBFP;
@@ -112,10 +111,10 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
   double* s_pg = smem + C::O_PG;
   double* s_gp = smem + C::O_GP;
   double* s_dphi = smem + C::O_DPHI;
-  TT* s_T = reinterpret_cast<TT*>(smem + C::O_T);
+  double* s_T = smem + C::O_T;
   int* s_node = reinterpret_cast<int*>(smem + C::O_END);  // [NR] row nodes, then table id
   const int tid = threadIdx.x;
-  const bool want_res = (MODE == M_RES || MODE == M_ERES || P.r != nullptr) && MODE != M_EJAC;
+  const bool want_res = MODE == M_ERES || (MODE == M_JAC && P.r != nullptr);
 
   for (int i = tid; i < NG * 4 * NPE; i += C::THREADS) s_gbf[i] = P.gbf_u[i];
   for (int i = tid; i < NG * 8; i += C::THREADS) s_gbfp[i] = P.gbf_p[i];
@@ -234,14 +233,14 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         }
       }
       if (JAC) {
-        TT Ct[6][6], St[6], Ft[3][3], ct[4];
+        double Ct[6][6], St[6], Ft[3][3], ct[4];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int j = 0; j < 3; ++j) Ft[i][j] = (TT)F[i][j];
+          for (int j = 0; j < 3; ++j) Ft[i][j] = F[i][j];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ct[i] = (TT)cc[i];
-        d_gauss_elasticity<TT>(P.law, ct, Ft, (TT)jznu, (TT)pg, Ct, St);
+        for (int i = 0; i < 4; ++i) ct[i] = cc[i];
+        d_gauss_elasticity<double>(P.law, ct, Ft, jznu, pg, Ct, St);
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
           rec[18 + i] = (double)St[i];
@@ -301,10 +300,10 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
     }
     if (!JAC) continue;
     // P5: Jacobian entries
-    TT acc_uu[C::EUU];
+    double acc_uu[C::EUU];
     double acc_pu[C::EPU];
 #pragma unroll
-    for (int j = 0; j < C::EUU; ++j) acc_uu[j] = TT(0);
+    for (int j = 0; j < C::EUU; ++j) acc_uu[j] = 0.0;
 #pragma unroll
     for (int j = 0; j < C::EPU; ++j) acc_pu[j] = 0.0;
     for (int g = 0; g < NG; ++g) {
@@ -315,16 +314,16 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         const int blk = i / NPE, b = i % NPE;
         const int nh = blk < 3 ? blk : (blk == 5 ? 1 : 0);
         const int mh = blk < 3 ? blk : (blk == 3 ? 1 : 2);
-        const TT jgw = (TT)rec[9];
-        TT sub[3][3];
+        const double jgw = rec[9];
+        double sub[3][3];
 #pragma unroll
         for (int r = 0; r < 3; ++r)
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const TT cv = (TT)rec[24 + t2v(r, mh) * 6 + t2v(c, nh)];
-            sub[r][c] = blk < 3 ? jgw * (cv + (TT)rec[18 + t2v(r, c)]) : jgw * cv;
+            const double cv = rec[24 + t2v(r, mh) * 6 + t2v(c, nh)];
+            sub[r][c] = blk < 3 ? jgw * (cv + rec[18 + t2v(r, c)]) : jgw * cv;
           }
-        const TT d0 = (TT)dpg[b * 3 + 0], d1 = (TT)dpg[b * 3 + 1], d2 = (TT)dpg[b * 3 + 2];
+        const double d0 = dpg[b * 3 + 0], d1 = dpg[b * 3 + 1], d2 = dpg[b * 3 + 2];
 #pragma unroll
         for (int r = 0; r < 3; ++r) s_T[i * 3 + r] = sub[r][0] * d0 + sub[r][1] * d1 + sub[r][2] * d2;
       }
@@ -336,8 +335,8 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         if (d >= 0) {
           const int R = d >> 8, Cc = d & 0xff;
           const int m = R / NPE, a = R % NPE, n = Cc / NPE, b = Cc % NPE;
-          const TT* tv = &s_T[(blk_of(m, n) * NPE + b) * 3];
-          const TT d0 = (TT)dpg[a * 3 + 0], d1 = (TT)dpg[a * 3 + 1], d2 = (TT)dpg[a * 3 + 2];
+          const double* tv = &s_T[(blk_of(m, n) * NPE + b) * 3];
+          const double d0 = dpg[a * 3 + 0], d1 = dpg[a * 3 + 1], d2 = dpg[a * 3 + 2];
           acc_uu[j] = acc_uu[j] + (d0 * tv[0] + d1 * tv[1] + d2 * tv[2]);
         }
       }
@@ -361,8 +360,8 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         const int d = e_uu[j];
         if (d >= 0) {
           const int R = d >> 8, Cc = d & 0xff;
-          out[(size_t)Cc * NROW + R] = (double)acc_uu[j];
-          out[(size_t)R * NROW + Cc] = (double)acc_uu[j];
+          out[(size_t)Cc * NROW + R] = acc_uu[j];
+          out[(size_t)R * NROW + Cc] = acc_uu[j];
         }
       }
 #pragma unroll
@@ -386,37 +385,22 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         const int m = R / NPE, a = R % NPE, n = Cc / NPE, b = Cc % NPE;
         const int na = s_node[a], nb = s_node[b];
         const uint16_t tab_ab = tab[a * NR + b], tab_ba = tab[b * NR + a];
-        const TT v = acc_uu[j];
-        if (MIX) {
-          const size_t p1 = (size_t)P.uu_row_ptr[(size_t)m * nu + na] + (size_t)n * P.wu[na] + (tab_ab & 0x7fff);
-          if (tab_ab & 0x8000)
-            P.vals_uu[p1] = (float)v;
+        const double v = acc_uu[j];
+        const size_t p1 = (size_t)P.row_ptr[(size_t)m * nu + na] + (size_t)n * P.wu[na] + (tab_ab & 0x7fff);
+        if (tab_ab & 0x8000)
+          P.vals[p1] = v;
+        else
+          atomicAdd(&P.vals[p1], v);
+        if (R != Cc) {
+          const size_t p2 = (size_t)P.row_ptr[(size_t)n * nu + nb] + (size_t)m * P.wu[nb] + (tab_ba & 0x7fff);
+          if (tab_ba & 0x8000)
+            P.vals[p2] = v;
           else
-            atomicAdd(&P.vals_uu[p1], (float)v);
-          if (R != Cc) {
-            const size_t p2 = (size_t)P.uu_row_ptr[(size_t)n * nu + nb] + (size_t)m * P.wu[nb] + (tab_ba & 0x7fff);
-            if (tab_ba & 0x8000)
-              P.vals_uu[p2] = (float)v;
-            else
-              atomicAdd(&P.vals_uu[p2], (float)v);
-          }
-        } else {
-          const size_t p1 = (size_t)P.row_ptr[(size_t)m * nu + na] + (size_t)n * P.wu[na] + (tab_ab & 0x7fff);
-          if (tab_ab & 0x8000)
-            P.vals[p1] = (double)v;
-          else
-            atomicAdd(&P.vals[p1], (double)v);
-          if (R != Cc) {
-            const size_t p2 = (size_t)P.row_ptr[(size_t)n * nu + nb] + (size_t)m * P.wu[nb] + (tab_ba & 0x7fff);
-            if (tab_ba & 0x8000)
-              P.vals[p2] = (double)v;
-            else
-              atomicAdd(&P.vals[p2], (double)v);
-          }
+            atomicAdd(&P.vals[p2], v);
         }
       }
     }
-    const int32_t* rp = MIX ? P.cp_row_ptr : P.row_ptr;
+    const int32_t* rp = P.row_ptr;
 #pragma unroll
     for (int j = 0; j < C::EPU; ++j) {
       const int d = e_pu[j];
@@ -433,8 +417,7 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
         else
           atomicAdd(&P.vals[p1], v);
         // mirror: displacement row (n, b), pressure column q
-        const size_t p2 = MIX ? (size_t)rp[(size_t)n * nu + nb] + (t_bq & 0x7fff)
-                              : (size_t)rp[(size_t)n * nu + nb] + 3 * (size_t)P.wu[nb] + (t_bq & 0x7fff);
+        const size_t p2 = (size_t)rp[(size_t)n * nu + nb] + 3 * (size_t)P.wu[nb] + (t_bq & 0x7fff);
         if ((t_bq & 0x8000))
           P.vals[p2] = v;
         else
@@ -447,8 +430,7 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
       const uint16_t t = tab[lq * NR + lq2];
       if (t & 0x8000) {
         const int pq = s_node[lq];
-        const size_t pos = MIX ? (size_t)rp[(size_t)3 * nu + pq] + 3 * (size_t)P.wp[pq] + (t & 0x7fff)
-                               : (size_t)rp[(size_t)3 * nu + pq] + 3 * (size_t)P.wp[pq] + (t & 0x7fff);
+        const size_t pos = (size_t)rp[(size_t)3 * nu + pq] + 3 * (size_t)P.wp[pq] + (t & 0x7fff);
         P.vals[pos] = 0.0;
       }
     }

@@ -193,12 +193,11 @@ int fe_set_high_precision(fe_handle h, int32_t mode);
  * FE_ASSEMBLY_STAGED (the default): every element stores its entries in a
  * per-element record on the device, and each CSR row is formed once from the
  * records of the elements around the row's node, in increasing element
- * number: in the same launch, by the block that assembles the node's last
- * element (where one row node's rows fit that kernel's shared memory), else
- * by a second kernel.  Every matrix sector is written once and never read.  The records take, per element, 4 (3 n_p)^2 +
- * 8 n_q 3 n_p + 8 (3 n_p + n_q) bytes (32 kB for a triquadratic element with
- * nodal pressure), allocated on the first staged evaluation and kept with
- * the handle.
+ * number, in the same launch, by the block that assembles the node's last
+ * element.  Every matrix sector is written once and never read.  The records
+ * take, per element, about 4 (3 n_p)^2 + 16 n_q 3 n_p + 8 (3 n_p + n_q) bytes
+ * (38 kB for a triquadratic element with nodal pressure), allocated on the
+ * first staged evaluation and kept with the handle.
  * FE_ASSEMBLY_COLOURED: one launch per element colour, each element adding
  * its entries straight into the CSR arrays (the first contributor in colour
  * order stores, later ones add).  No extra memory.
@@ -222,9 +221,8 @@ int fe_set_assembly_order(fe_handle h, int32_t order);
  * over the host link, without a device copy of the result.
  * FE_HOST_OUTPUT_AFTER: assembled into device staging, copied afterwards.
  * The values are the same bit for bit in every mode.  Where the streamed or
- * in-place mode does not apply (the coloured order; for streaming, a mesh
- * whose row neighbourhoods exceed the fused kernel's scratch; for in place,
- * pageable memory) the call copies after the assembly.  chunks: the launches of a
+ * in-place mode does not apply (the coloured order; for in place, pageable
+ * memory) the call copies after the assembly.  chunks: the launches of a
  * streamed assembly, 1..16 of equal element counts, or 0 for the wave plan
  * above. */
 #define FE_HOST_OUTPUT_STREAMED 0
@@ -271,9 +269,9 @@ int fe_batch_check(fe_batch b, void* stream);
 
 /* Launch configuration: variant (elements per group for triquadratic /
  * trilinear members: 0 = 4/8, 1 = 4/4, 2 = 2/4, 3 = 2/2, 4 = 3/2 compiled for
- * three CTAs per SM; 5 = no persistent launch but the single-set kernels, one
- * launch per member and colour, which the autotuner picks when the members
- * are large enough to fill the GPU on their own), CTAs per SM, and
+ * three CTAs per SM; 5 = no persistent launch but the single-set kernels, each
+ * member's launch on one of eight streams, forked from and joined to the
+ * caller's), CTAs per SM, and
  * consecutive element groups per work unit (both ignored by variant 5). */
 int fe_batch_set_config(fe_batch b, int32_t variant, int32_t ctas_per_sm, int32_t block_groups);
 int fe_batch_get_config(fe_batch b, int32_t* variant, int32_t* ctas_per_sm, int32_t* block_groups,
