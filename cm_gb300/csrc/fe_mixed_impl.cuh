@@ -1,5 +1,6 @@
-// libcm_fe: mixed-precision element assembly, device code shared by the
-// per-equations-set kernel (fe_mixed.cu) and the batched kernel (fe_batch.cu).
+// libcm_fe: element assembly, device code shared by the fused kernels
+// (fe_mixed.cu, fe_fp64.cu), the residual (fe_residual.cu), the launches per
+// colour (fe_mixed_coloured.cu) and the batched kernel (fe_batch.cu).
 //
 // Same arithmetic content as the reference's element residual and Jacobian
 // (FiniteElasticity_FiniteElement{Residual,Jacobian}Evaluate,
@@ -43,7 +44,7 @@ namespace {
 
 constexpr int align16(int x) { return (x + 15) & ~15; }
 
-// Default elements per group: 3 for triquadratic elements with nodal pressure
+// Elements per group of the launches per colour: 3 for triquadratic with nodal pressure
 // (about 72 KB of shared memory, so three 256-thread CTAs fit on an SM, which
 // measured 17 % faster than two CTAs of 4 elements despite the register
 // spills the 80-register budget causes), 4 for element-based pressure, 8 for

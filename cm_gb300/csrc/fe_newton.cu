@@ -13,19 +13,18 @@
 // The free-dof system is never extracted: vectors keep the full dof
 // numbering with zeros on the fixed dofs, and the matrix-vector product masks
 // rows and columns of fixed dofs.  Every reduction is a fixed-order two-pass
-// sum, so a solve is bit-identical from run to run.  The host drives the
-// iteration; it reads one small array per GMRES iteration (the new
-// Hessenberg column) to update the Givens rotations.
+// sum, so a solve is bit-identical from run to run.
 //
 // On the meshes this solver suits (its preconditioner is diagonal) a GMRES
 // iteration is a handful of vectors of a few thousand entries, bound by
-// launches and by the latency of FP64 reductions.  So an iteration is four
-// launches: dots, update with the second pass's dots, update with the norm,
-// the preconditioning and the Hessenberg column, matrix-vector product with
-// the scaling; a block owns a chunk of rows and its warps take different basis vectors, so
-// no dot waits on a block-wide reduction, and the sums over the at most 64
-// chunks are formed by the kernel that uses them.  The next iteration is queued
-// before the host waits for a column.
+// launches and by the latency of FP64 reductions.  While the rows fit the SMs'
+// shared memory, a whole cycle is one cooperative launch (k_cycle).  Else an
+// iteration is four launches: dots, update with the second pass's dots, update
+// with the norm, the preconditioning and the Hessenberg column, matrix-vector
+// product with the scaling; a block owns a chunk of rows and its warps take
+// different basis vectors, so no dot waits on a block-wide reduction, the sums
+// over the at most 64 chunks are formed by the kernel that uses them, the host
+// rotates the columns, and the next iteration is queued before it waits for one.
 #include "fe_internal.h"
 
 #include <cuda_runtime.h>
@@ -304,6 +303,11 @@ __global__ void __launch_bounds__(NT) k_update_norm(int64_t n, const double* __r
 // What crosses SMs is the preconditioned vector z and the blocks' shares of
 // the dots and the norm: three grid barriers an iteration (blocks that poll
 // the shares themselves until all have come take twice the time).
+//
+// Bound by the barriers (1.9 us each) and FP64 latency (an instruction holds a
+// quarter SM's pipe for 64 cycles): 17.5 us an iteration at 4,071 rows and
+// 700,000 entries, against 30 for four launches; a load step 21.0 against 31.4
+// ms, at 9,223 rows 54.3 against 89.0, at 525 rows 8.7 against 13.0.
 struct CycleArgs {
   int n, nb, restart, kmax, cap;
   int* bound;  // [nb + 1]
@@ -899,7 +903,9 @@ struct Solver {
   }
 
   // Rows and shared memory of k_cycle for this system; cyc_smem stays 0 when
-  // it has more rows than the blocks take.
+  // it has more rows than the blocks take: 64 each, a row per eight threads,
+  // with which the basis of the longest restart still fits.  Up to that line
+  // k_cycle is the faster one at every size (see there).
   void plan_cycle(int* ctl, int* bound) {
     int dev = 0, sms = 0, smem = 0, coop = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
