@@ -297,9 +297,16 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
     s_node[i] = v;
   }
   __syncthreads();
+  // positions from a node of the element: only their derivatives are wanted,
+  // and the lines below then round values of the element's size, not the
+  // mesh's (error against 64 bits relative to that of contracting over all
+  // Gauss points: FP64 Jacobian of the 16^3 box 1.5 -> 1.1, residual of the
+  // 32^3 box 1.15 -> 0.8; 635 -> 638 us)
   for (int i = tid; i < EG * 3 * NPE; i += C::THREADS) {
     const int el = i / (3 * NPE), c = (i / NPE) % 3, a = i % NPE;
-    s_z[i] = hval<H>(el < nvalid ? P.x[(size_t)c * nu + s_node[el * (NR + 1) + a]] : 0.0);
+    const int* nd = s_node + el * (NR + 1);
+    const double* x = P.x + (size_t)c * nu;
+    s_z[i] = hval<H>(el < nvalid ? x[nd[a]] - x[nd[NPE / 2]] : 0.0);
   }
   for (int i = tid; i < EG * NPP; i += C::THREADS) {
     const int el = i / NPP, q = i % NPP;
