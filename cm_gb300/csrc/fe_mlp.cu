@@ -95,13 +95,19 @@ static_assert(TWARPS * TBM * (TBN + 1) * 4 <= TSMEM, "reduction scratch");
 // Rows r0 .. r0 + ROWS of an operand (R rows in all), chunk [k0, k0 + TBK) of the
 // contraction (K long): all loads first (fetch), then into s[k][row] (put).  KC:
 // stored [row][K] (contraction contiguous), else [K][row].  Four values at a
-// time where the alignment and the sizes allow (vec).
-template <bool KC, int ROWS, int LD>
+// time where the alignment and the sizes allow (vec).  PAR: a parameter, else
+// written by a kernel before this one, maybe after this one started: read from
+// L2.
+template <bool KC, int ROWS, int LD, bool PAR>
 struct TileOperand {
   static constexpr int Q = ROWS * TBK / 4 / (32 * TWARPS);
   float4 v[Q];
   static __device__ __forceinline__ bool vec(const float* src, int64_t ld, int R, int K) {
     return (reinterpret_cast<uintptr_t>(src) & 15) == 0 && ld % 4 == 0 && (KC ? K : R) % 4 == 0;
+  }
+  template <class V>
+  static __device__ __forceinline__ V get(const V* p) {
+    return PAR ? *p : __ldcg(p);
   }
   static __device__ __forceinline__ void at(int u, int& r, int& k) {
     const int i = u * 32 * TWARPS + threadIdx.x;
@@ -117,13 +123,13 @@ struct TileOperand {
       v[u] = float4{0.f, 0.f, 0.f, 0.f};
       if (r0 + r < R && k0 + k < K) {
         if (vec) {
-          v[u] = *reinterpret_cast<const float4*>(p);
+          v[u] = get(reinterpret_cast<const float4*>(p));
         } else {
           const int left = KC ? K - k0 - k : R - r0 - r;
-          v[u].x = p[0];
-          if (left > 1) v[u].y = p[1];
-          if (left > 2) v[u].z = p[2];
-          if (left > 3) v[u].w = p[3];
+          v[u].x = get(p);
+          if (left > 1) v[u].y = get(p + 1);
+          if (left > 2) v[u].z = get(p + 2);
+          if (left > 3) v[u].w = get(p + 3);
         }
       }
     }
@@ -144,9 +150,21 @@ struct TileOperand {
   }
 };
 
+// Programmatic dependent launch along a training step: a kernel lets the next
+// one start at once, and the next one waits for the whole of it before it
+// touches anything that a kernel of the step writes.  Only the parameters (the
+// step's first kernel starts after all earlier work of the stream) are read
+// before the wait.  Without the launch attribute both do nothing.  The nine
+// launches of a step are bound by their latencies and the gaps between them:
+// 64 -> 46 us for the 4-256-256-256-64 network on 256 rows.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // The tile at (m0, n0).  Outputs go to out(m, n, value) for m < M, n < N; with
-// colsum, sum over the contraction of A's rows to csum(m, value).
-template <bool AKC, bool BKC, class Out, class Sum>
+// colsum, sum over the contraction of A's rows to csum(m, value).  BPAR: B is a
+// parameter, loaded before the wait for the previous kernel; else the wait is
+// the first thing.
+template <bool AKC, bool BKC, bool BPAR, class Out, class Sum>
 __device__ __forceinline__ void tile_product(int M, int N, int K, const float* A, int64_t lda, const float* B,
                                              int64_t ldb, int m0, int n0, bool colsum, Out out, Sum csum) {
   extern __shared__ __align__(16) float tsm[];
@@ -155,13 +173,15 @@ __device__ __forceinline__ void tile_product(int M, int N, int K, const float* A
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tr = lane >> 2, tc = lane & 3;  // rows tr + 8 i, columns 4 tc + j
   float acc[4][4] = {}, asum = 0.0f;
-  TileOperand<AKC, TBM, TLDA> ta;
-  TileOperand<BKC, TBN, TLDB> tb;
+  TileOperand<AKC, TBM, TLDA, false> ta;
+  TileOperand<BKC, TBN, TLDB, BPAR> tb;
   const bool va = ta.vec(A, lda, M, K), vb = tb.vec(B, ldb, N, K);
   for (int k0 = 0; k0 < K; k0 += TBK) {
     const int kn = min(TBK, K - k0);
-    ta.fetch(A, lda, m0, M, k0, K, va);
+    if (!BPAR && !k0) wait_for_previous();
     tb.fetch(B, ldb, n0, N, k0, K, vb);
+    if (BPAR && !k0) wait_for_previous();
+    ta.fetch(A, lda, m0, M, k0, K, va);
     if (k0) __syncthreads();
     ta.put(As, kn);
     tb.put(Bs, kn);
@@ -219,10 +239,11 @@ __global__ void __launch_bounds__(32 * TWARPS) linear_kernel(int n, int in, int 
                                                              const float* __restrict__ target, float* __restrict__ dz,
                                                              float* __restrict__ part) {
   __shared__ float sq[TWARPS];
+  let_next_start();
   const int tn = (out + TBN - 1) / TBN;
   const float inv2 = target ? 2.0f / ((float)n * (float)out) : 0.0f;
   float s = 0.0f;
-  tile_product<true, true>(
+  tile_product<true, true, true>(
       n, out, in, x, in, W, in, blockIdx.x / tn * TBM, blockIdx.x % tn * TBN, false,
       [&](int m, int c, float v) {
         v = act_fwd(v + (b ? b[c] : 0.0f), act);
@@ -257,15 +278,16 @@ __global__ void __launch_bounds__(32 * TWARPS) backward_kernel(int n, int in, in
                                                                float* __restrict__ dprev, int tw,
                                                                const float* __restrict__ part, int parts,
                                                                float* __restrict__ loss) {
+  let_next_start();
   if ((int)blockIdx.x < tw) {
     const int tn = (in + TBN - 1) / TBN;
     const int tm = blockIdx.x / tn, tc = blockIdx.x % tn;
-    tile_product<false, false>(
+    tile_product<false, false, false>(
         out, in, n, dz, out, h, in, tm * TBM, tc * TBN, tc == 0,
         [&](int o, int i, float v) { dW[(int64_t)o * in + i] = v; }, [&](int o, float v) { db[o] = v; });
     if (part && blockIdx.x == 0 && threadIdx.x < 32) {
       float s = 0.0f;
-      for (int c = threadIdx.x; c < parts; c += 32) s += part[c];
+      for (int c = threadIdx.x; c < parts; c += 32) s += __ldcg(part + c);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
       if (threadIdx.x == 0) *loss = s / ((float)n * (float)out);
@@ -273,14 +295,31 @@ __global__ void __launch_bounds__(32 * TWARPS) backward_kernel(int n, int in, in
     return;
   }
   const int t = blockIdx.x - tw, tn = (in + TBN - 1) / TBN;
-  tile_product<true, false>(
+  tile_product<true, false, true>(
       n, in, out, dz, out, W, in, t / tn * TBM, t % tn * TBN, false,
       [&](int m, int i, float v) {
         const int64_t at = (int64_t)m * in + i;
-        const float a = h[at];
+        const float a = __ldcg(h + at);
         dprev[at] = act == WS_ACT_TANH ? v * (1.0f - a * a) : v;
       },
       [](int, float) {});
+}
+
+// Launch that may start before the previous kernel of the stream has ended
+// (early) and then waits for it in the kernel.
+template <class... P, class... A>
+cudaError_t launch_next(void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t st, bool early, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 int tiles(int m, int n) { return ((m + TBM - 1) / TBM) * ((n + TBN - 1) / TBN); }
@@ -346,8 +385,9 @@ __global__ void __launch_bounds__(1024) mse_kernel(const float* p, const float* 
 
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
                             float eps, float c1, float c2) {
+  wait_for_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float gi = g[i];
+    const float gi = __ldcg(g + i);
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
@@ -527,17 +567,21 @@ int ws_mlp_loss_grad(int32_t n, int32_t layers, const int32_t* widths, const flo
     const int in = widths[l], out = widths[l + 1];
     const float* W = params + off[l];
     const bool last = l + 1 == layers;
-    linear_kernel<<<tiles(n, out), 32 * TWARPS, TSMEM, st>>>(
-        n, in, out, h[l], W, W + (int64_t)out * in, last ? WS_ACT_IDENTITY : WS_ACT_TANH,
-        last ? nullptr : const_cast<float*>(h[l + 1]), last ? target : nullptr, dz[l + 1], part);
+    const cudaError_t e =
+        launch_next(linear_kernel, tiles(n, out), 32 * TWARPS, TSMEM, st, l > 0, n, in, out, h[l], W,
+                    W + (int64_t)out * in, (int)(last ? WS_ACT_IDENTITY : WS_ACT_TANH),
+                    last ? nullptr : const_cast<float*>(h[l + 1]), last ? target : nullptr, dz[l + 1], part);
+    if (e != cudaSuccess) return cuda_status("ws_mlp_loss_grad");
   }
   for (int l = layers - 1; l >= 0; --l) {
     const int in = widths[l], out = widths[l + 1], tw = tiles(out, in);
     float* dW = grad + off[l];
     const bool last = l + 1 == layers;
-    backward_kernel<<<tw + (l > 0 ? tiles(n, in) : 0), 32 * TWARPS, TSMEM, st>>>(
-        n, in, out, dz[l + 1], h[l], params + off[l], WS_ACT_TANH, dW, dW + (int64_t)out * in, l > 0 ? dz[l] : nullptr,
-        tw, last ? part : nullptr, tiles(n, widths[layers]), loss);
+    const cudaError_t e =
+        launch_next(backward_kernel, tw + (l > 0 ? tiles(n, in) : 0), 32 * TWARPS, TSMEM, st, true, n, in, out, dz[l + 1],
+                    h[l], params + off[l], (int)WS_ACT_TANH, dW, dW + (int64_t)out * in, l > 0 ? dz[l] : nullptr, tw,
+                    last ? part : nullptr, tiles(n, widths[layers]), loss);
+    if (e != cudaSuccess) return cuda_status("ws_mlp_loss_grad");
   }
   return cuda_status("ws_mlp_loss_grad");
 }
@@ -572,8 +616,8 @@ int ws_adam(float* param, const float* grad, float* m, float* v, int64_t count, 
   if (!param || !grad || !m || !v || count < 0 || step < 1) return bad("ws_adam: bad arguments");
   if (count == 0) return FE_NO_ERROR;
   const float c1 = 1.0f - std::pow(beta1, (float)step), c2 = 1.0f - std::pow(beta2, (float)step);
-  adam_kernel<<<grid_for(count), 256, 0, (cudaStream_t)stream>>>(param, grad, m, v, count, lr, beta1, beta2, eps, c1,
-                                                                  c2);
+  launch_next(adam_kernel, grid_for(count), 256, 0, (cudaStream_t)stream, true, param, grad, m, v, count, lr, beta1, beta2,
+              eps, c1, c2);
   return cuda_status("ws_adam");
 }
 

@@ -188,3 +188,36 @@ def test_network_shapes(torch, widths, rows):
         assert _rel(a.cpu().numpy(), b) <= 2e-5
     if max(widths) <= 256:  # the widest layer it takes
         assert _rel(net.infer_bf16(xd).cpu().numpy(), hs[-1]) <= 2e-2
+
+
+@pytest.mark.parametrize("widths,rows", [((4, 64, 33, 5), 40), ((3, 2), 1)])
+def test_training_step_under_capture(torch, widths, rows):
+    """A recorded training step (its kernels start before their predecessors
+    have ended) gives the bits of the direct one, and steps in a row those of
+    steps with a wait after each call."""
+    from cm_gb300 import warmstart as W
+    g = torch.Generator().manual_seed(1)
+    x, y = torch.randn(rows, widths[0], generator=g).cuda(), torch.randn(rows, widths[-1], generator=g).cuda()
+    nets = [W.MLP(widths, seed=3, device="cuda") for _ in range(3)]
+
+    def step(net, wait):
+        loss = net.loss_and_grad(x, y)
+        if wait:
+            torch.cuda.synchronize()
+        net.adam_step(1e-2)
+        if wait:
+            torch.cuda.synchronize()
+        return loss
+
+    losses = [step(nets[0], True) for _ in range(20)]
+    assert all(torch.equal(a, b) for a, b in zip(losses, [step(nets[1], False) for _ in range(20)]))
+    assert torch.equal(nets[0].flat, nets[1].flat)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        loss = step(nets[2], False)
+    graph.replay()
+    assert torch.equal(loss, losses[0])
+    one = W.MLP(widths, seed=3, device="cuda")
+    step(one, True)
+    assert torch.equal(nets[2].flat, one.flat) and torch.equal(nets[2].grad, one.grad)
