@@ -6,7 +6,7 @@
 //
 // The FP64 pipe binds a large mesh: about 270 warp instructions per
 // triquadratic element, 19 cycles each, are 0.55 ms on the 32^3 box, which
-// takes 0.63 (0.86 in eight launches, one per element colour, with a third
+// takes 0.64 (0.86 in eight launches, one per element colour, with a third
 // more of them).  A small mesh is bound by the latency of one group, which the
 // eight launches paid eight times (9x7x8: 197 -> 23 us).
 #include "fe_mixed_impl.cuh"
