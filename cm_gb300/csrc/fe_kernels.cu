@@ -39,6 +39,7 @@
 
 #include "fe_internal.h"
 #include "fe_math.cuh"
+#include "fe_order.h"
 
 using cmfe::HostSetup;
 using cmfe::KParams;
@@ -697,21 +698,6 @@ bool capturing(cudaStream_t st) {
   return true;
 }
 
-// Work that uses buffers of the handle, on whatever streams, in call order:
-// the stream waits for the handle's previous such work, and the destructor
-// marks the end of what was queued since.
-struct HandleOrder {
-  cudaEvent_t* ev;
-  cudaStream_t st;
-  HandleOrder(cudaEvent_t* ev_, cudaStream_t st_) : ev(ev_), st(st_) {
-    if (!*ev) cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-    if (*ev) cudaStreamWaitEvent(st, *ev, 0);
-  }
-  ~HandleOrder() {
-    if (*ev) cudaEventRecord(*ev, st);
-  }
-};
-
 // The FP64 Jacobian (and the residual when kp.r) by the fused assembly.
 // *taken = false, without an error, where the records cannot be had (no
 // memory left, or the stream is being captured and its replays may run
@@ -721,7 +707,8 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   *taken = false;
   if (capturing(st)) return FE_NO_ERROR;
   if (ensure((void**)&h->d_rec64, cmfe::record_bytes_fp64(s) * (size_t)s.ne)) return FE_NO_ERROR;
-  HandleOrder order(&h->order_event, st);
+  cmfe::HandleOrder order(st);
+  CUDA_TRY(order.begin(&h->order_event));
   cmfe::FusedArgs fa;
   int rc;
   if ((rc = fused_args(h, &h->d_fuse64, st, &fa))) return rc == FE_ERR_OUT_OF_MEMORY ? FE_NO_ERROR : rc;
@@ -749,19 +736,19 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
     ev.push_back(e);
   }
   int* const work = fa.work;
-  if (n > 1) CUDA_TRY(cudaEventRecord(ev[0], st));
   int err = 0;
-  for (int c = n - 1; c >= 0 && !err; --c) {  // the last part on the caller's stream
-    fa.work = work + c;
-    fa.g0 = (int)((int64_t)groups * c / n);
-    fa.g1 = (int)((int64_t)groups * (c + 1) / n);
-    cudaStream_t t = c ? side[c - 1] : st;
-    if (c) CUDA_TRY(cudaStreamWaitEvent(t, ev[0], 0));
-    err = cmfe::launch_fp64_fused(s, kp, so, fa, h->num_sms, t);
-    if (!err) h->launches++;
-    if (c) CUDA_TRY(cudaEventRecord(ev[c], t));
+  {
+    cmfe::Fork fork(st);
+    if (n > 1) CUDA_TRY(cudaEventRecord(ev[0], st));
+    for (int c = n - 1; c >= 0 && !err; --c) {  // the last part on the caller's stream
+      fa.work = work + c;
+      fa.g0 = (int)((int64_t)groups * c / n);
+      fa.g1 = (int)((int64_t)groups * (c + 1) / n);
+      if (c) CUDA_TRY(fork.add(side[c - 1], ev[0], ev[c]));
+      err = cmfe::launch_fp64_fused(s, kp, so, fa, h->num_sms, c ? side[c - 1] : st);
+      if (!err) h->launches++;
+    }
   }
-  for (int c = 1; c < n; ++c) CUDA_TRY(cudaStreamWaitEvent(st, ev[c], 0));
   if (err) return set_error(FE_ERR_CUDA, std::string("FP64 kernel launch: ") + cudaGetErrorString((cudaError_t)err));
   *taken = true;
   return FE_NO_ERROR;
@@ -793,7 +780,8 @@ int residual_run(fe_handle h, const double* dx, double* dr, cudaStream_t st) {
   kp.res_only = 1;
   int rc;
   if (!capturing(st)) {
-    HandleOrder order(&h->residual_event, st);
+    cmfe::HandleOrder order(st);
+    CUDA_TRY(order.begin(&h->residual_event));
     const int nb = s.bnd_ptr.empty() ? 0 : s.bnd_ptr[s.ncolours];
     cmfe::FusedArgs fa;
     std::memset(&fa, 0, sizeof(fa));
@@ -1182,20 +1170,17 @@ int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t s
     // the single-set assembly of every member.  The members are independent,
     // so they run on several streams and small ones share the GPU (24 boxes of
     // 4 to 24 elements an edge: one after the other 3.4 ms, side by side 2.4)
-    const int nl = (int)b->lanes.size();
-    if (nl) CUDA_TRY(cudaEventRecord(b->lane_events[0], st));
-    for (int l = 0; l < nl; ++l) CUDA_TRY(cudaStreamWaitEvent(b->lanes[l], b->lane_events[0], 0));
     int rc = FE_NO_ERROR;
+    cmfe::Fork fork(st);
+    if (!b->lanes.empty()) CUDA_TRY(cudaEventRecord(b->lane_events[0], st));
+    for (size_t l = 0; l < b->lanes.size(); ++l)
+      CUDA_TRY(fork.add(b->lanes[l], b->lane_events[0], b->lane_events[l + 1]));
     for (size_t s = 0; s < b->members.size() && !rc; ++s) {
       const KParams& k = b->h_table[s].kp;
       fe_handle h = b->members[b->slot_member[s]];
       cudaStream_t t = b->slot_lane[s] ? b->lanes[b->slot_lane[s] - 1] : st;
       std::lock_guard<std::mutex> lk(h->mu);
       rc = mixed_assemble(h, k.x, k.vals_uu, k.vals, k.r, false, t, &b->launches);
-    }
-    for (int l = 0; l < nl; ++l) {  // also after an error: the caller's stream follows what was queued
-      CUDA_TRY(cudaEventRecord(b->lane_events[l + 1], b->lanes[l]));
-      CUDA_TRY(cudaStreamWaitEvent(st, b->lane_events[l + 1], 0));
     }
     return rc;
   }
