@@ -521,8 +521,10 @@ struct fe_equations_set {
           *d_u_inc_col = nullptr, *d_p_inc_col = nullptr;
   uint32_t* d_pat = nullptr;
   unsigned char* d_rec = nullptr;
-  // FP64 assembly: its records and counters, and the order of their uses
+  // FP64 assembly: its records and counters, the order of their uses, and
+  // whether there was no memory for them (until fe_set_assembly_order)
   unsigned char* d_rec64 = nullptr;
+  bool no_rec64 = false;
   int* d_fuse64 = nullptr;
   cudaEvent_t order_event = nullptr;
   // residual: its records and node counts (allocated at creation), and their order
@@ -654,6 +656,7 @@ int surface_after(fe_handle h, const KParams& kp, int c, int want_jac, cudaStrea
 }
 
 int ensure(void** buf, size_t bytes);
+cudaError_t try_ensure(void** buf, size_t bytes);
 
 // Group counters at the head of d_fuse: the most launches one fused assembly
 // is split into.
@@ -663,11 +666,13 @@ constexpr int kFuseChunks = 64;
 constexpr int kStreamChunks = 16;
 constexpr int kStreamAuto = 12;
 
+size_t fuse_counters(const HostSetup& s) { return kFuseChunks + (size_t)s.nu + (size_t)s.npn; }
+
 // The arguments of a fused launch of this handle, its counters (*fuse,
 // allocated on first use) set to zero on the stream.
 int fused_args(fe_handle h, int** fuse, cudaStream_t st, cmfe::FusedArgs* fa) {
   const auto& s = h->hs;
-  const size_t counters = kFuseChunks + (size_t)s.nu + (size_t)s.npn;
+  const size_t counters = fuse_counters(s);
   int rc;
   if ((rc = ensure((void**)fuse, sizeof(int) * counters))) return rc;
   CUDA_TRY(cudaMemsetAsync(*fuse, 0, sizeof(int) * counters, st));
@@ -699,19 +704,29 @@ bool capturing(cudaStream_t st) {
 }
 
 // The FP64 Jacobian (and the residual when kp.r) by the fused assembly.
-// *taken = false, without an error, where the records cannot be had (no
-// memory left, or the stream is being captured and its replays may run
-// beside other work of the handle): the caller then launches colour by colour.
+// *taken = false, without an error, where it is not to be: the handle's order
+// is the coloured one, the records cannot be had (found out once; every later
+// call then takes the same route, whose sums have another order), or the
+// stream is being captured, as its replays may run beside other work of the
+// handle.  The caller then launches colour by colour.
 int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   const auto& s = h->hs;
   *taken = false;
-  if (capturing(st)) return FE_NO_ERROR;
-  if (ensure((void**)&h->d_rec64, cmfe::record_bytes_fp64(s) * (size_t)s.ne)) return FE_NO_ERROR;
+  if (h->assembly_order != FE_ASSEMBLY_STAGED || h->no_rec64 || capturing(st)) return FE_NO_ERROR;
+  cudaError_t e = try_ensure((void**)&h->d_rec64, cmfe::record_bytes_fp64(s) * (size_t)s.ne);
+  if (e == cudaSuccess && (e = try_ensure((void**)&h->d_fuse64, sizeof(int) * fuse_counters(s))) != cudaSuccess) {
+    cudaFree(h->d_rec64);
+    h->d_rec64 = nullptr;
+  }
+  if (e != cudaSuccess) {
+    h->no_rec64 = e == cudaErrorMemoryAllocation;
+    return FE_NO_ERROR;
+  }
   cmfe::HandleOrder order(st);
   CUDA_TRY(order.begin(&h->order_event));
   cmfe::FusedArgs fa;
   int rc;
-  if ((rc = fused_args(h, &h->d_fuse64, st, &fa))) return rc == FE_ERR_OUT_OF_MEMORY ? FE_NO_ERROR : rc;
+  if ((rc = fused_args(h, &h->d_fuse64, st, &fa))) return rc;
   kp.elems = nullptr;
   kp.first_elem = 0;
   kp.count = s.ne;
@@ -1041,15 +1056,22 @@ bool mapped_host_ptr(const void* p, void** dptr) {
   return true;
 }
 
-int ensure(void** buf, size_t bytes) {
-  if (*buf) return FE_NO_ERROR;
-  cudaError_t e = cudaMalloc(buf, bytes);
+// Device memory at *buf unless it is there already; on failure *buf is NULL and
+// no error is recorded.
+cudaError_t try_ensure(void** buf, size_t bytes) {
+  if (*buf) return cudaSuccess;
+  const cudaError_t e = cudaMalloc(buf, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *buf = nullptr;
-    return set_error(FE_ERR_OUT_OF_MEMORY, std::string("device staging allocation failed: ") + cudaGetErrorString(e));
   }
-  return FE_NO_ERROR;
+  return e;
+}
+
+int ensure(void** buf, size_t bytes) {
+  const cudaError_t e = try_ensure(buf, bytes);
+  if (e == cudaSuccess) return FE_NO_ERROR;
+  return set_error(FE_ERR_OUT_OF_MEMORY, std::string("device staging allocation failed: ") + cudaGetErrorString(e));
 }
 
 int check_handle(fe_handle h) {
@@ -1769,6 +1791,7 @@ int fe_set_assembly_order(fe_handle h, int32_t order) {
     return set_error(FE_ERR_INVALID_ARGUMENT, "unknown assembly order");
   std::lock_guard<std::mutex> lk(h->mu);
   h->assembly_order = order;
+  h->no_rec64 = false;
   return FE_NO_ERROR;
 }
 

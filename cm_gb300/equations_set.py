@@ -237,7 +237,8 @@ class FiniteElasticityEquationsSet:
     def set_assembly_order(self, order):
         """fe_set_assembly_order: "staged" (per-element records and a row
         gather, the default) or "coloured" (element colours adding into the
-        CSR arrays) for jacobian_evaluate_mixed."""
+        CSR arrays, without records) for jacobian_evaluate and
+        jacobian_evaluate_mixed."""
         code = {"staged": _lib.FE_ASSEMBLY_STAGED, "coloured": _lib.FE_ASSEMBLY_COLOURED}[order]
         check(_lib.load().fe_set_assembly_order(self._h, code))
         self.assembly_order = order

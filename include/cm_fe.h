@@ -124,7 +124,15 @@ int fe_residual_evaluate(fe_handle h, const double* x, double* r, void* stream);
  * finite_elasticity_routines.f90:842-1175, and
  * EQUATIONS_MATRICES_JACOBIAN_ELEMENT_ADD, equations_matrices_routines.f90:
  * 3174-3225).  values is overwritten.  If r is not NULL the residual at x is
- * produced by the same pass. */
+ * produced by the same pass.
+ * In the staged order (fe_set_assembly_order) the first call takes device
+ * memory for element records, about 8 (3 n_p)^2 + 16 n_q 3 n_p + 8 (3 n_p + n_q)
+ * bytes per element (64 kB for a triquadratic element with nodal pressure,
+ * 2.1 GB for 32^3 of them), kept with the handle besides the records of the
+ * mixed assembly.  In the coloured order, on a stream that is being captured
+ * into a graph, and from a first call on that finds no memory for the records,
+ * the assembly runs colour by colour without them.  The two routes agree to
+ * rounding, not bit for bit; each is bit-reproducible. */
 int fe_jacobian_evaluate(fe_handle h, const double* x, double* values, double* r, void* stream);
 
 /* Mixed-precision Jacobian: the displacement-displacement block in FP32, the
@@ -186,18 +194,19 @@ int fe_set_materials(fe_handle h, const double* materials);
 #define FE_HIGH_PRECISION_DOUBLE_FLOAT 1
 int fe_set_high_precision(fe_handle h, int32_t mode);
 
-/* How fe_jacobian_evaluate_mixed adds the element contributions into the
- * CSR values and the residual (both deterministic; no counterpart in the
- * reference, which adds element by element, MATRIX_VALUES_ADD_DP2,
- * matrix_vector.f90:2756-2880).
+/* How fe_jacobian_evaluate and fe_jacobian_evaluate_mixed add the element
+ * contributions into the CSR values and the residual (both deterministic; no
+ * counterpart in the reference, which adds element by element,
+ * MATRIX_VALUES_ADD_DP2, matrix_vector.f90:2756-2880).
  * FE_ASSEMBLY_STAGED (the default): every element stores its entries in a
  * per-element record on the device, and each CSR row is formed once from the
  * records of the elements around the row's node, in increasing element
  * number, in the same launch, by the block that assembles the node's last
  * element.  Every matrix sector is written once and never read.  The records
- * take, per element, about 4 (3 n_p)^2 + 16 n_q 3 n_p + 8 (3 n_p + n_q) bytes
- * (38 kB for a triquadratic element with nodal pressure), allocated on the
- * first staged evaluation and kept with the handle.
+ * of the mixed assembly take, per element, about 4 (3 n_p)^2 + 16 n_q 3 n_p +
+ * 8 (3 n_p + n_q) bytes (38 kB for a triquadratic element with nodal
+ * pressure), allocated on the first staged evaluation and kept with the
+ * handle; those of the FP64 one: see fe_jacobian_evaluate.
  * FE_ASSEMBLY_COLOURED: one launch per element colour, each element adding
  * its entries straight into the CSR arrays (the first contributor in colour
  * order stores, later ones add).  No extra memory.

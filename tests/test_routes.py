@@ -1,0 +1,130 @@
+"""Routes that a call takes where its usual one does not apply: the coloured
+order, streams under capture, no memory for the element records."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from cm_gb300 import FiniteElasticityEquationsSet, _lib
+from cm_gb300 import mesh as M
+
+pytestmark = pytest.mark.gpu
+
+REL, FLOOR = 1e-12, 1e-13  # FP64 results per entry, as in the oracle parity tests
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch as _torch
+    if not _torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    _lib.load()
+    return _torch
+
+
+def box(torch, dims, nxi=3, pressure="node", load=False):
+    m = M.regular_box(*dims, lengths=tuple(0.5 * d for d in dims), nxi_u=nxi, pressure=pressure, law=M.MR,
+                      materials=(2.0, 6.0), perturb=0.05, seed=2)
+    sp = None
+    if load:
+        sp = np.zeros((3, m.nu))
+        i, j, k = m.node_ijk()
+        sp[2, k == 0] = 1.2
+        sp[0, i == i.max()] = -0.4
+    es = FiniteElasticityEquationsSet(m)
+    if load:
+        es.set_surface_pressure(sp)
+    x = M.deformed_state(m, stretch=1.05, shear=0.03, noise=0.02, pressure=-2.0, seed=4)
+    return m, es, x, torch.from_numpy(x).cuda(), sp
+
+
+def close(got, ref, what):
+    err = np.abs(got.cpu().numpy() - ref)
+    assert (err <= REL * np.abs(ref) + FLOOR * np.abs(ref).max()).all(), (what, err.max())
+
+
+def last_error():
+    buf = C.create_string_buffer(512)
+    _lib.load().fe_last_error(buf, 512)
+    return buf.value
+
+
+def test_coloured_order_takes_no_records(torch):
+    """In the coloured order the FP64 Jacobian allocates nothing on the device."""
+    _, warm, _, xw, _ = box(torch, (2, 2, 2))
+    _, es, _, x, _ = box(torch, (12, 12, 12))
+    for e in (warm, es):
+        e.set_assembly_order("coloured")
+    warm.jacobian_evaluate(xw)
+    v = torch.empty(es.nnz, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    es.jacobian_evaluate(x, v)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+
+
+def test_no_memory_for_the_records(torch):
+    """A first FP64 Jacobian that finds no memory for its records has the bits
+    of the coloured order and leaves no error behind; so do later ones, until
+    the order is set again."""
+    m, es, _, x, _ = box(torch, (12, 12, 12))  # records: 110 MB
+    new = lambda: torch.empty(es.nnz, dtype=torch.float64, device="cuda")  # noqa: E731
+    v, coloured, staged, r = new(), new(), new(), torch.empty_like(x)
+    other = FiniteElasticityEquationsSet(m)
+    other.jacobian_evaluate(x, staged, r)
+    other.set_assembly_order("coloured")
+    other.jacobian_evaluate(x, coloured, r)
+    torch.cuda.synchronize()
+    assert not torch.equal(staged, coloured)
+    torch.cuda.empty_cache()
+    error = last_error()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")
+    es.jacobian_evaluate(x, v, r)
+    torch.cuda.synchronize()
+    assert torch.equal(v, coloured) and last_error() == error
+    del rest
+    torch.cuda.empty_cache()
+    es.jacobian_evaluate(x, v.fill_(0.0), r)
+    assert torch.equal(v, coloured)
+    es.set_assembly_order("staged")
+    es.jacobian_evaluate(x, v.fill_(0.0), r)
+    assert torch.equal(v, staged)
+
+
+@pytest.mark.parametrize("load", [False, True])
+@pytest.mark.parametrize("nxi,pressure", [(2, "element"), (2, "node"), (3, "element"), (3, "node")])
+def test_captured_calls(torch, oracle, nxi, pressure, load):
+    """The FP64 Jacobian (with and without the residual) and the residual
+    recorded into a graph, at a state written after the recording: the
+    oracle's values, for the Jacobian the bits of the coloured order, for the
+    residual without a surface load those of the direct call."""
+    m, es, x, xd, sp = box(torch, (4, 3, 5), nxi, pressure, load)
+    P = oracle.Problem(m)
+    P.set_surface_pressure(sp)
+    rp, col = P.pattern()
+    vo, ro = P.assemble(x, rp, col, nthreads=8)
+    new = lambda n: torch.full((n,), float("nan"), dtype=torch.float64, device="cuda")  # noqa: E731
+    xin, v, v2, r, r2 = torch.empty_like(xd), new(es.nnz), new(es.nnz), new(es.ndofs), new(es.ndofs)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        es.jacobian_evaluate(xin, v, r)
+        es.jacobian_evaluate(xin, v2)
+        es.residual_evaluate(xin, r2)
+    xin.copy_(xd)
+    for _ in range(2):
+        for t in (v, v2, r, r2):
+            t.fill_(float("nan"))
+        graph.replay()
+        es.check_status(xd)
+        close(v, vo, "values")
+        close(r, ro, "residual of the Jacobian")
+        close(r2, ro, "residual")
+        assert torch.equal(v, v2)
+    direct = es.residual_evaluate(xd)
+    close(direct, ro, "direct residual")
+    if not load:
+        assert torch.equal(direct, r2)
+    es.set_assembly_order("coloured")
+    assert torch.equal(es.jacobian_evaluate(xd), v)
