@@ -92,6 +92,7 @@ SIGNATURES = {
     "fe_set_surface_pressure": [_vp, _vp],
     "fe_set_materials": [_vp, _vp],
     "fe_newton_options_default": [C.POINTER(FENewtonOptions)],
+    "fe_newton_set_barrier_limits": [_vp, C.c_uint32, C.c_uint32],
     "fe_newton_load_step": [_vp, _vp, _vp, _i64, _vp, C.POINTER(FENewtonOptions), C.POINTER(FENewtonReport), _vp],
     "fe_check": [_vp, _vp],
     "fe_launch_count": [_vp, C.POINTER(_i64)],

@@ -261,6 +261,8 @@ int launch_mixed_batch(int variant, unsigned mask, const BatchMember* members, i
 // (fe_kernels.cu), for the Newton driver (fe_newton.cu).
 int device_pattern(fe_handle h, const int32_t** row_ptr, const int32_t** col, int64_t* ndofs, int64_t* nnz,
                    int64_t* nu3);
+// Limits of the grid barriers of the GMRES cycle (fe_newton_set_barrier_limits).
+void newton_barrier_limits(fe_handle h, unsigned* polls, int* extra_from);
 
 // Records the text fe_last_error() returns (per calling thread) and returns code.
 int record_error(int code, const std::string& msg);

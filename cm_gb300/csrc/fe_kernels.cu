@@ -531,6 +531,8 @@ struct fe_equations_set {
   unsigned char* d_rec_r = nullptr;
   int* d_done_r = nullptr;
   cudaEvent_t residual_event = nullptr;
+  unsigned cycle_polls = 0;  // grid-barrier limits of the GMRES cycle (fe_newton_set_barrier_limits)
+  int cycle_extra_from = 0;
   std::vector<cudaStream_t> side_streams;  // parts of a small mesh's FP64 assembly
   std::vector<cudaEvent_t> side_events;
   int* d_fuse = nullptr;  // fused staged assembly: [0, kFuseChunks) group counters, then per-row-node counts
@@ -1323,6 +1325,11 @@ int device_pattern(fe_handle h, const int32_t** row_ptr, const int32_t** col, in
   *nu3 = 3 * (int64_t)h->hs.nu;
   return FE_NO_ERROR;
 }
+
+void newton_barrier_limits(fe_handle h, unsigned* polls, int* extra_from) {
+  *polls = h->cycle_polls;
+  *extra_from = h->cycle_extra_from;
+}
 }  // namespace cmfe
 
 extern "C" {
@@ -1792,6 +1799,17 @@ int fe_set_assembly_order(fe_handle h, int32_t order) {
   std::lock_guard<std::mutex> lk(h->mu);
   h->assembly_order = order;
   h->no_rec64 = false;
+  return FE_NO_ERROR;
+}
+
+int fe_newton_set_barrier_limits(fe_handle h, uint32_t polls, uint32_t extra_from) {
+  if (!h) return set_error(FE_ERR_INVALID_ARGUMENT, "NULL handle");
+  if (extra_from > INT32_MAX) return set_error(FE_ERR_INVALID_ARGUMENT, "extra_from out of range");
+  if (extra_from && (polls == 0 || polls > 4096))
+    return set_error(FE_ERR_INVALID_ARGUMENT, "an unreachable barrier needs a poll limit in 1..4096");
+  std::lock_guard<std::mutex> lk(h->mu);
+  h->cycle_polls = polls;
+  h->cycle_extra_from = (int)extra_from;
   return FE_NO_ERROR;
 }
 

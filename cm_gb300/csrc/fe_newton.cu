@@ -318,6 +318,8 @@ struct CycleArgs {
   double *res, *dx, *z, *part, *part2, *npart, *y;
   double* scale;  // 1 / norm of the newest basis vector, -1: converged
   int* ctl;       // barrier arrivals; zeroed before the launch
+  unsigned polls;  // of a barrier, before it gives up
+  int extra_from;  // > 0: barriers from this one on wait for one arrival more than there are
   double* host;  // page-locked: squared norm of the true residual, iterations, converged
 };
 
@@ -355,18 +357,18 @@ __global__ void __launch_bounds__(MAX_SHARES + 32) k_cycle_bounds(int n, int nb,
 }
 
 // Grid barrier number k = 1, 2, ... of the launch; false when it gave up.
-__device__ __forceinline__ bool cycle_barrier(int* arrivals, int k) {
+__device__ __forceinline__ bool cycle_barrier(const CycleArgs& A, int k) {
   __shared__ bool ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(arrivals, 1);
-    const int target = k * (int)gridDim.x;
+    atomicAdd(A.ctl, 1);
+    const int target = k * (int)gridDim.x + (A.extra_from > 0 && k >= A.extra_from);
     unsigned polls = 0;
     int v;
     do {
-      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(arrivals) : "memory");
-    } while (v < target && ++polls < CYCLE_POLLS);
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(A.ctl) : "memory");
+    } while (v < target && ++polls < A.polls);
     ok = v >= target;
     __threadfence();
   }
@@ -579,7 +581,7 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
     return fabs(g[k + 1]) <= A.tol || c[k + 1] <= A.breakdown;
   };
 
-  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (!cycle_barrier(A, ++bar)) return;
   int K = 0;
   bool converged = false;
   for (int k = 0;; ++k) {
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
       converged = rotate(k - 1);
       if (tid == 0) *A.scale = converged ? -1.0 : red[0];
     }
-    if (!cycle_barrier(A.ctl, ++bar)) return;
+    if (!cycle_barrier(A, ++bar)) return;
     // V_k, the product and its dots still lack the scale of V_k
     const double a = k ? __ldcg(A.scale) : 1.0;
     cycle_sums(A.part, A.nb, m, [&](int j, double s) { h[j] = j == k ? s * a * a : s * a; });
@@ -622,7 +624,7 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
     } else {
       for (int j = tid; j < m; j += CT) c[j] = h[j];
     }
-    if (!cycle_barrier(A.ctl, ++bar)) return;
+    if (!cycle_barrier(A, ++bar)) return;
     cycle_sums(A.part2, A.nb, m, [&](int j, double s) { h[j] = s; });
     __syncthreads();
     if (!givens) {
@@ -639,7 +641,7 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
     } else {
       for (int j = tid; j < m; j += CT) c[j] += h[j];
     }
-    if (!cycle_barrier(A.ctl, ++bar)) return;
+    if (!cycle_barrier(A, ++bar)) return;
     if (m == A.kmax) {
       if (givens) {
         if (warp == 0) {
@@ -664,14 +666,14 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
       __syncthreads();
     }
   }
-  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (!cycle_barrier(A, ++bar)) return;
   if (!givens) {
     for (int j = tid; j < K; j += CT) h[j] = __ldcg(A.y + j);
     __syncthreads();
     const double s = row_warp ? combine(K) : 0.0;
     if (grp < rows && q == 0) A.dx[r0 + grp] = fma(mi[grp], s, A.dx[r0 + grp]);
   }
-  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (!cycle_barrier(A, ++bar)) return;
   // the true residual and its norm
   if (!givens) {
     product(A.dx);
@@ -679,7 +681,7 @@ __global__ void __launch_bounds__(CT, 1) k_cycle(const __grid_constant__ CycleAr
     if (grp < rows && q == 0) A.res[r0 + grp] = t = A.b[r0 + grp] - wn[grp];
     norm_share(t);
   }
-  if (!cycle_barrier(A.ctl, ++bar)) return;
+  if (!cycle_barrier(A, ++bar)) return;
   if (givens && warp == 0) {
     const double r2 = cycle_norm(A.npart, A.nb);
     if (lane == 0) {
@@ -941,6 +943,9 @@ struct Solver {
     a.scale = scal;
     a.y = col_d;
     a.ctl = ctl;
+    unsigned polls = 0;
+    cmfe::newton_barrier_limits(h, &polls, &a.extra_from);
+    a.polls = polls ? polls : CYCLE_POLLS;
     a.bound = bound;
     a.host = pinned;
     k_cycle_bounds<<<1, MAX_SHARES + 32, 0, st>>>((int)n, nb, rp, bound);
@@ -948,7 +953,8 @@ struct Solver {
   }
 
   // One cycle of at most kmax iterations by k_cycle; *ran false when the GPU
-  // cannot hold its blocks at once.
+  // cannot hold its blocks at once or one of its barriers gave up, after which
+  // res and dx hold nothing of use.
   int cycle(const double* b, double* res, double* dx, double beta, double tol, int kmax, bool* ran, int* K,
             bool* converged, double* r2) {
     CycleArgs a = cyc;
@@ -970,8 +976,8 @@ struct Solver {
     }
     NT_TRY(e);
     NT_TRY(cudaStreamSynchronize(st));
-    if (pinned[1] < 0.0) return cmfe::record_error(FE_ERR_CUDA, "a grid barrier of the GMRES cycle gave up");
-    *ran = true;
+    *ran = pinned[1] >= 0.0;
+    if (!*ran) return FE_NO_ERROR;
     *r2 = pinned[0];
     *K = (int)pinned[1];
     *converged = pinned[2] != 0.0;
@@ -1007,7 +1013,12 @@ struct Solver {
           if (conv && beta <= rtol * bnorm) break;
           continue;
         }
+        // the four kernels, from the start of this solve
         cyc_smem = 0;
+        *its = 0;
+        beta = bnorm;
+        NT_TRY(cudaMemsetAsync(dx, 0, sizeof(double) * n, st));
+        NT_TRY(cudaMemcpyAsync(res, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
       }
       std::fill(g.begin(), g.end(), 0.0);
       g[0] = beta;

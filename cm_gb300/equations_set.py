@@ -279,6 +279,12 @@ class FiniteElasticityEquationsSet:
                                     C.byref(o), C.byref(rep), _stream(x)))
         return {k: getattr(rep, k) for k, _ in rep._fields_}
 
+    def set_newton_barrier_limits(self, polls=0, extra_from=0):
+        """fe_newton_set_barrier_limits: diagnostic of the failure path of the
+        one-launch GMRES cycle (barriers from number extra_from on give up
+        after `polls` polls; (0, 0) restores the default)."""
+        check(_lib.load().fe_newton_set_barrier_limits(self._h, polls, extra_from))
+
     def check_status(self, x=None):
         check(_lib.load().fe_check(self._h, _stream(x)))
 

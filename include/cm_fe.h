@@ -391,6 +391,15 @@ void fe_newton_options_default(fe_newton_options* options);
 int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fixed_values, int64_t num_fixed,
                         double* x, const fe_newton_options* options, fe_newton_report* report, void* stream);
 
+/* Diagnostic for the failure detection of the one-launch GMRES cycle that
+ * small systems take (no counterpart in the reference).  Its grid barriers poll
+ * at most `polls` times (0: the default, about a second) and then give up; the
+ * kernel returns, and the load step does that linear solve and the later ones
+ * with one launch per phase.  extra_from > 0 makes the barriers of a cycle from
+ * that number on wait for one arrival more than the grid can give, so that they
+ * give up; it needs polls in 1..4096.  (0, 0) restores the default. */
+int fe_newton_set_barrier_limits(fe_handle h, uint32_t polls, uint32_t extra_from);
+
 /* Waits for the handle's work on `stream` and reports numerical problems
  * seen by the kernels since the last call (FE_ERR_NUMERICAL) — the device
  * counterpart of the reference's error flags, set instead of trapping. */

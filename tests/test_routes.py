@@ -1,5 +1,6 @@
 """Routes that a call takes where its usual one does not apply: the coloured
-order, streams under capture, no memory for the element records."""
+order, streams under capture, no memory for the element records, a GMRES cycle
+whose grid barrier gives up."""
 import ctypes as C
 
 import numpy as np
@@ -128,3 +129,35 @@ def test_captured_calls(torch, oracle, nxi, pressure, load):
         assert torch.equal(direct, r2)
     es.set_assembly_order("coloured")
     assert torch.equal(es.jacobian_evaluate(xd), v)
+
+
+@pytest.mark.parametrize("restart,extra_from", [(30, 1), (30, 2), (30, 17), (4, 13), (4, 14), (4, 15), (4, 16), (4, 17)])
+def test_gmres_cycle_gives_up(torch, restart, extra_from):
+    """A load step in whose one-launch GMRES cycle a barrier gives up -- in its
+    first iterations, around the end of a short cycle where the solution and
+    the residual are updated, or in none when the cycle has fewer -- converges
+    to the state of an undisturbed one; so does the next step of the handle."""
+    from cm_gb300 import FEError, newton as N
+    m = M.regular_box(3, 2, 2, nxi_u=3, pressure="node", law=M.MR, materials=(2.0, 6.0))
+    bc = N.clamped_stretch_shear_conditions(m, 1.05, 0.02)
+    x0 = torch.from_numpy(N.initial_state(m)).cuda()
+
+    def step(es):
+        x = x0.clone()
+        rep = es.newton_load_step(x, bc.dofs, bc.full, ksp_restart=restart, ksp_max_iterations=4000)
+        assert rep["converged"] == 1 and rep["residual_norm"] <= 1e-10, rep
+        return x
+
+    es = FiniteElasticityEquationsSet(m)
+    ref = step(es)
+    es.set_newton_barrier_limits(4096, extra_from)
+    # converged states agree as in the other Newton tests: a residual norm of
+    # 1e-10 over a smallest stiffness of about 1e-2
+    x = step(es)
+    assert float((x - ref).abs().max()) <= 1e-8
+    # a cycle of four iterations has 16 barriers; the other route sums in another order
+    assert torch.equal(x, ref) == (extra_from == 17 and restart == 4)
+    es.set_newton_barrier_limits(0, 0)
+    assert torch.equal(step(es), ref)
+    with pytest.raises(FEError):
+        es.set_newton_barrier_limits(0, 1)
