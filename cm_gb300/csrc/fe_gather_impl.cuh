@@ -193,17 +193,20 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
         __syncwarp();
       }
     }
+    // row after row, so that the sectors a store begins or ends in are completed
+    // by the next one: over the host link (outputs in page-locked memory) every
+    // part of a sector is a write of its own (32^3 box 7.10 ms with the columns
+    // as the outer loop, 6.00 so; device outputs 1.81 and 1.80)
 #pragma unroll
-    for (int i = 0; i < GPOS / 32; ++i) {
-      const int pos = p0 + 32 * i + lane;
-      if (pos < wu) {
+    for (int m = 0; m < 3; ++m)
 #pragma unroll
-        for (int m = 0; m < 3; ++m)
+      for (int n = 0; n < 3; ++n)
 #pragma unroll
-          for (int n = 0; n < 3; ++n)
+        for (int i = 0; i < GPOS / 32; ++i) {
+          const int pos = p0 + 32 * i + lane;
+          if (pos < wu)
             du[m][n * wu + pos] = FULL ? (T)uacc[(3 * m + n) * GPOS + 32 * i + lane] : acc[FULL ? 0 : i][3 * m + n];
-      }
-    }
+        }
     if (q0 + lane < wc) {
 #pragma unroll
       for (int m = 0; m < 3; ++m) dc[m][q0 + lane] = cacc[m * GPP + lane];
