@@ -23,7 +23,7 @@
 // with the norm, the preconditioning and the Hessenberg column, matrix-vector
 // product with the scaling; a block owns a chunk of rows and its warps take
 // different basis vectors, so no dot waits on a block-wide reduction, the sums
-// over the at most 64 chunks are formed by the kernel that uses them, the host
+// over the chunks (row_chunks) are formed by the kernel that uses them, the host
 // rotates the columns, and the next iteration is queued before it waits for one.
 #include "fe_internal.h"
 
@@ -40,14 +40,18 @@ namespace {
 
 constexpr int NT = 256;
 constexpr int NWARP = NT / 32;
-constexpr int MAX_CHUNKS = 64;  // row chunks of a reduction: one block each
+constexpr int MAX_CHUNKS = 608;  // row chunks of a reduction: one block each
 
 // y = P A x on the free rows (P: the free-dof mask), 0 on the fixed ones, for
 // x zero on the fixed dofs; with scale: y and v scaled by *scale.  One warp
 // takes two rows, lanes over the entries, and reduces both with five
 // additions instead of ten: the FP64 pipe (19 cycles of an SM per warp
-// instruction) and two waits for memory bind it.  A row of a triquadratic box
-// has 100 to 400 entries; eight a lane are loaded at once.
+// instruction) and two waits for memory bind it.  U entries a lane are loaded
+// at once: eight for the rows of a triquadratic mesh (100 to 400 entries), four
+// for the shorter ones of a trilinear one, whose multiply-adds past the end of
+// the row would hold the pipe as long as real ones (a GMRES iteration on
+// 270,763 rows of about 80 entries: 243 against 315 us with eight).
+template <int U>
 __global__ void __launch_bounds__(NT) k_spmv(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
                                              const double* __restrict__ val, const uint8_t* __restrict__ free_dof,
                                              const double* __restrict__ x, double* __restrict__ y,
@@ -65,12 +69,12 @@ __global__ void __launch_bounds__(NT) k_spmv(int64_t n, const int32_t* __restric
       end[r] = in ? rp[i + r + 1] : 0;
     }
     while (__any_sync(0xffffffffu, at[0] < end[0] || at[1] < end[1])) {
-      double a[2][8];
-      int c[2][8];
+      double a[2][U];
+      int c[2][U];
 #pragma unroll
       for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < U; ++u) {
           const bool in = at[r] + 32 * u < end[r];
           a[r][u] = in ? val[at[r] + 32 * u] : 0.0;
           c[r][u] = in ? col[at[r] + 32 * u] : 0;
@@ -78,9 +82,9 @@ __global__ void __launch_bounds__(NT) k_spmv(int64_t n, const int32_t* __restric
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < U; ++u)
           if (at[r] + 32 * u < end[r]) s[r] = fma(a[r][u], x[c[r][u]], s[r]);
-        at[r] += 256;
+        at[r] += 32 * U;
       }
     }
     // lanes 0..15 go on with the first row, 16..31 with the second
@@ -743,6 +747,16 @@ __global__ void k_fix(int64_t m, const int32_t* __restrict__ dofs, const double*
   }
 }
 
+// Row chunks of a reduction: one, two or four to an SM of the 152.  Every block
+// adds up all chunks' shares (eight lanes to a sum), so more of them help only
+// where the rows are what takes the time.  A GMRES iteration with 64, 152, 304
+// and 608 chunks, us: 13,653 rows 51, 45, 47, 47; 49,072 rows 147, 108, 100,
+// 116; 216,024 rows 509, 351, 294, 295; 859,812 rows 2,510, 1,485, 1,136, 998.
+int row_chunks(int64_t n) {
+  const int64_t most = MAX_CHUNKS / 4 * (n < 24000 ? 1 : n < 200000 ? 2 : 4);
+  return (int)std::min<int64_t>((n + 63) / 64, most);
+}
+
 int blocks_for(int64_t n) {
   const int64_t b = (n + NT - 1) / NT;
   return (int)(b < 4096 ? (b < 1 ? 1 : b) : 4096);
@@ -824,7 +838,13 @@ struct Solver {
   }
 
   int spmv(const double* x, double* y) {
-    k_spmv<<<warp_blocks_for((n + 1) / 2), NT, 0, st>>>(n, rp, col, vals, free_dof, x, y, nullptr, nullptr);
+    return spmv(x, y, nullptr, nullptr, st);
+  }
+
+  // y = P A x; with scale, y and v scaled by it.
+  int spmv(const double* x, double* y, const double* scale, double* v, cudaStream_t t) {
+    auto kern = nnz <= 128 * n ? k_spmv<4> : k_spmv<8>;
+    kern<<<warp_blocks_for((n + 1) / 2), NT, 0, t>>>(n, rp, col, vals, free_dof, x, y, scale, v);
     NT_TRY(cudaGetLastError());
     return FE_NO_ERROR;
   }
@@ -868,10 +888,8 @@ struct Solver {
     k_update_dots<<<chunks, NT, 0, t>>>(n, V, n, m, part, wv, cd, part2);
     k_update_norm<<<chunks, NT, 0, t>>>(n, V, n, m, part2, wv, cd, npart, done, minv, z,
                                         pinned + (size_t)(k & 1) * (restart + 2));
-    if (m < restart)
-      k_spmv<<<warp_blocks_for((n + 1) / 2), NT, 0, t>>>(n, rp, col, vals, free_dof, z, V + (size_t)(m + 1) * n, cd + m, wv);
     NT_TRY(cudaGetLastError());
-    return FE_NO_ERROR;
+    return m < restart ? spmv(z, V + (size_t)(m + 1) * n, cd + m, wv, t) : FE_NO_ERROR;
   }
 
   // The same, from the second cycle on as one graph launch: single launches
@@ -1121,8 +1139,7 @@ int fe_newton_load_step(fe_handle h, const int32_t* fixed_dofs, const double* fi
   int* bound;
   const size_t rs = (size_t)S.restart;
   const size_t basis = rs + 1;
-  int64_t chunks = (n + 63) / 64;
-  S.chunks = (int)(chunks < MAX_CHUNKS ? chunks : MAX_CHUNKS);
+  S.chunks = row_chunks(n);
   W.add(&S.vals, (size_t)S.nnz);
   for (double** p : {&S.r, &S.rn, &S.d, &S.xs, &S.w, &S.minv, &S.diag, &S.z, &dx_state}) W.add(p, (size_t)n);
   W.add(&S.V, (basis + 1) * n);

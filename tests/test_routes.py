@@ -161,3 +161,50 @@ def test_gmres_cycle_gives_up(torch, restart, extra_from):
     assert torch.equal(step(es), ref)
     with pytest.raises(FEError):
         es.set_newton_barrier_limits(0, 1)
+
+
+@pytest.mark.parametrize("nxi,dims", [(2, (14, 13, 13)), (3, (10, 10, 10)), (2, (40, 40, 40))])
+def test_gmres_on_many_rows(torch, nxi, dims):
+    """Systems beyond the one-launch cycle, with one, two and four row chunks to
+    an SM and short and long rows: the first Newton step of a few GMRES
+    iterations against the same method in plain torch (FP64, an orthonormal
+    basis, least squares).  The two differ by the rounding of sums of 10^5
+    terms through a dozen well-conditioned steps."""
+    from cm_gb300 import newton as N
+    m = M.regular_box(*dims, nxi_u=nxi, pressure="node" if nxi == 3 else "element", law=M.MR, materials=(2.0, 6.0))
+    bc = N.clamped_stretch_shear_conditions(m, 1.05, 0.02) if nxi == 3 else N.uniaxial_symmetry_conditions(m, 1.05)
+    its = 12
+    es = FiniteElasticityEquationsSet(m)
+    x = torch.from_numpy(N.initial_state(m)).cuda()
+    got = x.clone()
+    rep = es.newton_load_step(got, bc.dofs, bc.full, ksp_max_iterations=its, max_iterations=1)
+    assert rep["linear_iterations"] == its
+    fixed = torch.as_tensor(np.asarray(bc.dofs, dtype=np.int64)).cuda()
+    x[fixed] = torch.as_tensor(np.asarray(bc.full, dtype=np.float64)).cuda()
+    free = torch.ones_like(x)
+    free[fixed] = 0.0
+    r = torch.empty_like(x)
+    vals = es.jacobian_evaluate(x, r=r)
+    rp, col = (torch.from_numpy(a.astype(np.int64)).cuda() for a in es.csr_pattern())
+    row = torch.repeat_interleave(torch.arange(es.ndofs, device="cuda"), rp[1:] - rp[:-1])
+    A = torch.sparse_csr_tensor(rp, col, vals * free[row] * free[col], size=(es.ndofs, es.ndofs))
+    nu3 = 3 * m.nu
+    diag = torch.zeros_like(x).index_add_(0, row[row == col], vals[row == col])
+    s = torch.zeros_like(x).index_add_(0, row, torch.where(col < nu3, vals * vals * free[col] / diag[col], 0.0))
+    minv = free * torch.where(torch.arange(es.ndofs, device="cuda") < nu3, 1.0 / diag, -1.0 / torch.where(s != 0, s, 1.0))
+    b = -r * free
+    V, H = [b / b.norm()], torch.zeros(its + 1, its, dtype=torch.float64, device="cuda")
+    for k in range(its):
+        w = A @ (minv * V[k])
+        for _ in range(2):
+            for j, v in enumerate(V):
+                h = v @ w
+                H[j, k] += h
+                w = w - h * v
+        H[k + 1, k] = w.norm()
+        V.append(w / H[k + 1, k])
+    e = torch.zeros(its + 1, 1, dtype=torch.float64)
+    e[0] = float(b.norm())
+    y = torch.linalg.lstsq(H.cpu(), e).solution[:, 0].cuda()
+    d = minv * sum(c * v for c, v in zip(y, V))
+    assert float((got - x - rep["last_lambda"] * d).norm()) <= 1e-9 * float(d.norm())
