@@ -521,11 +521,28 @@ int ws_gemm_f32(int32_t m, int32_t n, int32_t k, const float* a, int64_t a_sm, i
   return cuda_status("ws_gemm_f32");
 }
 
+// Many rows: the 64 x 64 tiles of gemm_kernel use their operands four times as
+// often as linear_kernel's 32 x 16 ones, whose split contraction and epilogue
+// are for the latency of few; the shorter the contraction, the sooner that
+// tells.  us, linear_kernel against gemm_kernel and bias_act_kernel, [in x out]:
+// 4 x 256 1,024 rows 12.4, 15.7, 2,048 rows 17.0, 16.1, 131,072 rows 509, 163;
+// 64 x 64 8,192 rows 20.9, 23.3, 16,384 rows 31.5, 29.2; 256 x 256 8,192 rows
+// 95, 100, 16,384 rows 181, 173, 131,072 rows 1,399, 1,096.
+static bool many_rows(int n, int in, int out) {
+  return tiles(n, out) >= 768 + 18 * (in < 256 ? in : 256) && (n + TM - 1) / TM <= 65535;
+}
+
 int ws_linear_f32(int32_t n, int32_t in, int32_t out, const float* x, const float* w, const float* bias, int32_t act,
                   float* y, void* stream) {
   if (n < 0 || in <= 0 || out <= 0 || !x || !w || !y || (act != WS_ACT_IDENTITY && act != WS_ACT_TANH))
     return bad("ws_linear_f32: bad arguments");
   if (n == 0) return FE_NO_ERROR;
+  if (many_rows(n, in, out)) {
+    gemm_kernel<<<dim3((out + TN - 1) / TN, (n + TM - 1) / TM), 256, 0, (cudaStream_t)stream>>>(n, out, in, x, in, 1, w,
+                                                                                                1, in, y, out, 0.0f);
+    bias_act_kernel<<<grid_for((int64_t)n * out), 256, 0, (cudaStream_t)stream>>>(y, bias, n, out, act);
+    return cuda_status("ws_linear_f32");
+  }
   const int rc = tile_attributes();
   if (rc) return rc;
   linear_kernel<<<tiles(n, out), 32 * TWARPS, TSMEM, (cudaStream_t)stream>>>(n, in, out, x, w, bias, act, y, nullptr,

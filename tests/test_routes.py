@@ -208,3 +208,21 @@ def test_gmres_on_many_rows(torch, nxi, dims):
     y = torch.linalg.lstsq(H.cpu(), e).solution[:, 0].cuda()
     d = minv * sum(c * v for c, v in zip(y, V))
     assert float((got - x - rep["last_lambda"] * d).norm()) <= 1e-9 * float(d.norm())
+
+
+@pytest.mark.parametrize("widths,rows", [((4, 256, 9), 2070), ((7, 64, 61), 16500), ((3, 256, 256), 12289)])
+def test_network_with_many_rows(torch, widths, rows):
+    """Layers of so many rows that they take the large tiles, and of one tile
+    of rows fewer, against FP64; the bar of the other network tests."""
+    from cm_gb300 import warmstart as W
+    net = W.MLP(widths, seed=3, device="cuda")
+    g = torch.Generator().manual_seed(2)
+    net.flat.add_(0.1 * torch.randn(net.flat.shape, generator=g).cuda())
+    x = torch.randn(rows, widths[0], generator=g).cuda()
+    for n in (rows, rows - 800):
+        h = x[:n].double()
+        for l, got in enumerate(net.forward(x[:n])[1:]):
+            h = h @ net.W(l).double().T + net.b(l).double()
+            if l + 1 < net.layers:
+                h = torch.tanh(h)
+            assert float((got - h).abs().max()) <= 2e-5 * float(h.abs().max())
