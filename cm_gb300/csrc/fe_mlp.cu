@@ -503,6 +503,52 @@ __global__ void __cluster_dims__(ICLUSTER, 1, 1) __launch_bounds__(32 * IW)
   }
 }
 
+// The same by one CTA of eight warps per 16 rows, which walks the layers' tiles
+// of 8 features and waits for their weights from L2: with enough rows to fill
+// the SMs that wait is hidden and there are no exchanges between CTAs.  The sums
+// and roundings are those of mlp_bf16_kernel.
+__global__ void __launch_bounds__(256) mlp_bf16_rows_kernel(MlpArgs a, int n, const float* __restrict__ x, int xcols,
+                                                            float* __restrict__ y, int act) {
+  __shared__ float buf[2][16][MAXW + 4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gq = lane >> 2, tq = lane & 3;
+  const int row0 = blockIdx.x * 16;
+  const int w0 = a.widths[0];
+  for (int i = threadIdx.x; i < 16 * w0; i += blockDim.x) {
+    const int r = i / w0, c = i % w0;
+    buf[0][r][c] = row0 + r < n && c < xcols ? x[(int64_t)(row0 + r) * xcols + c] : 0.0f;
+  }
+  __syncthreads();
+  for (int l = 0; l < a.layers; ++l) {
+    const int in = a.widths[l], out = a.widths[l + 1], cur = l & 1;
+    const bool last = l + 1 == a.layers;
+    for (int nt = warp; nt < out / 8; nt += 8) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint32_t* wr = a.w[l] + (int64_t)(8 * nt + gq) * in / 2;
+      for (int k0 = 0; k0 < in; k0 += 16) {
+        const float* A0 = &buf[cur][gq][k0 + 2 * tq];
+        const float* A1 = &buf[cur][gq + 8][k0 + 2 * tq];
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%0,%1,%2,%3};\n"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(pack2(A0[0], A0[1])), "r"(pack2(A1[0], A1[1])), "r"(pack2(A0[8], A0[9])), "r"(pack2(A1[8], A1[9])),
+              "r"(wr[k0 / 2 + tq]), "r"(wr[k0 / 2 + tq + 4]));
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int r = gq + (h >= 2 ? 8 : 0), c = 8 * nt + 2 * tq + (h & 1);
+        const float v = d[h] + a.b[l][c];
+        if (!last)
+          buf[cur ^ 1][r][c] = act_fwd(v, act);
+        else if (row0 + r < n)
+          y[(int64_t)(row0 + r) * out + c] = v;
+      }
+    }
+    __syncthreads();
+  }
+}
+
 int grid_for(int64_t n) {
   int64_t g = (n + 255) / 256;
   return (int)(g < 4096 ? (g < 1 ? 1 : g) : 4096);
@@ -670,7 +716,14 @@ int ws_mlp_forward_bf16_cols(int32_t n, int32_t layers, const int32_t* widths, c
   }
   if (x_cols <= 0 || x_cols > widths[0]) return bad("ws_mlp_forward_bf16: x has 1 to widths[0] columns");
   if (n == 0) return FE_NO_ERROR;
-  mlp_bf16_kernel<<<(n + 15) / 16 * ICLUSTER, 32 * IW, 0, (cudaStream_t)stream>>>(a, n, x, x_cols, y, act);
+  // A cluster per 16 rows or a CTA, us a call of the 4-256-256-256-64 network: 16
+  // rows 30 and 46, 256 rows 33 and 47, 1,024 rows 46 and 47, 2,048 rows 60 and
+  // 48, 16,384 rows 276 and 166, 131,072 rows 1,977 and 1,128; of 4-64-64-32:
+  // 1,024 rows 32 and 34, 2,048 rows 37 and 33, 131,072 rows 874 and 86.
+  if (n <= 1024)
+    mlp_bf16_kernel<<<(n + 15) / 16 * ICLUSTER, 32 * IW, 0, (cudaStream_t)stream>>>(a, n, x, x_cols, y, act);
+  else
+    mlp_bf16_rows_kernel<<<(n + 15) / 16, 256, 0, (cudaStream_t)stream>>>(a, n, x, x_cols, y, act);
   return cuda_status("ws_mlp_forward_bf16");
 }
 

@@ -226,3 +226,16 @@ def test_network_with_many_rows(torch, widths, rows):
             if l + 1 < net.layers:
                 h = torch.tanh(h)
             assert float((got - h).abs().max()) <= 2e-5 * float(h.abs().max())
+
+
+@pytest.mark.parametrize("widths", [(4, 256, 256, 64), (4, 24, 3), (9, 5)])
+def test_inference_with_many_rows(torch, widths):
+    """A row's BF16 prediction has the same bits whether it is asked for among
+    few rows (a cluster of blocks to 16 of them) or many (a block)."""
+    from cm_gb300 import warmstart as W
+    net = W.MLP(widths, seed=3, device="cuda")
+    x = torch.randn(2051, widths[0], generator=torch.Generator().manual_seed(2)).cuda()
+    y = net.infer_bf16(x)
+    parts = [net.infer_bf16(x[i:i + 1000]) for i in range(0, len(x), 1000)]
+    assert torch.equal(y, torch.cat(parts))
+    assert torch.equal(net.infer_bf16(x[:1024]), net.infer_bf16(x[:1025])[:1024])
