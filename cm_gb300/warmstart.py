@@ -169,6 +169,8 @@ class MLP:
             self._prepare_bf16()
         widths, _, _, W, Wp, Bp = self._bf16
         n, cols = x.shape
+        if cols == 0:  # nothing given: every input of the network is zero
+            x, cols = torch.zeros(n, 1, dtype=torch.float32, device=self.device), 1
         if x.dtype != torch.float32 or x.device != self.flat.device or not x.is_contiguous():
             xp = torch.empty(n, cols, dtype=torch.float32, device=self.device)
             xp.copy_(x)

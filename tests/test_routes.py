@@ -239,3 +239,17 @@ def test_inference_with_many_rows(torch, widths):
     parts = [net.infer_bf16(x[i:i + 1000]) for i in range(0, len(x), 1000)]
     assert torch.equal(y, torch.cat(parts))
     assert torch.equal(net.infer_bf16(x[:1024]), net.infer_bf16(x[:1025])[:1024])
+
+
+def test_inference_with_few_columns(torch):
+    """Inputs with fewer columns than the network has, down to none, and in
+    other types and layouts: the missing ones are zero."""
+    from cm_gb300 import warmstart as W
+    net = W.MLP((5, 32, 7), seed=3, device="cuda")
+    x = torch.randint(-2, 3, (19, 5), generator=torch.Generator().manual_seed(2)).float().cuda()
+    for cols in (0, 1, 3, 5):
+        full = torch.zeros_like(x)
+        full[:, :cols] = x[:, :cols]
+        ref = net.infer_bf16(full)
+        for given in (x[:, :cols], x[:, :cols].double(), x[:, :cols].int(), x[:, :cols].cpu(), x.T[:cols].T):
+            assert torch.equal(net.infer_bf16(given), ref)
