@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/cm_fe.h"
@@ -79,6 +80,14 @@ struct HostSetup {
   // and 0..q (pressure row nodes): once the elements below E are assembled,
   // every node a with u_last_prefix[a] < E has its rows complete
   std::vector<int32_t> u_last_prefix, p_last_prefix;
+
+  // Frees the arrays that only the device reads, once it has them: a clone
+  // copies what is left, a tenth.
+  void forget_uploaded() {
+    auto drop = [](auto&... v) { (std::decay_t<decltype(v)>().swap(v), ...); };
+    drop(elem_u, elem_p, wu, wp, colour_elems, tables, elem_table, geo, geo_rj, gbf_u, gbf_p, gw, bnd_mask, u_inc_ptr,
+         u_inc, p_inc_ptr, p_inc, u_inc_col, p_inc_col, u_inc_row, p_inc_row, u_pat, pat);
+  }
 };
 
 // Arguments of the element kernels (plain data; device pointers).

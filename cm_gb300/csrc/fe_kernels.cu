@@ -438,18 +438,9 @@ __global__ void __launch_bounds__(128) fe_element_kernel(KParams P) {
   }
 }
 
-// ------------------------------------------------------------ handle ----
-template <class T>
-int dev_upload(T** dst, const std::vector<T>& src) {
-  *dst = nullptr;
-  if (src.empty()) return FE_NO_ERROR;
-  CUDA_TRY(cudaMalloc(dst, src.size() * sizeof(T)));
-  CUDA_TRY(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return FE_NO_ERROR;
-}
-
 }  // namespace
 
+// ------------------------------------------------------------ handle ----
 namespace {
 // Host arrays to device memory in one allocation: small sets packed and copied
 // at once (an allocation and a copy take about 10 us each, and a mesh has
@@ -527,6 +518,7 @@ struct fe_equations_set {
   bool no_rec64 = false;
   int* d_fuse64 = nullptr;
   cudaEvent_t order_event = nullptr;
+  void* d_own = nullptr;  // the allocation that holds d_status, d_mat, d_done_r and d_rec_r
   // residual: its records and node counts (allocated at creation), and their order
   unsigned char* d_rec_r = nullptr;
   int* d_done_r = nullptr;
@@ -771,16 +763,25 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   return FE_NO_ERROR;
 }
 
-// The residual's records, node counts and event, at handle creation: residual
-// evaluations allocate nothing.
-int residual_buffers(fe_handle h) {
+// What a handle owns from its creation, in one allocation: status word,
+// materials, and the residual's node counts and records (residual evaluations
+// allocate nothing), with their event.  mat: the materials, host or device
+// memory.
+int own_buffers(fe_handle h, const double* mat) {
   const auto& s = h->hs;
-  const size_t counts = sizeof(int) * ((size_t)s.nu + (size_t)s.npn);
+  auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+  const size_t status = up(sizeof(unsigned)), counts = up(sizeof(int) * ((size_t)s.nu + (size_t)s.npn));
+  const size_t mat_bytes = sizeof(double) * s.mat.size();
+  char* p = nullptr;
   int rc;
-  if ((rc = ensure((void**)&h->d_rec_r, cmfe::record_bytes_residual(s) * (size_t)s.ne)) ||
-      (rc = ensure((void**)&h->d_done_r, counts)))
-    return rc;
-  CUDA_TRY(cudaMemset(h->d_done_r, 0, counts));
+  if ((rc = ensure((void**)&p, status + counts + up(mat_bytes) + cmfe::record_bytes_residual(s) * (size_t)s.ne))) return rc;
+  h->d_own = p;
+  h->d_status = reinterpret_cast<unsigned*>(p);
+  h->d_done_r = reinterpret_cast<int*>(p + status);
+  h->d_mat = reinterpret_cast<double*>(p + status + counts);
+  h->d_rec_r = reinterpret_cast<unsigned char*>(p + status + counts + up(mat_bytes));
+  CUDA_TRY(cudaMemset(p, 0, status + counts));
+  CUDA_TRY(cudaMemcpy(h->d_mat, mat, mat_bytes, cudaMemcpyDefault));
   CUDA_TRY(cudaEventCreateWithFlags(&h->residual_event, cudaEventDisableTiming));
   return FE_NO_ERROR;
 }
@@ -1394,16 +1395,14 @@ int fe_create(const fe_mesh_desc* desc, fe_handle* out) {
   up.add(&h->d_p_inc_row, s.p_inc_row);
   up.add(&h->d_u_pat, s.u_pat);
   up.add(&h->d_pat, s.pat);
-  if ((rc = up.run(&h->d_mesh)) || (rc = dev_upload(&h->d_mat, s.mat))) return fail(rc);
+  if ((rc = up.run(&h->d_mesh))) return fail(rc);
   {
     auto owner = std::make_shared<SharedDeviceSetup>();
     owner->ptrs = {h->d_mesh};
     h->shared = owner;
   }
-  if (cudaMalloc(&h->d_status, sizeof(unsigned)) != cudaSuccess ||
-      cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess)
-    return fail(set_error(FE_ERR_CUDA, "status allocation failed"));
-  if ((rc = residual_buffers(h))) return fail(rc);
+  if ((rc = own_buffers(h, s.mat.data()))) return fail(rc);
+  h->hs.forget_uploaded();
   {
     // Resolving the address of the allocation-free entry point's array loads
     // the module that holds it, which commits its 16 MiB on this device now,
@@ -1420,9 +1419,8 @@ int fe_destroy(fe_handle h) {
   if (!h) return FE_NO_ERROR;
   if (!h->shared && h->d_mesh) cudaFree(h->d_mesh);  // a handle whose creation failed part-way owns what it uploaded
   // per-handle state: materials, surface load, status word, staging and records
-  void* own[] = {h->d_surfp, h->d_mat, h->d_status, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
-                 h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64, h->d_rec_r,
-                 h->d_done_r};
+  void* own[] = {h->d_surfp, h->d_own, h->s_x, h->s_r, h->s_vals, h->s_cp, h->s_uu, h->s_elem,
+                 h->d_col, h->d_rec, h->d_fuse, h->d_rec64, h->d_fuse64};
   for (void* p : own)
     if (p) cudaFree(p);
   for (cudaEvent_t ev : h->chunk_events)
@@ -1486,13 +1484,7 @@ int fe_clone(fe_handle src, fe_handle* out) {
     fe_destroy(h);
     return code;
   };
-  const size_t mat_bytes = sizeof(double) * h->hs.mat.size();
-  if (cudaMalloc(&h->d_mat, mat_bytes) != cudaSuccess ||
-      cudaMemcpy(h->d_mat, src->d_mat, mat_bytes, cudaMemcpyDeviceToDevice) != cudaSuccess ||
-      cudaMalloc(&h->d_status, sizeof(unsigned)) != cudaSuccess ||
-      cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess)
-    return fail(set_error(FE_ERR_CUDA, "clone: device allocation failed"));
-  if ((rc = residual_buffers(h))) return fail(rc);
+  if ((rc = own_buffers(h, src->d_mat))) return fail(rc);
   if (src->has_surfp) {
     const size_t bytes = sizeof(double) * 3 * (size_t)h->hs.nu;
     if (cudaMalloc(&h->d_surfp, bytes) != cudaSuccess ||

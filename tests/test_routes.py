@@ -253,3 +253,29 @@ def test_inference_with_few_columns(torch):
         ref = net.infer_bf16(full)
         for given in (x[:, :cols], x[:, :cols].double(), x[:, :cols].int(), x[:, :cols].cpu(), x.T[:cols].T):
             assert torch.equal(net.infer_bf16(given), ref)
+
+
+def test_clones_of_clones(torch):
+    """A clone, a clone of it whose source is gone, and both with materials and
+    loads of their own: the bits of sets created from the mesh."""
+    m, es, x, xd, sp = box(torch, (4, 3, 5), load=True)
+    first = es.clone()
+    es.close()
+    second = first.clone(materials=(1.0, 3.0))
+    second.set_surface_pressure(None)
+    third = second.clone()
+    first.close()
+    for got, mats, load in ((second, (1.0, 3.0), None), (third, (1.0, 3.0), None), (third.clone((2.0, 6.0)), (2.0, 6.0), sp)):
+        ref = FiniteElasticityEquationsSet(m)
+        ref.set_materials(mats)
+        for e in (got, ref):
+            e.set_surface_pressure(load)
+        a, b = torch.empty_like(xd), torch.empty_like(xd)
+        assert torch.equal(got.residual_evaluate(xd), ref.residual_evaluate(xd))
+        assert torch.equal(got.jacobian_evaluate(xd, r=a), ref.jacobian_evaluate(xd, r=b)) and torch.equal(a, b)
+        for s, t in zip(got.jacobian_evaluate_mixed(xd, r=a), ref.jacobian_evaluate_mixed(xd, r=b)):
+            assert torch.equal(s, t)
+        assert torch.equal(a, b)
+        assert all(np.array_equal(s, t) for s, t in zip(got.csr_pattern(), ref.csr_pattern()))
+        ra = got.element_residuals(xd)
+        assert torch.equal(ra, ref.element_residuals(xd))
