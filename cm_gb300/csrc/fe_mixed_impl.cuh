@@ -273,6 +273,15 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
   T* s_D = reinterpret_cast<T*>(sm + C::O_R32);                // [el][g][UU_REC]
   T* s_mm = reinterpret_cast<T*>(sm + C::O_MM);
   int* s_node = reinterpret_cast<int*>(sm + (OUT == 2 ? C::O_NODE2 : OUT == 1 ? C::O_NODE1 : C::O_NODE0));  // [el][NR+1]
+  // Every scratch array ends inside its region (a region begins where the one
+  // before it ends, and what shares one is separated by barriers: the stages
+  // below; run thread by thread on the CPU, none leaves its array or races).
+  static_assert(sizeof(H) == 8 && EG * 3 * NPE * 8 <= C::O_P - C::O_Z && EG * 8 * 8 <= C::O_PG - C::O_P &&
+                    EG * NG * 8 <= C::O_R64 - C::O_PG && EG * NG * C::REC64 * 8 <= C::O_R32 - C::O_R64 &&
+                    EG * NG * 9 * 8 <= C::O_BASE - C::O_DZ,
+                "positions, pressures, Gauss-point records, gradients");
+  static_assert(OUT != 0 || (EG * 9 * NPE * 4 <= C::O_TAB - C::O_BASE && EG * NPE * NPE * 2 <= C::O_NODE0 - C::O_TAB),
+                "scatter addresses and rank tables");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // FP64 items are dealt to the warps from a different first warp in each
   // CTA of an SM: an SM sub-partition takes 64 cycles per FP64 warp
@@ -321,6 +330,7 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
     H* S1 = reinterpret_cast<H*>(sm + C::O_R32);  // [B|D][ec][g1][a2a3]
     H* S2 = S1 + EG * 3 * 2 * 3 * N2;             // [BB|BD|DB][ec][g1][g2][a3]
     constexpr int S1T = EG * 3 * 3 * N2, S2T = EG * 3 * 9 * N1;
+    static_assert((2 * S1T + 3 * S2T) * 8 <= C::O_DZ - C::O_R32, "scratch of the gradients");
     for (int i = vt; i < EG * 3 * N2; i += C::THREADS) {
       const int j = i % N2, ec = i / N2;
       H z[N1], B[3], D[3];
@@ -490,6 +500,9 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
       H* U1 = reinterpret_cast<H*>(sm + C::O_U1);  // [el][m][k][a1][g2 + 3 g3]
       H* U2 = reinterpret_cast<H*>(sm + C::O_U2);  // [W|U][el][m][a1 + N1 a2][g3]
       H* Lq = reinterpret_cast<H*>(sm + C::O_U3);  // residual pressure rows: [el][q1][j], then [el][q1 q2][g3]
+      static_assert(EG * 9 * N1 * 9 * 8 <= C::O_U2 - C::O_U1 && 2 * EG * 3 * N2 * 3 * 8 <= C::O_U3 - C::O_U2 &&
+                        (EG * 2 * 9 + EG * 4 * 3) * 8 <= C::O_BASE - C::O_U3,
+                    "scratch of the residual");
       auto sumfact = [&](int roff, bool prows, auto emit, auto emit_p) {
         for (int i = vt; i < EG * 81; i += C::THREADS) {
           const int j = i % 9, k = (i / 9) % 3, m = (i / 27) % 3, el = i / 81;
@@ -644,6 +657,8 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
         H* T1 = reinterpret_cast<H*>(sm + C::O_DZ);  // [n][el][k][q1 b1][g2 + 3 g3]
         H* W2 = T1 + EG * 9 * L2 * 9;                // [n][el][q1 b1][q2 b2][g3]
         H* V2 = W2 + EG * 3 * L2 * L2 * 3;           // the k = 2 terms
+        static_assert(!PM || (EG * 9 * L2 * 9 + 2 * EG * 3 * L2 * L2 * 3) * 8 <= C::O_BASE - C::O_DZ,
+                      "scratch of the coupling");
         for (int i = vt; i < EG * 81; i += C::THREADS) {
           const int j = i % 9, k = (i / 9) % 3, el = (i / 27) % EG, n = i / (27 * EG);
           const H* a = &s_r64[(el * NG + 3 * j) * C::REC64 + 9 + 3 * k + n];
@@ -705,6 +720,9 @@ __device__ __forceinline__ void mix_group(const KParams& P, const int32_t* elems
         int* s_base = reinterpret_cast<int*>(sm + C::O_BASE);
         uint16_t* s_tab = reinterpret_cast<uint16_t*>(sm + C::O_TAB);
         T* s1 = reinterpret_cast<T*>(sm + C::O_DZ) + (size_t)warp * UUCfg<N1>::S1;
+        static_assert(C::THREADS / 32 * UUCfg<N1>::S1 * (int)sizeof(T) <= C::O_BASE - C::O_DZ &&
+                          EG * NG * UU_REC * (int)sizeof(T) <= C::O_DZ - C::O_R32,
+                      "scratch of the displacement block");
         if constexpr (OUT == 0) {
           for (int i = tid; i < EG * 9 * NPE; i += C::THREADS) {
             const int a = i % NPE, mn = (i / NPE) % 9, el = i / (9 * NPE);

@@ -268,6 +268,7 @@ struct UUCfg {
   static constexpr int NP = N1 * N1;
   static constexpr int JP = N1;                                 // (a2, b2) pairs per lane
   static constexpr int S1 = N1 == 3 ? 2 * 6 * 81 : 4 * 9 * 36;  // stage-1 values of one warp task
+  static_assert(S1 >= (N1 == 3 ? 9 : 4 * 9) * NP * 9 && S1 >= (N1 == 3 ? 2 * 6 * NP * 9 : 0), "units of a warp task");
   static constexpr int MM = 4 * NP * 4;                         // table [t][a b][g], g padded to 4
   __host__ __device__ static constexpr int tasks(int nvalid) {
     return N1 == 3 ? 3 * nvalid + (3 * nvalid + 1) / 2 : (6 * nvalid + 3) / 4;
@@ -297,11 +298,9 @@ __device__ __forceinline__ void uu_load3(const T* p, T (&v)[3]) {
 }
 
 // One warp task: stages 1 to 3 of its units.  s_D: [el][g][UU_REC]; s1: this
-// warp's scratch (UUCfg::S1 values).  emit(el, m, n, a12, b12, base, mirrored)
-// is not used directly: out(el, blk, a12, b12, diag, K) receives, for one pair
-// of partial node indices a12 = a1 + N1 a2 and b12, the N1 x N1 values
-// K[a3][b3]; diag says that they lie on the a12 = b12 diagonal of a diagonal
-// block (then only a3 <= b3 count).
+// warp's scratch (UUCfg::S1 values).  out(el, blk, a12, b12, K) receives, for
+// one pair of partial node indices a12 = a1 + N1 a2 and b12, the N1 x N1 values
+// K[a3][b3].
 template <int N1, class T, class Out>
 __device__ __forceinline__ void uu_warp_task(const T* s_D, const T* s_mm, T* s1, int task, int nvalid, int lane, Out out) {
   using C = UUCfg<N1>;
