@@ -78,7 +78,7 @@ __device__ __forceinline__ int inv_at(uint32_t w, int j) { return (w >> (8 * j))
 
 // The three displacement rows of a u node, by one warp.  list: its first
 // GLIST incidences (element and local node, rank-table row).
-template <int NPE, int NPP, class T>
+template <int NPE, int NPP, class T, bool ROWS>
 __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe::StageOut& S, const cmfe::FusedArgs& F,
                                              const ReadyNode& rn, const int2* list, unsigned char* mine, int lane) {
   using R = cmfe::Rec<NPE, NPP, T>;
@@ -193,20 +193,19 @@ __device__ __forceinline__ void gather_unode(const cmfe::KParams& P, const cmfe:
         __syncwarp();
       }
     }
-    // row after row, so that the sectors a store begins or ends in are completed
-    // by the next one: over the host link (outputs in page-locked memory) every
-    // part of a sector is a write of its own (32^3 box 7.10 ms with the columns
-    // as the outer loop, 6.00 so; device outputs 1.81 and 1.80)
+    // Row after row (ROWS), so that the sectors a store begins or ends in are
+    // completed by the next one: over the host link (outputs in page-locked
+    // memory) every part of a sector is a write of its own (32^3 box 7.10 ms with
+    // the columns as the outer loop, 6.00 so; device outputs 1.80 and 1.78).  On
+    // meshes that are resident at once the columns go first (9x7x8 69.2 us, rows
+    // first 69.7).
+    constexpr int NC = GPOS / 32;
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
-#pragma unroll
-      for (int n = 0; n < 3; ++n)
-#pragma unroll
-        for (int i = 0; i < GPOS / 32; ++i) {
-          const int pos = p0 + 32 * i + lane;
-          if (pos < wu)
-            du[m][n * wu + pos] = FULL ? (T)uacc[(3 * m + n) * GPOS + 32 * i + lane] : acc[FULL ? 0 : i][3 * m + n];
-        }
+    for (int k = 0; k < 9 * NC; ++k) {
+      const int mn = ROWS ? k / NC : k % 9, i = ROWS ? k % NC : k / 9;
+      const int pos = p0 + 32 * i + lane;
+      if (pos < wu) du[mn / 3][mn % 3 * wu + pos] = FULL ? (T)uacc[mn * GPOS + 32 * i + lane] : acc[FULL ? 0 : i][mn];
+    }
     if (q0 + lane < wc) {
 #pragma unroll
       for (int m = 0; m < 3; ++m) dc[m][q0 + lane] = cacc[m * GPP + lane];
@@ -334,7 +333,7 @@ struct GroupGather {
       if (j >= nready) break;
       const ReadyNode rn = ready[j];
       if (rn.id < P.nu)
-        gather_unode<NPE, NPP, T>(P, S, F, rn, list + j * GLIST, mine, lane);
+        gather_unode<NPE, NPP, T, (EG > 2)>(P, S, F, rn, list + j * GLIST, mine, lane);
       else
         gather_pnode<NPE, NPP, T>(P, S, F, rn, list + j * GLIST, mine, lane);
     }
