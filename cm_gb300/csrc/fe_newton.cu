@@ -323,7 +323,7 @@ struct CycleArgs {
   double* scale;  // 1 / norm of the newest basis vector, -1: converged
   int* ctl;       // barrier arrivals; zeroed before the launch
   unsigned polls;  // of a barrier, before it gives up
-  int extra_from;  // > 0: barriers from this one on wait for one arrival more than there are
+  int extra_from;  // barriers from this one on wait for one arrival more than there are
   double* host;  // page-locked: squared norm of the true residual, iterations, converged
 };
 
@@ -365,14 +365,14 @@ __device__ __forceinline__ bool cycle_barrier(const CycleArgs& A, int k) {
   __shared__ bool ok;
   __syncthreads();
   if (threadIdx.x == 0) {
+    const int target = k * (int)gridDim.x + (k >= A.extra_from);
+    unsigned polls = A.polls;
+    int v;
     __threadfence();
     atomicAdd(A.ctl, 1);
-    const int target = k * (int)gridDim.x + (A.extra_from > 0 && k >= A.extra_from);
-    unsigned polls = 0;
-    int v;
     do {
       asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(A.ctl) : "memory");
-    } while (v < target && ++polls < A.polls);
+    } while (v < target && --polls);
     ok = v >= target;
     __threadfence();
   }
@@ -964,6 +964,7 @@ struct Solver {
     unsigned polls = 0;
     cmfe::newton_barrier_limits(h, &polls, &a.extra_from);
     a.polls = polls ? polls : CYCLE_POLLS;
+    if (!a.extra_from) a.extra_from = INT32_MAX;
     a.bound = bound;
     a.host = pinned;
     k_cycle_bounds<<<1, MAX_SHARES + 32, 0, st>>>((int)n, nb, rp, bound);
