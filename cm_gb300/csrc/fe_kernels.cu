@@ -731,7 +731,7 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   // colour-ordered assembly has (callers count them; a box has 8), side by side on streams
   // of the handle -- one after the other they would take one element's 50 us
   // each.
-  const int n = small ? std::min(std::min(s.ncolours, groups), 8) : 1;
+  const int n = small ? std::min(std::min(s.ncolours, groups), cmfe::Fork::MOST) : 1;
   std::vector<cudaStream_t>& side = h->side_streams;
   std::vector<cudaEvent_t>& ev = h->side_events;
   while ((int)side.size() < n - 1) {
@@ -1231,7 +1231,7 @@ int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t s
 // Deals the members to at most kLanes streams, the largest first, each to the
 // stream with the fewest elements so far; one handle stays on one stream (its
 // records and counters serve one launch at a time).
-constexpr int kLanes = 8;
+constexpr int kLanes = cmfe::Fork::MOST;
 int batch_lanes(fe_batch b) {
   const size_t n = b->members.size();
   std::vector<int> order(n);

@@ -6,9 +6,6 @@
 
 #include <cuda_runtime.h>
 
-#include <utility>
-#include <vector>
-
 namespace cmfe {
 
 // Uses of one set of buffers, on whatever streams, in call order: begin()
@@ -38,29 +35,38 @@ class HandleOrder {
   cudaEvent_t ev_ = nullptr;
 };
 
-// Streams forked from st; st follows the work queued on them when the scope
-// ends.
+// Streams forked from st, at most MOST; st follows the work queued on them when
+// the scope ends.  No allocation, so nothing here throws.
 class Fork {
  public:
+  static constexpr int MOST = 8;
   explicit Fork(cudaStream_t st) : st_(st) {}
   Fork(const Fork&) = delete;
   // side continues from the event `from` of st; `done` will mark its end.
   cudaError_t add(cudaStream_t side, cudaEvent_t from, cudaEvent_t done) {
+    if (n_ == MOST) return cudaErrorInvalidValue;
     const cudaError_t e = cudaStreamWaitEvent(side, from, 0);
-    if (e == cudaSuccess) sides_.push_back({side, done});
+    if (e == cudaSuccess) sides_[n_++] = {side, done};
     return e;
   }
   ~Fork() {
-    for (const auto& s : sides_)
-      if (cudaEventRecord(s.second, s.first) != cudaSuccess || cudaStreamWaitEvent(st_, s.second, 0) != cudaSuccess) {
+    for (int i = 0; i < n_; ++i) {
+      const Side& s = sides_[i];
+      if (cudaEventRecord(s.done, s.stream) != cudaSuccess || cudaStreamWaitEvent(st_, s.done, 0) != cudaSuccess) {
         cudaGetLastError();
-        cudaStreamSynchronize(s.first);
+        cudaStreamSynchronize(s.stream);
       }
+    }
   }
 
  private:
+  struct Side {
+    cudaStream_t stream;
+    cudaEvent_t done;
+  };
   cudaStream_t st_;
-  std::vector<std::pair<cudaStream_t, cudaEvent_t>> sides_;
+  int n_ = 0;
+  Side sides_[MOST];
 };
 
 }  // namespace cmfe

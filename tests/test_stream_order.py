@@ -15,7 +15,7 @@ CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "cm_gb300"
 FAKE = r"""
 #pragma once
 #include <set>
-enum cudaError_t { cudaSuccess, cudaErrorUnknown };
+enum cudaError_t { cudaSuccess, cudaErrorInvalidValue, cudaErrorUnknown };
 enum { cudaEventDisableTiming = 2 };
 typedef std::set<int> Work;
 struct Stream { Work seen; };  // the work that a stream's next item comes after, its own included
