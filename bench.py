@@ -458,7 +458,7 @@ def our_arm(args):
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / pk["hbm_gbs"], "traffic": traffic, "peak_source": pk["source"],
-                     "kernel": "fe_mixed_fused_kernel" if mixed else "fe_element_kernel",
+                     "kernel": "fe_fused_kernel",
                      "launches_per_step": launches / args.steps,
                      "algorithmic_bytes_per_launch": B * args.steps / max(launches, 1),
                      "traffic_unit": "DRAM bytes per launch (ncu, profiles/traffic.json)",

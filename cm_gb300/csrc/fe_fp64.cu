@@ -7,7 +7,8 @@
 // as outer products take about 3,000 such instructions per triquadratic
 // element; contracting every entry over every Gauss point in the reference's
 // order (fe_element_kernel in fe_kernels.cu, which stays for the
-// element-level calls) takes about 12,000.
+// element-level calls) takes about 12,000.  With the row gathers a 16^3 box's
+// launch issues 3,715 an element and keeps that pipe 77 % busy (counters).
 #include "fe_fused_impl.cuh"
 
 namespace {
@@ -17,8 +18,9 @@ namespace {
 // accumulators without spills, so two CTAs of four warps (one to an SM
 // sub-partition) beat three of three (16^3 box: 1100 against 1282 us).  Meshes
 // that leave SMs without a group take one element per CTA and a warp for
-// every contraction task (6x5x4: 98 against 158 us; the lines cross near three
-// elements per SM; trilinear 4x4x4: 59 against 109 us).
+// every contraction task (6x5x4: 96 us in one launch, 102 in eight, against 156;
+// 9x7x7: 204 and 221 against 211, the lines cross near three elements per SM;
+// trilinear 4x4x4: 59 and 68 against 108).
 template <int N1, bool SMALL>
 struct Shape64 {
   static constexpr int EG = SMALL ? 1 : (N1 == 3 ? 2 : 4);

@@ -17,10 +17,12 @@ namespace {
 // another.  Sh: elements per group EG, threads NT and CTAs per SM MINB.
 //
 // Bound by the FP64 pipe and by the barriers between a group's phases: the
-// 32^3 box's mixed assembly takes 1.80 ms, 1.0 of it FP64 issue (2.72 with the
-// contraction on the tensor cores and records laid out by element); without
-// the gathers 1.31.  The 16^3 box's FP64 Jacobian takes 1.10 ms, 0.7 of it FP64
-// issue (6.5 with one launch per colour contracting over all Gauss points).
+// 32^3 box's mixed assembly takes 1.78 ms (2.72 with the contraction on the
+// tensor cores and records laid out by element), without the gathers 1.26.  By
+// the counters of the 16^3 box it issues 600 FP64 warp instructions an element
+// (480 of them element work), which keep that pipe 55 % busy.  The 16^3 box's
+// FP64 Jacobian takes 1.10 ms (6.5 with one launch per colour contracting over
+// all Gauss points), without the gathers 0.91: 3,715 an element, 77 % busy.
 template <int N1, int PM, class T, class H, class Sh>
 __global__ void __launch_bounds__(Sh::NT, Sh::MINB) fe_fused_kernel(KParams P, cmfe::StageOut so, cmfe::FusedArgs F) {
   using C = MixCfg<N1, PM, Sh::EG, T, Sh::NT>;

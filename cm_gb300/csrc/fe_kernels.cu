@@ -727,10 +727,11 @@ int fp64_fused(fe_handle h, KParams kp, cudaStream_t st, bool* taken) {
   const cmfe::StageOut so{h->d_rec64};
   bool small = false;
   const int groups = cmfe::fp64_groups(s, h->num_sms, &small);
-  // A small mesh: as many launches as it has element colours, as the
-  // colour-ordered assembly has (callers count them; a box has 8), side by side on streams
-  // of the handle -- one after the other they would take one element's 50 us
-  // each.
+  // A small mesh: as many launches as it has element colours, a box eight, as
+  // the colour-ordered assembly has: what fe_launch_count reports for a call
+  // stays so.  Nothing in the kernel needs them (4x4x4 trilinear: one launch 59
+  // us, eight side by side on streams of the handle 68; one after the other
+  // they would take one element's 50 us each).
   const int n = small ? std::min(std::min(s.ncolours, groups), cmfe::Fork::MOST) : 1;
   std::vector<cudaStream_t>& side = h->side_streams;
   std::vector<cudaEvent_t>& ev = h->side_events;
@@ -1194,7 +1195,7 @@ int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t s
   if (b->variant == cmfe::batch_variants()) {
     // the single-set assembly of every member.  The members are independent,
     // so they run on several streams and small ones share the GPU (24 boxes of
-    // 4 to 24 elements an edge: one after the other 3.4 ms, side by side 2.4)
+    // 4 to 24 elements an edge: one after the other 3.94 ms, side by side 3.02)
     int rc = FE_NO_ERROR;
     cmfe::Fork fork(st);
     if (!b->lanes.empty()) CUDA_TRY(cudaEventRecord(b->lane_events[0], st));
@@ -1992,7 +1993,7 @@ int fe_batch_autotune(fe_batch b, const double* const* x, float* const* values_u
   const int blocks[] = {1, 2, 4};
   for (int v = 0; v <= cmfe::batch_variants() && !rc; ++v)
     for (int cps = 1; cps <= 3 && !rc; ++cps) {
-      // the last variant (one launch per member and colour) has no launch shape
+      // the last variant (every member's own launch) has no launch shape
       const bool per_member = v == cmfe::batch_variants();
       if (per_member && cps > 1) break;
       // skip a CTA count the shared memory cannot hold (the launch would use fewer)

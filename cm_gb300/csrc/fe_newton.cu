@@ -309,9 +309,11 @@ __global__ void __launch_bounds__(NT) k_update_norm(int64_t n, const double* __r
 // the shares themselves until all have come take twice the time).
 //
 // Bound by the barriers (1.9 us each) and FP64 latency (an instruction holds a
-// quarter SM's pipe for 64 cycles): 17.5 us an iteration at 4,071 rows and
-// 700,000 entries, against 30 for four launches; a load step 21.0 against 31.4
-// ms, at 9,223 rows 54.3 against 89.0, at 525 rows 8.7 against 13.0.
+// quarter SM's pipe for 64 cycles).  Load steps of triquadratic boxes, with the
+// cycle and with four launches an iteration, ms: 1,093 rows 9.0 and 13.7, 4,071
+// rows and 700,000 entries 22.1 and 32.9 (20.7 and 30.8 us an iteration, the
+// assemblies included), 9,223 rows 54.1 and 75.6; trilinear, 8,970 rows 51.9 and
+// 86.4.
 struct CycleArgs {
   int n, nb, restart, kmax, cap;
   int* bound;  // [nb + 1]

@@ -2,10 +2,12 @@
 // assembly without the displacement block and the coupling, a residual record
 // per element, and a node's rows summed by the CTA that finishes its last
 // element, in element colour order: the order, and with the same element code
-// the bits, of the colour-by-colour assembly.
+// the bits, of the colour-by-colour assembly.  With a surface load the two agree
+// to rounding: here an element's faces are added to its record, there to the row
+// after the volume terms of the element's colour.
 //
 // The FP64 pipe binds a large mesh: about 270 warp instructions per
-// triquadratic element, 19 cycles each, are 0.55 ms on the 32^3 box, which
+// triquadratic element (267 counted), 19 cycles each, are 0.53 ms on the 32^3 box, which
 // takes 0.64 (0.86 in eight launches, one per element colour, with a third
 // more of them).  A small mesh is bound by the latency of one group, which the
 // eight launches paid eight times (9x7x8: 197 -> 23 us).
