@@ -151,13 +151,14 @@ class ClockSampler:
         return {"sm_mhz": sm[len(sm) // 2], "sm_max_mhz": max(mx), "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def cpu_baseline(m, x, rp1, col1, budget_s=12.0):
+def cpu_baseline(m, x, rp1, col1, load=None, budget_s=12.0):
     """The FP64 CPU oracle (restatement of the reference's assembly loop with
     its bisection CSR add) timed with all host threads on whole assemblies of
-    the same mesh, repeated until about budget_s of CPU work."""
+    the same mesh and surface load, repeated until about budget_s of CPU work."""
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import oracle
     P = oracle.Problem(m)
+    P.set_surface_pressure(load)
     nt = os.cpu_count() or 1
     import numpy as np
     vals = np.zeros(int(rp1[-1]) - 1)
@@ -299,9 +300,11 @@ def our_arm(args):
     m, x, workload = config_mesh(args.config)
     mixed = args.config != "cfg1" and not args.fp64
     es = FiniteElasticityEquationsSet(m)
+    load = None
     if args.config == "cfg5":
         from cm_gb300.newton import bottom_face_pressure
-        es.set_surface_pressure(bottom_face_pressure(m, 2.0))
+        load = bottom_face_pressure(m, 2.0)
+        es.set_surface_pressure(load)
     dev = torch.device("cuda", local)
     xd = torch.from_numpy(x).to(dev)
     r = torch.empty(es.ndofs, dtype=torch.float64, device=dev)
@@ -479,7 +482,7 @@ def our_arm(args):
         torch.cuda.empty_cache()
     if world == 1 and not args.no_cpu:
         rp1, col1 = es.csr_pattern(base=1)
-        out["cpu_baseline"], vals_or, r_or = cpu_baseline(m, x, rp1, col1)
+        out["cpu_baseline"], vals_or, r_or = cpu_baseline(m, x, rp1, col1, load)
         out["error_vs_oracle"] = error_vs_oracle(es, mixed, vuh if mixed else vh, vch if mixed else None, rh,
                                                  vals_or, r_or)
     if world == 1 and args.loadstep:
