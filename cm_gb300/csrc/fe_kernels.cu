@@ -1231,17 +1231,19 @@ int batch_launch_from(fe_batch b, const cmfe::BatchMember* table, cudaStream_t s
 
 // Deals the members to at most kLanes streams, the largest first, each to the
 // stream with the fewest elements so far; one handle stays on one stream (its
-// records and counters serve one launch at a time).
+// records and counters serve one launch at a time).  Called when the variant
+// that uses them is first chosen or tried.
 constexpr int kLanes = cmfe::Fork::MOST;
 int batch_lanes(fe_batch b) {
   const size_t n = b->members.size();
+  if (!b->slot_lane.empty()) return FE_NO_ERROR;
   std::vector<int> order(n);
   for (size_t i = 0; i < n; ++i) order[i] = (int)i;
   auto ne = [&](int slot) { return b->members[b->slot_member[slot]]->hs.ne; };
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return ne(x) > ne(y); });
   std::vector<int64_t> load(kLanes, 0);
   std::unordered_map<fe_handle, int> lane_of;
-  b->slot_lane.assign(n, 0);
+  std::vector<int> slot_lane(n, 0);
   int used = 0;
   for (int slot : order) {
     fe_handle h = b->members[b->slot_member[slot]];
@@ -1249,19 +1251,20 @@ int batch_lanes(fe_batch b) {
     const int l = it != lane_of.end() ? it->second : (int)(std::min_element(load.begin(), load.end()) - load.begin());
     lane_of[h] = l;
     load[l] += ne(slot);
-    b->slot_lane[slot] = l;
+    slot_lane[slot] = l;
     used = std::max(used, l);
   }
-  for (int l = 0; l < used; ++l) {
+  while ((int)b->lanes.size() < used) {
     cudaStream_t s;
     CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     b->lanes.push_back(s);
   }
-  for (int l = 0; l <= used; ++l) {
+  while ((int)b->lane_events.size() <= used) {
     cudaEvent_t e;
     CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     b->lane_events.push_back(e);
   }
+  b->slot_lane = slot_lane;
   return FE_NO_ERROR;
 }
 
@@ -1885,7 +1888,6 @@ int fe_batch_create(const fe_handle* handles, int32_t count, fe_batch* out) {
         o[b->ncol + 1 + c] = hs.bnd_ptr[std::min(c, hs.ncolours)];
       }
     }
-    if (!rc) rc = batch_lanes(b);
     b->surf_sig.assign((size_t)count, nullptr);
     if (!rc) rc = fail(cudaMalloc(&b->d_offsets, offsets.size() * sizeof(int32_t)));
     if (!rc) rc = fail(cudaMemcpy(b->d_offsets, offsets.data(), offsets.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -1957,6 +1959,7 @@ int fe_batch_set_config(fe_batch b, int32_t variant, int32_t ctas_per_sm, int32_
   if (variant < 0 || variant > cmfe::batch_variants() || ctas_per_sm < 1 || ctas_per_sm > 4 || block_groups < 1)
     return set_error(FE_ERR_INVALID_ARGUMENT, "invalid batch configuration");
   std::lock_guard<std::mutex> lk(b->mu);
+  if (variant == cmfe::batch_variants() && (rc = batch_lanes(b))) return rc;
   b->variant = variant;
   b->ctas_per_sm = ctas_per_sm;
   b->block_groups = block_groups;
@@ -1980,7 +1983,7 @@ int fe_batch_autotune(fe_batch b, const double* const* x, float* const* values_u
   if (!x || !values_uu || !values_coupling || repeats < 1) return set_error(FE_ERR_INVALID_ARGUMENT, "bad arguments");
   std::lock_guard<std::mutex> lk(b->mu);
   cudaStream_t st = (cudaStream_t)stream;
-  if ((rc = batch_set_pointers(b, x, values_uu, values_coupling, r, st))) return rc;
+  if ((rc = batch_set_pointers(b, x, values_uu, values_coupling, r, st)) || (rc = batch_lanes(b))) return rc;
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
   CUDA_TRY(cudaEventCreate(&e1));
