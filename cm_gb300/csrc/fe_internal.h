@@ -224,7 +224,9 @@ int launch_surface(const HostSetup& s, const KParams& kp, const int32_t* belems,
                    int mode, int want_jac, int num_sms, void* stream);
 
 // Builds the set-up; returns FE_NO_ERROR or a FE_ERR_* code with msg filled.
-int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg);
+// Without `assembly`: the pattern and what decides whether a mesh is accepted,
+// not the arrays that only the staged assembly and the residual read.
+int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg, bool assembly = true);
 
 // Batched mixed assembly (fe_batch.cu).  The members' parameters live in a
 // constant-memory table of the batch module, one entry per member slot

@@ -1505,7 +1505,7 @@ int fe_structure_calculate(const fe_mesh_desc* desc, int32_t base, int64_t* num_
   if (base != 0 && base != 1) return set_error(FE_ERR_INVALID_ARGUMENT, "base must be 0 or 1");
   HostSetup s;
   std::string msg;
-  int rc = cmfe::build_setup(desc, s, msg);
+  int rc = cmfe::build_setup(desc, s, msg, false);
   if (rc) return set_error(rc, msg);
   if (num_dofs) *num_dofs = s.ndofs;
   if (nnz) *nnz = s.nnz;

@@ -177,9 +177,90 @@ void parallel_for(int n, F f) {
   for (auto& x : th) x.join();
 }
 
+// The incidences of every node: rank-table rows in element order, the
+// incidences again in colour order; and the column patterns of the u nodes' rows.
+int incidence_patterns(HostSetup& s, const std::vector<int32_t>& colour, std::string& msg) {
+  const int nr = s.nr;
+  if ((int64_t)s.ntables * nr >= (1ll << 31)) return fail(msg, "too many distinct rank tables");
+  s.u_inc_row.resize(s.u_inc.size());
+  s.p_inc_row.resize(s.p_inc.size());
+  s.u_inc_col = s.u_inc;
+  s.p_inc_col = s.p_inc;
+  std::vector<uint64_t> row_hash(s.nu);
+  parallel_for(s.nu + s.npn, [&](int i) {
+    const bool un = i < s.nu;
+    const int n = un ? i : i - s.nu, bits = un ? 5 : 3, off = un ? 0 : s.npe;
+    const auto& ptr = un ? s.u_inc_ptr : s.p_inc_ptr;
+    const auto& inc = un ? s.u_inc : s.p_inc;
+    auto& row = un ? s.u_inc_row : s.p_inc_row;
+    auto& col = un ? s.u_inc_col : s.p_inc_col;
+    uint64_t hash = 1469598103934665603ull;
+    for (int32_t k = ptr[n]; k < ptr[n + 1]; ++k) {
+      row[k] = s.elem_table[inc[k] >> bits] * nr + off + (inc[k] & ((1 << bits) - 1));
+      hash = (hash ^ (uint64_t)(uint32_t)row[k]) * 1099511628211ull;
+    }
+    if (un) row_hash[n] = hash;
+    std::sort(col.begin() + ptr[n], col.begin() + ptr[n + 1],
+              [&](int32_t x, int32_t y) { return colour[x >> bits] < colour[y >> bits]; });
+  });
+
+  // Column patterns of the u nodes' rows, shared by nodes with equal
+  // rank-table rows (a node's incidences in element order).
+  {
+    struct Seen {
+      int32_t node;  // a node with this pattern
+      int32_t next;  // next pattern with the same hash, or -1
+    };
+    std::unordered_map<uint64_t, int32_t> head;
+    std::vector<Seen> seen;
+    std::vector<int32_t> owner(s.nu);  // number of the pattern
+    auto row_of = [&](int32_t k) { return s.u_inc_row[k]; };
+    for (int n = 0; n < s.nu; ++n) {
+      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
+      auto it = head.emplace(row_hash[n], -1).first;
+      int32_t id = it->second;
+      for (; id >= 0; id = seen[id].next) {
+        const int32_t o0 = s.u_inc_ptr[seen[id].node];
+        bool same = s.u_inc_ptr[seen[id].node + 1] - o0 == cnt;
+        for (int32_t j = 0; same && j < cnt; ++j) same = row_of(o0 + j) == row_of(k0 + j);
+        if (same) break;
+      }
+      if (id < 0) {
+        id = (int32_t)seen.size();
+        seen.push_back({n, it->second});
+        it->second = id;
+      }
+      owner[n] = id;
+    }
+    const int pwords = 2 * s.npp;  // 4 * npp 16-bit ranks
+    std::vector<int64_t> at(seen.size() + 1, 0);
+    for (size_t i = 0; i < seen.size(); ++i) {
+      const int n = seen[i].node;
+      const int rounds = (s.u_inc_ptr[n + 1] - s.u_inc_ptr[n] + 3) / 4;
+      at[i + 1] = at[i] + (int64_t)rounds * (s.wu[n] + pwords);
+    }
+    if (at[seen.size()] >= (1ll << 31)) return fail(msg, "too many distinct node patterns");
+    s.pat.assign((size_t)at[seen.size()], 0xffffffffu);
+    parallel_for((int)seen.size(), [&](int i) {
+      const int n = seen[i].node;
+      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
+      for (int32_t j = 0; j < cnt; ++j) {
+        uint32_t* w = &s.pat[(size_t)at[i] + (size_t)(j / 4) * (s.wu[n] + pwords)];
+        const uint16_t* T = &s.tables[(size_t)row_of(k0 + j) * nr];
+        for (int b = 0; b < s.npe; ++b) reinterpret_cast<uint8_t*>(w + (T[b] & 0x7fff))[j % 4] = (uint8_t)b;
+        for (int q = 0; q < s.npp; ++q)
+          reinterpret_cast<uint16_t*>(w + s.wu[n])[(j % 4) * s.npp + q] = T[s.npe + q] & 0x7fff;
+      }
+    });
+    s.u_pat.resize(s.nu);
+    for (int n = 0; n < s.nu; ++n) s.u_pat[n] = (int32_t)at[owner[n]];
+  }
+  return FE_NO_ERROR;
+}
+
 }  // namespace
 
-int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
+int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg, bool assembly) {
   if (!d) return fail(msg, "mesh description is NULL");
   if (d->num_elements <= 0 || d->num_nodes_u <= 0) return fail(msg, "mesh has no elements or nodes");
   if (d->nodes_per_xi_u != 2 && d->nodes_per_xi_u != 3)
@@ -444,82 +525,8 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
     }
     s.ntables = (int)seen.size();
   }
-  if ((int64_t)s.ntables * nr >= (1ll << 31)) return fail(msg, "too many distinct rank tables");
-  // The incidences of every node: rank-table rows in element order, the
-  // incidences again in colour order, and a hash of a u node's rows.
-  s.u_inc_row.resize(s.u_inc.size());
-  s.p_inc_row.resize(s.p_inc.size());
-  s.u_inc_col = s.u_inc;
-  s.p_inc_col = s.p_inc;
-  std::vector<uint64_t> row_hash(s.nu);
-  parallel_for(s.nu + s.npn, [&](int i) {
-    const bool un = i < s.nu;
-    const int n = un ? i : i - s.nu, bits = un ? 5 : 3, off = un ? 0 : s.npe;
-    const auto& ptr = un ? s.u_inc_ptr : s.p_inc_ptr;
-    const auto& inc = un ? s.u_inc : s.p_inc;
-    auto& row = un ? s.u_inc_row : s.p_inc_row;
-    auto& col = un ? s.u_inc_col : s.p_inc_col;
-    uint64_t hash = 1469598103934665603ull;
-    for (int32_t k = ptr[n]; k < ptr[n + 1]; ++k) {
-      row[k] = s.elem_table[inc[k] >> bits] * nr + off + (inc[k] & ((1 << bits) - 1));
-      hash = (hash ^ (uint64_t)(uint32_t)row[k]) * 1099511628211ull;
-    }
-    if (un) row_hash[n] = hash;
-    std::sort(col.begin() + ptr[n], col.begin() + ptr[n + 1],
-              [&](int32_t x, int32_t y) { return colour[x >> bits] < colour[y >> bits]; });
-  });
-
-  // Column patterns of the u nodes' rows, shared by nodes with equal
-  // rank-table rows (a node's incidences in element order).
-  {
-    struct Seen {
-      int32_t node;  // a node with this pattern
-      int32_t next;  // next pattern with the same hash, or -1
-    };
-    std::unordered_map<uint64_t, int32_t> head;
-    std::vector<Seen> seen;
-    std::vector<int32_t> owner(s.nu);  // number of the pattern
-    auto row_of = [&](int32_t k) { return s.u_inc_row[k]; };
-    for (int n = 0; n < s.nu; ++n) {
-      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
-      auto it = head.emplace(row_hash[n], -1).first;
-      int32_t id = it->second;
-      for (; id >= 0; id = seen[id].next) {
-        const int32_t o0 = s.u_inc_ptr[seen[id].node];
-        bool same = s.u_inc_ptr[seen[id].node + 1] - o0 == cnt;
-        for (int32_t j = 0; same && j < cnt; ++j) same = row_of(o0 + j) == row_of(k0 + j);
-        if (same) break;
-      }
-      if (id < 0) {
-        id = (int32_t)seen.size();
-        seen.push_back({n, it->second});
-        it->second = id;
-      }
-      owner[n] = id;
-    }
-    const int pwords = 2 * s.npp;  // 4 * npp 16-bit ranks
-    std::vector<int64_t> at(seen.size() + 1, 0);
-    for (size_t i = 0; i < seen.size(); ++i) {
-      const int n = seen[i].node;
-      const int rounds = (s.u_inc_ptr[n + 1] - s.u_inc_ptr[n] + 3) / 4;
-      at[i + 1] = at[i] + (int64_t)rounds * (s.wu[n] + pwords);
-    }
-    if (at[seen.size()] >= (1ll << 31)) return fail(msg, "too many distinct node patterns");
-    s.pat.assign((size_t)at[seen.size()], 0xffffffffu);
-    parallel_for((int)seen.size(), [&](int i) {
-      const int n = seen[i].node;
-      const int32_t k0 = s.u_inc_ptr[n], cnt = s.u_inc_ptr[n + 1] - k0;
-      for (int32_t j = 0; j < cnt; ++j) {
-        uint32_t* w = &s.pat[(size_t)at[i] + (size_t)(j / 4) * (s.wu[n] + pwords)];
-        const uint16_t* T = &s.tables[(size_t)row_of(k0 + j) * nr];
-        for (int b = 0; b < s.npe; ++b) reinterpret_cast<uint8_t*>(w + (T[b] & 0x7fff))[j % 4] = (uint8_t)b;
-        for (int q = 0; q < s.npp; ++q)
-          reinterpret_cast<uint16_t*>(w + s.wu[n])[(j % 4) * s.npp + q] = T[s.npe + q] & 0x7fff;
-      }
-    });
-    s.u_pat.resize(s.nu);
-    for (int n = 0; n < s.nu; ++n) s.u_pat[n] = (int32_t)at[owner[n]];
-  }
+  if (assembly)
+    if (const int rc = incidence_patterns(s, colour, msg)) return rc;
 
   // Boundary faces: a local face (reference order -xi1, -xi2, -xi3, +xi1,
   // +xi2, +xi3) whose four corner nodes no other element holds.
@@ -578,7 +585,7 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
 
   // Geometric Gauss-point data.
   s.geo.assign((size_t)s.ne * NG * 10, 0.0);
-  s.geo_rj.assign((size_t)s.ne * NG, 0.0);
+  if (assembly) s.geo_rj.assign((size_t)s.ne * NG, 0.0);
   std::vector<char> degenerate(s.ne, 0);
   parallel_for(s.ne, [&](int e) {
     for (int g = 0; g < NG; ++g) {
@@ -608,7 +615,7 @@ int build_setup(const fe_mesh_desc* d, HostSetup& s, std::string& msg) {
         for (int j = 0; j < 3; ++j) out[i * 3 + j] = dn[i][j];
       out[9] = std::sqrt(std::fabs(det_gl));
       if (!(out[9] > 0.0)) degenerate[e] = 1;
-      s.geo_rj[(size_t)e * NG + g] = 1.0 / out[9];
+      if (assembly) s.geo_rj[(size_t)e * NG + g] = 1.0 / out[9];
     }
   });
   for (int e = 0; e < s.ne; ++e)
