@@ -19,9 +19,9 @@
 // result does not depend on scheduling.
 //
 // It serves the element-level calls, and the FP64 Jacobian where fe_fp64.cu's
-// launch has no records (no memory left, a stream under capture).  The other assemblies: fe_fp64.cu (FP64 Jacobian),
-// fe_residual.cu, fe_mixed.cu and fe_mixed_coloured.cu (mixed precision),
-// fe_batch.cu.
+// launch has no records (the coloured order, no memory left, a stream under
+// capture).  The other assemblies: fe_fp64.cu (FP64 Jacobian), fe_residual.cu,
+// fe_mixed.cu and fe_mixed_coloured.cu (mixed precision), fe_batch.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
